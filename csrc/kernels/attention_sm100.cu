@@ -79,11 +79,11 @@ extern "C" int opk_attn_fwd(const void* qkv, void* out, float* lse, int T, int H
   if (hd == 128) {
     static bool once = set_smem(opk::attn_fwd_kernel<128>, opk::FwdSmem<128>::BYTES);
     if (!once) return -3;
-    opk::launch(opk::attn_fwd_kernel<128>, grid, opk::kFwdThreads, opk::FwdSmem<128>::BYTES, st, 0, tm, tm_out, p);
+    opk::launch(opk::attn_fwd_kernel<128>, grid, opk::kFwdThreads, opk::FwdSmem<128>::BYTES, st, tm, tm_out, p);
   } else {
     static bool once = set_smem(opk::attn_fwd_kernel<64>, opk::FwdSmem<64>::BYTES);
     if (!once) return -3;
-    opk::launch(opk::attn_fwd_kernel<64>, grid, opk::kFwdThreads, opk::FwdSmem<64>::BYTES, st, 0, tm, tm_out, p);
+    opk::launch(opk::attn_fwd_kernel<64>, grid, opk::kFwdThreads, opk::FwdSmem<64>::BYTES, st, tm, tm_out, p);
   }
   return (int)cudaGetLastError();
 }
@@ -122,14 +122,14 @@ extern "C" int opk_attn_bwd(const void* qkv, const void* out, const void* dout, 
                        set_smem(opk::attn_dq128_kernel<128>, opk::Dq128Smem<128>::BYTES);
     if (!once) return -3;
     // the dQ kernel goes first: it also writes the row statistics (dsum, nlse2) that the dK/dV kernel reads
-    opk::launch(opk::attn_dq128_kernel<128>, n_kt * H, opk::kBwdThreads, opk::Dq128Smem<128>::BYTES, st, 0, tm128, tm128, tmdo128, tm_dq, tm_o128, p);
-    opk::launch(opk::attn_dkv_kernel<128>, dkv_grid, opk::kBwdThreads, opk::DkvSmem<128>::BYTES, st, 0, tm128, tm64, tmdo64, tm_part, p);
+    opk::launch(opk::attn_dq128_kernel<128>, n_kt * H, opk::kBwdThreads, opk::Dq128Smem<128>::BYTES, st, tm128, tm128, tmdo128, tm_dq, tm_o128, p);
+    opk::launch(opk::attn_dkv_kernel<128>, dkv_grid, opk::kBwdThreads, opk::DkvSmem<128>::BYTES, st, tm128, tm64, tmdo64, tm_part, p);
   } else {
     static bool once = set_smem(opk::attn_dkv_kernel<64>, opk::DkvSmem<64>::BYTES) &&
                        set_smem(opk::attn_dq128_kernel<64>, opk::Dq128Smem<64>::BYTES);
     if (!once) return -3;
-    opk::launch(opk::attn_dq128_kernel<64>, n_kt * H, opk::kBwdThreads, opk::Dq128Smem<64>::BYTES, st, 0, tm128, tm128, tmdo128, tm_dq, tm_o128, p);
-    opk::launch(opk::attn_dkv_kernel<64>, dkv_grid, opk::kBwdThreads, opk::DkvSmem<64>::BYTES, st, 0, tm128, tm64, tmdo64, tm_part, p);
+    opk::launch(opk::attn_dq128_kernel<64>, n_kt * H, opk::kBwdThreads, opk::Dq128Smem<64>::BYTES, st, tm128, tm128, tmdo128, tm_dq, tm_o128, p);
+    opk::launch(opk::attn_dkv_kernel<64>, dkv_grid, opk::kBwdThreads, opk::DkvSmem<64>::BYTES, st, tm128, tm64, tmdo64, tm_part, p);
   }
   if (p.part) {
     const int kvw = KV * hd;

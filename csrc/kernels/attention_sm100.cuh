@@ -274,7 +274,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  pdl_trigger();       // after this CTA's TMEM is allocated, as in the split GEMM
+  pdl_trigger();       // after this CTA's TMEM is allocated, as in the narrow GEMM
   pdl_wait();
   const uint32_t S_COL = 0, O_COL = 256;   // score buffers at 0 / 128, the two output accumulators at 256 / 384
 
@@ -841,7 +841,7 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  pdl_trigger();       // after this CTA's TMEM is allocated, as in the split GEMM
+  pdl_trigger();       // after this CTA's TMEM is allocated, as in the narrow GEMM
   pdl_wait();
   // columns: St buffers 0 / 64, dPt buffers 128 / 192, dV at 256, dK at 256 + HD
   const uint32_t ST_COL = 0, DPT_COL = 128, DV_COL = 256, DK_COL = 256 + HD;
@@ -1111,7 +1111,7 @@ attn_dq128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  pdl_trigger();       // after this CTA's TMEM is allocated, as in the split GEMM
+  pdl_trigger();       // after this CTA's TMEM is allocated, as in the narrow GEMM
   pdl_wait();
   const uint32_t S_COL = 0, DP_COL = 256, DQ_COL = 384;   // two S buffers at 0 / 128
 

@@ -1,5 +1,5 @@
 // Host side of the tcgen05 GEMM: builds the TMA tensor maps and launches the persistent kernel.
-#include "gemm_split_sm100.cuh"
+#include "gemm_narrow_sm100.cuh"
 #include "opk_api.h"
 #include "debug_bounds.cuh"
 
@@ -81,7 +81,7 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams& 
   const int tiles = ((p.M + 127) / 128) * ((p.N + BN - 1) / BN) * p.batch;
   int grid = max_ctas > 0 ? max_ctas : num_sms();
   if (grid > tiles) grid = tiles;
-  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::gemm1_epi_warps(EPI), Cfg::SMEM_BYTES, st, 0, ta, tb, p);
+  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::gemm1_epi_warps(EPI), Cfg::SMEM_BYTES, st, ta, tb, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
   return 0;
@@ -106,71 +106,59 @@ int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams&
   int grid = (max_ctas > 0 ? max_ctas : num_sms()) & ~1;   // whole CTA pairs
   if (grid < 2) grid = 2;
   if (grid > 2 * tiles) grid = 2 * tiles;
-  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::gemm_epi_warps(EPI) + (STAGE ? 32 * opk::kStageWarps : 0), Cfg::SMEM_BYTES, st, 0, ta, tb, p);
+  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::gemm_epi_warps(EPI) + (STAGE ? 32 * opk::kStageWarps : 0), Cfg::SMEM_BYTES, st, ta, tb, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
   return 0;
 }
 
-// How many clusters of S CTAs (one per SM) are resident at once. A cluster sits inside one GPC; pairs always find room,
-// larger ones leave SMs over (48 clusters of three measured like two waves, 24 of five like one).
-long long resident_clusters(int S) { return S <= 2 ? num_sms() / S : 16 / S * 8; }
-
 template <bool A_MN, bool B_MN, int BN, int EPI>
-int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams& p, int S, cudaStream_t st) {
-  using Cfg = opk::GemmSplitCfg<BN>;
-  auto kern = opk::gemm_split_kernel<A_MN, B_MN, BN, EPI>;
+int launch_narrow(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams& p, cudaStream_t st) {
+  using Cfg = opk::GemmNarrowCfg<BN>;
+  auto kern = opk::gemm_narrow_kernel<A_MN, B_MN, BN, EPI>;
   static bool attr_done = false;
   if (!attr_done) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::smem_bytes(Cfg::MANY));
     if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
     attr_done = true;
   }
-  const long long tiles = (long long)((p.M + 127) / 128) * ((p.N + BN - 1) / BN) * p.batch;
-  const int stages = tiles > resident_clusters(S) ? Cfg::FEW : Cfg::MANY;
-  const dim3 grid((unsigned)S, (unsigned)((p.N + BN - 1) / BN), (unsigned)(((p.M + 127) / 128) * p.batch));
-  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::kSplitEpiWarps, Cfg::smem_bytes(stages), st, S > 1 ? S : 0, ta, tb, p, S, stages);
+  const dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)(((p.M + 127) / 128) * p.batch));
+  const int stages = (long long)grid.x * grid.y > num_sms() ? Cfg::FEW : Cfg::MANY;
+  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::kNarrowEpiWarps, Cfg::smem_bytes(stages), st, ta, tb, p, stages);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
   return 0;
 }
 
-// Whether a product runs on the split kernel, with which tile width and how many CTAs per tile.
-struct SplitChoice { int bn, s; };    // bn == 0: one of the persistent kernels
-
-SplitChoice choose_split(const OpkGemmArgs* a, int bn, bool pair) {
-  SplitChoice best{0, 0};
-  if (!pair_mode() || a->tile_group || a->group_k || a->stage_dst || a->max_ctas > 0) return best;
+// Tile width of the narrow kernel for this product; 0: one of the persistent kernels. Never EPI_SUMSQ: a norm's fp32 partial
+// sums follow the tiles, and the clip factor of an example must not depend on which kernel its length favours.
+int choose_narrow(const OpkGemmArgs* a, int bn, bool pair) {
+  if (!pair_mode() || a->tile_group || a->group_k || a->stage_dst || a->max_ctas > 0) return 0;
   const int key = (a->a_mn ? 1 : 0) | (a->b_mn ? 2 : 0);
   const bool ok = a->epilogue == opk::EPI_STORE ? key != 1
-                  : a->epilogue == opk::EPI_SUMSQ ? key == 3
                   : a->epilogue == opk::EPI_SWIGLU ? key == 0
                   : a->epilogue == opk::EPI_SWIGLU_BWD ? key == 2 : false;
-  if (!ok || (a->fixed_order && a->epilogue == opk::EPI_SUMSQ)) return best;   // a norm's partial sums follow the tiles
+  if (!ok) return 0;
   auto ceil_div = [](long long x, long long y) { return (x + y - 1) / y; };
   const long long kb = ceil_div(a->K, 64), sms = num_sms();
   // Estimated nanoseconds, fitted to graph replays on B200 over 36 shapes (rows 40 .. 4096, columns 16 .. 16384, reductions
   // 16 .. 128256): a fixed part and a slope per 64-element block of the reduction and round of tiles.
-  //   tile            fixed   slope   measured at M x N x K (persistent kernel -> split kernel, us)
+  //   tile            fixed   slope   measured at M x N x K (persistent kernel -> narrow kernel, us)
   //   256 x 256 pair   6600     280
   //   128 x 256        5200     315   2048 x 2048 x 2048: 16.9 -> 16.3; 1024 x 3072 x 768: 10.3 -> 9.5
-  //   128 x 128        4200     235   1024 x 2304 x 768: 10.2 -> 7.6; 1024 x 768 x 3072 in two: 20.2 -> 12.3
-  //   128 x 64         3500     225   1024 x 768 x 768: 10.0 -> 6.3; 2048 x 64 x 2048 in four: 11.8 -> 7.2
-  // Below the line the persistent kernel is the better one: 1021 x 4096 x 4096 26.7 against 27.2 us, 3072 x 2048 x 317
-  // (weight gradient) 11.0 against 11.7. A split of the reduction pays its two cluster barriers and the exchange.
+  //   128 x 128        4200     235   1024 x 2304 x 768: 10.2 -> 7.6
+  //   128 x 64         3500     225   1024 x 768 x 768: 10.0 -> 6.3
+  // Below the line the persistent kernel is the better one: 1021 x 4096 x 4096 26.7 against 27.2 us.
   long long cost = pair ? ceil_div(ceil_div(a->M, 256) * ceil_div(a->N, 256) * a->batch, sms / 2) * kb * 280 + 6600
                         : ceil_div(ceil_div(a->M, 128) * ceil_div(a->N, bn) * a->batch, sms) * kb * 320 + 5300;
+  int best = 0;
   for (int w = 64; w <= 256; w *= 2) {
-    const long long tiles = ceil_div(a->M, 128) * ceil_div(a->N, w) * a->batch;
+    const long long per = ceil_div(ceil_div(a->M, 128) * ceil_div(a->N, w) * a->batch, sms);
+    if (per > 4) continue;
     const long long fixed = w == 256 ? 5200 : w == 128 ? 4200 : 3500, slope = w == 256 ? 315 : w == 128 ? 235 : 225;
     const long long round = w == 256 ? 4500 : w == 128 ? 1500 : 800;          // epilogue of every further round
-    const long long exchange = w == 256 ? 3500 : w == 128 ? 1700 : 1200;
-    for (int s = 1; s <= (a->fixed_order ? 1 : 5) && s <= kb; ++s) {
-      const long long per = ceil_div(tiles, resident_clusters(s));
-      if (per > 4) break;
-      const long long c = fixed + per * ceil_div(kb, s) * slope + (per - 1) * round + (s > 1 ? exchange + (w == 256 ? 250 : 150) * s : 0);
-      if (c < cost) { cost = c; best = SplitChoice{w, s}; }
-    }
+    const long long c = fixed + per * kb * slope + (per - 1) * round;
+    if (c < cost) { cost = c; best = w; }
   }
   return best;
 }
@@ -232,7 +220,7 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   if (!a || a->M <= 0 || a->N <= 0 || a->K <= 0 || a->batch <= 0) { set_err("opk_gemm: bad sizes"); return -1; }
   const int bn = pick_bn(a->N, a->epilogue);
   const bool pair = bn == 256 && !a->tile_group && !a->group_k && a->M >= 256 && pair_mode();
-  const SplitChoice split = choose_split(a, bn, pair);
+  const int narrow = choose_narrow(a, bn, pair);
   CUtensorMap ta, tb;
   // A: K-major -> {K, M, batch} box {64, 128}; MN-major -> {M, K, batch} box {64, 64}
   if (a->tile_group && (a->batch != 1 || a->n_groups <= 0)) { set_err("opk_gemm: tile_group needs batch == 1 and n_groups"); return -1; }
@@ -262,7 +250,7 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   } else if (a->b_mn) {
     if (!make_map(&tb, a->B, a->N, a->K, bbatch, a->ldb, a->strideB, 64)) return -2;
   } else {
-    if (!make_map(&tb, a->B, a->K, a->N, bbatch, a->ldb, a->strideB, split.bn ? split.bn : pair ? 128 : bn)) return -2;
+    if (!make_map(&tb, a->B, a->K, a->N, bbatch, a->ldb, a->strideB, narrow ? narrow : pair ? 128 : bn)) return -2;
   }
   opk::GemmParams p;
   memset(&p, 0, sizeof(p));
@@ -284,24 +272,22 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
     return a->b_mn ? launch2<false, true, opk::EPI_STORE, true>(ta, tb, p, mc, st)
                    : launch2<false, false, opk::EPI_STORE, true>(ta, tb, p, mc, st);
   }
-  if (split.bn) {
-    if (a->epilogue == opk::EPI_SUMSQ && !a->sumsq) { set_err("opk_gemm: sumsq pointer required"); return -1; }
+  if (narrow) {
     if (a->epilogue == opk::EPI_SWIGLU && (!a->act || (a->N & 1))) { set_err("opk_gemm: swiglu needs act and even N"); return -1; }
     if (a->epilogue == opk::EPI_SWIGLU_BWD && (!a->act || a->R || a->bias)) {
       set_err("opk_gemm: swiglu backward needs the saved pre-activations and takes no bias / residual");
       return -1;
     }
-#define OPK_SPLIT(AM, BM_, E) \
-  (split.bn == 256   ? launch_split<AM, BM_, 256, E>(ta, tb, p, split.s, st)          \
-   : split.bn == 128 ? launch_split<AM, BM_, 128, E>(ta, tb, p, split.s, st)          \
-                     : launch_split<AM, BM_, 64, E>(ta, tb, p, split.s, st))
-    if (a->epilogue == opk::EPI_SUMSQ) return OPK_SPLIT(true, true, opk::EPI_SUMSQ);
-    if (a->epilogue == opk::EPI_SWIGLU) return OPK_SPLIT(false, false, opk::EPI_SWIGLU);
-    if (a->epilogue == opk::EPI_SWIGLU_BWD) return OPK_SPLIT(false, true, opk::EPI_SWIGLU_BWD);
-    if (key == 0) return OPK_SPLIT(false, false, opk::EPI_STORE);
-    if (key == 2) return OPK_SPLIT(false, true, opk::EPI_STORE);
-    return OPK_SPLIT(true, true, opk::EPI_STORE);
-#undef OPK_SPLIT
+#define OPK_NARROW(AM, BM_, E) \
+  (narrow == 256   ? launch_narrow<AM, BM_, 256, E>(ta, tb, p, st)          \
+   : narrow == 128 ? launch_narrow<AM, BM_, 128, E>(ta, tb, p, st)          \
+                   : launch_narrow<AM, BM_, 64, E>(ta, tb, p, st))
+    if (a->epilogue == opk::EPI_SWIGLU) return OPK_NARROW(false, false, opk::EPI_SWIGLU);
+    if (a->epilogue == opk::EPI_SWIGLU_BWD) return OPK_NARROW(false, true, opk::EPI_SWIGLU_BWD);
+    if (key == 0) return OPK_NARROW(false, false, opk::EPI_STORE);
+    if (key == 2) return OPK_NARROW(false, true, opk::EPI_STORE);
+    return OPK_NARROW(true, true, opk::EPI_STORE);
+#undef OPK_NARROW
   }
   if (pair) {
     switch (a->epilogue) {

@@ -43,8 +43,6 @@ typedef struct OpkGemmArgs {
   // counters, one per band of 2048 rows of B (zeroed by opk_gemm on the stream before the launch).
   void* stage_dst;
   int32_t* stage_ready;
-  // != 0: an output element's products (and, EPI_SUMSQ, a tile's squares) are added in one order whatever the sizes
-  int32_t fixed_order;
   int32_t lce_parts;     // EPI_LCE_FWD: column parts per 256-column tile in pmax / psum (2, else 1)
 } OpkGemmArgs;
 

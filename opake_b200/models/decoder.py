@@ -34,12 +34,6 @@ class ExampleStats:
     n_tokens: torch.Tensor   # device scalar: number of supervised tokens
 
 
-def _fwd_gemm(*args, **kw):
-    # The forward pass keeps one order of summation for every sequence length: a token's logits, and the experts that a
-    # router picks from near-ties, do not depend on how many tokens are processed with it.
-    return G.gemm(*args, fixed_order=True, **kw)
-
-
 class DecoderRuntime:
     """Forward + per-example backward for dense decoders (Llama-style and GPT-2-style blocks)."""
 
@@ -89,10 +83,6 @@ class DecoderRuntime:
         self._vec_width = max([d] + [self.layout.slot(n).numel for n in self._vec_names])
         self._n_leaves = len(self.layout.slots)
         self._widest = max(s.numel for s in self.layout.slots)
-        # The backward pass keeps one order of summation too: rounding differences of one product grow to the level of bf16
-        # rounding over the layers below it, and the adaptive update of almost noise-free coordinates carries them into the
-        # next step's expert choices. An example's gradient does not depend on the kernels its length would favour.
-        self._fixed_order = True
 
     # slot-0 aliases (single-buffer users and tests)
     @property
@@ -199,11 +189,11 @@ class DecoderRuntime:
         """``out = dy^T x`` (+ squared norm) ordered after everything issued so far, on the weight-gradient stream."""
         side = self._wstream
         if side is None:
-            G.linear_wgrad(dy, x, out=out, sumsq=sumsq, fixed_order=self._fixed_order)
+            G.linear_wgrad(dy, x, out=out, sumsq=sumsq)
             return
         side.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(side):
-            G.linear_wgrad(dy, x, out=out, sumsq=sumsq, fixed_order=self._fixed_order)
+            G.linear_wgrad(dy, x, out=out, sumsq=sumsq)
 
     def _wgrad_call(self, fn) -> None:
         """Runs ``fn`` (a weight-gradient launch) on the weight-gradient stream, ordered after everything issued so far."""
@@ -272,7 +262,7 @@ class DecoderRuntime:
             p = f"layers.{li}."
             xn, st1 = self._norm_fwd(x, p + "norm1", out=a["xn"])
             wsrc, stg = self._wop(p + "wqkv")
-            _fwd_gemm(xn, wsrc, out=a["qkv"], bias=w.get(p + "bqkv"), stage=stg)
+            G.gemm(xn, wsrc, out=a["qkv"], bias=w.get(p + "bqkv"), stage=stg)
             stq = None
             if cfg.qk_norm == "head":
                 nq, nk = H * hd, KV * hd
@@ -296,43 +286,43 @@ class DecoderRuntime:
             _, actx = A.attention_fwd(a["qkv"], H, KV, hd, self.attn_impl, out=a["attn"])
             # output projection with the residual add fused into the GEMM epilogue
             wsrc, stg = self._wop(p + "wo")
-            _fwd_gemm(a["attn"], wsrc, out=a["x_mid"], residual=x, bias=w.get(p + "bo"), stage=stg)
+            G.gemm(a["attn"], wsrc, out=a["x_mid"], residual=x, bias=w.get(p + "bo"), stage=stg)
             xn2, st2 = self._norm_fwd(a["x_mid"], p + "norm2", out=a["xn2"])
             nxt = ws["layers"][li + 1]["x"] if li + 1 < cfg.n_layers else ws["x_last"]
             if cfg.n_experts and self.ep is not None:
                 self.ep.forward(li, xn2, a["x_mid"], nxt)
             elif cfg.n_experts:
                 plan = a["plan"]
-                _fwd_gemm(xn2, w[p + "router"], out=a["rlogits"])
+                G.gemm(xn2, w[p + "router"], out=a["rlogits"])
                 K.moe_route(a["rlogits"], plan, cfg.norm_topk_prob)
                 K.moe_gather(xn2, plan, a["xs"])
-                _fwd_gemm(a["xs"], w[p + "experts.wgu"], out=a["gu"], epilogue=G.EPI_SWIGLU, act=a["act"], tile_group=plan.tile_group)
-                _fwd_gemm(a["act"], w[p + "experts.wd"], out=a["ye"], tile_group=plan.tile_group)
+                G.gemm(a["xs"], w[p + "experts.wgu"], out=a["gu"], epilogue=G.EPI_SWIGLU, act=a["act"], tile_group=plan.tile_group)
+                G.gemm(a["act"], w[p + "experts.wd"], out=a["ye"], tile_group=plan.tile_group)
                 K.moe_combine(a["ye"], plan, nxt, wts=plan.wts, residual=a["x_mid"])
             elif cfg.act == "swiglu":
                 wsrc, stg = self._wop(p + "wgu")
-                _fwd_gemm(xn2, wsrc, out=a["gu"], epilogue=G.EPI_SWIGLU, act=a["act"], stage=stg)
+                G.gemm(xn2, wsrc, out=a["gu"], epilogue=G.EPI_SWIGLU, act=a["act"], stage=stg)
                 wsrc, stg = self._wop(p + "wd")
-                _fwd_gemm(a["act"], wsrc, out=nxt, residual=a["x_mid"], stage=stg)
+                G.gemm(a["act"], wsrc, out=nxt, residual=a["x_mid"], stage=stg)
             elif cfg.act == "geglu":
                 wsrc, stg = self._wop(p + "wgu")
-                _fwd_gemm(xn2, wsrc, out=a["gu"], stage=stg)
+                G.gemm(xn2, wsrc, out=a["gu"], stage=stg)
                 K.geglu_fwd(a["gu"], True, out=a["act"])
                 wsrc, stg = self._wop(p + "wd")
-                _fwd_gemm(a["act"], wsrc, out=nxt, residual=a["x_mid"], stage=stg)
+                G.gemm(a["act"], wsrc, out=nxt, residual=a["x_mid"], stage=stg)
             else:
                 wsrc, stg = self._wop(p + "wfc")
-                _fwd_gemm(xn2, wsrc, out=a["fc"], bias=w.get(p + "bfc"), stage=stg)
+                G.gemm(xn2, wsrc, out=a["fc"], bias=w.get(p + "bfc"), stage=stg)
                 K.gelu_fwd(a["fc"], out=a["act"])
                 wsrc, stg = self._wop(p + "wproj")
-                _fwd_gemm(a["act"], wsrc, out=nxt, residual=a["x_mid"], bias=w.get(p + "bproj"), stage=stg)
+                G.gemm(a["act"], wsrc, out=nxt, residual=a["x_mid"], bias=w.get(p + "bproj"), stage=stg)
             saved.append((st1, st2, actx, stq))
             x = nxt
         xf, stf = self._norm_fwd(x, "norm_f", out=ws["xf"])
         head = w["embed"] if cfg.tie_embeddings else w["lm_head"]
         nll = lse = None
         if labels is not None:
-            _fwd_gemm(xf, head, epilogue=G.EPI_LCE_FWD, labels=labels, pmax=ws["pmax"], psum=ws["psum"], tgt=ws["tgt"])
+            G.gemm(xf, head, epilogue=G.EPI_LCE_FWD, labels=labels, pmax=ws["pmax"], psum=ws["psum"], tgt=ws["tgt"])
             lse, nll = K.lce_finalize(ws["pmax"], ws["psum"], ws["tgt"], labels)
         return nll, lse, (saved, stf)
 
@@ -343,7 +333,7 @@ class DecoderRuntime:
         head = self.w["embed"] if self.cfg.tie_embeddings else self.w["lm_head"]
         Vp = (self.cfg.vocab_size + 7) // 8 * 8
         out = torch.empty(tok.numel(), Vp, dtype=_bf16, device=self.device)[:, : self.cfg.vocab_size]
-        return _fwd_gemm(ws["xf"], head, out=out)
+        return G.gemm(ws["xf"], head, out=out)
 
     # ------------------------------------------------------------------ forward + backward of one example
     def example_grad(self, tok: torch.Tensor, labels: torch.Tensor, *, loss_weight: torch.Tensor | None = None,
@@ -362,7 +352,6 @@ class DecoderRuntime:
         ws = ws or self.workspace(T)
         emb_ws = ws["embs"][slot]
         H, KV, hd = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim
-        fix = self._fixed_order
         nll, lse, (saved, stf) = self.forward(tok, labels, ws)
         coef, loss, ntok = ws["coef"], ws["loss"], ws["ntok"]
         K.loss_coef(labels, nll, coef, loss, ntok, weight=loss_weight)
@@ -378,7 +367,7 @@ class DecoderRuntime:
             self._wgrad(dlog, ws["xf"], ghead)                   # norm added after the embedding rows are merged
         else:
             self._wgrad(dlog, ws["xf"], ghead, sumsq)
-        dxf = G.gemm(dlog, head, b_mn=True, out=ws["dx2"], fixed_order=fix)
+        dxf = G.gemm(dlog, head, b_mn=True, out=ws["dx2"])
         x_last = ws["x_last"]
         dx = self._norm_bwd(ws, dxf, x_last, "norm_f", stf, None, ws["dx"])
 
@@ -405,8 +394,8 @@ class DecoderRuntime:
                 dxn2 = K.moe_combine(ws["dxs"], plan, ws["dx2"])
                 # router: d weights -> d logits -> router weight gradient and the second path into dxn2
                 K.moe_route_bwd(plan, ws["dwts"], ws["drl"], cfg.norm_topk_prob)
-                G.linear_wgrad(ws["drl"], a["xn2"], out=g[p + "router"], sumsq=sumsq, fixed_order=fix)
-                G.gemm(ws["drl"], w[p + "router"], b_mn=True, out=dxn2, residual=dxn2, fixed_order=fix)
+                G.linear_wgrad(ws["drl"], a["xn2"], out=g[p + "router"], sumsq=sumsq)
+                G.gemm(ws["drl"], w[p + "router"], b_mn=True, out=dxn2, residual=dxn2)
                 self._wgrad_join()            # dye / dgu are rewritten by the next layer, dx by the norm backward below
             elif cfg.act in ("swiglu", "geglu"):
                 self._wgrad(dx, a["act"], g[p + "wd"], sumsq)
@@ -417,7 +406,7 @@ class DecoderRuntime:
                     dact = G.gemm(dx, w[p + "wd"], b_mn=True, out=ws["dact"])
                     K.geglu_bwd(dact, a["gu"], True, out=dgu)
                 self._wgrad(dgu, a["xn2"], g[p + "wgu"], sumsq)
-                dxn2 = G.gemm(dgu, w[p + "wgu"], b_mn=True, out=ws["dx2"], fixed_order=fix)
+                dxn2 = G.gemm(dgu, w[p + "wgu"], b_mn=True, out=ws["dx2"])
                 self._wgrad_join()            # the norm backward below overwrites dx in place
             else:
                 G.linear_wgrad(dx, a["act"], out=g[p + "wproj"], sumsq=sumsq)
@@ -428,13 +417,13 @@ class DecoderRuntime:
                 G.linear_wgrad(dfc, a["xn2"], out=g[p + "wfc"], sumsq=sumsq)
                 if cfg.bias:
                     K.colsum_(dfc, self._vec(ws, p + "bfc"))
-                dxn2 = G.gemm(dfc, w[p + "wfc"], b_mn=True, out=ws["dx2"], fixed_order=fix)
+                dxn2 = G.gemm(dfc, w[p + "wfc"], b_mn=True, out=ws["dx2"])
             dx_mid = self._norm_bwd(ws, dxn2, a["x_mid"], p + "norm2", st2, dx, ws["dx"])  # in place over dres
             # ---- attention
             self._wgrad(dx_mid, a["attn"], g[p + "wo"], sumsq)
             if cfg.bias:
                 K.colsum_(dx_mid, self._vec(ws, p + "bo"))
-            dattn = G.gemm(dx_mid, w[p + "wo"], b_mn=True, out=ws["dattn"], fixed_order=fix)
+            dattn = G.gemm(dx_mid, w[p + "wo"], b_mn=True, out=ws["dattn"])
             dqkv = ws["dqkv"]
             A.attention_bwd(dattn, a["qkv"], a["attn"], actx, H, KV, hd, dqkv)
             if cfg.pos == "rope":
@@ -460,7 +449,7 @@ class DecoderRuntime:
             self._wgrad(dqkv, a["xn"], g[p + "wqkv"], sumsq)
             if cfg.bias or cfg.qkv_bias:
                 K.colsum_(dqkv, self._vec(ws, p + "bqkv"))
-            dxn = G.gemm(dqkv, w[p + "wqkv"], b_mn=True, out=ws["dx2"], fixed_order=fix)
+            dxn = G.gemm(dqkv, w[p + "wqkv"], b_mn=True, out=ws["dx2"])
             self._wgrad_join()                # dx_mid (read by the wo gradient) is overwritten in place below
             dx = self._norm_bwd(ws, dxn, a["x"], p + "norm1", st1, dx_mid, ws["dx"])
 

@@ -49,14 +49,13 @@ def gemm(
     sumsq_shared: bool = False,
     norm_only: bool = False,
     stage: tuple[torch.Tensor, torch.Tensor] | None = None,
-    fixed_order: bool = False,
 ) -> torch.Tensor | None:
     """General entry: ``out[b] = alpha * op(a[b]) @ op(b[b // b_batch_div])^T`` with an epilogue.
 
     ``a_mn=False``: ``a`` is ``[M, K]``; ``a_mn=True``: ``a`` is ``[K, M]`` (used as its transpose).
     ``b_mn=False``: ``b`` is ``[N, K]``; ``b_mn=True``: ``b`` is ``[K, N]``.
-    ``fixed_order``: every output element adds its products in the same order whatever the other sizes are. Without it a
-    product with few output tiles may split its reduction over several SMs, depending on the number of rows.
+    Every output element adds its products in the same order whatever the other sizes are: a row of ``a`` gives the same
+    bits alone and among thousands, whichever kernel the sizes favour.
     """
     _check2d(a, "a")
     _check2d(b, "b")
@@ -114,7 +113,7 @@ def gemm(
         args.strideB = b.stride(0)
     if group_k is not None:         # per-batch reduction ranges over un-batched operands (mixture of experts wgrad)
         args.group_k = group_k.data_ptr()
-    args.sumsq_shared, args.fixed_order = int(sumsq_shared), int(fixed_order)
+    args.sumsq_shared = int(sumsq_shared)
     if stage is not None:           # b lives on another GPU: (local scratch [N, K] bf16, int32 band counters)
         scratch, ready = stage
         if scratch.numel() < N * K or scratch.dtype != torch.bfloat16 or ready.dtype != torch.int32 or ready.numel() * 2048 < N:
@@ -134,23 +133,21 @@ def linear_dgrad(dy: torch.Tensor, w: torch.Tensor, *, out=None, residual=None) 
     return gemm(dy, w, b_mn=True, out=out, residual=residual)
 
 
-def swiglu_dgrad(dy: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor, *, out: torch.Tensor, tile_group=None,
-                 fixed_order: bool = False) -> torch.Tensor:
+def swiglu_dgrad(dy: torch.Tensor, w_down: torch.Tensor, gu: torch.Tensor, *, out: torch.Tensor, tile_group=None) -> torch.Tensor:
     """Backward through ``act = silu(gate) * up`` fused into the down projection's data gradient: the accumulator
     ``d_act = dy @ w_down`` (``dy [T, d]``, ``w_down [d, F]``) never reaches memory; the epilogue reads the saved
     interleaved pre-activations ``gu [T, 2F]`` and writes ``out [T, 2F]`` = interleaved ``(d_gate, d_up)``."""
-    return gemm(dy, w_down, b_mn=True, out=out, epilogue=EPI_SWIGLU_BWD, act=gu, tile_group=tile_group, fixed_order=fixed_order)
+    return gemm(dy, w_down, b_mn=True, out=out, epilogue=EPI_SWIGLU_BWD, act=gu, tile_group=tile_group)
 
 
-def linear_wgrad(dy: torch.Tensor, x: torch.Tensor, *, out=None, sumsq: torch.Tensor | None = None,
-                 fixed_order: bool = False) -> torch.Tensor:
+def linear_wgrad(dy: torch.Tensor, x: torch.Tensor, *, out=None, sumsq: torch.Tensor | None = None) -> torch.Tensor:
     """``dw = dy.T @ x`` with ``dy [T, N]``, ``x [T, K]`` -> ``[N, K]``.
 
     With ``sumsq`` (a float64 scalar tensor) the kernel also adds ``sum(dw**2)`` of the stored bf16 values to it,
     which is the per-example squared gradient norm contribution of this weight.
     """
     epi = EPI_SUMSQ if sumsq is not None else EPI_STORE
-    return gemm(dy, x, a_mn=True, b_mn=True, out=out, epilogue=epi, sumsq=sumsq, fixed_order=fixed_order)
+    return gemm(dy, x, a_mn=True, b_mn=True, out=out, epilogue=epi, sumsq=sumsq)
 
 
 def lce_tiles(n_vocab: int, parts: int = 1) -> int:

@@ -1,0 +1,69 @@
+"""One order of summation for every product: a row's result does not depend on how many rows are processed with it, although
+the number of rows decides which GEMM kernel and tile width run."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ROWS = (40, 128, 129, 317, 640)       # few rows: narrow tiles; 1024 rows (the comparison): wider tiles, pairs of SMs
+
+
+def _rand(shape, dev, scale=1.0):
+    return (torch.randn(shape, device=dev, dtype=torch.float32) * scale).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn"])
+@pytest.mark.parametrize("N,K", [(64, 2048), (512, 8192), (2048, 2048), (768, 3072), (8192, 2048)])
+def test_rows_of_plain_products(cuda, N, K, layout):
+    from opake_b200.ops import gemm as G
+    from opake_b200.ops._lib import raise_if_device_error
+
+    x, w, res = _rand((1024, K), cuda), _rand((N, K) if layout == "nt" else (K, N), cuda), _rand((1024, N), cuda)
+    whole = G.gemm(x, w, b_mn=layout == "nn", residual=res, out=torch.empty_like(res))
+    for M in ROWS:
+        part = G.gemm(x[:M], w, b_mn=layout == "nn", residual=res[:M], out=torch.empty(M, N, dtype=x.dtype, device=cuda))
+        assert torch.equal(part, whole[:M]), M
+    raise_if_device_error(cuda)
+
+
+@pytest.mark.parametrize("F,D", [(512, 2048), (8192, 2048), (1408, 4096)])
+def test_rows_of_gated_products(cuda, F, D):
+    from opake_b200.ops import gemm as G
+    from opake_b200.ops._lib import raise_if_device_error
+
+    x, w, dy, wd = _rand((1024, D), cuda), _rand((2 * F, D), cuda, D ** -0.5), _rand((1024, D), cuda), _rand((D, F), cuda, D ** -0.5)
+    act = torch.empty(1024, F, dtype=x.dtype, device=cuda)
+    gu = G.gemm(x, w, epilogue=G.EPI_SWIGLU, act=act)
+    dgu = G.swiglu_dgrad(dy, wd, gu, out=torch.empty_like(gu))
+    for M in ROWS:
+        a = torch.empty(M, F, dtype=x.dtype, device=cuda)
+        g = G.gemm(x[:M], w, epilogue=G.EPI_SWIGLU, act=a)
+        assert torch.equal(g, gu[:M]) and torch.equal(a, act[:M]), M
+        assert torch.equal(G.swiglu_dgrad(dy[:M], wd, gu[:M], out=torch.empty_like(g)), dgu[:M]), M
+    raise_if_device_error(cuda)
+
+
+@pytest.mark.parametrize("N,K", [(64, 2048), (768, 3072), (2304, 768)])
+def test_weight_gradient_with_and_without_norm(cuda, N, K):
+    """Products over the rows: the weight gradient has the same bits with the norm (persistent kernels) and without."""
+    from opake_b200.ops import gemm as G
+
+    for T in (64, 317, 1024):
+        dy, x = _rand((T, N), cuda), _rand((T, K), cuda)
+        ss = torch.zeros(1, dtype=torch.float64, device=cuda)
+        assert torch.equal(G.linear_wgrad(dy, x), G.linear_wgrad(dy, x, sumsq=ss))
+
+
+@pytest.mark.parametrize("T,D,V", [(129, 512, 8192), (65, 256, 4000)])
+def test_functional_gradients_do_not_depend_on_the_micro_batch(cuda, T, D, V):
+    from torch.func import grad, vmap
+
+    from opake_b200.ops.lce import opake_linear_cross_entropy_loss as lce
+
+    h, w = _rand((8, T, D), cuda), _rand((V, D), cuda, 0.02)
+    lab = torch.randint(0, V, (8, T), device=cuda)
+    f = vmap(grad(lambda a, b, l: lce(a, b, l), argnums=(0, 1)), in_dims=(0, None, 0))
+    dh, dw = f(h, w, lab)
+    for lo, hi in ((0, 1), (1, 4), (4, 8)):
+        ph, pw = f(h[lo:hi], w, lab[lo:hi])
+        assert torch.equal(ph, dh[lo:hi]) and torch.equal(pw, dw[lo:hi])

@@ -1,10 +1,10 @@
-"""Products with few output tiles (reduction split over a thread-block cluster) at the edges of tiles and splits."""
+"""Products with few output tiles (narrow tiles, one per CTA) at the edges of tiles and reductions."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-# (M, N, K): one tile, one element past a tile, ragged everything, more splits than is even, narrow N, single rows
+# (M, N, K): one tile, one element past a tile, ragged everything, long reductions, narrow N, single rows
 SHAPES = [(128, 128, 64), (129, 136, 72), (1, 8, 8), (317, 2048, 2048), (300, 264, 1032), (64, 2048, 2048), (1024, 768, 3072),
           (2048, 16, 520), (77, 50264, 64), (256, 40, 8192)]
 
@@ -38,7 +38,7 @@ def test_plain_products(cuda, M, N, K, layout):
     raise_if_device_error(cuda)
     _check(out, a, b)
     again = G.gemm(A, B, a_mn=layout == "tn", b_mn=layout != "nt")
-    assert torch.equal(out, again)            # partial sums meet in rank order
+    assert torch.equal(out, again)
 
 
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (317, 2048, 2048), (130, 264, 1032), (2048, 16, 520)])
