@@ -233,7 +233,9 @@ def lora_qkv(x, q, k, v):
 
 
 def _native_act(*ts) -> bool:
-    return all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 and t.numel() % 8 == 0 for t in ts)
+    # equal shapes: the kernel walks all buffers by one index (projections of other widths broadcast or fail in the formula)
+    return all(t.is_cuda and t.dtype == torch.bfloat16 and t.shape == ts[0].shape and t.is_contiguous() and t.data_ptr() % 16 == 0
+               and t.numel() % 8 == 0 for t in ts)
 
 
 def _act_fwd(g, u, act: str):
