@@ -625,6 +625,37 @@ __device__ __forceinline__ float gate_grad(float g) {
   return MODE == 1 ? gelu_erf_grad(g) : gelu_tanh_grad(g);
 }
 
+// MODE 3 = SwiGLU, 4 = GEGLU tanh with the library's exponential and every operation rounded by itself, in the order of the
+// formulas that they stand for in the LoRA operators: the result does not depend on whether a call reaches the kernel.
+template <int MODE>
+__device__ __forceinline__ float glu_value(float g, float u) {
+  if (MODE == 3) return __fmul_rn(__fdiv_rn(g, __fadd_rn(1.f, expf(-g))), u);
+  return MODE == 4 ? __fmul_rn(gelu_tanh(g), u) : gate_fn<MODE>(g) * u;
+}
+template <int MODE>
+__device__ __forceinline__ void glu_grads(float d, float g, float u, float& dg, float& du) {
+  if (MODE < 3) {
+    dg = d * u * gate_grad<MODE>(g);
+    du = d * gate_fn<MODE>(g);
+    return;
+  }
+  float a, da;
+  if (MODE == 3) {
+    const float s = __fdiv_rn(1.f, __fadd_rn(1.f, expf(-g)));
+    a = __fmul_rn(g, s);
+    da = __fmul_rn(s, __fadd_rn(1.f, __fmul_rn(g, __fadd_rn(1.f, -s))));
+  } else {
+    const float k = 0.7978845608028654f, h = __fmul_rn(0.5f, g);
+    const float t = tanhf(__fmul_rn(k, __fadd_rn(g, __fmul_rn(0.044715f, __fmul_rn(__fmul_rn(g, g), g)))));
+    const float t1 = __fadd_rn(1.f, t);
+    a = __fmul_rn(h, t1);
+    const float slope = __fadd_rn(1.f, __fmul_rn(__fmul_rn((float)(3 * 0.044715), g), g));
+    da = __fadd_rn(__fmul_rn(0.5f, t1), __fmul_rn(__fmul_rn(__fmul_rn(h, __fadd_rn(1.f, -__fmul_rn(t, t))), k), slope));
+  }
+  dg = __fmul_rn(__fmul_rn(d, u), da);
+  du = __fmul_rn(d, a);
+}
+
 // Gate and up either interleaved pairwise in one buffer (SPLIT = false: gate[2i], gate[2i+1] = gate, up of element i) or
 // in two buffers. A thread handles 8 elements with 16-byte accesses; n is a multiple of 8 in the vector kernels (rows are
 // multiples of 8 elements for every caller), the scalar kernel takes the rest. Bound by memory: 3 (forward) or 5
@@ -638,7 +669,7 @@ __global__ void __launch_bounds__(256) glu_fwd_kernel(const __nv_bfloat16* __res
       unpack8(reinterpret_cast<const bf16x8*>(gate)[i], a);
       unpack8(reinterpret_cast<const bf16x8*>(up)[i], b);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = gate_fn<MODE>(a[j]) * b[j];
+      for (int j = 0; j < 8; ++j) o[j] = glu_value<MODE>(a[j], b[j]);
     } else {
       unpack8(reinterpret_cast<const bf16x8*>(gate)[2 * i], a);
       unpack8(reinterpret_cast<const bf16x8*>(gate)[2 * i + 1], b);
@@ -659,7 +690,7 @@ __global__ void __launch_bounds__(256) glu_bwd_kernel(const __nv_bfloat16* __res
       unpack8(reinterpret_cast<const bf16x8*>(gate)[i], a);
       unpack8(reinterpret_cast<const bf16x8*>(up)[i], b);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { oa[j] = d[j] * b[j] * gate_grad<MODE>(a[j]); ob[j] = d[j] * gate_fn<MODE>(a[j]); }
+      for (int j = 0; j < 8; ++j) glu_grads<MODE>(d[j], a[j], b[j], oa[j], ob[j]);
       reinterpret_cast<bf16x8*>(dgate)[i] = pack8(oa);
       reinterpret_cast<bf16x8*>(dup)[i] = pack8(ob);
     } else {
@@ -1297,14 +1328,16 @@ extern "C" int opk_geglu_fwd(const void* gu, void* act, int T, int F, int approx
 extern "C" int opk_geglu_bwd(const void* dact, const void* gu, void* dgu, int T, int F, int approx, void* stream) {
   return approx ? glu_bwd<2>(dact, gu, dgu, (long long)T * F, ST(stream)) : glu_bwd<1>(dact, gu, dgu, (long long)T * F, ST(stream));
 }
-// Gate and up in separate buffers of n elements; kind 0 = SwiGLU, 1 = GEGLU (erf), 2 = GEGLU (tanh). n a multiple of 8,
-// every buffer 16-byte aligned.
+// Gate and up in separate buffers of n elements; kind 0 = SwiGLU, 1 = GEGLU (erf), 2 = GEGLU (tanh), 3 and 4 = 0 and 2 rounded
+// operation by operation. n a multiple of 8, every buffer 16-byte aligned.
 extern "C" int opk_glu_split_fwd(const void* gate, const void* up, void* act, int64_t n, int kind, void* stream) {
   if (n <= 0) return 0;
-  if (n % 8 || kind < 0 || kind > 2 || !aligned16(gate, up, act)) return -1;
+  if (n % 8 || kind < 0 || kind > 4 || !aligned16(gate, up, act)) return -1;
   const int g = grid_for(n >> 3, 256);
   if (kind == 0) glu_fwd_kernel<0, true><<<g, 256, 0, ST(stream)>>>(BF(gate), BF(up), BFM(act), n >> 3);
   else if (kind == 1) glu_fwd_kernel<1, true><<<g, 256, 0, ST(stream)>>>(BF(gate), BF(up), BFM(act), n >> 3);
+  else if (kind == 3) glu_fwd_kernel<3, true><<<g, 256, 0, ST(stream)>>>(BF(gate), BF(up), BFM(act), n >> 3);
+  else if (kind == 4) glu_fwd_kernel<4, true><<<g, 256, 0, ST(stream)>>>(BF(gate), BF(up), BFM(act), n >> 3);
   else glu_fwd_kernel<2, true><<<g, 256, 0, ST(stream)>>>(BF(gate), BF(up), BFM(act), n >> 3);
   OPK_LAUNCH_CHECK();
   return 0;
@@ -1312,10 +1345,12 @@ extern "C" int opk_glu_split_fwd(const void* gate, const void* up, void* act, in
 extern "C" int opk_glu_split_bwd(const void* dact, const void* gate, const void* up, void* dgate, void* dup, int64_t n, int kind,
                                  void* stream) {
   if (n <= 0) return 0;
-  if (n % 8 || kind < 0 || kind > 2 || !aligned16(dact, gate, up, dgate, dup)) return -1;
+  if (n % 8 || kind < 0 || kind > 4 || !aligned16(dact, gate, up, dgate, dup)) return -1;
   const int g = grid_for(n >> 3, 256);
   if (kind == 0) glu_bwd_kernel<0, true><<<g, 256, 0, ST(stream)>>>(BF(dact), BF(gate), BF(up), BFM(dgate), BFM(dup), n >> 3);
   else if (kind == 1) glu_bwd_kernel<1, true><<<g, 256, 0, ST(stream)>>>(BF(dact), BF(gate), BF(up), BFM(dgate), BFM(dup), n >> 3);
+  else if (kind == 3) glu_bwd_kernel<3, true><<<g, 256, 0, ST(stream)>>>(BF(dact), BF(gate), BF(up), BFM(dgate), BFM(dup), n >> 3);
+  else if (kind == 4) glu_bwd_kernel<4, true><<<g, 256, 0, ST(stream)>>>(BF(dact), BF(gate), BF(up), BFM(dgate), BFM(dup), n >> 3);
   else glu_bwd_kernel<2, true><<<g, 256, 0, ST(stream)>>>(BF(dact), BF(gate), BF(up), BFM(dgate), BFM(dup), n >> 3);
   OPK_LAUNCH_CHECK();
   return 0;

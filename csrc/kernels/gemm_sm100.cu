@@ -252,11 +252,12 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   } else {
     if (!make_map(&tb, a->B, a->K, a->N, bbatch, a->ldb, a->strideB, narrow ? narrow : pair ? 128 : bn)) return -2;
   }
+  if (a->stepwise && (a->epilogue != opk::EPI_STORE || a->bias)) { set_err("opk_gemm: stepwise rounding takes a plain store without a bias"); return -1; }
   opk::GemmParams p;
   memset(&p, 0, sizeof(p));
   p.M = a->M; p.N = a->N; p.K = a->K; p.batch = a->batch; p.b_batch_div = bdiv;
   p.ldc = a->ldc; p.strideC = a->strideC; p.C = a->C; p.R = a->R; p.bias = a->bias;
-  p.alpha = a->alpha; p.sumsq = a->sumsq; p.act = a->act; p.ld_act = a->ld_act; p.labels = a->labels;
+  p.alpha = a->alpha; p.stepwise = a->stepwise; p.sumsq = a->sumsq; p.act = a->act; p.ld_act = a->ld_act; p.labels = a->labels;
   p.pmax = a->pmax; p.psum = a->psum; p.tgt = a->tgt; p.lse = a->lse; p.coef = a->coef; p.softcap = a->softcap;
   p.err = a->err;
   p.tile_group = a->tile_group; p.group_k = a->group_k; p.sumsq_stride = a->sumsq_shared ? 0 : 1;

@@ -38,6 +38,7 @@ struct GemmParams {
   const void* R;         // optional residual, same layout as C (may alias C)
   const void* bias;      // optional bf16 [N]
   float alpha;
+  int stepwise;          // EPI_STORE: the product is rounded to bf16, scaled and rounded again before R is added
   double* sumsq;         // EPI_SUMSQ: one accumulator per batch entry (sumsq[b])
   void* act;             // EPI_SWIGLU: bf16 [M][ld_act] (written); EPI_SWIGLU_BWD: saved pre-activations (read)
   long long ld_act;
@@ -209,7 +210,10 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, EpiState& e, floa
   if (ncols <= 0) return;
   const bool full = ncols == 32 && e.vec_ok;
   __nv_bfloat16* Crow = e.C + (long long)(threadIdx.x & 31) * p.ldc + col0;
-  if (p.alpha != 1.f) {
+  if (EPI == EPI_STORE && p.stepwise) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = bf16_round(__fmul_rn(bf16_round(v[j]), p.alpha));
+  } else if (p.alpha != 1.f) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] *= p.alpha;
   }

@@ -43,6 +43,7 @@ typedef struct OpkGemmArgs {
   // counters, one per band of 2048 rows of B (zeroed by opk_gemm on the stream before the launch).
   void* stage_dst;
   int32_t* stage_ready;
+  int32_t stepwise;      // epilogue 0 without a bias: C = round(round(alpha * round(acc)) + R), as separate bf16 operations give it
   int32_t lce_parts;     // EPI_LCE_FWD: column parts per 256-column tile in pmax / psum (2, else 1)
 } OpkGemmArgs;
 
@@ -96,7 +97,8 @@ int opk_swiglu_bwd(const void* dact, const void* gu, void* dgu, int T, int F, vo
 // GEGLU (tanh approximation when approx != 0), same interleaved layout.
 int opk_geglu_fwd(const void* gu, void* act, int T, int F, int approx, void* stream);
 int opk_geglu_bwd(const void* dact, const void* gu, void* dgu, int T, int F, int approx, void* stream);
-// Gate and up in separate buffers (kind 0 SwiGLU, 1 GEGLU erf, 2 GEGLU tanh); n a multiple of 8, 16-byte aligned buffers.
+// Gate and up in separate buffers (kind 0 SwiGLU, 1 GEGLU erf, 2 GEGLU tanh; 3 and 4: 0 and 2 with every operation rounded by
+// itself); n a multiple of 8, 16-byte aligned buffers.
 int opk_glu_split_fwd(const void* gate, const void* up, void* act, int64_t n, int kind, void* stream);
 int opk_glu_split_bwd(const void* dact, const void* gate, const void* up, void* dgate, void* dup, int64_t n, int kind, void* stream);
 // GELU (GPT-2 "gelu_new" tanh form): y = gelu(x); backward dx = dy * gelu'(x).

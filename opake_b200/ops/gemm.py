@@ -49,13 +49,15 @@ def gemm(
     sumsq_shared: bool = False,
     norm_only: bool = False,
     stage: tuple[torch.Tensor, torch.Tensor] | None = None,
+    stepwise: bool = False,
 ) -> torch.Tensor | None:
     """General entry: ``out[b] = alpha * op(a[b]) @ op(b[b // b_batch_div])^T`` with an epilogue.
 
     ``a_mn=False``: ``a`` is ``[M, K]``; ``a_mn=True``: ``a`` is ``[K, M]`` (used as its transpose).
     ``b_mn=False``: ``b`` is ``[N, K]``; ``b_mn=True``: ``b`` is ``[K, N]``.
     Every output element adds its products in the same order whatever the other sizes are: a row of ``a`` gives the same
-    bits alone and among thousands, whichever kernel the sizes favour.
+    bits alone and among thousands, whichever kernel the sizes favour. ``stepwise`` (plain store): rounded like the separate
+    operations ``residual + alpha * (a @ b)`` on bf16 tensors, product, scaling and sum each to bf16.
     """
     _check2d(a, "a")
     _check2d(b, "b")
@@ -113,7 +115,7 @@ def gemm(
         args.strideB = b.stride(0)
     if group_k is not None:         # per-batch reduction ranges over un-batched operands (mixture of experts wgrad)
         args.group_k = group_k.data_ptr()
-    args.sumsq_shared = int(sumsq_shared)
+    args.sumsq_shared, args.stepwise = int(sumsq_shared), int(stepwise)
     if stage is not None:           # b lives on another GPU: (local scratch [N, K] bf16, int32 band counters)
         scratch, ready = stage
         if scratch.numel() < N * K or scratch.dtype != torch.bfloat16 or ready.dtype != torch.int32 or ready.numel() * 2048 < N:

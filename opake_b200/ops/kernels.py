@@ -154,7 +154,8 @@ def geglu_bwd(dact, gu, approximate: bool = True, out=None):
 
 
 def glu_split_fwd(gate, up, kind: int):
-    """``act(gate) * up`` of two contiguous bf16 buffers (a multiple of 8 elements); kind 0 SwiGLU, 1 GEGLU, 2 GEGLU tanh."""
+    """``act(gate) * up`` of two contiguous bf16 buffers (a multiple of 8 elements); kind 0 SwiGLU, 1 GEGLU, 2 GEGLU tanh;
+    3 and 4: 0 and 2 with every fp32 operation rounded by itself (library exponential)."""
     act = torch.empty_like(gate)
     _chk(_L().opk_glu_split_fwd(_p(gate), _p(up), _p(act), gate.numel(), kind, _s(gate)), "glu_split_fwd")
     return act

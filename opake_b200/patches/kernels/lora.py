@@ -40,22 +40,23 @@ def _native_pair(a: torch.Tensor, b: torch.Tensor, n: int) -> bool:
 
 
 def _adapted(x, W, xa, B, s):
-    """``x W^T + s (xa B^T)``; on the tcgen05 GEMM the base product enters as the residual of the adapter's epilogue."""
+    """``x W^T + s (xa B^T)``; on the tcgen05 GEMM the base product enters as the residual of the adapter's epilogue. The
+    epilogue rounds where the formula does: whether a call has the rows and widths for the kernel does not show in its result."""
     y = _mm(x, W)
     if _native_pair(xa, B, B.shape[0]) and y.dtype == torch.bfloat16 and y.shape[1] % 8 == 0:
         from ...ops import gemm as G
-        return G.gemm(xa.contiguous(), B.contiguous(), out=y, residual=y, alpha=s)
+        return G.gemm(xa.contiguous(), B.contiguous(), out=y, residual=y, alpha=s, stepwise=True)
     return y + s * _mm(xa, B)
 
 
 def _adapted_nn(dy, W, dyB, A, s, dx=None):
-    """``(dx +) dy W + s (dyB A)``."""
+    """``(dx +) dy W + s (dyB A)``, added from the left; ``dx`` may be overwritten."""
     if (_native_pair(dy, W, W.shape[1]) and _native_pair(dyB, A, A.shape[1]) and (dx is None or dx.dtype == torch.bfloat16)):
         from ...ops import gemm as G
-        out = G.gemm(dy.contiguous(), W.contiguous(), b_mn=True, out=dx, residual=dx)
-        return G.gemm(dyB.contiguous(), A.contiguous(), b_mn=True, out=out, residual=out, alpha=s)
-    part = _mm_nn(dy, W) + s * _mm_nn(dyB, A)
-    return part if dx is None else dx + part
+        out = G.gemm(dy.contiguous(), W.contiguous(), b_mn=True, out=dx, residual=dx, stepwise=True)
+        return G.gemm(dyB.contiguous(), A.contiguous(), b_mn=True, out=out, residual=out, alpha=s, stepwise=True)
+    base = _mm_nn(dy, W)
+    return (base if dx is None else dx + base) + s * _mm_nn(dyB, A)
 
 
 class _LoRABwd(torch.autograd.Function):
@@ -159,7 +160,8 @@ class _LoRAQKVBwd(torch.autograd.Function):
         dx, grads = None, []
         for dy, xa, W, A, B, s in ((dq, xaq, Wq, Aq, Bq, sq), (dk, xak, Wk, Ak, Bk, sk), (dv, xav, Wv, Av, Bv, sv)):
             dyB, dA, dB = _adapter_grads(dy, x, xa, A, B, s, n)
-            dx = _adapted_nn(dy, W, dyB, A, s, dx)
+            part = _adapted_nn(dy, W, dyB, A, s)
+            dx = part if dx is None else dx + part
             grads += [dA, dB]
         return (dx, *grads)
 
@@ -241,7 +243,7 @@ def _native_act(*ts) -> bool:
 def _act_fwd(g, u, act: str):
     if _native_act(g, u):
         from ...ops import kernels as K
-        return K.glu_split_fwd(g, u, 0 if act == "silu" else 2)
+        return K.glu_split_fwd(g, u, 3 if act == "silu" else 4)
     gf = g.float()
     a = torch.nn.functional.silu(gf) if act == "silu" else torch.nn.functional.gelu(gf, approximate="tanh")
     return (a * u.float()).to(g.dtype)
@@ -250,7 +252,7 @@ def _act_fwd(g, u, act: str):
 def _act_bwd(dh, g, u, act: str):
     if _native_act(dh, g, u):
         from ...ops import kernels as K
-        return K.glu_split_bwd(dh, g, u, 0 if act == "silu" else 2)
+        return K.glu_split_bwd(dh, g, u, 3 if act == "silu" else 4)
     gf, uf, dhf = g.float(), u.float(), dh.float()
     if act == "silu":
         sig = torch.sigmoid(gf)
