@@ -986,7 +986,8 @@ __device__ __forceinline__ int ce_head(const void* p, long long base, int n) {
   return h < n ? h : n;
 }
 
-// One CTA per row, online (max, sum) per thread: one exponential per element plus one per vector.
+// One CTA per row, online (max, sum) per thread: one exponential per element plus one per vector. Entries of -inf that come
+// before any other value are passed over (the sum stays 0); a NaN is not, although fmaxf ignores it: the row's loss is NaN.
 template <bool FP32>
 __global__ void __launch_bounds__(NT) ce_fwd_kernel(const void* __restrict__ logits, const int* __restrict__ labels,
                                                     float* __restrict__ nll, float* __restrict__ lse, int V,
@@ -999,7 +1000,7 @@ __global__ void __launch_bounds__(NT) ce_fwd_kernel(const void* __restrict__ log
   auto one = [&](float raw) {
     const float z = cap(raw, scale, softcap);
     const float nm = fmaxf(m, z);
-    if (nm == -INFINITY) return;          // every logit so far is -inf: the running sum stays 0
+    if (nm == -INFINITY && z == -INFINITY) return;
     s = s * __expf(m - nm) + __expf(z - nm);
     m = nm;
   };
@@ -1014,7 +1015,12 @@ __global__ void __launch_bounds__(NT) ce_fwd_kernel(const void* __restrict__ log
     float nm = m;
 #pragma unroll
     for (int j = 0; j < VW; ++j) { z[j] = cap(z[j], scale, softcap); nm = fmaxf(nm, z[j]); }
-    if (nm == -INFINITY) continue;
+    if (nm == -INFINITY) {
+      float t = z[0];
+#pragma unroll
+      for (int j = 1; j < VW; ++j) t += z[j];
+      if (t == -INFINITY) continue;       // all of them -inf, no NaN among them
+    }
     float add = 0.f;
 #pragma unroll
     for (int j = 0; j < VW; ++j) add += __expf(z[j] - nm);
@@ -1030,7 +1036,7 @@ __global__ void __launch_bounds__(NT) ce_fwd_kernel(const void* __restrict__ log
   __syncthreads();
   float bm = sh[0];
   for (int w = 1; w < NT / 32; ++w) bm = fmaxf(bm, sh[w]);
-  const float tot = block_sum<NT>(m == -INFINITY ? 0.f : s * __expf(m - bm), sh);
+  const float tot = block_sum<NT>(m == -INFINITY ? s : s * __expf(m - bm), sh);   // m = -inf: s is 0, or NaN
   if (threadIdx.x == 0) {
     const float l = bm + logf(tot);
     if (lse) lse[row] = l;

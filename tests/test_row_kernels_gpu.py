@@ -134,3 +134,32 @@ def test_cross_entropy_rows(cuda, dtype, V, softcap):
     assert bool(((nll.double() - ref).abs() <= ref.abs() * 1e-5 + 2e-5).all())
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-5
     assert bool(((g.double() - want).abs() <= want.abs() * eps + 2e-6).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [7, 256, 4001, 32000, 50257])
+@pytest.mark.parametrize("softcap", [0.0, 30.0])
+def test_cross_entropy_keeps_nan(cuda, dtype, V, softcap):
+    """A NaN anywhere in a row (before its first 16-byte boundary, in a vector, a whole vector, after the last vector, behind
+    masked entries, everywhere) makes the row's loss and gradient NaN and touches no other row."""
+    from opake_b200.patches.kernels import opake_cross_entropy
+
+    base = torch.randn(12, V, device=cuda) * 3
+    spots = [slice(0, 1), slice(V - 1, V), slice(V // 2, V // 2 + 1), slice(0, min(16, V)), slice(max(0, V - 16), V), slice(0, V)]
+    rows = [1, 3, 5, 7, 9, 11]                       # odd rows of an odd width start off the 16-byte boundary
+    for r, s in zip(rows, spots):
+        base[r, s] = float("nan")
+    if V > 20:
+        base[3, : V - 1] = float("-inf")             # NaN after nothing but masked entries
+        base[2, : V - 1] = float("-inf")             # one entry left: its loss is 0
+    logits = base.to(dtype).requires_grad_()
+    labels = torch.full((12,), V - 1, device=cuda)
+    nll = opake_cross_entropy(logits, labels, logit_softcapping=softcap)
+    (g,) = torch.autograd.grad(nll.sum(), logits)
+    bad = torch.zeros(12, dtype=torch.bool, device=cuda)
+    bad[rows] = True
+    assert torch.equal(nll.isnan(), bad)
+    assert torch.equal(g.isnan().any(1), bad)
+    z = softcap * torch.tanh(logits.detach().double() / softcap) if softcap else logits.detach().double()
+    ref = torch.nn.functional.cross_entropy(z, labels, reduction="none")
+    assert bool(((nll.double() - ref).abs() <= ref.abs() * 1e-5 + 2e-5)[~bad].all())
