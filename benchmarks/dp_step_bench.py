@@ -4,9 +4,11 @@
         -m benchmarks.dp_step_bench [--model llama32_1b] [--iters 5]
 
 For every shard mode the engine's own ``apply_update()`` (barriers, the fused ``opk_dp_step`` kernel, zeroing of the
-sums) is timed with CUDA events on the launching stream after warm-up, as the maximum over ranks, on the engine's
+sums where the mode has it) is timed with CUDA events on the launching stream after warm-up, as the maximum over ranks, on the engine's
 real buffers (their total is far larger than L2). Modes:
 
+``local``  one rank: what a step of more than one accumulation group ends with. The kernel adds the last group of clipped
+           gradients itself and the sums are not zeroed.
 ``state``  sums and parameters replicated, moments sharded: the kernel reduce-scatters by loading every peer's fp32
            sums over NVLink and all-gathers by storing the new bf16 parameters into every replica.
 ``full``   sums and parameters sharded as well: the reduction happened during the backward (pushes into the owners'
@@ -42,7 +44,7 @@ def main() -> None:
     ap = argparse.ArgumentParser()
     ap.add_argument("--model", default="llama32_1b")
     ap.add_argument("--iters", type=int, default=5)
-    ap.add_argument("--modes", default="state,full,nccl")
+    ap.add_argument("--modes", default="", help="default: local on one rank, state,full,nccl on more")
     a = ap.parse_args()
     from opake_b200.parallel import comm
 
@@ -55,18 +57,32 @@ def main() -> None:
 
     mcfg = getattr(C, a.model)()
     hbm, src = _hbm_gbs()
-    for mode in a.modes.split(","):
-        if mode == "nccl" and world == 1:
+    for mode in (a.modes or ("local" if world == 1 else "state,full,nccl")).split(","):
+        if (mode == "local") != (world == 1):
             continue
         kw = dict(shard_params=mode == "full", shard_sums=mode == "full", comm_backend="nccl" if mode == "nccl" else "peer")
         eng = ShardedDPEngine(mcfg, EngineConfig(logical_batch=world, noise_multiplier=0.9, use_cuda_graph=False, seq_len=128, **kw), dev)
         P, n = eng.layout.total, eng.shard_len
-        eng.acc.normal_()                      # something to reduce; the step's cost does not depend on the values
+        dense = eng.layout.dense_total
+
+        def fill():
+            # the state that a step leaves for its update (values do not change the cost): sums, or gradients not yet in them
+            if world == 1:
+                eng._last_group, eng._have_sums = eng.group, True
+
+        if world == 1:
+            for g, s in zip(eng.runtime.Gs, eng.runtime.scales):
+                g.normal_(std=1e-3)
+                s.fill_(1.0)
+        else:
+            eng.acc.normal_()
         for _ in range(3):
+            fill()
             eng.apply_update()
         torch.cuda.synchronize(dev)
         times = []
         for _ in range(a.iters):
+            fill()
             if world > 1:
                 dist.barrier()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -81,7 +97,10 @@ def main() -> None:
             dist.all_reduce(t, op=dist.ReduceOp.MAX)
         ms = float(t)
         # bytes per rank, from the algorithm: moments 16 n (read + write), parameter read 2 n; mode-specific rest
-        if mode == "state":
+        if mode == "local":
+            hbm_b = 16 * n + 2 * n + 4 * n + 2 * n + 2 * eng.group * dense          # m,v; p read; sum read; p write; last group
+            link_in = link_out = 0
+        elif mode == "state":
             hbm_b = 16 * n + 2 * n + 4 * n + 2 * n + 4 * P + 4 * n * (world - 1) + 2 * n * (world - 1)
             #        m,v      p read  own sum  own p   zero    peers read my sums   peers write my replica
             link_in, link_out = 4 * n * (world - 1), 2 * n * (world - 1)

@@ -99,12 +99,12 @@ class ShardedDPEngine:
         self.params = self.params_pb.local
         if self.shard_sums:
             longest = max(self.bounds[r + 1] - self.bounds[r] for r in range(self.world))
-            self.acc_pb = comm.alloc_peer_buffer(max(longest, 8), torch.float32, device)    # this rank's shard only
+            self._acc_pb = comm.alloc_peer_buffer(max(longest, 8), torch.float32, device)    # this rank's shard only
         else:
-            self.acc_pb = comm.alloc_peer_buffer(total, torch.float32, device)
-        self.acc = self.acc_pb.local
+            self._acc_pb = comm.alloc_peer_buffer(total, torch.float32, device)
+        self._acc = self._acc_pb.local
         init_params_(model_cfg, self.params, self.layout, seed=init_seed)  # same seed on every rank -> same replica
-        self.acc.zero_()
+        self._acc.zero_()
         self.m = torch.zeros(self.shard_len, dtype=torch.float32, device=device)
         self.v = torch.zeros(self.shard_len, dtype=torch.float32, device=device)
         self.master = None
@@ -135,8 +135,10 @@ class ShardedDPEngine:
         # One rank: the dense part of the sums is never zeroed. The first group of a step overwrites it, and the last group
         # is added inside the step kernel, which does not read the sums at all when there was only one group.
         self._fuse_last_group = self.world == 1
+        # The sums are then not what `acc` promises: a caller who asks for that buffer gets settled sums and, from there on, the
+        # separate passes (see `acc`).
         self._last_group = 0          # gradient slots that the next update adds itself
-        self._have_sums = False       # the sums hold earlier groups of this step
+        self._have_sums = False       # the sums hold groups that no update has applied yet (else: stale values)
         self._rs_out = torch.empty(self.shard_len, dtype=torch.float32, device=device) if self.nccl_step else None
         self._stale = False      # shard_params: the replica's remote parts are older than their owners' copies
         self._refresh: dict[int, tuple] = {}
@@ -218,18 +220,44 @@ class ShardedDPEngine:
         self._refresh[T] = plan
         return plan
 
+    def _settle_sums(self) -> None:
+        """Brings the dense sums of one rank up to date: zero where nothing is pending, the last group added."""
+        dense = self._acc[: self.layout.dense_total]
+        if self._last_group:
+            n = self._last_group
+            K.clip_accumulate_group(self.runtime.Gs[:n], self.runtime.scales[:n], dense, overwrite=not self._have_sums)
+        elif not self._have_sums:
+            dense.zero_()
+        self._last_group, self._have_sums = 0, True
+
+    @property
+    def acc(self) -> torch.Tensor:
+        """The fp32 sums of the clipped gradients (this rank's shard of them with ``shard_sums``): zero after an update, and
+        whatever a caller adds to them is part of the next one, with or without a step in between. On one rank the steps
+        do without most passes over this buffer; once it has been asked for, they run all of them."""
+        if self._fuse_last_group:
+            self._settle_sums()
+            self._fuse_last_group = False
+        return self._acc
+
+    @property
+    def acc_pb(self):
+        """The peer-addressable buffer behind :attr:`acc`."""
+        self.acc
+        return self._acc_pb
+
     def _accumulate(self, ws, n: int, toks, overwrite: bool = False) -> None:
         """Adds the clipped gradients held in slots ``0 .. n-1`` to the fp32 sums (local pass, or reductions into the
         owners' shards when the sums are sharded)."""
         if not self.shard_sums:
-            self.runtime.accumulate_group(self.acc, ws, n, toks=toks, overwrite=overwrite)
+            self.runtime.accumulate_group(self._acc, ws, n, toks=toks, overwrite=overwrite)
             return
         emb_acc = None
         if not self.model_cfg.tie_embeddings:
             emb = self.layout.slot("embed")
             owner = self.layout.owner_of("embed", self.bounds)
-            emb_acc = self.acc_pb.peer_view(owner, emb.shape, offset=emb.offset - self.bounds[owner])
-        self.runtime.accumulate_group_sharded(self.acc_pb.ptrs, self.bounds, self.rank, ws, n, emb_acc=emb_acc, toks=toks)
+            emb_acc = self._acc_pb.peer_view(owner, emb.shape, offset=emb.offset - self.bounds[owner])
+        self.runtime.accumulate_group_sharded(self._acc_pb.ptrs, self.bounds, self.rank, ws, n, emb_acc=emb_acc, toks=toks)
 
     def _example_body(self, ws, slot: int, drain_prev: bool, refresh: bool = False, first: bool = False) -> None:
         """Gradient of the example staged in slot ``slot``; meanwhile (side stream) the clipped accumulation of the
@@ -286,7 +314,10 @@ class ShardedDPEngine:
         ws = self.runtime.workspace(T)
         slot = index % self.group
         drain = index > 0
-        first = index == self.group and self._fuse_last_group       # drains the first group of the step
+        drains = drain and slot == 0
+        first = drains and self._fuse_last_group and not self._have_sums       # the sums hold nothing that counts
+        if drains:
+            self._have_sums = True
         refresh = index == 0 and self._stale
         if refresh:
             self._stale = False
@@ -302,14 +333,14 @@ class ShardedDPEngine:
 
             if not self._warm.get((T, refresh)):
                 # eager warm-up (lazy workspaces, library autotuning) on a side stream, state restored afterwards
-                saved = (ws["loss_sum"].clone(), self.acc.clone() if self.acc.numel() < (1 << 28) else None)
+                saved = ws["loss_sum"].clone()
                 s = torch.cuda.Stream(device=self.device)
                 s.wait_stream(torch.cuda.current_stream(self.device))
                 with torch.cuda.stream(s):
                     self._example_body(ws, slot, False, refresh)
                 torch.cuda.current_stream(self.device).wait_stream(s)
                 torch.cuda.synchronize(self.device)
-                ws["loss_sum"].copy_(saved[0])
+                ws["loss_sum"].copy_(saved)
                 self.runtime.clip_count.zero_()
                 if self.ep is not None:
                     # warm-ups only ever happen on the first example of a step, where the expert sums are still zero
@@ -343,6 +374,8 @@ class ShardedDPEngine:
             # the exchange kernels wait for their peers with a bounded budget: start every step together
             torch.cuda.synchronize(self.device)
             dist.barrier()
+        if self._last_group:
+            self._settle_sums()       # left over from an update that was not applied: the gradient slots are refilled now
         ws = self.runtime.workspace(tokens.shape[1])
         if "loss_sum" not in ws:
             ws["loss_sum"] = torch.zeros(1, dtype=torch.float32, device=self.device)
@@ -356,8 +389,8 @@ class ShardedDPEngine:
         # example that followed it
         n_last = B_local % self.group or min(self.group, B_local)
         if n_last and self._fuse_last_group:
-            self.runtime.accumulate_embeddings(self.acc, ws, n_last, toks=self._group_toks(ws, n_last))
-            self._last_group, self._have_sums = n_last, B_local > n_last
+            self.runtime.accumulate_embeddings(self._acc, ws, n_last, toks=self._group_toks(ws, n_last))
+            self._last_group = n_last
         elif n_last:
             self._accumulate(ws, n_last, self._group_toks(ws, n_last))
         loss_sum = ws["loss_sum"].clone()
@@ -368,6 +401,7 @@ class ShardedDPEngine:
         return loss_sum
 
     def apply_update(self) -> None:
+        """The optimizer step on the sums: those of the last ``step`` call, and what a caller added to :attr:`acc`."""
         cfg = self.cfg
         t = self.step_count + 1
         b1, b2 = cfg.betas
@@ -381,12 +415,12 @@ class ShardedDPEngine:
             self._apply_update_nccl(sigma, step_key, phi_hat, t)
             return
         if self.world > 1:
-            self.acc_pb.barrier()       # every rank finished accumulating before anyone reads (or owns) the sums
+            self._acc_pb.barrier()       # every rank finished accumulating before anyone reads (or owns) the sums
         if self.shard_sums:
             # the owner's shard already holds the sum over all ranks; addressed with global offsets like a full buffer
-            grad_src = [self.acc.data_ptr() - 4 * self.shard_begin]
+            grad_src = [self._acc.data_ptr() - 4 * self.shard_begin]
         else:
-            grad_src = self._rotate(self.acc_pb.ptrs)
+            grad_src = self._rotate(self._acc_pb.ptrs)
         # sharded parameters: only the owner's copy is written here, the other ranks fetch it in their next forward pass
         param_dst = [self.params.data_ptr()] if self.shard_params else self._rotate(self.params_pb.ptrs)
         fused = {}
@@ -394,7 +428,6 @@ class ShardedDPEngine:
             n = self._last_group
             fused = dict(group=self.runtime.Gs[:n], group_scales=self.runtime.scales[:n], group_len=self.layout.dense_total,
                          skip_sum=not self._have_sums)
-            self._last_group, self._have_sums = 0, False
         K.dp_step(
             grad_src=grad_src, shard_begin=self.shard_begin, shard_len=self.shard_len,
             inv_batch=1.0 / cfg.logical_batch, sigma=sigma, seed=step_key.seed, step=self.step_count,
@@ -403,6 +436,7 @@ class ShardedDPEngine:
             bc2=1.0 - b2**t, phi_hat=phi_hat, zero_grad=self.shard_sums, blt_state=self.blt_state, blt_decay=self.blt_decay,
             blt_scale=self.blt_scale, toep_state=self.toep_state, toep_coef=self.toep_coef, toep_pos=self.toep_pos,
             sgd_mode=(cfg.optimizer == "sgd"), device=self.device, **fused)
+        self._last_group, self._have_sums = 0, False
         if self.ep is not None:
             self.ep.apply_update(noise_offset=self.layout.total, inv_batch=1.0 / cfg.logical_batch, sigma=sigma, seed=step_key.seed,
                                  step=self.step_count, lr=cfg.lr, beta1=b1, beta2=b2, eps=cfg.eps, weight_decay=cfg.weight_decay,
@@ -413,9 +447,9 @@ class ShardedDPEngine:
             self.params_pb.barrier()    # the new parameters (and, sharded sums, the zeroed shards) are in place everywhere
         if self._fuse_last_group:
             if not self.model_cfg.tie_embeddings:
-                self.acc[self.layout.dense_total :].zero_()      # embedding rows are added to
+                self._acc[self.layout.dense_total :].zero_()      # embedding rows are added to
         elif not self.shard_sums:
-            self.acc.zero_()
+            self._acc.zero_()
         if self.shard_params:
             self._stale = True
         self.step_count += 1
@@ -427,7 +461,7 @@ class ShardedDPEngine:
         cfg = self.cfg
         b1, b2 = cfg.betas
         with nvtx_range("opake::dp_step/nccl"):
-            dist.reduce_scatter_tensor(self._rs_out, self.acc[: self.shard_len * self.world], op=dist.ReduceOp.SUM)
+            dist.reduce_scatter_tensor(self._rs_out, self._acc[: self.shard_len * self.world], op=dist.ReduceOp.SUM)
             K.dp_step(
                 grad_src=[self._rs_out.data_ptr() - 4 * self.shard_begin], shard_begin=self.shard_begin, shard_len=self.shard_len,
                 inv_batch=1.0 / cfg.logical_batch, sigma=sigma, seed=step_key.seed, step=self.step_count,
@@ -440,7 +474,7 @@ class ShardedDPEngine:
                 self.toep_pos = (self.toep_pos - 1) % self.toep_state.shape[0]
             mine = self.params[self.shard_begin : self.shard_begin + self.shard_len]
             dist.all_gather_into_tensor(self.params[: self.shard_len * self.world], mine)
-        self.acc.zero_()
+        self._acc.zero_()
         self.step_count += 1
 
     def gather_params(self) -> None:

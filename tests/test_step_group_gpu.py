@@ -59,3 +59,100 @@ def test_engine_steps_of_changing_batch_sizes(cuda, graph):
             e.step(tok, lab) if B else e.apply_update()
     a, b = engines
     assert torch.equal(a.params, b.params) and torch.equal(a.m, b.m) and torch.equal(a.v, b.v)
+
+
+@pytest.mark.parametrize("tied", [False, True])
+@pytest.mark.parametrize("graph", [False, True])
+def test_sums_that_a_caller_fills_are_applied(cuda, graph, tied):
+    """`acc` is zero between steps, and what a caller adds to it is part of the next update, with or without a step in between:
+    equal to an engine that runs every pass from its first step on."""
+    from dataclasses import replace
+
+    from opake_b200.models.config import tiny_llama
+    from opake_b200.parallel.engine import EngineConfig, ShardedDPEngine
+
+    cfg = replace(tiny_llama(), tie_embeddings=tied)
+    engines = []
+    for fused in (True, False):
+        e = ShardedDPEngine(cfg, EngineConfig(logical_batch=4, noise_multiplier=0.1, accumulate_group=2, use_cuda_graph=graph), cuda)
+        e._fuse_last_group = fused
+        engines.append(e)
+    gen = torch.Generator().manual_seed(0)
+    add = [torch.randn(engines[0].layout.total, generator=torch.Generator().manual_seed(i)).to(cuda) for i in range(2)]
+
+    def step(B):
+        tok = torch.randint(0, cfg.vocab_size, (B, 64), dtype=torch.int32, generator=gen).pin_memory()
+        for e in engines:
+            e.step(tok, torch.roll(tok, -1, 1).clone())
+
+    def same():
+        a, b = engines
+        assert torch.equal(a.params, b.params) and torch.equal(a.m, b.m) and torch.equal(a.v, b.v)
+
+    step(5)
+    same()
+    before = engines[0].m.clone()
+    for e in engines:
+        assert not bool(e.acc.any())
+        e.acc.copy_(add[0])
+        e.apply_update()
+        assert not bool(e.acc.any())
+    same()
+    assert float((engines[0].m - 0.9 * before).norm()) > 0.02 * float(add[0].norm()) / 4        # the sums were applied, not noise alone
+    for e in engines:
+        e.acc.add_(add[1])
+    step(3)
+    same()
+    step(2)
+    same()
+
+
+def test_sums_seen_by_an_update_that_looks_at_them(cuda):
+    """A subclass that reads the sums before they are applied sees all groups of the step."""
+    from opake_b200.models.config import tiny_llama
+    from opake_b200.parallel.engine import EngineConfig, ShardedDPEngine
+
+    cfg = tiny_llama()
+    seen = {}
+
+    class Looking(ShardedDPEngine):
+        def apply_update(self):
+            seen.setdefault(self.tag, []).append(self.acc.clone())
+            super().apply_update()
+
+    gen = torch.Generator().manual_seed(0)
+    batches = [torch.randint(0, cfg.vocab_size, (B, 64), dtype=torch.int32, generator=gen).pin_memory() for B in (3, 1, 4)]
+    for tag, fused in (("a", True), ("b", False)):
+        e = Looking(cfg, EngineConfig(logical_batch=4, noise_multiplier=0.1, accumulate_group=2), cuda)
+        e.tag, e._fuse_last_group = tag, fused
+        for tok in batches:
+            e.step(tok, torch.roll(tok, -1, 1).clone())
+    for x, y in zip(seen["a"], seen["b"]):
+        assert bool(x.any()) and torch.equal(x, y)
+
+
+def test_step_after_an_update_that_failed(cuda):
+    """The groups of a step whose update raised stay in the sums, as they do in separate passes."""
+    from opake_b200.models.config import tiny_llama
+    from opake_b200.parallel.engine import EngineConfig, ShardedDPEngine
+
+    cfg = tiny_llama()
+    gen = torch.Generator().manual_seed(0)
+    batches = [torch.randint(0, cfg.vocab_size, (B, 64), dtype=torch.int32, generator=gen).pin_memory() for B in (3, 1, 4)]
+    engines = []
+    for fused in (True, False):
+        e = ShardedDPEngine(cfg, EngineConfig(logical_batch=4, noise_multiplier=0.1, accumulate_group=2), cuda)
+        e._fuse_last_group = fused
+        engines.append(e)
+        update = e.apply_update
+        for i, tok in enumerate(batches):
+            def fail():
+                raise OSError("interrupted")
+
+            e.apply_update = fail if i == 0 else update
+            try:
+                e.step(tok, torch.roll(tok, -1, 1).clone())
+            except OSError:
+                assert i == 0
+    a, b = engines
+    assert torch.equal(a.params, b.params) and torch.equal(a.m, b.m)
