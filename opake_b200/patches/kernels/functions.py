@@ -298,7 +298,7 @@ class _CE(torch.autograd.Function):
     def forward(logits, labels, scale, softcap):
         from ...ops import kernels as K
         V = logits.shape[-1]
-        lab = labels.reshape(-1).to(torch.int32).contiguous()
+        lab = labels.reshape(-1).to(torch.int32, copy=True).contiguous()      # kept for the backward pass: never the caller's buffer
         nll, lse = K.cross_entropy_fwd(logits.reshape(-1, V), lab, scale, softcap)
         return nll.view(labels.shape), lse.view(labels.shape), lab.view(labels.shape)
 

@@ -163,3 +163,17 @@ def test_cross_entropy_keeps_nan(cuda, dtype, V, softcap):
     z = softcap * torch.tanh(logits.detach().double() / softcap) if softcap else logits.detach().double()
     ref = torch.nn.functional.cross_entropy(z, labels, reduction="none")
     assert bool(((nll.double() - ref).abs() <= ref.abs() * 1e-5 + 2e-5)[~bad].all())
+
+
+def test_cross_entropy_label_buffer_may_be_refilled(cuda):
+    from opake_b200.patches.kernels import opake_cross_entropy
+
+    logits = torch.randn(9, 128, device=cuda).to(torch.bfloat16).requires_grad_()
+    labels = torch.arange(9, dtype=torch.int32, device=cuda)
+    (want,) = torch.autograd.grad(opake_cross_entropy(logits, labels.long()).sum(), logits)
+    nll = opake_cross_entropy(logits, labels)
+    labels.zero_()
+    (got,) = torch.autograd.grad(nll.sum(), logits)
+    assert torch.equal(got, want)
+    f = torch.func.vmap(torch.func.grad(lambda z, l: opake_cross_entropy(z, l).sum()))
+    assert torch.equal(f(logits.detach().view(3, 3, 128), torch.arange(9, dtype=torch.int32, device=cuda).view(3, 3)).view(9, 128), want)
