@@ -8,6 +8,7 @@ nothing is cached between calls.
 from __future__ import annotations
 
 import struct
+from ctypes import c_float
 
 import torch
 
@@ -57,7 +58,8 @@ def _pack(rows) -> bytes:
                 ptrs[i] = t.data_ptr()
                 if t.dtype is torch.bfloat16:
                     mask |= 1 << i
-        out += _LEAF.pack(*ptrs, n, aux, s, mask)
+        # c_float rounds and overflows to infinity like a scalar next to an fp32 tensor; struct refuses what is out of range
+        out += _LEAF.pack(*ptrs, n, aux, c_float(s).value, mask)
     return bytes(out)
 
 

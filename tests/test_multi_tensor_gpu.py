@@ -121,3 +121,15 @@ def test_rope_of_a_batch(cuda):
     assert torch.equal(torch.func.vmap(lambda t: opake_rope_qk(t, table, H, hd))(x), one)
     nested = torch.func.vmap(torch.func.vmap(lambda t: opake_rope_qk(t, table, H, hd)))(x[:4].view(2, 2, T, -1))
     assert torch.equal(nested.view(4, T, -1), one[:4])
+
+
+def test_noise_of_a_huge_standard_deviation(cuda):
+    """Beyond the fp32 range the leaf-by-leaf formula gives infinities; so does the kernel."""
+    from opake_b200.dpsgd.noise import add_gaussian_noise_tree
+    from opake_b200.engine.random import key
+
+    tree = {"a": torch.zeros(1000, device=cuda), "b": torch.ones(33, device=cuda, dtype=torch.bfloat16)}
+    got = add_gaussian_noise_tree(tree, 1e39, key(0))
+    ref = add_gaussian_noise_tree({**tree, "c": torch.zeros(4, device=cuda, dtype=torch.float64)}, 1e39, key(0))     # leaf by leaf
+    for n in tree:
+        assert torch.equal(got[n], ref[n]) and bool(got[n].isinf().all())
