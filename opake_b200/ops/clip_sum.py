@@ -38,6 +38,7 @@ def fused_clip_sum(leaves: Sequence[torch.Tensor], clipping_norm: float, *, with
     of earlier micro-batches that this one is added to; ``scale`` multiplies the result."""
     from ..engine.clipping import numerics as N
     leaves = [l.contiguous() for l in leaves]
+    prev = None if prev is None else [p.contiguous() for p in prev]       # the portable path may leave other strides
     dev = leaves[0].device
     B = leaves[0].shape[0]
     outs = [torch.empty(l.shape[1:], dtype=torch.float32, device=dev) for l in leaves]

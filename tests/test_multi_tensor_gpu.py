@@ -133,3 +133,30 @@ def test_noise_of_a_huge_standard_deviation(cuda):
     ref = add_gaussian_noise_tree({**tree, "c": torch.zeros(4, device=cuda, dtype=torch.float64)}, 1e39, key(0))     # leaf by leaf
     for n in tree:
         assert torch.equal(got[n], ref[n]) and bool(got[n].isinf().all())
+
+
+def test_earlier_sums_of_any_strides(cuda):
+    from opake_b200.ops.clip_sum import fused_clip_sum
+
+    leaves = [torch.randn(3, 40, 24, device=cuda), torch.randn(3, 7, device=cuda).to(torch.bfloat16)]
+    prev = [torch.randn(24, 40, device=cuda).t(), torch.randn(7, device=cuda)]
+    got = fused_clip_sum(leaves, 1.0, prev=prev, scale=0.5)[0]
+    want = fused_clip_sum(leaves, 1.0, prev=[p.clone(memory_format=torch.contiguous_format) for p in prev], scale=0.5)[0]
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_micro_batches_on_either_side_of_the_kernel_limit(cuda):
+    """65,540 examples go through the portable path, the last 3 through the kernel: equal to one portable pass."""
+    from opake_b200 import patches
+    from opake_b200.dpsgd.clipping import clipped_grad
+
+    patches.apply_runtime_patches(compat=False)
+    p = {"w": torch.randn(3, 5, device=cuda)}
+    x = torch.randn(65543, 5, device=cuda)
+    loss = lambda q, xe: ((xe @ q["w"].t()) ** 2).sum()
+    sums = []
+    for micro in (65540, 65543):
+        fn, st = clipped_grad(loss, clipping_norm=1.0, normalize_by=65543.0, microbatch_size=micro)
+        sums.append(fn(p, x, state=st)[0].pytree["w"])
+    # fp32 sums of 65,543 terms of at most 1 in another order
+    assert float((sums[0] - sums[1]).abs().max()) <= 65543 ** 0.5 * 2.0 ** -23
