@@ -259,6 +259,11 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   p.ldc = a->ldc; p.strideC = a->strideC; p.C = a->C; p.R = a->R; p.bias = a->bias;
   p.alpha = a->alpha; p.stepwise = a->stepwise; p.sumsq = a->sumsq; p.act = a->act; p.ld_act = a->ld_act; p.labels = a->labels;
   p.pmax = a->pmax; p.psum = a->psum; p.tgt = a->tgt; p.lse = a->lse; p.coef = a->coef; p.softcap = a->softcap;
+  if (a->softcap > 0.f) {
+    const double inv = 1.0 / (double)a->softcap;
+    p.inv_cap = (float)inv;
+    p.inv_cap_lo = (float)(inv - (double)p.inv_cap);
+  }
   p.err = a->err;
   p.tile_group = a->tile_group; p.group_k = a->group_k; p.sumsq_stride = a->sumsq_shared ? 0 : 1;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
