@@ -841,7 +841,7 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, l
   double acc = 0.0;
   float part = 0.f;
   int cnt = 0;
-  // 16-byte loads, two vectors in flight, when the base allows it; fp32 partials of at most 64 squares as below
+  // 16-byte loads, four vectors in flight, when the base allows it; fp32 partials of at most 64 squares as below
   constexpr int VW = FP32 ? 4 : 8;
   const long long nvec = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / VW : 0;
 #pragma unroll 4
@@ -874,11 +874,6 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, l
     atomicAdd(out, t);
   }
   (void)sh;
-}
-
-__global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = __float2bfloat16(in[i]);
 }
 
 // ------------------------------------------------------------------------------------------- cross entropy
@@ -1281,7 +1276,7 @@ extern "C" int opk_layernorm_bwd(const void* dy, const void* x, const void* w, c
   return 0;
 }
 // period > 0: row t sits at position t % period (sequences of `period` rows one after the other).
-extern "C" int opk_rope_batch(void* qk, const float* cs, const int32_t* pos, int period, int64_t T, int n_rot_heads, int head_dim,
+extern "C" int opk_rope(void* qk, const float* cs, const int32_t* pos, int period, int64_t T, int n_rot_heads, int head_dim,
                               int64_t ld, float sign, void* stream) {
   const long long n = (long long)T * n_rot_heads * (head_dim / 2);
   if (n <= 0) return 0;
@@ -1293,10 +1288,6 @@ extern "C" int opk_rope_batch(void* qk, const float* cs, const int32_t* pos, int
     rope_kernel<<<grid_for(n, 256), 256, 0, ST(stream)>>>(BFM(qk), cs, pos, period, T, n_rot_heads, head_dim, ld, sign);
   OPK_LAUNCH_CHECK();
   return 0;
-}
-extern "C" int opk_rope(void* qk, const float* cs, const int32_t* pos, int T, int n_rot_heads, int head_dim, int64_t ld,
-                        float sign, void* stream) {
-  return opk_rope_batch(qk, cs, pos, 0, T, n_rot_heads, head_dim, ld, sign, stream);
 }
 namespace {
 bool aligned16(const void* a, const void* b, const void* c = nullptr, const void* d = nullptr, const void* e = nullptr) {
@@ -1465,18 +1456,7 @@ extern "C" int opk_sumsq(const void* x, int is_fp32, int round_bf16, int64_t n, 
   OPK_LAUNCH_CHECK();
   return 0;
 }
-extern "C" int opk_cast_f32_bf16(const float* in, void* out, int64_t n, void* stream) {
-  if (n <= 0) return 0;
-  cast_f32_bf16_kernel<<<grid_for(n, 256), 256, 0, ST(stream)>>>(in, BFM(out), n);
-  OPK_LAUNCH_CHECK();
-  return 0;
-}
-
-extern "C" int opk_scatter_rows_cast_sumsq(const float* src, void* dst_base, const int64_t* offsets, int R, int D,
-                                           double* sumsq, void* stream) {
-  return opk_scatter_rows_cast_sumsq_ragged(src, dst_base, offsets, nullptr, R, D, sumsq, stream);
-}
-extern "C" int opk_scatter_rows_cast_sumsq_ragged(const float* src, void* dst_base, const int64_t* offsets, const int32_t* widths, int R,
+extern "C" int opk_scatter_rows_cast_sumsq(const float* src, void* dst_base, const int64_t* offsets, const int32_t* widths, int R,
                                                   int D, double* sumsq, void* stream) {
   if (R <= 0) return 0;
   scatter_rows_cast_sumsq_kernel<<<R, NT, 0, ST(stream)>>>(src, BFM(dst_base), reinterpret_cast<const long long*>(offsets), widths, D, sumsq);

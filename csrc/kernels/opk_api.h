@@ -87,10 +87,9 @@ int opk_layernorm_bwd(const void* dy, const void* x, const void* w, const float*
                       const void* dres, void* dx_out, float* dw, float* db, int T, int D, void* stream);
 // In-place rotary embedding on the first n_rot_heads heads of each row (heads are head_dim wide, row pitch ld).
 // cs = [T][head_dim/2][2] fp32 (cos, sin); pos = optional int32 [T] row -> table row. sign = +1 forward, -1 backward.
-int opk_rope(void* qk, const float* cs, const int32_t* pos, int T, int n_rot_heads, int head_dim, int64_t ld,
+// Without pos, row t sits at position t % period (sequences of `period` rows one after the other; period 0: at position t).
+int opk_rope(void* qk, const float* cs, const int32_t* pos, int period, int64_t T, int n_rot_heads, int head_dim, int64_t ld,
              float sign, void* stream);
-int opk_rope_batch(void* qk, const float* cs, const int32_t* pos, int period, int64_t T, int n_rot_heads, int head_dim, int64_t ld,
-                   float sign, void* stream);
 // SwiGLU on interleaved (gate, up) columns. fwd: act[T][F]; bwd: dgu[T][2F] from dact[T][F] and gu[T][2F].
 int opk_swiglu_fwd(const void* gu, void* act, int T, int F, void* stream);
 int opk_swiglu_bwd(const void* dact, const void* gu, void* dgu, int T, int F, void* stream);
@@ -137,19 +136,15 @@ int opk_cross_entropy_bwd(const void* logits, int is_fp32, const int32_t* labels
                           void* dlogits, int T, int V, int64_t ld, float scale, float softcap, void* stream);
 // sum(x^2) of a bf16/fp32 vector (x rounded to bf16 first when round_bf16) added to *sumsq (double).
 int opk_sumsq(const void* x, int is_fp32, int round_bf16, int64_t n, double* sumsq, void* stream);
-// fp32 rows -> bf16 at dst_base + offsets[r] (device int64 array), with sum of squares of the stored values.
-int opk_scatter_rows_cast_sumsq(const float* src, void* dst_base, const int64_t* offsets, int R, int D, double* sumsq,
-                                void* stream);
-// Only the first widths[r] columns of row r (D = row pitch of src); widths == NULL: all D of every row.
-int opk_scatter_rows_cast_sumsq_ragged(const float* src, void* dst_base, const int64_t* offsets, const int32_t* widths, int R, int D,
-                                       double* sumsq, void* stream);
+// fp32 rows -> bf16 at dst_base + offsets[r] (device int64 array), with sum of squares of the stored values: the first widths[r]
+// columns of row r (device int32 array, D = row pitch of src); widths == NULL: all D of every row.
+int opk_scatter_rows_cast_sumsq(const float* src, void* dst_base, const int64_t* offsets, const int32_t* widths, int R, int D,
+                                double* sumsq, void* stream);
 // out[n] += sum_t dy[t][n] (out fp32, zeroed by the caller)
 int opk_colsum(const void* dy, float* out, int T, int N, int64_t ld, void* stream);
 // Tied embeddings: dense[tok[t]] += gc[t] for first-occurrence rows (bf16 read-modify-write).
 int opk_embedding_add_rows(const int32_t* tok, const int32_t* rep, const float* gc, void* dense, int T, int D,
                            void* stream);
-// out_bf16 = bf16(in_fp32)
-int opk_cast_f32_bf16(const float* in, void* out, int64_t n, void* stream);
 
 // ---- causal GQA flash attention on the fused projection buffer (csrc/kernels/attention_sm100.cu) -------------
 // qkv bf16 [T][(H+2KV)*hd] (row pitch ld), out bf16 [T][H*hd] (row pitch ldo), lse fp32 [H][T]. hd in {64, 128}.
@@ -164,7 +159,7 @@ int opk_attn_bwd(const void* qkv, const void* out, const void* dout, const float
                  void* stream);
 
 // ---- multi-tensor kernels of the functional API (csrc/kernels/multi_tensor.cu) ---------------------------------
-// `leaves`: HOST array of n_leaves records of opk_mt_leaf_bytes() = 72 bytes: six buffer addresses, elements (int64; per
+// `leaves`: HOST array of n_leaves records of opk_mt_leaf_bytes() bytes (72, checked by the caller): six buffer addresses, elements (int64; per
 // example where there are examples), an int64 and a float parameter, and a mask of the buffers that hold bf16 (else fp32).
 int opk_mt_leaf_bytes(void);
 int opk_mt_sumsq_tile(void);   // elements of one example per entry of `partial`

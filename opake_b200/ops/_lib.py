@@ -12,6 +12,7 @@ from functools import lru_cache
 import torch
 
 import os
+import struct
 
 from .._build import KERNEL_LIB, KERNEL_LIB_DEBUG, build_kernels
 
@@ -64,7 +65,7 @@ def lib() -> ctypes.CDLL:
 
 def _declare_optional(L: ctypes.CDLL) -> None:
     """Attach prototypes for the non-GEMM kernels (declared in csrc/kernels/opk_api.h)."""
-    from ._protos import PROTOTYPES
+    from ._protos import MT_LEAF, PROTOTYPES
 
     for name, (restype, argtypes) in PROTOTYPES.items():
         fn = getattr(L, name, None)
@@ -72,6 +73,8 @@ def _declare_optional(L: ctypes.CDLL) -> None:
             raise KernelLibraryError(f"symbol {name} missing from {KERNEL_LIB}; rebuild with opake_b200._build")
         fn.restype = restype
         fn.argtypes = argtypes
+    if L.opk_mt_leaf_bytes() != struct.calcsize(MT_LEAF):
+        raise KernelLibraryError(f"{KERNEL_LIB} packs the leaves of the multi-tensor kernels differently; rebuild with opake_b200._build")
 
 
 LAUNCHES = [0]  # number of native kernel entry-point calls issued by this process

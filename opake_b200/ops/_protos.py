@@ -3,6 +3,9 @@ from ctypes import POINTER, Structure, c_char_p, c_double, c_float, c_int32, c_i
 
 P, I, L, F = c_void_p, c_int32, c_int64, c_float
 
+# one leaf of the multi-tensor kernels: six buffers, elements, int64 and float parameter, bf16 mask
+MT_LEAF = "<6Qqqfi"
+
 
 class DpStepArgs(Structure):
     _fields_ = [
@@ -54,8 +57,7 @@ PROTOTYPES: dict = {
     "opk_rmsnorm_bwd": (I, [P, P, P, P, P, P, P, P, I, I, I, F, P]),
     "opk_layernorm_fwd": (I, [P, P, P, P, P, P, I, I, F, P]),
     "opk_layernorm_bwd": (I, [P, P, P, P, P, P, P, P, P, I, I, P]),
-    "opk_rope": (I, [P, P, P, I, I, I, L, F, P]),
-    "opk_rope_batch": (I, [P, P, P, I, L, I, I, L, F, P]),
+    "opk_rope": (I, [P, P, P, I, L, I, I, L, F, P]),
     "opk_swiglu_fwd": (I, [P, P, I, I, P]),
     "opk_swiglu_bwd": (I, [P, P, P, I, I, P]),
     "opk_geglu_fwd": (I, [P, P, I, I, I, P]),
@@ -91,11 +93,9 @@ PROTOTYPES: dict = {
     "opk_mt_adam": (I, [c_char_p, I, F, F, F, F, c_double, c_double, F, I, P]),
     "opk_mt_finish_update": (I, [c_char_p, I, F, F, P]),
     "opk_mt_add_update": (I, [c_char_p, I, P]),
-    "opk_scatter_rows_cast_sumsq": (I, [P, P, P, I, I, P, P]),
-    "opk_scatter_rows_cast_sumsq_ragged": (I, [P, P, P, P, I, I, P, P]),
+    "opk_scatter_rows_cast_sumsq": (I, [P, P, P, P, I, I, P, P]),
     "opk_colsum": (I, [P, P, I, I, L, P]),
     "opk_embedding_add_rows": (I, [P, P, P, P, I, I, P]),
-    "opk_cast_f32_bf16": (I, [P, P, L, P]),
     "opk_clip_scale": (I, [P, F, I, F, I, L, P, P, P, I, P]),
     "opk_clip_accumulate": (I, [P, P, P, L, P]),
     "opk_clip_accumulate2": (I, [P, P, P, L, I, P]),

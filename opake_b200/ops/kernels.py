@@ -119,7 +119,7 @@ def rope_table(seq_len: int, head_dim: int, theta: float = 10000.0, device=None,
 def rope_(qk, table, n_heads: int, head_dim: int, pos=None, backward: bool = False, period: int = 0):
     """Rotate the first ``n_heads`` heads of every row of ``qk`` in place (rotate-half convention). Row ``t`` sits at
     position ``pos[t]``, else ``t % period`` (``period`` rows per sequence), else ``t``."""
-    _chk(_L().opk_rope_batch(_p(qk), _p(table), _p(pos), period, qk.shape[0], n_heads, head_dim, qk.stride(0),
+    _chk(_L().opk_rope(_p(qk), _p(table), _p(pos), period, qk.shape[0], n_heads, head_dim, qk.stride(0),
                              -1.0 if backward else 1.0, _s(qk)), "rope")
     return qk
 
@@ -264,7 +264,7 @@ def scatter_rows_cast_sumsq(src, dst_base, offsets, sumsq, widths=None):
     """fp32 rows ``src[r]`` (their first ``widths[r]`` columns, int32, when given) -> bf16 at ``dst_base + offsets[r]``;
     ``sumsq += sum(stored**2)``."""
     R, D = src.shape
-    _chk(_L().opk_scatter_rows_cast_sumsq_ragged(_p(src), _p(dst_base), _p(offsets), _p(widths), R, D, _p(sumsq), _s(src)),
+    _chk(_L().opk_scatter_rows_cast_sumsq(_p(src), _p(dst_base), _p(offsets), _p(widths), R, D, _p(sumsq), _s(src)),
          "scatter_rows_cast_sumsq")
 
 
@@ -276,10 +276,6 @@ def colsum_(dy, out):
 def embedding_add_rows(tok, ws, dense, T: int):
     _chk(_L().opk_embedding_add_rows(_p(tok), _p(ws.rep), _p(ws.gc), _p(dense), T, dense.shape[1], _s(dense)),
          "embedding_add_rows")
-
-
-def cast_f32_bf16(src, dst):
-    _chk(_L().opk_cast_f32_bf16(_p(src), _p(dst), src.numel(), _s(src)), "cast_f32_bf16")
 
 
 def clip_scale(sumsq, clip: float, *, scale_out, norm_out=None, counters=None, auto: bool = False, gamma: float = 0.01,

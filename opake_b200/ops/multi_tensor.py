@@ -7,14 +7,15 @@ nothing is cached between calls.
 """
 from __future__ import annotations
 
+import functools
 import struct
 from ctypes import c_float
 
 import torch
 
-from . import _lib
+from . import _lib, _protos
 
-_LEAF = struct.Struct("<6Qqqfi")        # six buffers, elements, aux, scalar, bf16 mask
+_LEAF = struct.Struct(_protos.MT_LEAF)
 _DTYPES = (torch.float32, torch.bfloat16)
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
 
@@ -68,8 +69,11 @@ def _call(name: str, device, *args) -> None:
         _lib.check(getattr(_lib.lib(), name)(*args, _lib.stream_ptr(device)), name)
 
 
-def _tiles(leaves, tile: int) -> int:
-    return sum((l[0].numel() + tile - 1) // tile for l in leaves)
+@functools.cache
+def _clip_tiles() -> tuple[int, int]:
+    """Elements per entry of the kernels' partial sums before and after clipping: constants of the library."""
+    lib = _lib.lib()
+    return lib.opk_mt_sumsq_tile(), lib.opk_mt_apply_tile()
 
 
 def clip_and_sum(leaves, clip: float, guards, outs, *, prev=None, scale: float = 1.0, with_postsq: bool = False):
@@ -79,9 +83,8 @@ def clip_and_sum(leaves, clip: float, guards, outs, *, prev=None, scale: float =
     dev, B = leaves[0].device, leaves[0].shape[0]
     n = [l[0].numel() for l in leaves]
     blob = _pack([((l, o, None if prev is None else prev[i]), n[i], 0, 0.0) for i, (l, o) in enumerate(zip(leaves, outs))])
-    L = _lib.lib()
-    n_sq = sum((k + L.opk_mt_sumsq_tile() - 1) // L.opk_mt_sumsq_tile() for k in n)
-    n_ap = sum((k + L.opk_mt_apply_tile() - 1) // L.opk_mt_apply_tile() for k in n)
+    t_sq, t_ap = _clip_tiles()
+    n_sq, n_ap = sum((k + t_sq - 1) // t_sq for k in n), sum((k + t_ap - 1) // t_ap for k in n)
     partial = torch.empty(B, max(n_sq, 1), dtype=torch.float64, device=dev)
     factors = torch.empty(2, B, dtype=torch.float32, device=dev)
     norms = torch.empty(B, dtype=torch.float64, device=dev)
