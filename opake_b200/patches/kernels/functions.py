@@ -226,7 +226,8 @@ class _GluBwd(torch.autograd.Function):
 
 
 class _Glu(torch.autograd.Function):
-    """Element-wise on two buffers: gate and up are read where the projections left them (no interleaved copy)."""
+    """Element-wise on two buffers: gate and up are read where the projections left them (no interleaved copy), and saved as they
+    are: editing one of them in place before the backward pass raises, as it does with the plain formula."""
 
     @staticmethod
     def forward(gate, up, kind):
