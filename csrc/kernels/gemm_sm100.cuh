@@ -73,10 +73,12 @@ struct GemmParams {
 // quadrant, each taking half of the tile's columns) for the SwiGLU-backward epilogue, which reads and writes four
 // times the bytes of a plain store per accumulator column, and for the cross-entropy epilogues that are a long chain of
 // dependent instructions per column (one warp per scheduler leaves it idle most of the time): the backward one, and the
-// forward one with a soft cap's hyperbolic tangents. (With eight warps the store-only kernels measured 3-5 % slower; the
+// forward one with a soft cap's hyperbolic tangents. The forward SwiGLU epilogue (an exponential and a division per pair)
+// takes eight too: with four it set the pace up to K = 4096 (2048 x 16384 x 2048 116 us, 97 with eight; 2048 x 28672 x 4096
+// 324 and 319). (With eight warps the store-only kernels measured 3-5 % slower; the
 // plain forward cross-entropy hides under its main loop with four.)
 __host__ __device__ constexpr int gemm_epi_warps(int epi) {
-  return epi == EPI_SWIGLU_BWD || epi == EPI_LCE_FWD2 || epi == EPI_LCE_BWD ? 8 : 4;
+  return epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD || epi == EPI_LCE_FWD2 || epi == EPI_LCE_BWD ? 8 : 4;
 }
 // The single-CTA kernel serves the grouped (mixture-of-experts) modes, whose per-expert reductions are only a few
 // k-blocks long while every tile is still written in full: there the epilogue, not the main loop, sets the pace.
@@ -213,7 +215,7 @@ __device__ __forceinline__ EpiState epi_begin(const GemmParams& p, uint8_t* scr,
 template <int EPI>
 __device__ __forceinline__ void epi_chunk(const GemmParams& p, EpiState& e, float (&v)[32], int col0) {
   const int ncols = min(32, p.N - col0);
-  if (ncols <= 0) return;
+  if (ncols <= 0 || e.rows_left <= 0) return;      // the same in all lanes
   const bool full = ncols == 32 && e.vec_ok;
   __nv_bfloat16* Crow = e.C + (long long)(threadIdx.x & 31) * p.ldc + col0;
   if (EPI == EPI_STORE && p.stepwise) {
@@ -282,11 +284,18 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, EpiState& e, floa
     }
     if (EPI == EPI_SWIGLU) {
       float a[16];
+      // Not for rows past M: their accumulators are zero, and a division of zero leaves the fast path of the whole warp (with
+      // four epilogue warps 1021 x 16384 x 2048 took 101 us so and 72 without them, 317 x 16384 x 2048 72 and 42).
+      if (e.row_ok) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        // match the stored (bf16-rounded) pre-activations so backward recomputes the same values
-        const float g = bf16_round(v[2 * j]), u = bf16_round(v[2 * j + 1]);
-        a[j] = g / (1.f + __expf(-g)) * u;
+        for (int j = 0; j < 16; ++j) {
+          // match the stored (bf16-rounded) pre-activations so backward recomputes the same values
+          const float g = bf16_round(v[2 * j]), u = bf16_round(v[2 * j + 1]);
+          a[j] = g / (1.f + __expf(-g)) * u;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) a[j] = 0.f;
       }
       const int lane = threadIdx.x & 31;
       __nv_bfloat16* act0 = reinterpret_cast<__nv_bfloat16*>(p.act) + (long long)(e.row - lane) * p.ld_act + (col0 >> 1);

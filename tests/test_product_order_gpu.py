@@ -5,7 +5,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-ROWS = (40, 128, 129, 317, 640)       # few rows: narrow tiles; 1024 rows (the comparison): wider tiles, pairs of SMs
+ROWS = (1, 31, 40, 128, 129, 317, 640)       # few rows: narrow tiles; 1024 rows (the comparison): wider tiles, pairs of SMs
 
 
 def _rand(shape, dev, scale=1.0):
