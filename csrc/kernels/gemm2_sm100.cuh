@@ -74,6 +74,8 @@ struct Gemm2Cfg {
 };
 
 constexpr int kStageWarps = 8;     // copier warps per CTA of the staged variant
+// The staged variant keeps four epilogue warps: with eight next to its copier warps a thread would have 112 registers.
+__host__ __device__ constexpr int gemm2_epi_warps(int epi, bool stage) { return stage ? 4 : gemm_epi_warps(epi); }
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;
@@ -82,7 +84,7 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
 }
 
 template <bool A_MN, bool B_MN, int EPI, bool STAGE = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * gemm_epi_warps(EPI) + (STAGE ? 32 * kStageWarps : 0), 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * gemm2_epi_warps(EPI, STAGE) + (STAGE ? 32 * kStageWarps : 0), 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   using Cfg = Gemm2Cfg;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES;
@@ -107,7 +109,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 2 * gemm_epi_warps(EPI));    // the epilogue warps of both CTAs
+      mbar_init(&tempty[b], 2 * gemm2_epi_warps(EPI, STAGE));    // the epilogue warps of both CTAs
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -214,9 +216,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
     __syncwarp();
-  } else if (STAGE && warp >= 2 + gemm_epi_warps(EPI)) {
+  } else if (STAGE && warp >= 2 + gemm2_epi_warps(EPI, STAGE)) {
     // ------------------------------------------------------------ copiers: remote B -> local scratch, band by band
-    const int ctid = (warp - 2 - gemm_epi_warps(EPI)) * 32 + lane;
+    const int ctid = (warp - 2 - gemm2_epi_warps(EPI, STAGE)) * 32 + lane;
     const long long nthreads = (long long)gridDim.x * (32 * kStageWarps);
     const long long gtid = (long long)blockIdx.x * (32 * kStageWarps) + ctid;
     // K-major B ([N][K], a band = 2048 whole rows) or MN-major B ([K][N], a band = 2048 columns of every row)
@@ -260,7 +262,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs, own 128 rows each)
     const int quad = warp & 3;
-    constexpr int CSPLIT = gemm_epi_warps(EPI) / 4;
+    constexpr int CSPLIT = gemm2_epi_warps(EPI, STAGE) / 4;
     const int c_begin = ((warp - 2) >> 2) * (BN / CSPLIT), c_end = c_begin + BN / CSPLIT;
     uint8_t* scratch = smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * kEpiScratch;
     int it = 0;
@@ -299,7 +301,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tc_fence_after();
     tmem_dealloc2(tmem_base, Cfg::TMEM_COLS);
   }
-  if (EPI == EPI_SUMSQ && threadIdx.x == 0) epi_flush_sq(p, sq_slots, gemm_epi_warps(EPI));
+  if (EPI == EPI_SUMSQ && threadIdx.x == 0) epi_flush_sq(p, sq_slots, gemm2_epi_warps(EPI, STAGE));
   if (threadIdx.x == 0 && *abort_flag && p.err) atomicExch(p.err, 1);
 }
 

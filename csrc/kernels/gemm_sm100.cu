@@ -106,7 +106,7 @@ int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams&
   int grid = (max_ctas > 0 ? max_ctas : num_sms()) & ~1;   // whole CTA pairs
   if (grid < 2) grid = 2;
   if (grid > 2 * tiles) grid = 2 * tiles;
-  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::gemm_epi_warps(EPI) + (STAGE ? 32 * opk::kStageWarps : 0), Cfg::SMEM_BYTES, st, ta, tb, p);
+  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::gemm2_epi_warps(EPI, STAGE) + (STAGE ? 32 * opk::kStageWarps : 0), Cfg::SMEM_BYTES, st, ta, tb, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
   return 0;
