@@ -62,16 +62,11 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   pdl_trigger();       // after this CTA's TMEM is allocated: a successor that allocates next can only wait for a running grid
   pdl_wait();
 
-  // grid = (column tiles, row tiles x batch): no divisions before the first load (the persistent kernels' tile
-  // arithmetic, cold in the instruction cache, costs 1,400 cycles there)
+  // grid = (row tiles, column tiles, batch): no divisions before the first load (the persistent kernels' tile arithmetic, cold
+  // in the instruction cache, costs 1,400 cycles there), and the row tiles of a column follow each other, so that a weight
+  // matrix larger than the L2 is read once (the other order read it per row tile: 317 x 28672 x 4096 129 us)
   const int kblocks = (p.K + BK - 1) / BK;
-  const int tn = blockIdx.x;
-  int tm = blockIdx.y, b = 0;
-  if (p.batch > 1) {
-    const int tiles_m = (p.M + BM - 1) / BM;
-    b = tm / tiles_m;
-    tm -= b * tiles_m;
-  }
+  const int tm = blockIdx.x, tn = blockIdx.y, b = blockIdx.z;
   if (warp == 0) {
     int s = 0;
     uint32_t ph = 0;

@@ -122,8 +122,8 @@ int launch_narrow(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmP
     if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
     attr_done = true;
   }
-  const dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)(((p.M + 127) / 128) * p.batch));
-  const int stages = (long long)grid.x * grid.y > num_sms() ? Cfg::FEW : Cfg::MANY;
+  const dim3 grid((unsigned)((p.M + 127) / 128), (unsigned)((p.N + BN - 1) / BN), (unsigned)p.batch);
+  const int stages = (long long)grid.x * grid.y * grid.z > num_sms() ? Cfg::FEW : Cfg::MANY;
   cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::kNarrowEpiWarps, Cfg::smem_bytes(stages), st, ta, tb, p, stages);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
