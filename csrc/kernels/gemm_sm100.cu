@@ -154,7 +154,9 @@ int choose_narrow(const OpkGemmArgs* a, int bn, bool pair) {
   int best = 0;
   for (int w = 64; w <= 256; w *= 2) {
     const long long per = ceil_div(ceil_div(a->M, 128) * ceil_div(a->N, w) * a->batch, sms);
-    if (per > 4) continue;
+    // Fewer than 32 rows: many CTAs that ask for the same few lines of A at once wait for them. 8 x 6144 x 4096 took 28.4 us on
+    // 96 tiles, 18.5 on 48, 22.6 on the persistent kernel; 8 x 8192 x 2048 16.5 on 128, 13.7 persistent (32 rows: 9.5).
+    if (per > 4 || (a->M < 32 && ceil_div(a->N, w) > 48)) continue;
     const long long fixed = w == 256 ? 5200 : w == 128 ? 4200 : 3500, slope = w == 256 ? 315 : w == 128 ? 235 : 225;
     const long long round = w == 256 ? 4500 : w == 128 ? 1500 : 800;          // epilogue of every further round
     const long long c = fixed + per * kb * slope + (per - 1) * round;
