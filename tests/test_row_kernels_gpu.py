@@ -177,3 +177,22 @@ def test_cross_entropy_label_buffer_may_be_refilled(cuda):
     assert torch.equal(got, want)
     f = torch.func.vmap(torch.func.grad(lambda z, l: opake_cross_entropy(z, l).sum()))
     assert torch.equal(f(logits.detach().view(3, 3, 128), torch.arange(9, dtype=torch.int32, device=cuda).view(3, 3)).view(9, 128), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("V", [512, 513, 2047, 2056, 4104, 8190, 12345])
+def test_cross_entropy_row_forms(cuda, dtype, V):
+    """Around the widths where rows change from single elements to vectors, and from one round of loads to several."""
+    from opake_b200.patches.kernels import opake_cross_entropy
+
+    logits = (torch.randn(5, V, device=cuda) * 3).to(dtype).requires_grad_()
+    labels = torch.randint(0, V, (5,), device=cuda)
+    c = torch.rand(5, device=cuda)
+    nll = opake_cross_entropy(logits, labels)
+    (g,) = torch.autograd.grad(nll, logits, c)
+    ld = logits.detach().double().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(ld, labels, reduction="none")
+    (want,) = torch.autograd.grad(ref, ld, c.double())
+    assert bool(((nll.double() - ref).abs() <= ref.abs() * 1e-5 + 2e-5).all())
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-5
+    assert bool(((g.double() - want).abs() <= want.abs() * eps + 2e-6).all())
