@@ -196,3 +196,22 @@ def test_cross_entropy_row_forms(cuda, dtype, V):
     assert bool(((nll.double() - ref).abs() <= ref.abs() * 1e-5 + 2e-5).all())
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-5
     assert bool(((g.double() - want).abs() <= want.abs() * eps + 2e-6).all())
+
+
+@pytest.mark.parametrize("kind", ["silu", "gelu", "gelu_tanh"])
+@pytest.mark.parametrize("n,offset", [(1, 0), (1000, 0), (1000, 1), (131072, 0), (131080, 0), (131073, 0), (200_000, 1), (12_582_920, 0)])
+def test_interleaved_activation_forms(cuda, kind, n, offset):
+    """One element per thread or eight, buffers on 16-byte and on 2-byte boundaries."""
+    from opake_b200.ops import kernels as K
+
+    gu = _rand((2 * n + offset,), cuda, 2.0)[offset:].view(1, 2 * n)
+    d = _rand((n + offset,), cuda)[offset:].view(1, n)
+    if kind == "silu":
+        act, dgu = K.swiglu_fwd(gu), K.swiglu_bwd(d, gu)
+    else:
+        act, dgu = K.geglu_fwd(gu, kind == "gelu_tanh"), K.geglu_bwd(d, gu, kind == "gelu_tanh")
+    g, u, dd = gu[0, 0::2].double().requires_grad_(), gu[0, 1::2].double().requires_grad_(), d[0].double()
+    f = torch.nn.functional.silu(g) if kind == "silu" else torch.nn.functional.gelu(g, approximate="tanh" if kind == "gelu_tanh" else "none")
+    dg, du = torch.autograd.grad(f * u, (g, u), dd)
+    for a, b in ((act[0], (f * u).detach()), (dgu[0, 0::2], dg), (dgu[0, 1::2], du)):
+        assert bool(((a.double() - b).abs() <= b.abs() * 2.0 ** -7 + 1e-4).all())
