@@ -581,12 +581,16 @@ extern "C" int opk_clip_accumulate(const void* g, const float* scale, float* acc
 }
 
 // One round of resident CTAs walks the shard: every CTA gets the same share. (A fixed 8 CTAs per SM ran as 2.7 rounds of the
-// variants that fit three at a time: 8.1 ms at 1.49e9 parameters.)
-template <class Kernel>
-void launch_dp_step(Kernel kernel, long long nq, cudaStream_t st, const OpkDpStepArgs& args, const PeerTable& pt, const StepGroup& grp) {
-  int per_sm = 0, dev = 0, sms = 148;
+// variants that fit three at a time: 8.1 ms at 1.49e9 parameters.) Eight per SM where that is the faster grid (2^26 elements, one
+// round -> eight per SM): SGD 150 -> 142 us, with two gradient buffers 208 -> 199; AdamW with master weights, without buffers and
+// correlation, on large shards 351 -> 337 us (2^20 elements: 5.6 -> 6.6; with buffers 381 -> 397; correlated noise 627 -> 660).
+template <bool ADAM, bool MASTER, int CORR, int NG>
+void launch_dp_step(long long nq, cudaStream_t st, const OpkDpStepArgs& args, const PeerTable& pt, const StepGroup& grp) {
+  auto kernel = dp_step_kernel<ADAM, MASTER, CORR, NG>;
+  int per_sm = 8, dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess || per_sm < 1) per_sm = 2;
+  const bool eight = !ADAM || (MASTER && CORR == CORR_NONE && NG == 0 && nq > (1ll << 21));
+  if (!eight && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess || per_sm < 1)) per_sm = 2;
   kernel<<<grid_for((nq + 1) / 2, 256, sms * per_sm), 256, 0, st>>>(args, pt, grp);
 }
 
@@ -635,9 +639,9 @@ extern "C" int opk_dp_step(const OpkDpStepArgs* args, void* stream) {
   // a group and zeroing take 1,880 us together for two buffers, 1,907 for three, 2,356 for eight.
 #define OPK_DP_STEP_LAUNCH(A, M, C)                                                  \
   do {                                                                               \
-    if (!group) launch_dp_step(dp_step_kernel<A, M, C, 0>, nq, st, *args, pt, grp);   \
-    else if (grp.n <= 2) launch_dp_step(dp_step_kernel<A, M, C, 2>, nq, st, *args, pt, grp); \
-    else launch_dp_step(dp_step_kernel<A, M, C, OPK_ACC_GROUP_MAX>, nq, st, *args, pt, grp); \
+    if (!group) launch_dp_step<A, M, C, 0>(nq, st, *args, pt, grp);   \
+    else if (grp.n <= 2) launch_dp_step<A, M, C, 2>(nq, st, *args, pt, grp); \
+    else launch_dp_step<A, M, C, OPK_ACC_GROUP_MAX>(nq, st, *args, pt, grp); \
   } while (0)
 #define OPK_DP_STEP_CORR(A, M)                                      \
   do {                                                              \
