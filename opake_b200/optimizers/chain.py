@@ -79,13 +79,15 @@ def apply_updates(params: Any, updates: Any, *, inplace: bool = False) -> Any:
 
 def _fused(*trees):
     """``(multi_tensor, treedef, leaf lists)`` when all trees have one structure of plain fp32 / bf16 CUDA tensors."""
-    flat = [tree_flatten(t) for t in trees]
-    leaves, td = flat[0]
-    if not leaves or not all(isinstance(t, torch.Tensor) and t.is_cuda for t in leaves) or any(f[1] != td for f in flat[1:]):
+    leaves, td = tree_flatten(trees[0])
+    if not leaves or not all(isinstance(t, torch.Tensor) and t.is_cuda for t in leaves):
+        return None
+    flat = [tree_flatten(t) for t in trees[1:]]
+    if any(f[1] != td for f in flat):
         return None
     from ..ops import multi_tensor as MT
 
-    lists = [f[0] for f in flat]
+    lists = [leaves, *(f[0] for f in flat)]
     return (MT, td, lists) if MT.usable(*lists) else None
 
 
