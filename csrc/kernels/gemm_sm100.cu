@@ -264,7 +264,7 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   if (a->softcap > 0.f) {
     const double inv = 1.0 / (double)a->softcap;
     p.inv_cap = (float)inv;
-    p.inv_cap_lo = (float)(inv - (double)p.inv_cap);
+    p.inv_cap_lo = p.inv_cap <= 3.4028234e38f ? (float)(inv - (double)p.inv_cap) : 0.f;      // 1 / cap beyond fp32: no low part
   }
   p.err = a->err;
   p.tile_group = a->tile_group; p.group_k = a->group_k; p.sumsq_stride = a->sumsq_shared ? 0 : 1;

@@ -148,9 +148,9 @@ __device__ __forceinline__ void load_pieces(uint8_t* scr, const __nv_bfloat16* b
 
 // v / cap with the reciprocal carried in two floats (48 bits): one rounding, as in a division. A division costs the epilogue of
 // the soft-capped cross-entropy 0.27 ms of 2.73 (4 x 1024 x 2048 x 50257, both directions), the product with a reciprocal of 24
-// bits has a second rounding. Values whose tanh is 1 anyway are handed on: infinity times the low part would be NaN.
+// bits has a second rounding. Infinities are handed on (their tanh is 1): infinity times the low part would be NaN.
 __device__ __forceinline__ float cap_quotient(const GemmParams& p, float v) {
-  return fabsf(v) < 1e30f ? __fmaf_rn(v, p.inv_cap, __fmul_rn(v, p.inv_cap_lo)) : v;
+  return fabsf(v) < INFINITY ? __fmaf_rn(v, p.inv_cap, __fmul_rn(v, p.inv_cap_lo)) : v;
 }
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
 

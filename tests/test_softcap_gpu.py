@@ -5,7 +5,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cap", [30.0, 50.0, 7.3])
+@pytest.mark.parametrize("cap", [30.0, 50.0, 7.3, 1e35, 1e-6])
 @pytest.mark.parametrize("parts", [1, 2])
 def test_cap_is_divided_by(cuda, cap, parts):
     """One column and a one-hot reduction: the epilogue's running maximum is cap * tanh(z / cap) of a known z, bit for bit (the
