@@ -248,7 +248,7 @@ def cross_entropy_fwd(logits, labels, scale: float = 1.0, softcap: float = 0.0):
 
 def cross_entropy_bwd(logits, labels, lse, coef, scale: float = 1.0, softcap: float = 0.0):
     T, V = logits.shape
-    d = torch.empty_like(logits)
+    d = torch.empty_strided(logits.shape, logits.stride(), dtype=logits.dtype, device=logits.device)    # the kernel uses one row pitch
     _chk(_L().opk_cross_entropy_bwd(_p(logits), int(logits.dtype == torch.float32), _p(labels), _p(lse), _p(coef), _p(d),
                                     T, V, logits.stride(0), scale, softcap, _s(logits)), "cross_entropy_bwd")
     return d

@@ -215,3 +215,18 @@ def test_interleaved_activation_forms(cuda, kind, n, offset):
     dg, du = torch.autograd.grad(f * u, (g, u), dd)
     for a, b in ((act[0], (f * u).detach()), (dgu[0, 0::2], dg), (dgu[0, 1::2], du)):
         assert bool(((a.double() - b).abs() <= b.abs() * 2.0 ** -7 + 1e-4).all())
+
+
+def test_cross_entropy_of_padded_rows(cuda):
+    from opake_b200.ops import kernels as K
+
+    wide = torch.randn(9, 520, device=cuda)
+    lab, c = torch.arange(9, dtype=torch.int32, device=cuda), torch.rand(9, device=cuda)
+    for V in (515, 37):
+        z = wide[:, :V]
+        nll, lse = K.cross_entropy_fwd(z, lab)
+        d = K.cross_entropy_bwd(z, lab, lse, c)
+        zc = z.contiguous()
+        nll2, lse2 = K.cross_entropy_fwd(zc, lab)
+        d2 = K.cross_entropy_bwd(zc, lab, lse2, c)
+        assert torch.allclose(nll, nll2, rtol=1e-6, atol=1e-6) and torch.allclose(d, d2, rtol=1e-5, atol=1e-7)
