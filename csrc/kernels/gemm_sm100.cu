@@ -1,5 +1,6 @@
 // Host side of the tcgen05 GEMM: builds the TMA tensor maps and launches the persistent kernel.
 #include "gemm_narrow_sm100.cuh"
+#include "lce_grad.cuh"
 #include "opk_api.h"
 #include "debug_bounds.cuh"
 
@@ -261,6 +262,7 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   p.ldc = a->ldc; p.strideC = a->strideC; p.C = a->C; p.R = a->R; p.bias = a->bias;
   p.alpha = a->alpha; p.stepwise = a->stepwise; p.sumsq = a->sumsq; p.act = a->act; p.ld_act = a->ld_act; p.labels = a->labels;
   p.pmax = a->pmax; p.psum = a->psum; p.tgt = a->tgt; p.lse = a->lse; p.coef = a->coef; p.softcap = a->softcap;
+  p.z = a->z;
   if (a->softcap > 0.f) {
     const double inv = 1.0 / (double)a->softcap;
     p.inv_cap = (float)inv;
@@ -367,6 +369,28 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   }
   set_err("opk_gemm: unsupported (layout, epilogue) combination");
   return -3;
+}
+
+extern "C" int64_t opk_lce_logits_floats(int M, int N) {
+  return M > 0 && N > 0 ? (int64_t)((M + 31) / 32) * ((N + 31) / 32) * 1024 : 0;
+}
+
+extern "C" int opk_lce_grad(const float* z, const int32_t* labels, const float* lse, const float* coef, void* out, int64_t ld, int M,
+                            int N, float softcap, void* stream) {
+  if (M <= 0 || N <= 0 || ld < N || !z || !labels || !lse || !coef || !out || (reinterpret_cast<uintptr_t>(z) & 15)) {
+    set_err("opk_lce_grad: bad arguments");
+    return -1;
+  }
+  opk::GemmParams p;
+  memset(&p, 0, sizeof(p));
+  p.M = M; p.N = N; p.batch = 1; p.alpha = 1.f; p.C = out; p.ldc = ld;
+  p.z = const_cast<float*>(z); p.labels = labels; p.lse = lse; p.coef = coef; p.softcap = softcap;
+  const long long groups = ((N + 31) / 32 + opk::kLceGradChunks - 1) / opk::kLceGradChunks;
+  const long long items = groups * ((M + 31) / 32);
+  opk::lce_grad_kernel<<<(unsigned)((items + 7) / 8), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
+  return 0;
 }
 
 // ------------------------------------------------------------------------------------------------ wait self-test

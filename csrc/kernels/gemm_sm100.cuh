@@ -27,6 +27,7 @@ enum GemmEpilogue : int {
   EPI_LCE_BWD = 4,  // C = (exp(z - lse[m]) - [n == label[m]]) * coef[m]
   EPI_SWIGLU_BWD = 5,  // acc = d(act); act = saved (gate, up) pairs [M][2N]; C[m][2n], C[m][2n+1] = d(gate), d(up)
   EPI_LCE_FWD2 = 6,    // EPI_LCE_FWD with two column parts per tile (twice the epilogue warps), chosen by lce_parts == 2
+  EPI_LCE_GRAD = 7,    // EPI_LCE_BWD on logits that the forward pass stored (lce_grad_kernel): no product
 };
 
 struct GemmParams {
@@ -46,6 +47,7 @@ struct GemmParams {
   float* pmax;           // EPI_LCE_FWD: [M][parts * tiles_n], parts = 1 (EPI_LCE_FWD) or 2 (EPI_LCE_FWD2)
   float* psum;           // EPI_LCE_FWD: [M][parts * tiles_n], parts = 1 (EPI_LCE_FWD) or 2 (EPI_LCE_FWD2)
   float* tgt;            // EPI_LCE_FWD: [M] target logit (written by the tile that owns the label)
+  float* z;              // EPI_LCE_FWD, optional: fp32 logits for the backward pass in blocks of 32 x 32 (see z_block)
   const float* lse;      // EPI_LCE_BWD: [M]
   const float* coef;     // EPI_LCE_BWD: [M] per-row scale (mask / divisor * upstream grad)
   float softcap;         // EPI_LCE_*: 0 = off, else z = cap * tanh(z / cap)
@@ -152,6 +154,12 @@ __device__ __forceinline__ void load_pieces(uint8_t* scr, const __nv_bfloat16* b
 __device__ __forceinline__ float cap_quotient(const GemmParams& p, float v) {
   return fabsf(v) < INFINITY ? __fmaf_rn(v, p.inv_cap, __fmul_rn(v, p.inv_cap_lo)) : v;
 }
+// Stored logits: [ceil(M / 32)][ceil(N / 32)] blocks of 1,024 floats, element (r, c) of a block at (c / 4) * 128 + r * 4 + c % 4.
+// A thread that owns row r of the block moves 16 bytes at a time and the 32 threads of a warp 512 contiguous ones, in the
+// epilogue that writes the block as in the kernel that reads it, without a pass through shared memory.
+__device__ __forceinline__ float4* z_block(float* z, int N, int row0, int col0) {
+  return reinterpret_cast<float4*>(z) + ((long long)(row0 >> 5) * ((N + 31) >> 5) + (col0 >> 5)) * 256 + (threadIdx.x & 31);
+}
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
 
 // L2 prefetch of the 2 * BN saved pre-activation values (gate / up pairs) that the SwiGLU-backward epilogue of this
@@ -204,9 +212,9 @@ __device__ __forceinline__ EpiState epi_begin(const GemmParams& p, uint8_t* scr,
   e.run_sum = 0.f;
   e.label = -1;
   e.lse = e.coef = 0.f;
-  if (EPI == EPI_LCE_FWD || EPI == EPI_LCE_FWD2 || EPI == EPI_LCE_BWD) {
+  if (EPI == EPI_LCE_FWD || EPI == EPI_LCE_FWD2 || EPI == EPI_LCE_BWD || EPI == EPI_LCE_GRAD) {
     if (e.row_ok) e.label = p.labels[e.row];
-    if (EPI == EPI_LCE_BWD && e.row_ok) { e.lse = p.lse[e.row]; e.coef = p.coef[e.row]; }
+    if ((EPI == EPI_LCE_BWD || EPI == EPI_LCE_GRAD) && e.row_ok) { e.lse = p.lse[e.row]; e.coef = p.coef[e.row]; }
   }
   return e;
 }
@@ -218,7 +226,9 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, EpiState& e, floa
   if (ncols <= 0 || e.rows_left <= 0) return;      // the same in all lanes
   const bool full = ncols == 32 && e.vec_ok;
   __nv_bfloat16* Crow = e.C + (long long)(threadIdx.x & 31) * p.ldc + col0;
-  if (EPI == EPI_STORE && p.stepwise) {
+  if (EPI == EPI_LCE_GRAD) {
+    // the stored values are scaled already
+  } else if (EPI == EPI_STORE && p.stepwise) {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = bf16_round(__fmul_rn(bf16_round(v[j]), p.alpha));
   } else if (p.alpha != 1.f) {
@@ -360,7 +370,16 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, EpiState& e, floa
   } else if (EPI == EPI_LCE_FWD || EPI == EPI_LCE_FWD2) {
     if (p.softcap > 0.f) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = p.softcap * tanhf(cap_quotient(p, v[j]));
+      for (int j = 0; j < 32; ++j) v[j] = tanhf(cap_quotient(p, v[j]));
+    }
+    if (p.z) {      // the scaled logit, or the hyperbolic tangent of the soft cap: what EPI_LCE_GRAD starts from
+      float4* z = z_block(p.z, p.N, e.row - (int)(threadIdx.x & 31), col0);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) __stcs(z + 32 * q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+    }
+    if (p.softcap > 0.f) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] *= p.softcap;
     }
     float cmax = -INFINITY;
 #pragma unroll
@@ -377,11 +396,11 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, EpiState& e, floa
       for (int j = 0; j < 32; ++j) if (col0 + j == e.label) t = v[j];
       p.tgt[e.row] = t;
     }
-  } else {  // EPI_LCE_BWD
+  } else {  // EPI_LCE_BWD, EPI_LCE_GRAD
     if (p.softcap > 0.f) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        const float th = tanhf(cap_quotient(p, v[j]));
+        const float th = EPI == EPI_LCE_GRAD ? v[j] : tanhf(cap_quotient(p, v[j]));
         const float pr = __expf(p.softcap * th - e.lse);
         v[j] = (pr - ((col0 + j == e.label) ? 1.f : 0.f)) * e.coef * (1.f - th * th);
       }

@@ -45,10 +45,16 @@ typedef struct OpkGemmArgs {
   int32_t* stage_ready;
   int32_t stepwise;      // epilogue 0 without a bias: C = round(round(alpha * round(acc)) + R), as separate bf16 operations give it
   int32_t lce_parts;     // EPI_LCE_FWD: column parts per 256-column tile in pmax / psum (2, else 1)
+  float* z;              // EPI_LCE_FWD, optional: the logits are stored here (opk_lce_logits_floats floats, 16-byte aligned)
 } OpkGemmArgs;
 
 int opk_gemm(const OpkGemmArgs* args, void* stream);
 int opk_gemm_tiles_n(int N, int epilogue);  // number of column tiles the kernel uses (LCE partial buffers; epilogue 6: in two parts each)
+// Logits stored by epilogue 3 (`z`), in a layout of the library's own, and the gradient with respect to them:
+// out[m][n] = (softmax - [n == label[m]]) * coef[m] in bf16 (row pitch ld), the bits of epilogue 4.
+int64_t opk_lce_logits_floats(int M, int N);
+int opk_lce_grad(const float* z, const int32_t* labels, const float* lse, const float* coef, void* out, int64_t ld, int M, int N,
+                 float softcap, void* stream);
 int opk_num_sms(void);
 // Two-CTA (cta_group::2) kernel for eligible products: on by default, OPK_GEMM_PAIR=0 or set_pair_mode(0) turns it off.
 void opk_gemm_set_pair_mode(int on);

@@ -173,6 +173,24 @@ class DecoderRuntime:
         self._ws[T] = ws
         return ws
 
+    def _logits_buffer(self, ws: dict, T: int) -> torch.Tensor | None:
+        """fp32 logits that the loss leaves for its backward pass, which then needs no second product with the head. ``None``,
+        for good, where the product is the cheaper one or they would take more than a quarter of the memory that is free."""
+        if "z" in ws or self.device.type != "cuda":
+            return ws.get("z")
+        if torch.cuda.is_current_stream_capturing():
+            return None
+        dev = self.device
+        free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+        n = G.lce_logits_floats(T, self.cfg.vocab_size)
+        ws["z"] = None
+        if 16 * n <= free and G.lce_keeps_logits(T, self.cfg.vocab_size, self.cfg.d_model):
+            try:
+                ws["z"] = self._alloc(n, dtype=torch.float32, name=f"logits[T={T}]")
+            except torch.cuda.OutOfMemoryError:
+                pass
+        return ws["z"]
+
     def _rope_table(self, T: int):
         cfg = self.cfg
         if self._rope is None or self._rope.shape[0] < T:
@@ -246,8 +264,8 @@ class DecoderRuntime:
         return T >= 256 and n > 128 and n % 8 == 0 and k % 8 == 0 and G.pair_mode()
 
     # ------------------------------------------------------------------ forward
-    def forward(self, tok: torch.Tensor, labels: torch.Tensor | None, ws: dict | None = None):
-        """Runs the decoder on one sequence. Returns ``(per-token nll [T], lse, saved)``.
+    def forward(self, tok: torch.Tensor, labels: torch.Tensor | None, ws: dict | None = None, z: torch.Tensor | None = None):
+        """Runs the decoder on one sequence. Returns ``(per-token nll [T], lse, saved)``; ``z``: buffer for the logits.
 
         ``labels`` are already shifted (``labels[t]`` is the target of position ``t``; negative = ignored).
         """
@@ -322,7 +340,7 @@ class DecoderRuntime:
         head = w["embed"] if cfg.tie_embeddings else w["lm_head"]
         nll = lse = None
         if labels is not None:
-            G.gemm(xf, head, epilogue=G.EPI_LCE_FWD, labels=labels, pmax=ws["pmax"], psum=ws["psum"], tgt=ws["tgt"])
+            G.gemm(xf, head, epilogue=G.EPI_LCE_FWD, labels=labels, pmax=ws["pmax"], psum=ws["psum"], tgt=ws["tgt"], z=z)
             lse, nll = K.lce_finalize(ws["pmax"], ws["psum"], ws["tgt"], labels)
         return nll, lse, (saved, stf)
 
@@ -352,7 +370,8 @@ class DecoderRuntime:
         ws = ws or self.workspace(T)
         emb_ws = ws["embs"][slot]
         H, KV, hd = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim
-        nll, lse, (saved, stf) = self.forward(tok, labels, ws)
+        z = self._logits_buffer(ws, T)
+        nll, lse, (saved, stf) = self.forward(tok, labels, ws, z)
         coef, loss, ntok = ws["coef"], ws["loss"], ws["ntok"]
         K.loss_coef(labels, nll, coef, loss, ntok, weight=loss_weight)
         ws["vec"].zero_()
@@ -360,7 +379,10 @@ class DecoderRuntime:
 
         head = w["embed"] if cfg.tie_embeddings else w["lm_head"]
         ghead = g["embed"] if cfg.tie_embeddings else g["lm_head"]
-        dlog = G.gemm(ws["xf"], head, out=ws["dlogits"], epilogue=G.EPI_LCE_BWD, labels=labels, lse=lse, coef=coef)
+        if z is not None:
+            dlog = G.lce_grad(z, labels, lse, coef, ws["dlogits"])
+        else:
+            dlog = G.gemm(ws["xf"], head, out=ws["dlogits"], epilogue=G.EPI_LCE_BWD, labels=labels, lse=lse, coef=coef)
         if before_wgrad is not None:
             before_wgrad()
         if cfg.tie_embeddings:

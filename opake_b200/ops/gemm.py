@@ -50,6 +50,7 @@ def gemm(
     norm_only: bool = False,
     stage: tuple[torch.Tensor, torch.Tensor] | None = None,
     stepwise: bool = False,
+    z: torch.Tensor | None = None,
 ) -> torch.Tensor | None:
     """General entry: ``out[b] = alpha * op(a[b]) @ op(b[b // b_batch_div])^T`` with an epilogue.
 
@@ -57,7 +58,8 @@ def gemm(
     ``b_mn=False``: ``b`` is ``[N, K]``; ``b_mn=True``: ``b`` is ``[K, N]``.
     Every output element adds its products in the same order whatever the other sizes are: a row of ``a`` gives the same
     bits alone and among thousands, whichever kernel the sizes favour. ``stepwise`` (plain store): rounded like the separate
-    operations ``residual + alpha * (a @ b)`` on bf16 tensors, product, scaling and sum each to bf16.
+    operations ``residual + alpha * (a @ b)`` on bf16 tensors, product, scaling and sum each to bf16. ``z`` (forward
+    cross-entropy): fp32 buffer of :func:`lce_logits_floats` values, filled with the logits for :func:`lce_grad`.
     """
     _check2d(a, "a")
     _check2d(b, "b")
@@ -108,6 +110,10 @@ def gemm(
     args.lse, args.coef = _lib.ptr(lse), _lib.ptr(coef)
     if pmax is not None:
         args.lce_parts = 2 if pmax.shape[-1] == lce_tiles(N, parts=2) else 1
+    if z is not None:
+        if epilogue != EPI_LCE_FWD or z.dtype != torch.float32 or z.numel() < lce_logits_floats(M, N):
+            raise ValueError("z: fp32 buffer of lce_logits_floats() values, filled by the forward cross-entropy epilogue")
+        args.z = z.data_ptr()
     args.err = _lib.err_word(a.device).data_ptr()
     args.max_ctas = max_ctas
     if tile_group is not None:      # row-grouped A / C, B batched per group (mixture of experts forward / dgrad)
@@ -157,6 +163,32 @@ def lce_tiles(n_vocab: int, parts: int = 1) -> int:
     halves by twice the warps, the faster form when a soft cap's hyperbolic tangents set the pace (the width of the
     buffers tells :func:`gemm` which form to run)."""
     return _lib.lib().opk_gemm_tiles_n(n_vocab, 6 if parts == 2 else EPI_LCE_FWD)
+
+
+def lce_logits_floats(rows: int, n_vocab: int) -> int:
+    """Size of the fp32 buffer in which the forward cross-entropy product leaves its logits (blocked layout) for
+    :func:`lce_grad`."""
+    return _lib.lib().opk_lce_logits_floats(rows, n_vocab)
+
+
+def lce_keeps_logits(rows: int, n_vocab: int, dim: int, softcap: float = 0.0) -> bool:
+    """Whether storing the logits and reading them back is cheaper than forming them again (both passes, us, product -> stored):
+    2048 x 128256 over 4096 columns 2860 -> 1758, over 2048 1344 -> 969, 4092 x 50257 x 2048 1188 -> 864 and with a soft cap
+    1406 -> 944. Below 1024 columns it depends on the cache: 2040 x 8192 x 512 (67 MB) 89 -> 78, 1024 x 50257 x 768 (206 MB)
+    151 -> 154."""
+    return dim >= 1024 or softcap > 0 or 4 * rows * n_vocab <= 128 << 20
+
+
+def lce_grad(z: torch.Tensor, labels: torch.Tensor, lse: torch.Tensor, coef: torch.Tensor, out: torch.Tensor,
+             softcap: float = 0.0) -> torch.Tensor:
+    """``out [M, N] = (softmax - onehot) * coef`` from stored logits: the bits of ``EPI_LCE_BWD`` without its product."""
+    M, N = out.shape
+    _check2d(out, "out")
+    if z.numel() < lce_logits_floats(M, N):
+        raise ValueError("z holds fewer logits than out has elements")
+    _lib.check(_lib.lib().opk_lce_grad(z.data_ptr(), labels.data_ptr(), lse.data_ptr(), coef.data_ptr(), out.data_ptr(), out.stride(0),
+                                       M, N, softcap, _lib.stream_ptr(out.device)), "opk_lce_grad")
+    return out
 
 
 def set_pair_mode(on: bool) -> None:

@@ -3,9 +3,10 @@
 Counterpart of ``opake_linear_cross_entropy_loss`` (packages/opake-patches/src/opake/api/patches/kernels/
 linear_cross_entropy.py:1223-1276, kernels :101-247 and :292-528). The reference tiles the vocabulary inside a Triton
 program and merges partial log-sum-exps under a spin lock; here the vocabulary GEMM runs on the tcgen05 kernel with
-two epilogues: the forward epilogue reduces every 128-column tile to (max, sum-exp, target logit) per row, a tiny
+two epilogues: the forward epilogue reduces every 256-column tile to (max, sum-exp, target logit) per row, a tiny
 finalize kernel merges the tiles, and the backward epilogue recomputes the logits tile and writes
-``coef * (softmax - onehot)`` in bf16, from which dH and dW are two more GEMMs.
+``coef * (softmax - onehot)`` in bf16, from which dH and dW are two more GEMMs. Up to ``KEEP_BYTES`` of logits are left
+behind by the forward epilogue for one backward pass instead (same bits, a pass over memory in place of the product).
 
 Both directions are ``torch.autograd.Function`` objects with ``vmap`` rules so that ``vmap(grad(loss))`` works: a
 batch of examples sharing one weight is flattened into rows for the forward and dH; the per-example weight gradient
@@ -17,6 +18,17 @@ from __future__ import annotations
 import torch
 
 IGNORE_INDEX = -100
+
+# Logits of one loss that may wait for its backward pass. They are twice the bf16 gradient that the backward pass
+# writes anyway; beyond this size the second product is the smaller price.
+KEEP_BYTES = 1 << 30
+
+
+def _keep_logits(hidden, weight) -> bool:
+    """Whether the forward pass leaves its logits for a backward pass: one is coming, and nobody is moving or replacing what
+    autograd saves (offloading hooks would carry the logits around)."""
+    return (torch.is_grad_enabled() and (hidden.requires_grad or weight.requires_grad)
+            and torch._C._autograd._top_saved_tensors_default_hooks(True) is None)
 
 
 def native_available(hidden: torch.Tensor, weight: torch.Tensor) -> bool:
@@ -41,25 +53,34 @@ def _chunked_nll(hidden, weight, labels, logit_scale, softcap, chunk: int = 4096
 
 
 # ------------------------------------------------------------------------------------------- native forward
-def _native_fwd(hidden, weight, labels, logit_scale, softcap):
+def _native_fwd(hidden, weight, labels, logit_scale, softcap, keep):
+    """``(nll, lse, int32 labels, logits)``; the last one is empty unless ``keep`` and the size allows it."""
     from . import gemm as G, kernels as K
-    T = hidden.shape[0]
-    tiles = G.lce_tiles(weight.shape[0], parts=2 if softcap else 1)
+    T, V = hidden.shape[0], weight.shape[0]
+    tiles = G.lce_tiles(V, parts=2 if softcap else 1)
     pmax = torch.empty(T, tiles, dtype=torch.float32, device=hidden.device)
     psum = torch.empty_like(pmax)
     tgt = torch.empty(T, dtype=torch.float32, device=hidden.device)
     lab = labels.to(torch.int32).contiguous()
+    n = G.lce_logits_floats(T, V)
+    try:
+        keep = keep and 4 * n <= KEEP_BYTES and G.lce_keeps_logits(T, V, hidden.shape[1], softcap)
+        z = torch.empty(n if keep else 0, dtype=torch.float32, device=hidden.device)
+    except torch.cuda.OutOfMemoryError:
+        z = torch.empty(0, dtype=torch.float32, device=hidden.device)
     G.gemm(hidden, weight, epilogue=G.EPI_LCE_FWD, labels=lab, pmax=pmax, psum=psum, tgt=tgt, alpha=logit_scale,
-           softcap=softcap)
+           softcap=softcap, z=z if z.numel() else None)
     lse, nll = K.lce_finalize(pmax, psum, tgt, lab)
-    return nll, lse, lab
+    return nll, lse, lab, z
 
 
-def _native_dlogits(hidden, weight, lab, lse, coef, logit_scale, softcap):
+def _native_dlogits(hidden, weight, lab, lse, z, coef, logit_scale, softcap):
     from . import gemm as G
     T, V = hidden.shape[0], weight.shape[0]
     Vp = (V + 7) // 8 * 8
     dlog = torch.empty(T, Vp, dtype=torch.bfloat16, device=hidden.device)[:, :V]
+    if z.numel():
+        return G.lce_grad(z, lab, lse, coef.contiguous(), dlog, softcap)
     G.gemm(hidden, weight, out=dlog, epilogue=G.EPI_LCE_BWD, labels=lab, lse=lse, coef=coef.contiguous(),
            alpha=logit_scale, softcap=softcap)
     return dlog
@@ -69,10 +90,10 @@ class _LinearCEBackward(torch.autograd.Function):
     """Backward of the fused loss as its own Function so that it can carry a vmap rule (per-example dW)."""
 
     @staticmethod
-    def forward(grad_nll, hidden, weight, lab, lse, logit_scale, softcap):
+    def forward(grad_nll, hidden, weight, lab, lse, z, logit_scale, softcap):
         from . import gemm as G
         coef = (grad_nll.to(torch.float32) * (lab >= 0)).contiguous()
-        dlog = _native_dlogits(hidden, weight, lab, lse, coef, logit_scale, softcap)
+        dlog = _native_dlogits(hidden, weight, lab, lse, z, coef, logit_scale, softcap)
         # dlog is the gradient with respect to logit_scale * (hidden @ weight.T)
         d_hidden = G.gemm(dlog, weight, b_mn=True, alpha=logit_scale)
         d_weight = G.linear_wgrad(dlog, hidden)
@@ -89,7 +110,7 @@ class _LinearCEBackward(torch.autograd.Function):
         raise NotImplementedError("second-order differentiation of the fused linear cross-entropy is not supported")
 
     @staticmethod
-    def vmap(info, in_dims, grad_nll, hidden, weight, lab, lse, logit_scale, softcap):
+    def vmap(info, in_dims, grad_nll, hidden, weight, lab, lse, z, logit_scale, softcap):
         from . import gemm as G
         if in_dims[2] is not None:
             raise NotImplementedError("fused linear cross-entropy under vmap needs one shared weight")
@@ -103,7 +124,10 @@ class _LinearCEBackward(torch.autograd.Function):
         hf = h.reshape(B * T, D).contiguous()
         labf = lb.reshape(B * T).contiguous()
         coef = (g.to(torch.float32).reshape(B * T) * (labf >= 0)).contiguous()
-        dlog = _native_dlogits(hf, weight, labf, ls.reshape(B * T).contiguous(), coef, logit_scale, softcap)
+        # the stored logits have the rows of the whole batch when the forward pass ran under this vmap, which shows in lse; with
+        # a vmap over cotangents alone they are one example's
+        zf = z if in_dims[4] is not None and in_dims[5] is None else z.new_empty(0)
+        dlog = _native_dlogits(hf, weight, labf, ls.reshape(B * T).contiguous(), zf, coef, logit_scale, softcap)
         d_hidden = G.gemm(dlog, weight, b_mn=True, alpha=logit_scale).view(B, T, D)
         V = weight.shape[0]
         d_weight = torch.empty(B, V, D, dtype=torch.bfloat16, device=hidden.device)
@@ -115,34 +139,33 @@ class _LinearCEBackward(torch.autograd.Function):
 
 class _LinearCE(torch.autograd.Function):
     @staticmethod
-    def forward(hidden, weight, labels, logit_scale, softcap):
-        nll, lse, lab = _native_fwd(hidden.contiguous(), weight, labels, logit_scale, softcap)
-        return nll, lse, lab
+    def forward(hidden, weight, labels, logit_scale, softcap, keep):
+        return _native_fwd(hidden.contiguous(), weight, labels, logit_scale, softcap, keep)
 
     @staticmethod
     def setup_context(ctx, inputs, output):
-        hidden, weight, _labels, logit_scale, softcap = inputs
-        _nll, lse, lab = output
-        ctx.save_for_backward(hidden, weight, lab, lse)
-        ctx.mark_non_differentiable(lse, lab)
+        hidden, weight, _labels, logit_scale, softcap, _keep = inputs
+        _nll, lse, lab, z = output
+        ctx.save_for_backward(hidden, weight, lab, lse, z)
+        ctx.mark_non_differentiable(lse, lab, z)
         ctx.logit_scale, ctx.softcap = logit_scale, softcap
 
     @staticmethod
-    def backward(ctx, g_nll, _g_lse, _g_lab):
-        hidden, weight, lab, lse = ctx.saved_tensors
-        d_hidden, d_weight = _LinearCEBackward.apply(g_nll, hidden, weight, lab, lse, ctx.logit_scale, ctx.softcap)
-        return d_hidden, d_weight, None, None, None
+    def backward(ctx, g_nll, _g_lse, _g_lab, _g_z):
+        hidden, weight, lab, lse, z = ctx.saved_tensors
+        d_hidden, d_weight = _LinearCEBackward.apply(g_nll, hidden, weight, lab, lse, z, ctx.logit_scale, ctx.softcap)
+        return d_hidden, d_weight, None, None, None, None
 
     @staticmethod
-    def vmap(info, in_dims, hidden, weight, labels, logit_scale, softcap):
+    def vmap(info, in_dims, hidden, weight, labels, logit_scale, softcap, keep):
         if in_dims[1] is not None:
             raise NotImplementedError("fused linear cross-entropy under vmap needs one shared weight")
         B = info.batch_size
         h = hidden.movedim(in_dims[0], 0) if in_dims[0] is not None else hidden.unsqueeze(0).expand(B, *hidden.shape)
         lb = labels.movedim(in_dims[2], 0) if in_dims[2] is not None else labels.unsqueeze(0).expand(B, *labels.shape)
         T, D = h.shape[1], h.shape[2]
-        nll, lse, lab = _native_fwd(h.reshape(B * T, D).contiguous(), weight, lb.reshape(B * T), logit_scale, softcap)
-        return (nll.view(B, T), lse.view(B, T), lab.view(B, T)), (0, 0, 0)
+        nll, lse, lab, z = _native_fwd(h.reshape(B * T, D).contiguous(), weight, lb.reshape(B * T), logit_scale, softcap, keep)
+        return (nll.view(B, T), lse.view(B, T), lab.view(B, T), z), (0, 0, 0, None)
 
 
 def linear_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor, *, logit_scale: float = 1.0,
@@ -157,7 +180,7 @@ def linear_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, labels: tor
     if hidden.dim() != 2:
         raise ValueError("hidden must be [T, D]; flatten leading dimensions first")
     if not force_portable and native_available(hidden, weight):
-        nll, _lse, _lab = _LinearCE.apply(hidden, weight, labels, float(logit_scale), float(logit_softcapping))
+        nll = _LinearCE.apply(hidden, weight, labels, float(logit_scale), float(logit_softcapping), _keep_logits(hidden, weight))[0]
     else:
         nll = _chunked_nll(hidden, weight, labels, float(logit_scale), float(logit_softcapping))
     if use_token_scaling:
