@@ -74,8 +74,11 @@ struct Gemm2Cfg {
 };
 
 constexpr int kStageWarps = 8;     // copier warps per CTA of the staged variant
+enum Gemm2Variant : int { G2_PLAIN = 0, G2_STAGE = 1, G2_WIDE = 2 };      // G2_WIDE: eight epilogue warps (see wide_epilogue)
 // The staged variant keeps four epilogue warps: with eight next to its copier warps a thread would have 112 registers.
-__host__ __device__ constexpr int gemm2_epi_warps(int epi, bool stage) { return stage ? 4 : gemm_epi_warps(epi); }
+__host__ __device__ constexpr int gemm2_epi_warps(int epi, int variant) {
+  return variant == G2_STAGE ? 4 : variant == G2_WIDE ? 8 : gemm_epi_warps(epi);
+}
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;
@@ -83,10 +86,12 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   return v;
 }
 
-template <bool A_MN, bool B_MN, int EPI, bool STAGE = false>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * gemm2_epi_warps(EPI, STAGE) + (STAGE ? 32 * kStageWarps : 0), 1)
+template <bool A_MN, bool B_MN, int EPI, int VARIANT = G2_PLAIN>
+__global__ void __cluster_dims__(2, 1, 1)
+__launch_bounds__(64 + 32 * gemm2_epi_warps(EPI, VARIANT) + (VARIANT == G2_STAGE ? 32 * kStageWarps : 0), 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   using Cfg = Gemm2Cfg;
+  constexpr bool STAGE = VARIANT == G2_STAGE;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -109,7 +114,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 2 * gemm2_epi_warps(EPI, STAGE));    // the epilogue warps of both CTAs
+      mbar_init(&tempty[b], 2 * gemm2_epi_warps(EPI, VARIANT));    // the epilogue warps of both CTAs
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -216,9 +221,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
     __syncwarp();
-  } else if (STAGE && warp >= 2 + gemm2_epi_warps(EPI, STAGE)) {
+  } else if (STAGE && warp >= 2 + gemm2_epi_warps(EPI, VARIANT)) {
     // ------------------------------------------------------------ copiers: remote B -> local scratch, band by band
-    const int ctid = (warp - 2 - gemm2_epi_warps(EPI, STAGE)) * 32 + lane;
+    const int ctid = (warp - 2 - gemm2_epi_warps(EPI, VARIANT)) * 32 + lane;
     const long long nthreads = (long long)gridDim.x * (32 * kStageWarps);
     const long long gtid = (long long)blockIdx.x * (32 * kStageWarps) + ctid;
     // K-major B ([N][K], a band = 2048 whole rows) or MN-major B ([K][N], a band = 2048 columns of every row)
@@ -262,7 +267,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs, own 128 rows each)
     const int quad = warp & 3;
-    constexpr int CSPLIT = gemm2_epi_warps(EPI, STAGE) / 4;
+    constexpr int CSPLIT = gemm2_epi_warps(EPI, VARIANT) / 4;
     const int c_begin = ((warp - 2) >> 2) * (BN / CSPLIT), c_end = c_begin + BN / CSPLIT;
     uint8_t* scratch = smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * kEpiScratch;
     int it = 0;
@@ -301,7 +306,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tc_fence_after();
     tmem_dealloc2(tmem_base, Cfg::TMEM_COLS);
   }
-  if (EPI == EPI_SUMSQ && threadIdx.x == 0) epi_flush_sq(p, sq_slots, gemm2_epi_warps(EPI, STAGE));
+  if (EPI == EPI_SUMSQ && threadIdx.x == 0) epi_flush_sq(p, sq_slots, gemm2_epi_warps(EPI, VARIANT));
   if (threadIdx.x == 0 && *abort_flag && p.err) atomicExch(p.err, 1);
 }
 

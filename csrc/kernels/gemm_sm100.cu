@@ -93,10 +93,11 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams& 
 int g_pair_mode = 1;
 bool pair_mode() { return g_pair_mode == 1; }
 
-template <bool A_MN, bool B_MN, int EPI, bool STAGE = false>
+template <bool A_MN, bool B_MN, int EPI, int VARIANT = opk::G2_PLAIN>
 int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams& p, int max_ctas, cudaStream_t st) {
   using Cfg = opk::Gemm2Cfg;
-  auto kern = opk::gemm2_bf16_kernel<A_MN, B_MN, EPI, STAGE>;
+  auto kern = opk::gemm2_bf16_kernel<A_MN, B_MN, EPI, VARIANT>;
+  constexpr int kThreads = 64 + 32 * opk::gemm2_epi_warps(EPI, VARIANT) + (VARIANT == opk::G2_STAGE ? 32 * opk::kStageWarps : 0);
   static bool attr_done = false;
   if (!attr_done) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
@@ -107,7 +108,7 @@ int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams&
   int grid = (max_ctas > 0 ? max_ctas : num_sms()) & ~1;   // whole CTA pairs
   if (grid < 2) grid = 2;
   if (grid > 2 * tiles) grid = 2 * tiles;
-  cudaError_t e = opk::launch(kern, grid, 64 + 32 * opk::gemm2_epi_warps(EPI, STAGE) + (STAGE ? 32 * opk::kStageWarps : 0), Cfg::SMEM_BYTES, st, ta, tb, p);
+  cudaError_t e = opk::launch(kern, grid, kThreads, Cfg::SMEM_BYTES, st, ta, tb, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
   return 0;
@@ -164,6 +165,18 @@ int choose_narrow(const OpkGemmArgs* a, int bn, bool pair) {
     if (c < cost) { cost = c; best = w; }
   }
   return best;
+}
+
+// Whether the pair kernel takes eight epilogue warps for a plain store. Where the main loop covers the epilogue of the tile before,
+// four are as good and draw less power; eight pay where the epilogue sets the pace (us, four -> eight):
+//   weight gradients over few rows   16384 x 2048 over 317: 28.8 -> 24.3, with norm 35.2 -> 28.7; over 64 25.4 -> 20.4; over 1024
+//                                    51.0 -> 50.4; 128256 x 2048 over 317 189 -> 164 (its 525 MB take 170 us in a copy)
+//   a residual to read               4096 x 768 x 3072 40 -> 33; 2048 x 16384 x 2048 111 -> 103; 1021 x 4096 x 4096 37 -> 33
+//   one round of tiles               the only epilogue is exposed: 2304 x 768 over 1024 16.6 -> 13.1
+// By the tiles of one batch entry: the number of examples in a launch must not choose how a norm is summed.
+bool wide_epilogue(const OpkGemmArgs* a) {
+  const long long tiles = (long long)((a->M + 255) / 256) * ((a->N + 255) / 256);
+  return a->R || (a->a_mn && a->K <= 512) || tiles <= num_sms() / 2;
 }
 
 int pick_bn(int N, int epilogue) {
@@ -278,9 +291,9 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
     cudaError_t e = cudaMemsetAsync(a->stage_ready, 0, sizeof(int32_t) * n_bands, st);
     if (e != cudaSuccess) { set_err(cudaGetErrorString(e)); return (int)e; }
     p.stage_src = a->B; p.stage_ld = a->ldb; p.stage_dst = a->stage_dst; p.stage_ready = a->stage_ready;
-    if (a->epilogue == opk::EPI_SWIGLU) return launch2<false, false, opk::EPI_SWIGLU, true>(ta, tb, p, mc, st);
-    return a->b_mn ? launch2<false, true, opk::EPI_STORE, true>(ta, tb, p, mc, st)
-                   : launch2<false, false, opk::EPI_STORE, true>(ta, tb, p, mc, st);
+    if (a->epilogue == opk::EPI_SWIGLU) return launch2<false, false, opk::EPI_SWIGLU, opk::G2_STAGE>(ta, tb, p, mc, st);
+    return a->b_mn ? launch2<false, true, opk::EPI_STORE, opk::G2_STAGE>(ta, tb, p, mc, st)
+                   : launch2<false, false, opk::EPI_STORE, opk::G2_STAGE>(ta, tb, p, mc, st);
   }
   if (narrow) {
     if (a->epilogue == opk::EPI_SWIGLU && (!a->act || (a->N & 1))) { set_err("opk_gemm: swiglu needs act and even N"); return -1; }
@@ -302,12 +315,19 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   if (pair) {
     switch (a->epilogue) {
       case opk::EPI_STORE:
+        if (wide_epilogue(a)) {
+          if (key == 0) return launch2<false, false, opk::EPI_STORE, opk::G2_WIDE>(ta, tb, p, mc, st);
+          if (key == 2) return launch2<false, true, opk::EPI_STORE, opk::G2_WIDE>(ta, tb, p, mc, st);
+          if (key == 3) return launch2<true, true, opk::EPI_STORE, opk::G2_WIDE>(ta, tb, p, mc, st);
+          break;
+        }
         if (key == 0) return launch2<false, false, opk::EPI_STORE>(ta, tb, p, mc, st);
         if (key == 2) return launch2<false, true, opk::EPI_STORE>(ta, tb, p, mc, st);
         if (key == 3) return launch2<true, true, opk::EPI_STORE>(ta, tb, p, mc, st);
         break;
       case opk::EPI_SUMSQ:
         if (!a->sumsq) { set_err("opk_gemm: sumsq pointer required"); return -1; }
+        if (key == 3 && wide_epilogue(a)) return launch2<true, true, opk::EPI_SUMSQ, opk::G2_WIDE>(ta, tb, p, mc, st);
         if (key == 3) return launch2<true, true, opk::EPI_SUMSQ>(ta, tb, p, mc, st);
         break;
       case opk::EPI_SWIGLU:
