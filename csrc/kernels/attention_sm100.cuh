@@ -1,6 +1,8 @@
 // Causal grouped-query flash attention for sm_100a on tcgen05 / TMEM, operating in place on the fused projection
 // buffer qkv[T][(H + 2*KV) * hd] (bf16, row pitch ld): Q head h at column h*hd, K head g at (H+g)*hd, V head g at
-// (H+KV+g)*hd. head_dim is 64 or 128. One example (sequence) per launch; heads are the parallel dimension.
+// (H+KV+g)*hd. head_dim is 64 or 128. A launch takes one or several sequences of T rows, one after the other (blockIdx.y); the
+// CTAs of a sequence take the same items in the same order as in a launch of its own, so its result has the same bits. All
+// tensor maps have the sequence as their last dimension: rows past T read as zero and are not written.
 //
 // Shared design of the three kernels (forward, dK/dV, dQ):
 //   * 384 threads: warp 0 = TMA producer (Q, K), warp 1 = TMEM owner + issuer of the score products, warps 2..9 =
@@ -24,7 +26,7 @@ struct AttnParams {
   int T, H, KV, hd;
   long long ld;            // row pitch of qkv / dqkv (elements)
   long long ldo;           // row pitch of out / dout (elements)
-  void* out;               // fwd: bf16 [T][H*hd]
+  void* out;               // fwd: bf16 [T][H*hd] (every buffer holds one such part per sequence)
   float* lse;              // [H][T] natural-log-sum-exp of scaled scores
   const void* dout;        // bwd: bf16 [T][H*hd]
   const float* dsum;       // bwd: [H][T64] rowsum(dO * O), T64 = T rounded up to a multiple of 64
@@ -41,18 +43,10 @@ __device__ __forceinline__ uint32_t swz_off(int r, int c) {
   return (uint32_t)(r * 128 + ((((c >> 3) ^ (r & 7)) << 4) | ((c & 7) << 1)));
 }
 
-// 2-D TMA load of a {64 cols, rows} box (the tensor map fixes the box shape).
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-      : "memory");
-}
-
-// 2-D TMA store of a {64 cols, rows} box from shared memory (rows outside the tensor are clipped), as one bulk group.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* smem_src, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
-               "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
+// TMA store of a {64 cols, rows} box from shared memory (rows past the end of the sequence are clipped), as one bulk group.
+__device__ __forceinline__ void tma_store_seq(const CUtensorMap* map, const void* smem_src, int c0, int c1, int seq) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map),
+               "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(seq)
                : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
@@ -240,7 +234,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* xchg = reinterpret_cast<float*>(bars + 32);   // [2 groups][128 rows] running maxima, then [2][128] row sums
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, seq = (int)blockIdx.y;
   const int n_qt = (p.T + 127) / 128;
   const int n_items = n_qt * p.H;
   const int G = (int)gridDim.x, cta = (int)blockIdx.x;
@@ -265,9 +259,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
     tma_prefetch_desc(&tm);
     pdl_wait();
     mbar_expect_tx(q_full, SM::TILE);
-    for (int c = 0; c < HD / 64; ++c) tma_load_2d(smem + SM::Q_OFF + c * 16384, &tm, q_full, it.h * HD + c * 64, it.qt * 128);
+    for (int c = 0; c < HD / 64; ++c) tma_load_3d(smem + SM::Q_OFF + c * 16384, &tm, q_full, it.h * HD + c * 64, it.qt * 128, seq);
     mbar_expect_tx(&k_full[0], SM::TILE);
-    for (int c = 0; c < HD / 64; ++c) tma_load_2d(smem + SM::K_OFF + c * 16384, &tm, &k_full[0], k_col0 + it.g * HD + c * 64, 0);
+    for (int c = 0; c < HD / 64; ++c) tma_load_3d(smem + SM::K_OFF + c * 16384, &tm, &k_full[0], k_col0 + it.g * HD + c * 64, 0, seq);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
@@ -296,7 +290,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
         if (k > 0) {
           if (!mbar_wait(q_empty, (uint32_t)((k - 1) & 1), abort_flag)) break;
           mbar_expect_tx(q_full, SM::TILE);
-          for (int c = 0; c < HD / 64; ++c) tma_load_2d(smem + SM::Q_OFF + c * 16384, &tm, q_full, q_col + c * 64, it.qt * 128);
+          for (int c = 0; c < HD / 64; ++c) tma_load_3d(smem + SM::Q_OFF + c * 16384, &tm, q_full, q_col + c * 64, it.qt * 128, seq);
         }
         for (int j = (k == 0 ? 1 : 0); j < it.n_kv; ++j) {   // K(0) of the first item was requested during the setup
           const int t = t_base + j, s = t & 1;
@@ -305,7 +299,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
           if (k == OPK_TRACE_K) OPK_TRACE(0, j, 0);
           mbar_expect_tx(&k_full[s], SM::TILE);
           for (int c = 0; c < HD / 64; ++c)
-            tma_load_2d(smem + SM::K_OFF + s * SM::TILE + c * 16384, &tm, &k_full[s], k_col + c * 64, j * 128);
+            tma_load_3d(smem + SM::K_OFF + s * SM::TILE + c * 16384, &tm, &k_full[s], k_col + c * 64, j * 128, seq);
         }
         t_base += it.n_kv;
       }
@@ -328,7 +322,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
           if (k == OPK_TRACE_K) OPK_TRACE(0, j, 1);
           mbar_expect_tx(&v_full[s], SM::TILE);
           for (int c = 0; c < HD / 64; ++c)
-            tma_load_2d(smem + SM::V_OFF + s * SM::TILE + c * 16384, &tm, &v_full[s], v_col + c * 64, j * 128);
+            tma_load_3d(smem + SM::V_OFF + s * SM::TILE + c * 16384, &tm, &v_full[s], v_col + c * 64, j * 128, seq);
         }
         t_base += it.n_kv;
       }
@@ -462,7 +456,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
       // probability buffer (free: its last P*V is complete); the other group's own buffer already holds the
       // probabilities of the next item, so it borrows the second half of the owner's. HD = 64: written directly.
       uint8_t* stage = owner ? p_smem : smem + SM::P_OFF + (grp ^ 1) * SM::P_BYTES + 16384;
-      __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) + (long long)row * p.ldo + h * HD + grp * (HD / 2);
+      __nv_bfloat16* orow = reinterpret_cast<__nv_bfloat16*>(p.out) + ((long long)seq * p.T + row) * p.ldo + h * HD + grp * (HD / 2);
 #pragma unroll
       for (int c0 = 0; c0 < HD / 2; c0 += 32) {
         uint32_t ra[32], rb[32];
@@ -498,7 +492,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
         fence_proxy_async();
         __syncwarp();
         if (lane == 0 && qt * 128 + quad * 32 < p.T)
-          tma_store_2d(&tm_out, stage + quad * 32 * 128, h * HD + grp * 64, qt * 128 + quad * 32);
+          tma_store_seq(&tm_out, stage + quad * 32 * 128, h * HD + grp * 64, qt * 128 + quad * 32, seq);
       }
       if (!owner) {                               // hand the borrowed half back once the store has read it
         if (lane == 0) {
@@ -507,7 +501,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm, const __grid_constant__ 
         }
       }
       __syncwarp();
-      if (grp == 0 && row < p.T) p.lse[(long long)h * p.T + row] = m_tot * p.scale + logf(l_tot);
+      if (grp == 0 && row < p.T) p.lse[((long long)seq * p.H + h) * p.T + row] = m_tot * p.scale + logf(l_tot);
       if (e_k == OPK_TRACE_K && quad == 2 && lane == 0) OPK_TRACE(2, 100 + grp, 1);
       if (quad == 2 && lane == 0 && grp == 0) OPK_TRACE_ITEM(e_w, 1);
       return true;
@@ -698,6 +692,8 @@ __device__ __forceinline__ void store_acc_rows(uint32_t tmem_addr, __nv_bfloat16
 // dqkv[t][K | V columns] = bf16(sum over the G partials), summed in index order (deterministic).
 __global__ void attn_dkv_reduce_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ dqkv, int T, int G,
                                        int kvw, long long ld, int k_col0) {
+  part += (long long)blockIdx.y * 2 * G * T * kvw;        // one sequence per grid row
+  dqkv += (long long)blockIdx.y * T * ld;
   // eight columns per thread and step: 2 * G independent 16-byte loads in flight, one 16-byte store
   const long long n8 = (long long)T * (kvw / 8) * 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
@@ -801,7 +797,7 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pd_free + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, seq = (int)blockIdx.y;
   const int G = p.H / p.KV;
   // Two work splits: one CTA per (key tile, KV head) that loops over the G query heads of the group and stores
   // bf16 results directly; or, with a partial buffer, one CTA per (key tile, query head) that stores fp32 partials
@@ -832,8 +828,8 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant
     pdl_wait();
     mbar_expect_tx(kv_full, 2 * SM::KV_TILE);
     for (int c = 0; c < HD / 64; ++c) {
-      tma_load_2d(smem + SM::K_OFF + c * 16384, &tm_kv, kv_full, k_col + c * 64, kt * 128);
-      tma_load_2d(smem + SM::V_OFF + c * 16384, &tm_kv, kv_full, v_col + c * 64, kt * 128);
+      tma_load_3d(smem + SM::K_OFF + c * 16384, &tm_kv, kv_full, k_col + c * 64, kt * 128, seq);
+      tma_load_3d(smem + SM::V_OFF + c * 16384, &tm_kv, kv_full, v_col + c * 64, kt * 128, seq);
     }
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
@@ -855,11 +851,11 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant
         const int h = h_first + i / per_head, q64 = q_first + i % per_head;
         if (!mbar_wait(&q_empty[s], ph ^ 1u, abort_flag)) break;
         mbar_expect_tx(&q_full[s], 2 * SM::Q_TILE + 512);
-        bulk_load_1d(smem + SM::ROW_OFF + s * 512, p.nlse2 + (long long)h * p.T64 + q64 * 64, 256, &q_full[s]);
-        bulk_load_1d(smem + SM::ROW_OFF + s * 512 + 256, p.dsum + (long long)h * p.T64 + q64 * 64, 256, &q_full[s]);
+        bulk_load_1d(smem + SM::ROW_OFF + s * 512, p.nlse2 + ((long long)seq * p.H + h) * p.T64 + q64 * 64, 256, &q_full[s]);
+        bulk_load_1d(smem + SM::ROW_OFF + s * 512 + 256, p.dsum + ((long long)seq * p.H + h) * p.T64 + q64 * 64, 256, &q_full[s]);
         for (int c = 0; c < HD / 64; ++c) {
-          tma_load_2d(smem + SM::Q_OFF + s * SM::Q_TILE + c * 8192, &tm_q, &q_full[s], h * HD + c * 64, q64 * 64);
-          tma_load_2d(smem + SM::DO_OFF + s * SM::Q_TILE + c * 8192, &tm_do, &q_full[s], h * HD + c * 64, q64 * 64);
+          tma_load_3d(smem + SM::Q_OFF + s * SM::Q_TILE + c * 8192, &tm_q, &q_full[s], h * HD + c * 64, q64 * 64, seq);
+          tma_load_3d(smem + SM::DO_OFF + s * SM::Q_TILE + c * 8192, &tm_do, &q_full[s], h * HD + c * 64, q64 * 64, seq);
         }
       }
     }
@@ -981,13 +977,13 @@ attn_dkv_kernel(const __grid_constant__ CUtensorMap tm_kv, const __grid_constant
 #pragma unroll
             for (int b = 0; b < NB; ++b)
               tma_store_3d_nocommit(&tm_part, stage + (m * NB + b) * 4096, g * HD + half * (HD / 2) + b * 32,
-                                    kt * 128 + quad * 32, m * G + (h_first % G));
+                                    kt * 128 + quad * 32, (2 * seq + m) * G + (h_first % G));
           tma_store_commit();
           tma_store_wait_read();
         }
         __syncwarp();
       } else {
-        __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.dqkv) + (long long)key * p.ld + half * (HD / 2);
+        __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(p.dqkv) + ((long long)seq * p.T + key) * p.ld + half * (HD / 2);
         store_acc_rows<HD / 2>(tmem + lane_base + DV_COL + half * (HD / 2), base + v_col, key < p.T, 1.f);
         store_acc_rows<HD / 2>(tmem + lane_base + DK_COL + half * (HD / 2), base + k_col, key < p.T, p.scale);
       }
@@ -1069,7 +1065,7 @@ attn_dq128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_read + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, seq = (int)blockIdx.y;
   const int n_qt = (p.T + 127) / 128;
   const int h = blockIdx.x % p.H;
   const int qt = n_qt - 1 - (int)(blockIdx.x / p.H);     // heavy (late) query tiles first
@@ -1097,14 +1093,14 @@ attn_dq128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     pdl_wait();
     mbar_expect_tx(q_full, 2 * SM::Q_TILE);
     for (int c = 0; c < HD / 64; ++c) {
-      tma_load_2d(smem + SM::Q_OFF + c * 16384, &tm_q, q_full, q_col + c * 64, qt * 128);
-      tma_load_2d(smem + SM::DO_OFF + c * 16384, &tm_do, q_full, q_col + c * 64, qt * 128);
+      tma_load_3d(smem + SM::Q_OFF + c * 16384, &tm_q, q_full, q_col + c * 64, qt * 128, seq);
+      tma_load_3d(smem + SM::DO_OFF + c * 16384, &tm_do, q_full, q_col + c * 64, qt * 128, seq);
     }
     mbar_expect_tx(&k_full[0], SM::KV_TILE);
-    for (int c = 0; c < HD / 64; ++c) tma_load_2d(smem + SM::K_OFF + c * 16384, &tm_kv, &k_full[0], k_col + c * 64, 0);
+    for (int c = 0; c < HD / 64; ++c) tma_load_3d(smem + SM::K_OFF + c * 16384, &tm_kv, &k_full[0], k_col + c * 64, 0, seq);
     // the O tile of these rows goes into the dS buffer, which is idle until the first score gradients are stored
     mbar_expect_tx(o_full, SM::Q_TILE);
-    for (int c = 0; c < HD / 64; ++c) tma_load_2d(smem + SM::DS_OFF + c * 16384, &tm_o, o_full, q_col + c * 64, qt * 128);
+    for (int c = 0; c < HD / 64; ++c) tma_load_3d(smem + SM::DS_OFF + c * 16384, &tm_o, o_full, q_col + c * 64, qt * 128, seq);
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
@@ -1123,7 +1119,7 @@ attn_dq128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if (!mbar_wait(&k_empty[s], (uint32_t)((i / NS) & 1) ^ 1u, abort_flag)) break;
         mbar_expect_tx(&k_full[s], SM::KV_TILE);
         for (int c = 0; c < HD / 64; ++c)
-          tma_load_2d(smem + SM::K_OFF + s * SM::KV_TILE + c * 16384, &tm_kv, &k_full[s], k_col + c * 64, i * 128);
+          tma_load_3d(smem + SM::K_OFF + s * SM::KV_TILE + c * 16384, &tm_kv, &k_full[s], k_col + c * 64, i * 128, seq);
       }
     }
     __syncwarp();
@@ -1134,7 +1130,7 @@ attn_dq128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if (!mbar_wait(v_empty, (uint32_t)(i & 1) ^ 1u, abort_flag)) break;
         mbar_expect_tx(v_full, SM::KV_TILE);
         for (int c = 0; c < HD / 64; ++c)
-          tma_load_2d(smem + SM::V_OFF + c * 16384, &tm_kv, v_full, v_col + c * 64, i * 128);
+          tma_load_3d(smem + SM::V_OFF + c * 16384, &tm_kv, v_full, v_col + c * 64, i * 128, seq);
       }
     }
     __syncwarp();
@@ -1226,11 +1222,11 @@ attn_dq128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(o_read);
-    const float nl_r = qvalid ? -p.lse[(long long)h * p.T + qrow] * 1.4426950408889634f : -INFINITY;   // invalid rows give P = 0
+    const float nl_r = qvalid ? -p.lse[((long long)seq * p.H + h) * p.T + qrow] * 1.4426950408889634f : -INFINITY;   // invalid rows give P = 0
     if (!qvalid) d_r = 0.f;
     if (half == 0 && qrow < p.T64) {
-      const_cast<float*>(p.dsum)[(long long)h * p.T64 + qrow] = d_r;
-      const_cast<float*>(p.nlse2)[(long long)h * p.T64 + qrow] = nl_r;
+      const_cast<float*>(p.dsum)[((long long)seq * p.H + h) * p.T64 + qrow] = d_r;
+      const_cast<float*>(p.nlse2)[((long long)seq * p.H + h) * p.T64 + qrow] = nl_r;
     }
     for (int i = 0; i < n_it && ok; ++i) {
       const int b = i & 1;
@@ -1304,12 +1300,12 @@ attn_dq128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         fence_proxy_async();
         __syncwarp();
         if (lane == 0 && qt * 128 + quad * 32 < p.T) {
-          tma_store_2d(&tm_dq, chunk + quad * 32 * 128, q_col + half * 64, qt * 128 + quad * 32);
+          tma_store_seq(&tm_dq, chunk + quad * 32 * 128, q_col + half * 64, qt * 128 + quad * 32, seq);
           tma_store_wait_read();
         }
         __syncwarp();
       } else {
-        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.dqkv) + (long long)qrow * p.ld + q_col + half * (HD / 2);
+        __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.dqkv) + ((long long)seq * p.T + qrow) * p.ld + q_col + half * (HD / 2);
         store_acc_rows<HD / 2>(tmem + lane_base + DQ_COL + half * (HD / 2), dst, qvalid, p.scale);
       }
     }

@@ -52,10 +52,11 @@ __global__ void philox_normal_kernel(float* __restrict__ out, long long n, uint6
 // is <= clip. AUTO-S (mode_auto): R / (norm + gamma) with the same guard and no clamp to one.
 __global__ void clip_scale_kernel(double* sumsq, float clip, int mode_auto, float gamma, int n_leaves,
                                   long long widest_leaf, float* scale_out, float* norm_out, int* counters, int reset) {
-  const double sq = *sumsq;
-  if (reset) *sumsq = 0.0;
+  const int j = threadIdx.x;             // one example per thread
+  const double sq = sumsq[j];
+  if (reset) sumsq[j] = 0.0;
   const double norm = sqrt(sq > 0.0 ? sq : 0.0);
-  if (norm_out) *norm_out = (float)norm;
+  if (norm_out) norm_out[j] = (float)norm;
   const double c = clip > 0.f ? (double)clip : 0.0;
   double ratio;
   if (mode_auto) ratio = c / (norm + (double)gamma);
@@ -78,7 +79,7 @@ __global__ void clip_scale_kernel(double* sumsq, float clip, int mode_auto, floa
   // round the fp32 factor toward zero so the cast itself cannot enlarge it
   float sf = (float)s;
   if ((double)sf > s) sf = nextafterf(sf, 0.0f);
-  *scale_out = sf;
+  scale_out[j] = sf;
 }
 
 struct alignas(16) bf16x8 { __nv_bfloat162 h[4]; };
@@ -517,8 +518,9 @@ extern "C" int opk_philox_normal(float* out, int64_t n, uint64_t seed, uint32_t 
 }
 
 extern "C" int opk_clip_scale(double* sumsq, float clip, int mode_auto, float gamma, int n_leaves, int64_t widest_leaf,
-                              float* scale_out, float* norm_out, int32_t* counters, int reset, void* stream) {
-  clip_scale_kernel<<<1, 1, 0, ST(stream)>>>(sumsq, clip, mode_auto, gamma, n_leaves, widest_leaf, scale_out, norm_out,
+                              float* scale_out, float* norm_out, int32_t* counters, int reset, int batch, void* stream) {
+  if (batch < 1 || batch > 32) return -1;
+  clip_scale_kernel<<<1, batch, 0, ST(stream)>>>(sumsq, clip, mode_auto, gamma, n_leaves, widest_leaf, scale_out, norm_out,
                                             counters, reset);
   OPK_LAUNCH_CHECK();
   return 0;

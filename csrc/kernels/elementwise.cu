@@ -210,7 +210,8 @@ __global__ void __launch_bounds__(NT) add_rmsnorm_fwd_kernel(const __nv_bfloat16
 
 // RMSNorm backward. A CTA of 512 threads walks rows with a grid stride; every thread owns the same columns for
 // all rows (ITERS vectors of 8), so the weight gradient accumulates in registers without atomics and is written once
-// per CTA to partial[blockIdx][D]. A second kernel adds the column sums of `partial` into dw.
+// per CTA to partial[CTA][D]. A second kernel adds the column sums of `partial` into dw. gridDim.y examples of T rows each:
+// an example's rows meet the same CTAs in the same order as in a launch of its own, so its weight gradient has the same bits.
 constexpr int MAX_COL_ITERS = 8;  // layernorm backward: D <= 8 * 2048
 constexpr int RMS_BWD_NT = 512;
 template <int ITERS>
@@ -225,6 +226,7 @@ __global__ void __launch_bounds__(RMS_BWD_NT) rmsnorm_bwd_kernel(const __nv_bflo
                                                                  long long ld_dx) {
   __shared__ float sh[32];
   const int nv = D >> 3;
+  const long long first = (long long)blockIdx.y * T;
   float wv[ITERS][8], acc[ITERS][8];
 #pragma unroll
   for (int it = 0; it < ITERS; ++it) {
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(RMS_BWD_NT) rmsnorm_bwd_kernel(const __nv_bflo
     }
   }
   int par = 0;
-  for (long long row = blockIdx.x; row < T; row += gridDim.x) {
+  for (long long row = first + blockIdx.x; row < first + T; row += gridDim.x) {
     const bf16x8* dyr = reinterpret_cast<const bf16x8*>(dy + row * ld_dy);
     const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * ldx);
     const float rs = rstd[row];
@@ -290,7 +292,7 @@ __global__ void __launch_bounds__(RMS_BWD_NT) rmsnorm_bwd_kernel(const __nv_bflo
     for (int it = 0; it < ITERS; ++it) {
       const int v = threadIdx.x + it * RMS_BWD_NT;
       if (v < nv) {
-        float4* dst = reinterpret_cast<float4*>(partial + (long long)blockIdx.x * D + v * 8);
+        float4* dst = reinterpret_cast<float4*>(partial + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * D + v * 8);
         dst[0] = make_float4(acc[it][0], acc[it][1], acc[it][2], acc[it][3]);
         dst[1] = make_float4(acc[it][4], acc[it][5], acc[it][6], acc[it][7]);
       }
@@ -298,10 +300,12 @@ __global__ void __launch_bounds__(RMS_BWD_NT) rmsnorm_bwd_kernel(const __nv_bflo
   }
 }
 
-// dst[c] += sum_r partial[r][c]; CTA = 32 columns x 8 row groups.
+// dst[b][c] += sum_r partial[b][r][c] (b = blockIdx.y); CTA = 32 columns x 8 row groups.
 __global__ void __launch_bounds__(256) colsum_add_kernel(const float* __restrict__ partial, float* __restrict__ dst,
-                                                         int rows, int D) {
+                                                         int rows, int D, long long dst_stride) {
   opk::pdl_trigger();
+  partial += (long long)blockIdx.y * rows * D;
+  dst += blockIdx.y * dst_stride;
   __shared__ float sh[8][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -369,16 +373,17 @@ __global__ void __launch_bounds__(NT) layernorm_bwd_kernel(const __nv_bfloat16* 
                                                            const float* __restrict__ rstd,
                                                            const __nv_bfloat16* __restrict__ dres,
                                                            __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
-                                                           float* __restrict__ db, int T, int D) {
+                                                           float* __restrict__ db, int T, int D, long long stride) {
   __shared__ float sh[32];
   const int nv = D >> 3;
+  const long long first = (long long)blockIdx.y * T;       // gridDim.y examples of T rows, gradients `stride` floats apart
   float dwp[MAX_COL_ITERS][8], dbp[MAX_COL_ITERS][8];
 #pragma unroll
   for (int c = 0; c < MAX_COL_ITERS; ++c)
 #pragma unroll
     for (int j = 0; j < 8; ++j) { dwp[c][j] = 0.f; dbp[c][j] = 0.f; }
   const bf16x8* wr = reinterpret_cast<const bf16x8*>(w);
-  for (long long row = blockIdx.x; row < T; row += gridDim.x) {
+  for (long long row = first + blockIdx.x; row < first + T; row += gridDim.x) {
     const bf16x8* dyr = reinterpret_cast<const bf16x8*>(dy + row * D);
     const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * D);
     const float rs = rstd[row], mu = mean[row];
@@ -431,8 +436,8 @@ __global__ void __launch_bounds__(NT) layernorm_bwd_kernel(const __nv_bfloat16* 
     if (i < nv) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        if (dw) atomicAdd(&dw[i * 8 + j], dwp[c][j]);
-        if (db) atomicAdd(&db[i * 8 + j], dbp[c][j]);
+        if (dw) atomicAdd(&dw[blockIdx.y * stride + i * 8 + j], dwp[c][j]);
+        if (db) atomicAdd(&db[blockIdx.y * stride + i * 8 + j], dbp[c][j]);
       }
     }
   }
@@ -451,8 +456,9 @@ __global__ void __launch_bounds__(256) layernorm_bwd_warp_kernel(const __nv_bflo
                                                                  const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean,
                                                                  const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dres,
                                                                  __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
-                                                                 float* __restrict__ db, int T, int D) {
+                                                                 float* __restrict__ db, int T, int D, long long stride) {
   opk::pdl_trigger();
+  const long long first = (long long)blockIdx.y * T;       // gridDim.y examples of T rows, gradients `stride` floats apart
   constexpr int W = VPL * 256;
   __shared__ float sh[8 * W];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = D >> 3;
@@ -461,7 +467,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_warp_kernel(const __nv_bflo
   for (int i = 0; i < VPL; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) { gw[i][j] = 0.f; gb[i][j] = 0.f; }
-  for (long long row = blockIdx.x * 8ll + warp; row < T; row += gridDim.x * 8ll) {
+  for (long long row = first + blockIdx.x * 8ll + warp; row < first + T; row += gridDim.x * 8ll) {
     const bf16x8* dyr = reinterpret_cast<const bf16x8*>(dy + row * D);
     const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * D);
     const bf16x8* drr = dres ? reinterpret_cast<const bf16x8*>(dres + row * D) : nullptr;
@@ -534,7 +540,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_warp_kernel(const __nv_bflo
       for (int k = 0; k < 8; ++k)
 #pragma unroll
         for (int j = 0; j < 4; ++j) a[j] += sh[k * W + c + j];
-      red_add_v4(out + c, a);
+      red_add_v4(out + blockIdx.y * stride + c, a);
     }
   }
 }
@@ -764,13 +770,13 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const __nv_bfloat16* __re
 // ------------------------------------------------------------------------------------------- embedding
 __global__ void embedding_fwd_kernel(const int* __restrict__ tok, const __nv_bfloat16* __restrict__ table,
                                      const __nv_bfloat16* __restrict__ pos_table, __nv_bfloat16* __restrict__ out,
-                                     int D, int vocab) {
+                                     int D, int vocab, int period) {
   const long long t = blockIdx.x;
   // an id outside the table yields a zero embedding row: never an address outside the table
   const bool in_table = tok[t] >= 0 && tok[t] < vocab;
   (void)OPK_IDX_OK(tok[t], vocab);
   const bf16x8* src = reinterpret_cast<const bf16x8*>(table + (long long)(in_table ? tok[t] : 0) * D);
-  const bf16x8* ps = pos_table ? reinterpret_cast<const bf16x8*>(pos_table + t * D) : nullptr;
+  const bf16x8* ps = pos_table ? reinterpret_cast<const bf16x8*>(pos_table + (t % period) * D) : nullptr;
   bf16x8* dst = reinterpret_cast<bf16x8*>(out + t * D);
   for (int i = threadIdx.x; i < (D >> 3); i += blockDim.x) {
     if (ps || !in_table) {
@@ -792,14 +798,22 @@ __device__ __forceinline__ bool emb_tok_ok(int tok, int vocab) {
   return (unsigned)tok < (unsigned)vocab;
 }
 OPK_DEBUG_BOUNDS_UNIT();
+// gridDim.y examples of T tokens each, with a first-occurrence table, representatives and rows of their own.
 __global__ void emb_first_pos_kernel(const int* __restrict__ tok, int* __restrict__ first_pos, int T, int vocab) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  tok += (long long)blockIdx.y * T;
+  first_pos += (long long)blockIdx.y * vocab;
   if (t < T && emb_tok_ok(tok[t], vocab)) atomicMin(&first_pos[tok[t]], t);
 }
 __global__ void emb_scatter_kernel(const int* __restrict__ tok, const __nv_bfloat16* __restrict__ dx,
                                    const int* __restrict__ first_pos, int* __restrict__ rep, float* __restrict__ gc,
-                                   int D, int vocab) {
-  const long long t = blockIdx.x;
+                                   int T, int D, int vocab) {
+  const long long t = blockIdx.x, first = (long long)blockIdx.y * T;
+  tok += first;
+  rep += first;
+  dx += first * D;
+  gc += first * D;
+  first_pos += (long long)blockIdx.y * vocab;
   if (!emb_tok_ok(tok[t], vocab)) {
     if (threadIdx.x == 0) rep[t] = -1;
     return;
@@ -812,6 +826,8 @@ __global__ void emb_scatter_kernel(const int* __restrict__ tok, const __nv_bfloa
 }
 __global__ void emb_reset_kernel(const int* __restrict__ tok, int* __restrict__ first_pos, int T, int vocab) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  tok += (long long)blockIdx.y * T;
+  first_pos += (long long)blockIdx.y * vocab;
   if (t < T && emb_tok_ok(tok[t], vocab)) first_pos[tok[t]] = INT_MAX;
 }
 // ATOMIC: the rows of acc are shared with other GPUs' kernels (sharded sums, acc may be peer-mapped), so the add is a
@@ -846,9 +862,10 @@ __device__ __forceinline__ void load_vec16(const void* p, long long i, float (&f
   }
 }
 template <bool FP32, bool ROUND>
-__global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, long long n, double* out) {
-  __shared__ float sh[32];
+__global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, long long n, double* out, long long stride) {
   double acc = 0.0;
+  x = reinterpret_cast<const char*>(x) + blockIdx.y * stride * (FP32 ? 4 : 2);       // gridDim.y buffers, one sum each
+  out += blockIdx.y;
   float part = 0.f;
   int cnt = 0;
   // 16-byte loads, four vectors in flight, when the base allows it; fp32 partials of at most 64 squares as below
@@ -883,7 +900,6 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, l
     for (int w = 0; w < NT / 32; ++w) t += shd[w];
     atomicAdd(out, t);
   }
-  (void)sh;
 }
 
 // ------------------------------------------------------------------------------------------- cross entropy
@@ -936,6 +952,9 @@ __global__ void __launch_bounds__(1024) loss_coef_kernel(const int* __restrict__
                                                          const float* __restrict__ weight, float* __restrict__ coef,
                                                          float* __restrict__ loss, float* __restrict__ ntok, int T) {
   opk::pdl_trigger();
+  labels += (long long)blockIdx.x * T;         // one CTA per example
+  nll += (long long)blockIdx.x * T;
+  coef += (long long)blockIdx.x * T;
   __shared__ float red[32];
   __shared__ float bcast;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -967,8 +986,8 @@ __global__ void __launch_bounds__(1024) loss_coef_kernel(const int* __restrict__
   if (threadIdx.x == 0) {
     float s = 0.f;
     for (int wi = 0; wi < (int)(blockDim.x >> 5); ++wi) s += red[wi];
-    *loss = s;
-    if (ntok) *ntok = n;
+    loss[blockIdx.x] = s;
+    if (ntok) ntok[blockIdx.x] = n;
   }
 }
 
@@ -1140,11 +1159,12 @@ __global__ void __launch_bounds__(NT) ce_bwd_kernel(const void* __restrict__ log
 __global__ void __launch_bounds__(NT) scatter_rows_cast_sumsq_kernel(const float* __restrict__ src,
                                                                      __nv_bfloat16* __restrict__ dst_base,
                                                                      const long long* __restrict__ offsets,
-                                                                     const int* __restrict__ widths, int D, double* sumsq) {
+                                                                     const int* __restrict__ widths, int D, double* sumsq,
+                                                                     long long dst_stride) {
   __shared__ float sh[32];
   const long long r = blockIdx.x;
-  const float* s = src + r * D;
-  __nv_bfloat16* d = dst_base + offsets[r];
+  const float* s = src + ((long long)blockIdx.y * gridDim.x + r) * D;         // gridDim.y examples
+  __nv_bfloat16* d = dst_base + blockIdx.y * dst_stride + offsets[r];
   const int n = widths ? widths[r] : D;
   float part = 0.f;
   for (int i = threadIdx.x; i < n; i += NT) {
@@ -1154,13 +1174,16 @@ __global__ void __launch_bounds__(NT) scatter_rows_cast_sumsq_kernel(const float
     part += f * f;
   }
   const float tot = block_sum<NT>(part, sh);
-  if (threadIdx.x == 0 && sumsq) atomicAdd(sumsq, (double)tot);
+  if (threadIdx.x == 0 && sumsq) atomicAdd(sumsq + blockIdx.y, (double)tot);
 }
 
 // out[n] (+)= sum_t dy[t][n]  (bias gradient)
-__global__ void colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ out, int T, int N, long long ld) {
+__global__ void colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ out, int T, int N, long long ld,
+                              long long out_stride) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
+  dy += (long long)blockIdx.z * T * ld;        // gridDim.z examples of T rows
+  out += blockIdx.z * out_stride;
   float a = 0.f;
   for (int t = blockIdx.y; t < T; t += gridDim.y) a += __bfloat162float(dy[(long long)t * ld + n]);
   atomicAdd(&out[n], a);
@@ -1171,8 +1194,10 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __res
 // four columns and CTA. (2-byte loads and one atomic per column and row chunk measured 9.2 us on average over the
 // GPT-2-small bias gradients, 1024 x 768 .. 3072.)
 __global__ void __launch_bounds__(256) colsum_vec_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ out, int T, int N,
-                                                         long long ld, int rows_per_cta) {
+                                                         long long ld, int rows_per_cta, long long out_stride) {
   opk::pdl_trigger();
+  dy += (long long)blockIdx.z * T * ld;
+  out += blockIdx.z * out_stride;
   __shared__ float sh[8][256 + 4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = blockIdx.x * 256, c = c0 + lane * 8;
@@ -1204,11 +1229,12 @@ __global__ void __launch_bounds__(256) colsum_vec_kernel(const __nv_bfloat16* __
 
 // tied embeddings: dense[tok[t]] += gc[t] for representative rows (no two representatives share a row)
 __global__ void emb_add_rows_kernel(const int* __restrict__ tok, const int* __restrict__ rep,
-                                    const float* __restrict__ gc, __nv_bfloat16* __restrict__ dense, int D) {
-  const long long t = blockIdx.x;
-  if (rep[t] != (int)t) return;
-  const float* src = gc + t * D;
-  __nv_bfloat16* dst = dense + (long long)tok[t] * D;
+                                    const float* __restrict__ gc, __nv_bfloat16* __restrict__ dense, int T, int D,
+                                    long long dense_stride) {
+  const long long t = blockIdx.x, first = (long long)blockIdx.y * T;
+  if (rep[first + t] != (int)t) return;
+  const float* src = gc + (first + t) * D;
+  __nv_bfloat16* dst = dense + blockIdx.y * dense_stride + (long long)tok[first + t] * D;
   for (int d = threadIdx.x; d < D; d += blockDim.x) dst[d] = __float2bfloat16(__bfloat162float(dst[d]) + src[d]);
 }
 
@@ -1262,13 +1288,15 @@ extern "C" int opk_add_rmsnorm_fwd(const void* x, const void* r, const void* w, 
 }
 extern "C" int opk_rmsnorm_bwd_ld(const void* dy, int64_t ld_dy, const void* x, int64_t ldx, const void* w, const float* rstd,
                                   const void* dres, void* dx_out, int64_t ld_dx, float* dw, float* workspace, int ws_rows,
-                                  int T, int D, float w_offset, void* stream) {
-  if (T <= 0) return 0;
+                                  int T, int D, float w_offset, int batch, int64_t dw_stride, void* stream) {
+  if (T <= 0 || batch <= 0) return 0;
+  if (batch > 65535) return -1;
   if (D % 8 || D > 3 * RMS_BWD_NT * 8) return -1;
   if (ld_dy % 8 || ldx % 8 || ld_dx % 8 || ld_dy < D || ldx < D || ld_dx < D) return -1;
-  if (dw && (!workspace || ws_rows < 1)) return -1;
-  int grid = T < 148 * 2 ? T : 148 * 2;
-  if (dw && grid > ws_rows) grid = ws_rows;
+  if (dw && (!workspace || ws_rows < batch)) return -1;
+  int ctas = T < 148 * 2 ? T : 148 * 2;
+  if (dw && ctas > ws_rows / batch) ctas = ws_rows / batch;
+  const dim3 grid((unsigned)ctas, (unsigned)batch);
   float* part = dw ? workspace : nullptr;
   const int iters = (D / 8 + RMS_BWD_NT - 1) / RMS_BWD_NT;
   if (iters == 1)
@@ -1279,7 +1307,7 @@ extern "C" int opk_rmsnorm_bwd_ld(const void* dy, int64_t ld_dy, const void* x, 
     rmsnorm_bwd_kernel<3><<<grid, RMS_BWD_NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), rstd, BF(dres), BFM(dx_out), part, T, D, w_offset, ld_dy, ldx, ld_dx);
   OPK_LAUNCH_CHECK();
   if (dw) {
-    colsum_add_kernel<<<(D + 31) / 32, 256, 0, ST(stream)>>>(part, dw, grid, D);
+    colsum_add_kernel<<<dim3((D + 31) / 32, batch), 256, 0, ST(stream)>>>(part, dw, ctas, D, dw_stride);
     OPK_LAUNCH_CHECK();
   }
   return 0;
@@ -1287,7 +1315,7 @@ extern "C" int opk_rmsnorm_bwd_ld(const void* dy, int64_t ld_dy, const void* x, 
 extern "C" int opk_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,
                                void* dx_out, float* dw, float* workspace, int ws_rows, int T, int D, float w_offset,
                                void* stream) {
-  return opk_rmsnorm_bwd_ld(dy, D, x, D, w, rstd, dres, dx_out, D, dw, workspace, ws_rows, T, D, w_offset, stream);
+  return opk_rmsnorm_bwd_ld(dy, D, x, D, w, rstd, dres, dx_out, D, dw, workspace, ws_rows, T, D, w_offset, 1, 0, stream);
 }
 extern "C" int opk_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int T,
                                  int D, float eps, void* stream) {
@@ -1298,13 +1326,14 @@ extern "C" int opk_layernorm_fwd(const void* x, const void* w, const void* b, vo
   return 0;
 }
 extern "C" int opk_layernorm_bwd(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
-                                 const void* dres, void* dx_out, float* dw, float* db, int T, int D, void* stream) {
-  if (T <= 0) return 0;
-  if (D % 8 || D > MAX_COL_ITERS * NT * 8) return -1;
-  if (D <= 1024 && (reinterpret_cast<uintptr_t>(dw) & 15) == 0 && (reinterpret_cast<uintptr_t>(db) & 15) == 0) {
+                                 const void* dres, void* dx_out, float* dw, float* db, int T, int D, int batch, int64_t stride,
+                                 void* stream) {
+  if (T <= 0 || batch <= 0) return 0;
+  if (D % 8 || D > MAX_COL_ITERS * NT * 8 || batch > 65535) return -1;
+  if (D <= 1024 && (batch == 1 || stride % 4 == 0) && (reinterpret_cast<uintptr_t>(dw) & 15) == 0 && (reinterpret_cast<uintptr_t>(db) & 15) == 0) {
     const int g = (T + 7) / 8 < 148 ? (T + 7) / 8 : 148;
 #define OPK_LN_BWD(V) \
-  layernorm_bwd_warp_kernel<V><<<g, 256, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db, T, D)
+  layernorm_bwd_warp_kernel<V><<<dim3(g, batch), 256, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db, T, D, stride)
     if (D <= 256) OPK_LN_BWD(1);
     else if (D <= 512) OPK_LN_BWD(2);
     else if (D <= 768) OPK_LN_BWD(3);
@@ -1313,8 +1342,8 @@ extern "C" int opk_layernorm_bwd(const void* dy, const void* x, const void* w, c
     OPK_LAUNCH_CHECK();
     return 0;
   }
-  const int grid = T < 148 * 2 ? T : 148 * 2;
-  layernorm_bwd_kernel<<<grid, NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db, T, D);
+  const dim3 grid(T < 148 * 2 ? T : 148 * 2, batch);
+  layernorm_bwd_kernel<<<grid, NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db, T, D, stride);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1424,24 +1453,26 @@ extern "C" int opk_gelu_bwd(const void* dy, const void* x, void* dx, int64_t n, 
   return 0;
 }
 extern "C" int opk_embedding_fwd(const int32_t* tok, const void* table, const void* pos_table, void* out, int T, int D,
-                                 int vocab, void* stream) {
+                                 int vocab, int period, void* stream) {
   if (T <= 0) return 0;
   if (D % 8 || vocab <= 0) return -1;
-  embedding_fwd_kernel<<<T, 128, 0, ST(stream)>>>(tok, BF(table), BF(pos_table), BFM(out), D, vocab);
+  embedding_fwd_kernel<<<T, 128, 0, ST(stream)>>>(tok, BF(table), BF(pos_table), BFM(out), D, vocab, period > 0 ? period : T);
   OPK_LAUNCH_CHECK();
   return 0;
 }
 extern "C" int opk_embedding_bwd_compact(const int32_t* tok, const void* dx, int32_t* first_pos, int32_t* rep,
-                                         float* gc, double* sumsq, int T, int D, int vocab, void* stream) {
-  if (T <= 0) return 0;
-  if (vocab <= 0) return -1;
+                                         float* gc, double* sumsq, int T, int D, int vocab, int batch, void* stream) {
+  if (T <= 0 || batch <= 0) return 0;
+  if (vocab <= 0 || batch > 65535) return -1;
   cudaStream_t st = ST(stream);
-  cudaError_t e = cudaMemsetAsync(gc, 0, sizeof(float) * (size_t)T * D, st);
+  cudaError_t e = cudaMemsetAsync(gc, 0, sizeof(float) * (size_t)batch * T * D, st);
   if (e != cudaSuccess) return (int)e;
-  emb_first_pos_kernel<<<(T + 255) / 256, 256, 0, st>>>(tok, first_pos, T, vocab);
-  emb_scatter_kernel<<<T, 256, 0, st>>>(tok, BF(dx), first_pos, rep, gc, D, vocab);
-  emb_reset_kernel<<<(T + 255) / 256, 256, 0, st>>>(tok, first_pos, T, vocab);
-  if (sumsq) sumsq_kernel<true, true><<<grid_for((long long)T * D, NT, 148 * 4), NT, 0, st>>>(gc, (long long)T * D, sumsq);
+  const dim3 by_token((T + 255) / 256, batch);
+  emb_first_pos_kernel<<<by_token, 256, 0, st>>>(tok, first_pos, T, vocab);
+  emb_scatter_kernel<<<dim3(T, batch), 256, 0, st>>>(tok, BF(dx), first_pos, rep, gc, T, D, vocab);
+  emb_reset_kernel<<<by_token, 256, 0, st>>>(tok, first_pos, T, vocab);
+  const long long n = (long long)T * D;
+  if (sumsq) sumsq_kernel<true, true><<<dim3(grid_for(n, NT, 148 * 4), batch), NT, 0, st>>>(gc, n, sumsq, n);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1478,9 +1509,9 @@ extern "C" int opk_rmsnorm_dw_per_example(const void* dy, const void* x, const f
   return 0;
 }
 extern "C" int opk_loss_coef(const int32_t* labels, const float* nll, const float* weight, float* coef, float* loss, float* ntok,
-                             int T, void* stream) {
-  if (T <= 0 || !labels || !nll || !coef || !loss) return -1;
-  loss_coef_kernel<<<1, 1024, 0, ST(stream)>>>(labels, nll, weight, coef, loss, ntok, T);
+                             int T, int batch, void* stream) {
+  if (T <= 0 || batch <= 0 || !labels || !nll || !coef || !loss) return -1;
+  loss_coef_kernel<<<batch, 1024, 0, ST(stream)>>>(labels, nll, weight, coef, loss, ntok, T);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1505,45 +1536,50 @@ extern "C" int opk_cross_entropy_bwd(const void* logits, int is_fp32, const int3
   OPK_LAUNCH_CHECK();
   return 0;
 }
-extern "C" int opk_sumsq(const void* x, int is_fp32, int round_bf16, int64_t n, double* sumsq, void* stream) {
-  if (n <= 0) return 0;
-  const int g = grid_for(n, NT, 148 * 8);
+extern "C" int opk_sumsq(const void* x, int is_fp32, int round_bf16, int64_t n, double* sumsq, int batch, int64_t stride, void* stream) {
+  if (n <= 0 || batch <= 0) return 0;
+  // the 16-byte form is chosen by the base, so every buffer of a batch has to lie on the same boundary
+  if (batch > 65535 || (batch > 1 && stride % 8)) return -1;
+  const dim3 g(grid_for(n, NT, 148 * 8), batch);
   if (is_fp32) {
-    if (round_bf16) sumsq_kernel<true, true><<<g, NT, 0, ST(stream)>>>(x, n, sumsq);
-    else sumsq_kernel<true, false><<<g, NT, 0, ST(stream)>>>(x, n, sumsq);
+    if (round_bf16) sumsq_kernel<true, true><<<g, NT, 0, ST(stream)>>>(x, n, sumsq, stride);
+    else sumsq_kernel<true, false><<<g, NT, 0, ST(stream)>>>(x, n, sumsq, stride);
   } else {
-    sumsq_kernel<false, false><<<g, NT, 0, ST(stream)>>>(x, n, sumsq);
+    sumsq_kernel<false, false><<<g, NT, 0, ST(stream)>>>(x, n, sumsq, stride);
   }
   OPK_LAUNCH_CHECK();
   return 0;
 }
 extern "C" int opk_scatter_rows_cast_sumsq(const float* src, void* dst_base, const int64_t* offsets, const int32_t* widths, int R,
-                                                  int D, double* sumsq, void* stream) {
-  if (R <= 0) return 0;
-  scatter_rows_cast_sumsq_kernel<<<R, NT, 0, ST(stream)>>>(src, BFM(dst_base), reinterpret_cast<const long long*>(offsets), widths, D, sumsq);
+                                                  int D, double* sumsq, int batch, int64_t dst_stride, void* stream) {
+  if (R <= 0 || batch <= 0) return 0;
+  if (batch > 65535) return -1;
+  scatter_rows_cast_sumsq_kernel<<<dim3(R, batch), NT, 0, ST(stream)>>>(src, BFM(dst_base), reinterpret_cast<const long long*>(offsets), widths, D, sumsq, dst_stride);
   OPK_LAUNCH_CHECK();
   return 0;
 }
-extern "C" int opk_colsum(const void* dy, float* out, int T, int N, int64_t ld, void* stream) {
-  if (T <= 0 || N <= 0) return 0;
-  if (N % 8 == 0 && ld % 8 == 0 && aligned16(dy, out)) {
+extern "C" int opk_colsum(const void* dy, float* out, int T, int N, int64_t ld, int batch, int64_t out_stride, void* stream) {
+  if (T <= 0 || N <= 0 || batch <= 0) return 0;
+  if (batch > 65535) return -1;
+  if (N % 8 == 0 && ld % 8 == 0 && aligned16(dy, out) && (batch == 1 || out_stride % 4 == 0)) {
     // about one CTA per SM over all column blocks, at least 8 rows (one per warp) each
     const int cols = (N + 255) / 256;
     int rows = (int)(((long long)T * cols + 147) / 148);
     rows = rows < 8 ? 8 : (rows + 7) / 8 * 8;
-    colsum_vec_kernel<<<dim3(cols, (T + rows - 1) / rows), 256, 0, ST(stream)>>>(BF(dy), out, T, N, ld, rows);
+    colsum_vec_kernel<<<dim3(cols, (T + rows - 1) / rows, batch), 256, 0, ST(stream)>>>(BF(dy), out, T, N, ld, rows, out_stride);
     OPK_LAUNCH_CHECK();
     return 0;
   }
-  dim3 grid((N + 127) / 128, T < 32 ? T : 32);
-  colsum_kernel<<<grid, 128, 0, ST(stream)>>>(BF(dy), out, T, N, ld);
+  dim3 grid((N + 127) / 128, T < 32 ? T : 32, batch);
+  colsum_kernel<<<grid, 128, 0, ST(stream)>>>(BF(dy), out, T, N, ld, out_stride);
   OPK_LAUNCH_CHECK();
   return 0;
 }
 extern "C" int opk_embedding_add_rows(const int32_t* tok, const int32_t* rep, const float* gc, void* dense, int T, int D,
-                                      void* stream) {
-  if (T <= 0) return 0;
-  emb_add_rows_kernel<<<T, 256, 0, ST(stream)>>>(tok, rep, gc, BFM(dense), D);
+                                      int batch, int64_t dense_stride, void* stream) {
+  if (T <= 0 || batch <= 0) return 0;
+  if (batch > 65535) return -1;
+  emb_add_rows_kernel<<<dim3(T, batch), 256, 0, ST(stream)>>>(tok, rep, gc, BFM(dense), T, D, dense_stride);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1592,9 +1628,9 @@ extern "C" int opk_embedding_bwd_compact_noalloc(const int32_t* tok, const void*
   // (possibly one that was interrupted) left behind
   emb_reset_kernel<<<(T + 255) / 256, 256, 0, st>>>(tok, first_pos, T, vocab);
   emb_first_pos_kernel<<<(T + 255) / 256, 256, 0, st>>>(tok, first_pos, T, vocab);
-  emb_scatter_kernel<<<T, 256, 0, st>>>(tok, BF(dx), first_pos, rep, gc, D, vocab);
+  emb_scatter_kernel<<<T, 256, 0, st>>>(tok, BF(dx), first_pos, rep, gc, T, D, vocab);
   emb_reset_kernel<<<(T + 255) / 256, 256, 0, st>>>(tok, first_pos, T, vocab);
-  if (sumsq) sumsq_kernel<true, true><<<grid_for((long long)T * D, NT, 148 * 4), NT, 0, st>>>(gc, (long long)T * D, sumsq);
+  if (sumsq) sumsq_kernel<true, true><<<grid_for((long long)T * D, NT, 148 * 4), NT, 0, st>>>(gc, (long long)T * D, sumsq, 0);
   OPK_LAUNCH_CHECK();
   return 0;
 }

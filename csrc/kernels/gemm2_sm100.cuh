@@ -69,7 +69,7 @@ struct Gemm2Cfg {
   static constexpr int B_BYTES = (BN / 2) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;          // 32 KB
   static constexpr int STAGES = 6;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 8 * kEpiScratch;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 8 * kEpiScratch + 8 * 8 * 8;
   static constexpr int TMEM_COLS = 2 * BN;                        // two accumulator buffers
 };
 
@@ -101,7 +101,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint64_t* tempty = tfull + 2;                                                     // used in the even CTA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  double* sq_slots = reinterpret_cast<double*>(tmem_slot + 2);      // EPI_SUMSQ: one per epilogue warp
+  double* sq_slots = reinterpret_cast<double*>(smem + STAGES * Cfg::STAGE_BYTES + 256 + 8 * kEpiScratch);   // EPI_SUMSQ: [warp][kSqSums]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
@@ -271,7 +271,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int c_begin = ((warp - 2) >> 2) * (BN / CSPLIT), c_end = c_begin + BN / CSPLIT;
     uint8_t* scratch = smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * kEpiScratch;
     int it = 0;
-    double sq_total = 0.0;
+    double* sq = sq_slots + (warp - 2) * kSqSums;
+    if (EPI == EPI_SUMSQ) epi_zero_sq(sq);
     for (int tile = cluster_id; tile < total; tile += n_clusters, ++it) {
       const int b = tile / per_batch;
       const int r = tile - b * per_batch;
@@ -293,9 +294,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         if (lane == 0) mbar_arrive_cluster_relaxed(mapa_u32(smem_u32(&tempty[buf]), 0));
       });
       epi_end<EPI>(p, e, tn * CSPLIT + c_begin / (BN / CSPLIT), tiles_n * CSPLIT);
-      if (EPI == EPI_SUMSQ) epi_add_sq(p, e, b, sq_total);
+      if (EPI == EPI_SUMSQ) epi_add_sq(p, e, b, sq);
     }
-    if (EPI == EPI_SUMSQ && lane == 0) sq_slots[warp - 2] = sq_total;
   }
 
   // ---------------------------------------------------------------- teardown
@@ -306,7 +306,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tc_fence_after();
     tmem_dealloc2(tmem_base, Cfg::TMEM_COLS);
   }
-  if (EPI == EPI_SUMSQ && threadIdx.x == 0) epi_flush_sq(p, sq_slots, gemm2_epi_warps(EPI, VARIANT));
+  if (EPI == EPI_SUMSQ) epi_flush_sq(p, sq_slots, gemm2_epi_warps(EPI, VARIANT));
   if (threadIdx.x == 0 && *abort_flag && p.err) atomicExch(p.err, 1);
 }
 

@@ -96,7 +96,7 @@ struct GemmCfg {
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (BN == 256) ? 4 : 6;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + 8 * kEpiScratch;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + 8 * kEpiScratch + 8 * 8 * 8 /*norm sums*/;
   static constexpr int TMEM_COLS = 2 * BN;
 };
 
@@ -432,20 +432,31 @@ __device__ __forceinline__ void epi_end(const GemmParams& p, const EpiState& e, 
 // Squared norm of one finished tile. All tiles of a launch usually add to ONE double, and atomics on one address are served
 // one after the other (about 5 ns each: 4,096 of them, one per tile and warp of a 16384 x 2048 gradient, took 20 us, and
 // the 65,536 of an OLMoE expert gradient 320 us, longer than the products). So lane 0 of every epilogue warp keeps a
-// running double, and the CTA adds its warps' sums once, when it is done (epi_flush_sq). Only launches with one sum per
-// batch entry (sumsq_stride != 0) add per tile.
-__device__ __forceinline__ void epi_add_sq(const GemmParams& p, const EpiState& e, int b, double& total) {
+// running double per sum in shared memory (`slots`, kSqSums per warp), and the CTA adds its warps' sums once, when it is done
+// (epi_flush_sq). Only launches with more than kSqSums sums (one per batch entry, sumsq_stride != 0) add per tile.
+constexpr int kSqSums = 8;
+__device__ __forceinline__ int sq_sums(const GemmParams& p) { return p.sumsq_stride == 0 ? 1 : p.batch; }
+__device__ __forceinline__ void epi_zero_sq(double* slots) {
+  const int lane = threadIdx.x & 31;
+  if (lane < kSqSums) slots[lane] = 0.0;
+  __syncwarp();
+}
+__device__ __forceinline__ void epi_add_sq(const GemmParams& p, const EpiState& e, int b, double* slots) {
   float w = e.sq;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-  if (p.sumsq_stride == 0 || p.batch == 1) total += (double)w;
-  else if ((threadIdx.x & 31) == 0) atomicAdd(&p.sumsq[b * p.sumsq_stride], (double)w);
+  if ((threadIdx.x & 31) == 0) {
+    if (sq_sums(p) <= kSqSums) slots[p.sumsq_stride == 0 ? 0 : b] += (double)w;
+    else atomicAdd(&p.sumsq[b * p.sumsq_stride], (double)w);
+  }
 }
-// Call between the warps' stores to `slots` (one per epilogue warp) and their reuse: after a CTA barrier, by one thread.
-__device__ __forceinline__ void epi_flush_sq(const GemmParams& p, const double* slots, int n) {
+// After a CTA barrier behind the warps' last tiles, by the first kSqSums threads: `slots` of all `warps` epilogue warps.
+__device__ __forceinline__ void epi_flush_sq(const GemmParams& p, const double* slots, int warps) {
+  const int n = sq_sums(p);
+  if (n > kSqSums || (int)threadIdx.x >= n) return;
   double t = 0.0;
-  for (int i = 0; i < n; ++i) t += slots[i];
-  if (t != 0.0) atomicAdd(p.sumsq, t);
+  for (int i = 0; i < warps; ++i) t += slots[i * kSqSums + threadIdx.x];
+  if (t != 0.0) atomicAdd(p.sumsq + threadIdx.x, t);
 }
 
 // Columns [c_begin, c_end) of one accumulator tile, read from TMEM (tmem_tile = lane-adjusted address of the tile).
@@ -511,7 +522,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  double* sq_slots = reinterpret_cast<double*>(tmem_slot + 2);      // EPI_SUMSQ: one per epilogue warp
+  double* sq_slots = reinterpret_cast<double*>(smem + STAGES * Cfg::STAGE_BYTES + 256 + 8 * kEpiScratch);   // EPI_SUMSQ: [warp][kSqSums]
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -633,7 +644,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int c_begin = ((warp - 2) >> 2) * (BN / CSPLIT), c_end = c_begin + BN / CSPLIT;
     uint8_t* scratch = smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * kEpiScratch;
     int it = 0;
-    double sq_total = 0.0;
+    double* sq = sq_slots + (warp - 2) * kSqSums;
+    if (EPI == EPI_SUMSQ) epi_zero_sq(sq);
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
       const int b = tile / per_batch;
       const int r = tile - b * per_batch;
@@ -658,9 +670,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) mbar_arrive_relaxed(&tempty[buf]);
       });
       epi_end<EPI>(p, e, tn * CSPLIT + c_begin / (BN / CSPLIT), tiles_n * CSPLIT);
-      if (EPI == EPI_SUMSQ) epi_add_sq(p, e, b, sq_total);
+      if (EPI == EPI_SUMSQ) epi_add_sq(p, e, b, sq);
     }
-    if (EPI == EPI_SUMSQ && lane == 0) sq_slots[warp - 2] = sq_total;
   }
 
   // ---------------------------------------------------------------- teardown
@@ -670,7 +681,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
-  if (EPI == EPI_SUMSQ && threadIdx.x == 0) epi_flush_sq(p, sq_slots, gemm1_epi_warps(EPI));
+  if (EPI == EPI_SUMSQ) epi_flush_sq(p, sq_slots, gemm1_epi_warps(EPI));
   if (threadIdx.x == 0 && *abort_flag && p.err) atomicExch(p.err, 1);
 }
 

@@ -75,9 +75,10 @@ int opk_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int T, i
 // QKV activation. x and y may alias.
 int opk_rmsnorm_fwd_ld(const void* x, int64_t ldx, const void* w, void* y, int64_t ldy, float* rstd, int T, int D, float eps,
                        float w_offset, void* stream);
+// `batch` examples of T rows one after the other, each with a weight gradient of its own (dw_stride floats apart).
 int opk_rmsnorm_bwd_ld(const void* dy, int64_t ld_dy, const void* x, int64_t ldx, const void* w, const float* rstd,
                        const void* dres, void* dx_out, int64_t ld_dx, float* dw, float* workspace, int ws_rows, int T, int D,
-                       float w_offset, void* stream);
+                       float w_offset, int batch, int64_t dw_stride, void* stream);
 // s = x + r (stored to sum_out), then RMSNorm of s.
 int opk_add_rmsnorm_fwd(const void* x, const void* r, const void* w, void* sum_out, void* y, float* rstd, int T, int D,
                         float eps, float w_offset, void* stream);
@@ -90,7 +91,8 @@ int opk_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* r
 int opk_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int T, int D,
                       float eps, void* stream);
 int opk_layernorm_bwd(const void* dy, const void* x, const void* w, const float* mean, const float* rstd,
-                      const void* dres, void* dx_out, float* dw, float* db, int T, int D, void* stream);
+                      const void* dres, void* dx_out, float* dw, float* db, int T, int D, int batch, int64_t stride,
+                      void* stream);   // `batch` examples of T rows, gradients `stride` floats apart
 // In-place rotary embedding on the first n_rot_heads heads of each row (heads are head_dim wide, row pitch ld).
 // cs = [T][head_dim/2][2] fp32 (cos, sin); pos = optional int32 [T] row -> table row. sign = +1 forward, -1 backward.
 // Without pos, row t sits at position t % period (sequences of `period` rows one after the other; period 0: at position t).
@@ -109,15 +111,16 @@ int opk_glu_split_bwd(const void* dact, const void* gate, const void* up, void* 
 // GELU (GPT-2 "gelu_new" tanh form): y = gelu(x); backward dx = dy * gelu'(x).
 int opk_gelu_fwd(const void* x, void* y, int64_t n, void* stream);
 int opk_gelu_bwd(const void* dy, const void* x, void* dx, int64_t n, void* stream);
-// out[t] = table[tok[t]] (+ pos_table[t] when given)
+// out[t] = table[tok[t]] (+ pos_table[t] when given; with period > 0 pos_table[t % period]: sequences one after the other)
 int opk_embedding_fwd(const int32_t* tok, const void* table, const void* pos_table, void* out, int T, int D, int vocab,
-                      void* stream);
+                      int period, void* stream);
 // Per-example embedding gradient without a dense [V][D] buffer: rows with equal tokens are summed into the row of
 // their first occurrence. first_pos is an int32 [V] scratch that must hold INT32_MAX on entry and is restored.
 // Outputs: rep[T] (first position of the same token), gc[T][D] fp32 (zeroed here), sumsq += sum(bf16(gc)^2).
 // vocab is the length of first_pos; a token id outside [0, vocab) is skipped (rep[t] = -1, no row written).
+// `batch` examples of T tokens: every buffer holds one such part per example, sumsq one sum each.
 int opk_embedding_bwd_compact(const int32_t* tok, const void* dx, int32_t* first_pos, int32_t* rep, float* gc,
-                              double* sumsq, int T, int D, int vocab, void* stream);
+                              double* sumsq, int T, int D, int vocab, int batch, void* stream);
 // acc[tok[t]] += bf16(gc[t] * scale) for the representative rows (rep[t] == t).
 int opk_embedding_accumulate(const int32_t* tok, const int32_t* rep, const float* gc, const float* scale, float* acc,
                              int T, int D, void* stream);
@@ -132,36 +135,40 @@ int opk_lce_finalize(const float* pmax, const float* psum, const float* tgt, con
 // rows b*rows .. (b+1)*rows - 1), rstd [B * rows]; dw [B][D] fp32 is ACCUMULATED into (zero it first).
 int opk_rmsnorm_dw_per_example(const void* dy, const void* x, const float* rstd, float* dw, int B, int rows, int D, void* stream);
 // Per-example loss bookkeeping: ntok = max(1, number of labels >= 0); coef[t] = (label >= 0) / ntok, times *weight when
-// weight != NULL; *loss = sum_t nll[t] * coef[t]; *ntok (may be NULL) = ntok. One CTA.
+// weight != NULL; *loss = sum_t nll[t] * coef[t]; *ntok (may be NULL) = ntok. `batch` examples of T tokens, one CTA each.
 int opk_loss_coef(const int32_t* labels, const float* nll, const float* weight, float* coef, float* loss, float* ntok, int T,
-                  void* stream);
+                  int batch, void* stream);
 // Row-wise cross entropy over materialised logits (bf16 or fp32): nll[t], optional lse[t]; softcap / scale as LCE.
 int opk_cross_entropy_fwd(const void* logits, int is_fp32, const int32_t* labels, float* nll, float* lse, int T, int V,
                           int64_t ld, float scale, float softcap, void* stream);
 int opk_cross_entropy_bwd(const void* logits, int is_fp32, const int32_t* labels, const float* lse, const float* coef,
                           void* dlogits, int T, int V, int64_t ld, float scale, float softcap, void* stream);
-// sum(x^2) of a bf16/fp32 vector (x rounded to bf16 first when round_bf16) added to *sumsq (double).
-int opk_sumsq(const void* x, int is_fp32, int round_bf16, int64_t n, double* sumsq, void* stream);
+// sum(x^2) of a bf16/fp32 vector (x rounded to bf16 first when round_bf16) added to *sumsq (double). `batch` vectors of n
+// elements, `stride` elements (a multiple of 8) apart, with one sum each.
+int opk_sumsq(const void* x, int is_fp32, int round_bf16, int64_t n, double* sumsq, int batch, int64_t stride, void* stream);
 // fp32 rows -> bf16 at dst_base + offsets[r] (device int64 array), with sum of squares of the stored values: the first widths[r]
-// columns of row r (device int32 array, D = row pitch of src); widths == NULL: all D of every row.
+// columns of row r (device int32 array, D = row pitch of src); widths == NULL: all D of every row. `batch` examples of R rows,
+// destinations dst_stride elements apart, one sum each.
 int opk_scatter_rows_cast_sumsq(const float* src, void* dst_base, const int64_t* offsets, const int32_t* widths, int R, int D,
-                                double* sumsq, void* stream);
-// out[n] += sum_t dy[t][n] (out fp32, zeroed by the caller)
-int opk_colsum(const void* dy, float* out, int T, int N, int64_t ld, void* stream);
-// Tied embeddings: dense[tok[t]] += gc[t] for first-occurrence rows (bf16 read-modify-write).
-int opk_embedding_add_rows(const int32_t* tok, const int32_t* rep, const float* gc, void* dense, int T, int D,
-                           void* stream);
+                                double* sumsq, int batch, int64_t dst_stride, void* stream);
+// out[n] += sum_t dy[t][n] (out fp32, zeroed by the caller); `batch` examples of T rows, sums out_stride floats apart
+int opk_colsum(const void* dy, float* out, int T, int N, int64_t ld, int batch, int64_t out_stride, void* stream);
+// Tied embeddings: dense[tok[t]] += gc[t] for first-occurrence rows (bf16 read-modify-write); `batch` examples of T tokens,
+// matrices dense_stride elements apart.
+int opk_embedding_add_rows(const int32_t* tok, const int32_t* rep, const float* gc, void* dense, int T, int D, int batch,
+                           int64_t dense_stride, void* stream);
 
 // ---- causal GQA flash attention on the fused projection buffer (csrc/kernels/attention_sm100.cu) -------------
 // qkv bf16 [T][(H+2KV)*hd] (row pitch ld), out bf16 [T][H*hd] (row pitch ldo), lse fp32 [H][T]. hd in {64, 128}.
-int opk_attn_fwd(const void* qkv, void* out, float* lse, int T, int H, int KV, int hd, int64_t ld, int64_t ldo,
+// n_seq sequences of T rows one after the other; every buffer holds one such part per sequence (dsum: of each of its halves).
+int opk_attn_fwd(const void* qkv, void* out, float* lse, int T, int H, int KV, int hd, int n_seq, int64_t ld, int64_t ldo,
                  float scale, int32_t* err, void* stream);
 // Backward: dqkv (same layout as qkv) receives dQ, dK, dV. dsum is a 16-byte-aligned fp32 work buffer of
 // 2 * H * T64 elements, T64 = T rounded up to a multiple of 64 (rowsum(dO * O), then -lse * log2 e).
 // part (optional, 16-byte aligned, 2 * (H/KV) * T * KV*hd floats): with grouped-query attention the dK / dV kernel
 // then runs one CTA per query head, writes fp32 partials there and a reduce kernel sums them in a fixed order.
 int opk_attn_bwd(const void* qkv, const void* out, const void* dout, const float* lse, float* dsum, void* dqkv,
-                 float* part, int T, int H, int KV, int hd, int64_t ld, int64_t ldo, float scale, int32_t* err,
+                 float* part, int T, int H, int KV, int hd, int n_seq, int64_t ld, int64_t ldo, float scale, int32_t* err,
                  void* stream);
 
 // ---- multi-tensor kernels of the functional API (csrc/kernels/multi_tensor.cu) ---------------------------------
@@ -261,9 +268,10 @@ int opk_moe_combine_bwd(const void* dy, const void* y, const int32_t* dest, int 
 
 // ---- DP clipping / noise / optimizer (csrc/kernels/dp_step.cu) ---------------------------------------------
 // scale = guarded min(1, C / sqrt(sumsq)) (fixed) or R / (sqrt(sumsq) + gamma) (auto); see dp_step.cu.
-// Also: norm_out[0] = sqrt(sumsq), counters[0] += (norm > C), and *sumsq is reset to 0 when reset != 0.
+// Also: norm_out[0] = sqrt(sumsq), counters[0] += (norm > C), and *sumsq is reset to 0 when reset != 0. `batch` (1 .. 32)
+// consecutive sums, factors and norms.
 int opk_clip_scale(double* sumsq, float clip, int mode_auto, float gamma, int n_leaves, int64_t widest_leaf,
-                   float* scale_out, float* norm_out, int32_t* counters, int reset, void* stream);
+                   float* scale_out, float* norm_out, int32_t* counters, int reset, int batch, void* stream);
 // acc[i] += float(bf16(float(g[i]) * scale)) with bf16 subnormals that rounded up flushed to zero.
 int opk_clip_accumulate(const void* g, const float* scale, float* acc, int64_t n, void* stream);
 // Same with overwrite != 0 meaning acc = bf16(g * scale) (first example of a step: no separate zeroing pass).

@@ -56,14 +56,23 @@ class DecoderRuntime:
         # With two slots the clipped accumulation of example i can run on a side stream while example i+1 is
         # being computed into the other slot.
         self.n_slots = n_slots
-        self.Gs = [self._alloc(self.layout.dense_total, dtype=_bf16, name=f"grad_slot{i}") for i in range(n_slots)]
+        # The slots are one buffer, so that one launch can write the gradients of several (guard bands need them apart).
+        if canaries is None:
+            self.G_all = torch.empty(n_slots, self.layout.dense_total, dtype=_bf16, device=self.device)
+            self.Gs = list(self.G_all.unbind(0))
+        else:
+            self.G_all = None
+            self.Gs = [self._alloc(self.layout.dense_total, dtype=_bf16, name=f"grad_slot{i}") for i in range(n_slots)]
         self.gs = [self.layout.views(G_, dense_only=True) for G_ in self.Gs]
+        self._g_stacks: dict[tuple[int, int], dict] = {}
         self.attn_impl = attn_impl
-        self.sumsqs = [torch.zeros(1, dtype=torch.float64, device=self.device) for _ in range(n_slots)]
-        self.scales = [torch.zeros(1, dtype=torch.float32, device=self.device) for _ in range(n_slots)]
-        self.norms = [torch.zeros(1, dtype=torch.float32, device=self.device) for _ in range(n_slots)]
+        self.sumsq_all = torch.zeros(n_slots, dtype=torch.float64, device=self.device)
+        self.scale_all = torch.zeros(n_slots, dtype=torch.float32, device=self.device)
+        self.norm_all = torch.zeros(n_slots, dtype=torch.float32, device=self.device)
+        self.sumsqs, self.scales, self.norms = (list(t.split(1)) for t in (self.sumsq_all, self.scale_all, self.norm_all))
         self.clip_count = torch.zeros(1, dtype=torch.int32, device=self.device)
-        self._ws: dict[int, dict] = {}
+        self._ws: dict[tuple[int, int], dict] = {}
+        self._parts: dict[tuple, dict] = {}
         self._rope = None
         # weights to pull from their owner during the NEXT forward pass (name -> the owner's copy, a peer-mapped
         # tensor): the consuming GEMM copies the matrix into this rank's replica band by band while it multiplies
@@ -81,6 +90,7 @@ class DecoderRuntime:
         self._vec_row = {n: i for i, n in enumerate(self._vec_names)}
         d = cfg.d_model
         self._vec_width = max([d] + [self.layout.slot(n).numel for n in self._vec_names])
+        self._norm_scratch: dict[int, torch.Tensor] = {}
         self._n_leaves = len(self.layout.slots)
         self._widest = max(s.numel for s in self.layout.slots)
 
@@ -92,6 +102,11 @@ class DecoderRuntime:
     @property
     def g(self):
         return self.gs[0]
+
+    def can_join(self) -> bool:
+        """Whether several sequences can go through the model in one pass: dense blocks, native attention, slots in one buffer."""
+        impl = A.resolve_impl(self.cfg.head_dim) if self.attn_impl == "auto" else self.attn_impl
+        return self.G_all is not None and not self.cfg.n_experts and impl == "flash" and self.device.type == "cuda"
 
     @property
     def sumsq(self):
@@ -111,12 +126,18 @@ class DecoderRuntime:
         return torch.empty(*shape, dtype=dtype, device=self.device)
 
     # ------------------------------------------------------------------ workspaces
-    def workspace(self, T: int) -> dict:
-        ws = self._ws.get(T)
+    def workspace(self, T: int, n: int = 1) -> dict:
+        """Buffers for sequences of ``T`` tokens, ``n`` of them going through the model together: one set of ``n * T`` rows
+        per length. A smaller ``n`` gets views of a larger set."""
+        ws = self._ws.get((T, n))
         if ws is not None:
             return ws
+        wider = [m for t, m in self._ws if t == T and m > n]
+        if wider:
+            return self.part(self._ws[(T, max(wider))], n)
         cfg, dev = self.cfg, self.device
         d, F, L = cfg.d_model, cfg.ffn, cfg.n_layers
+        seq, T = T, n * T
 
         def e(*shape, dtype=_bf16):
             return self._alloc(*shape, dtype=dtype, name=f"workspace[T={T}]#{len(self.canaries) if self.canaries is not None else 0}")
@@ -153,13 +174,15 @@ class DecoderRuntime:
             "dx": e(T, d), "dx2": e(T, d), "dact": e(T, max(F, 8)), "dqkv": e(T, cfg.qkv_dim),
             "dwide": e(T, max(2 * F if cfg.act in ("swiglu", "geglu") else F, 8)),
             "dattn": e(T, cfg.n_heads * cfg.head_dim),
-            "vec": torch.zeros(len(self._vec_names), self._vec_width, dtype=torch.float32, device=dev),
-            "embs": [K.EmbeddingGradWorkspace(cfg.vocab_size, T, d, dev) for _ in range(self.n_slots)],
-            "toks": [torch.zeros(T, dtype=torch.int32, device=dev) for _ in range(self.n_slots)],
+            "vec": torch.zeros(n, len(self._vec_names), self._vec_width, dtype=torch.float32, device=dev),
+            "emb_all": K.EmbeddingGradWorkspace(cfg.vocab_size, seq, d, dev, examples=self.n_slots),
+            "tok_all": torch.zeros(self.n_slots, seq, dtype=torch.int32, device=dev),
             "labels": torch.zeros(T, dtype=torch.int32, device=dev),
-            "loss": torch.zeros(1, dtype=torch.float32, device=dev), "ntok": torch.zeros(1, dtype=torch.float32, device=dev),
-            "coef": torch.zeros(T, dtype=torch.float32, device=dev),
+            "loss": torch.zeros(n, dtype=torch.float32, device=dev), "ntok": torch.zeros(n, dtype=torch.float32, device=dev),
+            "coef": torch.zeros(T, dtype=torch.float32, device=dev), "n": n, "key": (seq, n),
         }
+        ws["embs"] = [ws["emb_all"].examples(j, 1) for j in range(self.n_slots)]
+        ws["toks"] = list(ws["tok_all"].unbind(0))
         ws["vec_offsets"] = torch.tensor([self.layout.slot(n).offset for n in self._vec_names], dtype=torch.int64,
                                          device=dev)
         widths = [self.layout.slot(n).numel for n in self._vec_names]
@@ -170,12 +193,30 @@ class DecoderRuntime:
             R, I = layers[0]["plan"].R, cfg.expert_ffn
             ws.update(dye=e(R, d), dgu=e(R, 2 * I).zero_(), dxs=e(R, d).zero_(),
                       dwts=e(T, cfg.top_k, dtype=torch.float32), drl=e(T, cfg.n_experts))
-        self._ws[T] = ws
+        self._ws[(seq, n)] = ws
         return ws
 
-    def _logits_buffer(self, ws: dict, T: int) -> torch.Tensor | None:
+    def part(self, ws: dict, n: int) -> dict:
+        """The first ``n`` sequences of a workspace (views)."""
+        if n == ws["n"]:
+            return ws
+        out = self._parts.get((ws["key"], n))
+        if out is not None:
+            return out
+        out = self._parts[(ws["key"], n)] = dict(ws, n=n)
+        rows = n * ws["key"][0]
+        out["layers"] = [{k: v[:rows] for k, v in a.items()} for a in ws["layers"]]
+        for k in ("x_last", "xf", "pmax", "psum", "tgt", "dlogits", "dx", "dx2", "dact", "dqkv", "dwide", "dattn", "labels", "coef"):
+            out[k] = ws[k][:rows]
+        for k in ("vec", "loss", "ntok"):
+            out[k] = ws[k][:n]
+        return out
+
+    def _logits_buffer(self, ws: dict) -> torch.Tensor | None:
         """fp32 logits that the loss leaves for its backward pass, which then needs no second product with the head. ``None``,
         for good, where the product is the cheaper one or they would take more than a quarter of the memory that is free."""
+        ws = self._ws[ws["key"]]          # the whole set, T its rows
+        T = ws["labels"].numel()
         if "z" in ws or self.device.type != "cuda":
             return ws.get("z")
         if torch.cuda.is_current_stream_capturing():
@@ -186,7 +227,7 @@ class DecoderRuntime:
         ws["z"] = None
         if 16 * n <= free and G.lce_keeps_logits(T, self.cfg.vocab_size, self.cfg.d_model):
             try:
-                ws["z"] = self._alloc(n, dtype=torch.float32, name=f"logits[T={T}]")
+                ws["z"] = self._alloc(n, dtype=torch.float32, name=f"logits[rows={T}]")
             except torch.cuda.OutOfMemoryError:
                 pass
         return ws["z"]
@@ -199,19 +240,42 @@ class DecoderRuntime:
         return self._rope
 
     def _vec(self, ws, name: str) -> torch.Tensor:
-        n = self.layout.slot(name).numel
-        return ws["vec"][self._vec_row[name], :n]
+        """Gradient of a vector parameter: ``[numel]``, or ``[n, numel]`` for ``n`` sequences."""
+        v = ws["vec"][:, self._vec_row[name], : self.layout.slot(name).numel]
+        return v[0] if ws["n"] == 1 else v
+
+    def _scratch(self, ws: dict) -> torch.Tensor:
+        """Scratch of the norm backward kernels, kept per number of sequences: a graph may hold on to it."""
+        n = ws["n"]
+        s = self._norm_scratch.get(n)
+        if s is None:
+            s = self._norm_scratch[n] = K.rmsnorm_bwd_scratch(self._vec_width, n, self.device)
+        return s
 
     # ------------------------------------------------------------------ second stream for weight gradients
-    def _wgrad(self, dy, x, out, sumsq=None) -> None:
-        """``out = dy^T x`` (+ squared norm) ordered after everything issued so far, on the weight-gradient stream."""
-        side = self._wstream
+    def _wgrad(self, dy, x, out, sumsq=None, main: bool = False) -> None:
+        """``out = dy^T x`` (+ squared norm) ordered after everything issued so far, on the weight-gradient stream (``main``: on
+        the current one). ``out [n, N, K]``: the rows are ``n`` sequences, each with a gradient (and norm) of its own."""
+        if out.dim() == 3:
+            dy, x = dy.unflatten(0, (out.shape[0], -1)), x.unflatten(0, (out.shape[0], -1))
+        side = None if main else self._wstream
         if side is None:
             G.linear_wgrad(dy, x, out=out, sumsq=sumsq)
             return
         side.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(side):
             G.linear_wgrad(dy, x, out=out, sumsq=sumsq)
+
+    def _grads(self, slot: int, n: int) -> tuple[dict, torch.Tensor]:
+        """Gradient views and squared norms of slots ``slot .. slot+n-1``; several slots: stacked, ``[n, *shape]``."""
+        if n == 1:
+            return self.gs[slot], self.sumsqs[slot]
+        g = self._g_stacks.get((slot, n))
+        if g is None:
+            part = self.G_all[slot : slot + n]
+            g = self._g_stacks[(slot, n)] = {s.name: part[:, s.offset : s.offset + s.numel].unflatten(1, s.shape)
+                                             for s in self.layout.slots if s.offset < self.layout.dense_total}
+        return g, self.sumsq_all[slot : slot + n]
 
     def _wgrad_call(self, fn) -> None:
         """Runs ``fn`` (a weight-gradient launch) on the weight-gradient stream, ordered after everything issued so far."""
@@ -241,7 +305,7 @@ class DecoderRuntime:
         cfg, w = self.cfg, self.w
         if cfg.norm == "rms":
             return K.rmsnorm_bwd(dy, x, w[prefix + ".weight"], stats[0], dres=dres, dw=self._vec(ws, prefix + ".weight"),
-                                 out=out)
+                                 out=out, scratch=self._scratch(ws))
         return K.layernorm_bwd(dy, x, w[prefix + ".weight"], stats[0], stats[1], dres=dres,
                                dw=self._vec(ws, prefix + ".weight"), db=self._vec(ws, prefix + ".bias"), out=out)
 
@@ -265,15 +329,19 @@ class DecoderRuntime:
 
     # ------------------------------------------------------------------ forward
     def forward(self, tok: torch.Tensor, labels: torch.Tensor | None, ws: dict | None = None, z: torch.Tensor | None = None):
-        """Runs the decoder on one sequence. Returns ``(per-token nll [T], lse, saved)``; ``z``: buffer for the logits.
+        """Runs the decoder on one sequence, or on the ``ws["n"]`` sequences of equal length that ``tok`` holds one after the
+        other. Returns ``(per-token nll [T], lse, saved)``; ``z``: buffer for the logits.
 
         ``labels`` are already shifted (``labels[t]`` is the target of position ``t``; negative = ignored).
         """
         cfg, w = self.cfg, self.w
         T = tok.numel()
         ws = ws or self.workspace(T)
+        n_seq = ws["n"]
+        seq = T // n_seq
+        period = seq if n_seq > 1 else 0
         H, KV, hd = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim
-        x = K.embedding_fwd(tok, w["embed"], w.get("wpe") if cfg.pos == "learned" else None, out=ws["layers"][0]["x"])
+        x = K.embedding_fwd(tok, w["embed"], w.get("wpe") if cfg.pos == "learned" else None, out=ws["layers"][0]["x"], period=period)
         saved = []
         for li in range(cfg.n_layers):
             a = ws["layers"][li]
@@ -300,8 +368,8 @@ class DecoderRuntime:
                 _, rk = K.rmsnorm_fwd(a["qk_raw"][:, nq:], w[p + "k_norm.weight"], cfg.norm_eps, out=a["qkv"][:, nq : nq + nk])
                 stq = (rq, rk)
             if cfg.pos == "rope":
-                K.rope_(a["qkv"], self._rope_table(T), H + KV, hd)
-            _, actx = A.attention_fwd(a["qkv"], H, KV, hd, self.attn_impl, out=a["attn"])
+                K.rope_(a["qkv"], self._rope_table(seq), H + KV, hd, period=period)
+            _, actx = A.attention_fwd(a["qkv"], H, KV, hd, self.attn_impl, out=a["attn"], n_seq=n_seq)
             # output projection with the residual add fused into the GEMM epilogue
             wsrc, stg = self._wop(p + "wo")
             G.gemm(a["attn"], wsrc, out=a["x_mid"], residual=x, bias=w.get(p + "bo"), stage=stg)
@@ -361,16 +429,21 @@ class DecoderRuntime:
         ``before_wgrad`` (optional callable) runs once, after the forward pass and right before the first kernel that
         writes the slot's gradient buffer: the place to wait for a consumer of the buffer's previous contents.
 
+        A workspace for ``n`` sequences (``workspace(T, n)``): ``tok`` and ``labels`` hold them one after the other, their
+        gradients go to slots ``slot .. slot+n-1``. Every kernel treats a sequence as it would alone.
+
         The example loss is the mean NLL over supervised tokens (per-example divisor, as
         packages/opake-alignment/src/opake/api/alignment/sft/loss/_nll.py:43-88).
         """
-        cfg, w, g = self.cfg, self.w, self.gs[slot]
-        sumsq, emb_ws = self.sumsqs[slot], None
+        cfg, w = self.cfg, self.w
         T = tok.numel()
         ws = ws or self.workspace(T)
-        emb_ws = ws["embs"][slot]
+        n = ws["n"]
+        seq = T // n
+        g, sumsq = self._grads(slot, n)
+        emb_ws = ws["emb_all"].examples(slot, n)
         H, KV, hd = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim
-        z = self._logits_buffer(ws, T)
+        z = self._logits_buffer(ws)
         nll, lse, (saved, stf) = self.forward(tok, labels, ws, z)
         coef, loss, ntok = ws["coef"], ws["loss"], ws["ntok"]
         K.loss_coef(labels, nll, coef, loss, ntok, weight=loss_weight)
@@ -431,12 +504,12 @@ class DecoderRuntime:
                 dxn2 = G.gemm(dgu, w[p + "wgu"], b_mn=True, out=ws["dx2"])
                 self._wgrad_join()            # the norm backward below overwrites dx in place
             else:
-                G.linear_wgrad(dx, a["act"], out=g[p + "wproj"], sumsq=sumsq)
+                self._wgrad(dx, a["act"], g[p + "wproj"], sumsq, main=True)
                 if cfg.bias:
                     K.colsum_(dx, self._vec(ws, p + "bproj"))
                 dact = G.gemm(dx, w[p + "wproj"], b_mn=True, out=ws["dact"])
                 dfc = K.gelu_bwd(dact, a["fc"], out=ws["dwide"])
-                G.linear_wgrad(dfc, a["xn2"], out=g[p + "wfc"], sumsq=sumsq)
+                self._wgrad(dfc, a["xn2"], g[p + "wfc"], sumsq, main=True)
                 if cfg.bias:
                     K.colsum_(dfc, self._vec(ws, p + "bfc"))
                 dxn2 = G.gemm(dfc, w[p + "wfc"], b_mn=True, out=ws["dx2"])
@@ -449,7 +522,7 @@ class DecoderRuntime:
             dqkv = ws["dqkv"]
             A.attention_bwd(dattn, a["qkv"], a["attn"], actx, H, KV, hd, dqkv)
             if cfg.pos == "rope":
-                K.rope_(dqkv, self._rope_table(T), H + KV, hd, backward=True)
+                K.rope_(dqkv, self._rope_table(seq), H + KV, hd, backward=True, period=seq if n > 1 else 0)
             if cfg.qk_norm == "head":
                 nq, nk = H * hd, KV * hd
                 dq_c = a["qk_raw"].view(-1)[: T * nq].view(T, nq)           # the normalised copies are dead by now
@@ -457,17 +530,17 @@ class DecoderRuntime:
                 dq_c.copy_(dqkv[:, :nq])
                 dk_c.copy_(dqkv[:, nq : nq + nk])
                 K.rmsnorm_bwd(dq_c.view(T * H, hd), a["q_raw"].view(T * H, hd), w[p + "q_norm.weight"], stq[0],
-                              dw=self._vec(ws, p + "q_norm.weight"), out=dq_c.view(T * H, hd))
+                              dw=self._vec(ws, p + "q_norm.weight"), scratch=self._scratch(ws), out=dq_c.view(T * H, hd))
                 K.rmsnorm_bwd(dk_c.view(T * KV, hd), a["k_raw"].view(T * KV, hd), w[p + "k_norm.weight"], stq[1],
-                              dw=self._vec(ws, p + "k_norm.weight"), out=dk_c.view(T * KV, hd))
+                              dw=self._vec(ws, p + "k_norm.weight"), scratch=self._scratch(ws), out=dk_c.view(T * KV, hd))
                 dqkv[:, :nq].copy_(dq_c)
                 dqkv[:, nq : nq + nk].copy_(dk_c)
             elif cfg.qk_norm:      # in place on the query and key columns of dqkv
                 nq, nk = H * hd, KV * hd
                 K.rmsnorm_bwd(dqkv[:, :nq], a["qk_raw"][:, :nq], w[p + "q_norm.weight"], stq[0],
-                              dw=self._vec(ws, p + "q_norm.weight"), out=dqkv[:, :nq])
+                              dw=self._vec(ws, p + "q_norm.weight"), scratch=self._scratch(ws), out=dqkv[:, :nq])
                 K.rmsnorm_bwd(dqkv[:, nq : nq + nk], a["qk_raw"][:, nq:], w[p + "k_norm.weight"], stq[1],
-                              dw=self._vec(ws, p + "k_norm.weight"), out=dqkv[:, nq : nq + nk])
+                              dw=self._vec(ws, p + "k_norm.weight"), scratch=self._scratch(ws), out=dqkv[:, nq : nq + nk])
             self._wgrad(dqkv, a["xn"], g[p + "wqkv"], sumsq)
             if cfg.bias or cfg.qkv_bias:
                 K.colsum_(dqkv, self._vec(ws, p + "bqkv"))
@@ -477,23 +550,31 @@ class DecoderRuntime:
 
         self._wgrad_join()
         # ---- embeddings
-        K.embedding_bwd_compact(tok, dx, emb_ws, None if cfg.tie_embeddings else sumsq)
+        K.embedding_bwd_compact(tok, dx, emb_ws, None if cfg.tie_embeddings else sumsq, examples=n)
         if cfg.pos == "learned":
             gw = g["wpe"]
-            gw[:T].copy_(dx)
-            gw[T:].zero_()
-            K.sumsq_(gw[:T], sumsq)
+            if n > 1:
+                gw[:, :seq].copy_(dx.unflatten(0, (n, seq)))
+                gw[:, seq:].zero_()
+                K.sumsq_(gw[:, :seq], sumsq)
+            else:
+                gw[:T].copy_(dx)
+                gw[T:].zero_()
+                K.sumsq_(gw[:T], sumsq)
         if cfg.tie_embeddings:
-            K.embedding_add_rows(tok, emb_ws, ghead, T)
+            K.embedding_add_rows(tok, emb_ws, ghead, seq)
             K.sumsq_(ghead, sumsq)
         # ---- vector parameters (norm weights, biases): fp32 rows -> bf16 slots of G, with their norm
-        K.scatter_rows_cast_sumsq(ws["vec"], self.Gs[slot], ws["vec_offsets"], sumsq, ws["vec_widths"])
+        if n > 1:
+            K.scatter_rows_cast_sumsq(ws["vec"], self.G_all[slot : slot + n], ws["vec_offsets"], sumsq, ws["vec_widths"])
+        else:
+            K.scatter_rows_cast_sumsq(ws["vec"][0], self.Gs[slot], ws["vec_offsets"], sumsq, ws["vec_widths"])
         return ExampleStats(loss=loss, n_tokens=ntok)
 
     # ------------------------------------------------------------------ clip + accumulate
-    def clip_factor(self, clip: float, *, auto: bool = False, gamma: float = 0.01, slot: int = 0) -> None:
-        """Turns the slot's squared norm into the guarded clip factor (device scalar) and resets the accumulator."""
-        K.clip_scale(self.sumsqs[slot], clip, scale_out=self.scales[slot], norm_out=self.norms[slot],
+    def clip_factor(self, clip: float, *, auto: bool = False, gamma: float = 0.01, slot: int = 0, n: int = 1) -> None:
+        """Turns the squared norms of ``n`` slots into the guarded clip factors (device scalars) and resets the accumulators."""
+        K.clip_scale(self.sumsq_all[slot : slot + n], clip, scale_out=self.scales[slot], norm_out=self.norms[slot],
                      counters=self.clip_count, auto=auto, gamma=gamma, n_leaves=self._n_leaves,
                      widest_leaf=self._widest, reset=True)
 

@@ -54,11 +54,11 @@ PROTOTYPES: dict = {
     "opk_lce_grad": (I, [P, P, P, P, P, L, I, I, F, P]),
     "opk_rmsnorm_fwd": (I, [P, P, P, P, I, I, F, F, P]),
     "opk_rmsnorm_fwd_ld": (I, [P, L, P, P, L, P, I, I, F, F, P]),
-    "opk_rmsnorm_bwd_ld": (I, [P, L, P, L, P, P, P, P, L, P, P, I, I, I, F, P]),
+    "opk_rmsnorm_bwd_ld": (I, [P, L, P, L, P, P, P, P, L, P, P, I, I, I, F, I, L, P]),
     "opk_add_rmsnorm_fwd": (I, [P, P, P, P, P, P, I, I, F, F, P]),
     "opk_rmsnorm_bwd": (I, [P, P, P, P, P, P, P, P, I, I, I, F, P]),
     "opk_layernorm_fwd": (I, [P, P, P, P, P, P, I, I, F, P]),
-    "opk_layernorm_bwd": (I, [P, P, P, P, P, P, P, P, P, I, I, P]),
+    "opk_layernorm_bwd": (I, [P, P, P, P, P, P, P, P, P, I, I, I, L, P]),
     "opk_rope": (I, [P, P, P, I, L, I, I, L, F, P]),
     "opk_swiglu_fwd": (I, [P, P, I, I, P]),
     "opk_swiglu_bwd": (I, [P, P, P, I, I, P]),
@@ -68,15 +68,15 @@ PROTOTYPES: dict = {
     "opk_glu_split_bwd": (I, [P, P, P, P, P, L, I, P]),
     "opk_gelu_fwd": (I, [P, P, L, P]),
     "opk_gelu_bwd": (I, [P, P, P, L, P]),
-    "opk_embedding_fwd": (I, [P, P, P, P, I, I, I, P]),
-    "opk_embedding_bwd_compact": (I, [P, P, P, P, P, P, I, I, I, P]),
+    "opk_embedding_fwd": (I, [P, P, P, P, I, I, I, I, P]),
+    "opk_embedding_bwd_compact": (I, [P, P, P, P, P, P, I, I, I, I, P]),
     "opk_embedding_accumulate": (I, [P, P, P, P, P, I, I, P]),
     "opk_lce_finalize": (I, [P, P, P, P, P, P, I, I, P]),
-    "opk_loss_coef": (I, [P, P, P, P, P, P, I, P]),
+    "opk_loss_coef": (I, [P, P, P, P, P, P, I, I, P]),
     "opk_rmsnorm_dw_per_example": (I, [P, P, P, P, I, I, I, P]),
     "opk_cross_entropy_fwd": (I, [P, I, P, P, P, I, I, L, F, F, P]),
     "opk_cross_entropy_bwd": (I, [P, I, P, P, P, P, I, I, L, F, F, P]),
-    "opk_sumsq": (I, [P, I, I, L, P, P]),
+    "opk_sumsq": (I, [P, I, I, L, P, I, L, P]),
     "opk_moe_route": (I, [P, L, I, I, I, I, P, P, P, P]),
     "opk_moe_route_bwd": (I, [P, P, P, I, I, I, I, P, L, P]),
     "opk_moe_rows_capacity": (I, [I, I]),
@@ -95,10 +95,10 @@ PROTOTYPES: dict = {
     "opk_mt_adam": (I, [c_char_p, I, F, F, F, F, c_double, c_double, F, I, P]),
     "opk_mt_finish_update": (I, [c_char_p, I, F, F, P]),
     "opk_mt_add_update": (I, [c_char_p, I, P]),
-    "opk_scatter_rows_cast_sumsq": (I, [P, P, P, P, I, I, P, P]),
-    "opk_colsum": (I, [P, P, I, I, L, P]),
-    "opk_embedding_add_rows": (I, [P, P, P, P, I, I, P]),
-    "opk_clip_scale": (I, [P, F, I, F, I, L, P, P, P, I, P]),
+    "opk_scatter_rows_cast_sumsq": (I, [P, P, P, P, I, I, P, I, L, P]),
+    "opk_colsum": (I, [P, P, I, I, L, I, L, P]),
+    "opk_embedding_add_rows": (I, [P, P, P, P, I, I, I, L, P]),
+    "opk_clip_scale": (I, [P, F, I, F, I, L, P, P, P, I, I, P]),
     "opk_clip_accumulate": (I, [P, P, P, L, P]),
     "opk_clip_accumulate2": (I, [P, P, P, L, I, P]),
     "opk_clip_accumulate_group": (I, [POINTER(c_void_p), POINTER(c_void_p), I, P, L, I, P]),

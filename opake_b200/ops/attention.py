@@ -25,15 +25,23 @@ def have_flash() -> bool:
     return hasattr(L, "opk_attn_fwd") and hasattr(L, "opk_attn_bwd")
 
 
-def attention_fwd(qkv: torch.Tensor, H: int, KV: int, hd: int, impl: str = "auto", out: torch.Tensor | None = None):
-    """Returns ``(out [T, H*hd] bf16, ctx)``; ``ctx`` is what :func:`attention_bwd` needs."""
+def resolve_impl(hd: int) -> str:
+    return "flash" if (have_flash() and hd in (64, 128)) else "sdpa"
+
+
+def attention_fwd(qkv: torch.Tensor, H: int, KV: int, hd: int, impl: str = "auto", out: torch.Tensor | None = None,
+                  n_seq: int = 1):
+    """Returns ``(out [T, H*hd] bf16, ctx)``; ``ctx`` is what :func:`attention_bwd` needs. ``n_seq``: the rows are that many
+    sequences of equal length, one after the other (``flash`` only)."""
     if impl == "auto":
-        impl = "flash" if (have_flash() and hd in (64, 128)) else "sdpa"
+        impl = resolve_impl(hd)
     if impl == "flash":
         from .flash import flash_fwd
 
-        out, lse = flash_fwd(qkv, H, KV, hd, out=out)
-        return out, ("flash", lse)
+        out, lse = flash_fwd(qkv, H, KV, hd, out=out, n_seq=n_seq)
+        return out, ("flash", (lse, n_seq))
+    if n_seq != 1:
+        raise ValueError("several sequences per call need the native kernels")
     q, k, v = _split(qkv, H, KV, hd)
     qh = q.transpose(0, 1).unsqueeze(0).detach().requires_grad_()
     kh = k.transpose(0, 1).unsqueeze(0).detach().requires_grad_()
@@ -58,7 +66,8 @@ def attention_bwd(dout: torch.Tensor, qkv: torch.Tensor, out: torch.Tensor, ctx,
     if kind == "flash":
         from .flash import flash_bwd
 
-        return flash_bwd(dout, qkv, out, saved, H, KV, hd, dqkv)
+        lse, n_seq = saved
+        return flash_bwd(dout, qkv, out, lse, H, KV, hd, dqkv, n_seq=n_seq)
     o, qh, kh, vh = saved
     go = dout.view(T, H, hd).transpose(0, 1).unsqueeze(0)
     dq, dk, dv = torch.autograd.grad(o, (qh, kh, vh), go)

@@ -17,30 +17,34 @@ def _fn(name, argtypes):
     return f
 
 
-def flash_fwd(qkv: torch.Tensor, H: int, KV: int, hd: int, out: torch.Tensor | None = None):
-    """Causal GQA attention over the fused projection buffer. Returns ``(out [T, H*hd], lse [H, T])``."""
-    T = qkv.shape[0]
+def flash_fwd(qkv: torch.Tensor, H: int, KV: int, hd: int, out: torch.Tensor | None = None, n_seq: int = 1):
+    """Causal GQA attention over the fused projection buffer. Returns ``(out [rows, H*hd], lse [n_seq * H, T])``: ``n_seq``
+    sequences of ``T`` rows one after the other."""
+    rows = qkv.shape[0]
+    T = rows // n_seq
+    if T * n_seq != rows:
+        raise ValueError("the rows are not sequences of equal length")
     if out is None:
-        out = torch.empty(T, H * hd, dtype=torch.bfloat16, device=qkv.device)
-    lse = torch.empty(H, T, dtype=torch.float32, device=qkv.device)
-    f = _fn("opk_attn_fwd", [_P, _P, _P, _I, _I, _I, _I, _L, _L, _F, _P, _P])
-    rc = f(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), T, H, KV, hd, qkv.stride(0), out.stride(0), hd**-0.5,
+        out = torch.empty(rows, H * hd, dtype=torch.bfloat16, device=qkv.device)
+    lse = torch.empty(n_seq * H, T, dtype=torch.float32, device=qkv.device)
+    f = _fn("opk_attn_fwd", [_P, _P, _P, _I, _I, _I, _I, _I, _L, _L, _F, _P, _P])
+    rc = f(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), T, H, KV, hd, n_seq, qkv.stride(0), out.stride(0), hd**-0.5,
            _lib.err_word(qkv.device).data_ptr(), _lib.stream_ptr(qkv.device))
     _lib.check(rc, "opk_attn_fwd")
     return out, lse
 
 
-def flash_bwd(dout, qkv, out, lse, H: int, KV: int, hd: int, dqkv: torch.Tensor, split_heads: bool = True):
+def flash_bwd(dout, qkv, out, lse, H: int, KV: int, hd: int, dqkv: torch.Tensor, split_heads: bool = True, n_seq: int = 1):
     """Gradient with respect to the fused projection buffer (dQ, dK, dV written into ``dqkv``)."""
-    T = qkv.shape[0]
+    T = qkv.shape[0] // n_seq
     t64 = (T + 63) // 64 * 64
-    dsum = torch.empty(2, H, t64, dtype=torch.float32, device=qkv.device)   # rowsum(dO*O), then -lse*log2(e)
+    dsum = torch.empty(2, n_seq * H, t64, dtype=torch.float32, device=qkv.device)   # rowsum(dO*O), then -lse*log2(e)
     part = None
     if H > KV and split_heads:
-        part = torch.empty(2 * (H // KV) * T * KV * hd, dtype=torch.float32, device=qkv.device)
-    f = _fn("opk_attn_bwd", [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _L, _L, _F, _P, _P])
+        part = torch.empty(n_seq * 2 * (H // KV) * T * KV * hd, dtype=torch.float32, device=qkv.device)
+    f = _fn("opk_attn_bwd", [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _L, _L, _F, _P, _P])
     rc = f(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), dsum.data_ptr(), dqkv.data_ptr(),
-           None if part is None else part.data_ptr(), T, H, KV, hd,
+           None if part is None else part.data_ptr(), T, H, KV, hd, n_seq,
            qkv.stride(0), out.stride(0), hd**-0.5, _lib.err_word(qkv.device).data_ptr(), _lib.stream_ptr(qkv.device))
     _lib.check(rc, "opk_attn_bwd")
     return dqkv

@@ -59,26 +59,43 @@ _RMS_WS: dict = {}
 _RMS_WS_ROWS = 296
 
 
-def _rms_workspace(device, D: int) -> torch.Tensor:
+def _rms_workspace(device, floats: int) -> torch.Tensor:
     """Per-device scratch for the per-CTA partial weight gradients of the norm backward kernel. Calls on one device
     share it, so they must be ordered on one stream (the model runtimes issue every example on a single stream)."""
     key = device.index
     ws = _RMS_WS.get(key)
-    if ws is None or ws.numel() < _RMS_WS_ROWS * D:
-        ws = torch.empty(_RMS_WS_ROWS * D, dtype=torch.float32, device=device)
+    if ws is None or ws.numel() < floats:
+        ws = torch.empty(floats, dtype=torch.float32, device=device)
         _RMS_WS[key] = ws
     return ws
 
 
-def rmsnorm_bwd(dy, x, w, rstd, dres=None, dw=None, w_offset: float = 0.0, out=None):
-    """Returns ``dx`` (plus ``dres`` when given); accumulates the weight gradient into fp32 ``dw`` when given."""
+def _per_example(dw) -> tuple[int, int]:
+    """Examples and pitch of a per-example fp32 output: ``[n]`` (one example) or ``[examples, n]``."""
+    return (1, 0) if dw is None or dw.dim() == 1 else (dw.shape[0], dw.stride(0))
+
+
+def rmsnorm_bwd_scratch(D: int, examples: int, device) -> torch.Tensor:
+    """Scratch of :func:`rmsnorm_bwd` for a caller that keeps its own (one per stream, and one that a graph may hold on to)."""
+    return torch.empty(_RMS_WS_ROWS * examples * D, dtype=torch.float32, device=device)
+
+
+def rmsnorm_bwd(dy, x, w, rstd, dres=None, dw=None, w_offset: float = 0.0, out=None, scratch=None):
+    """Returns ``dx`` (plus ``dres`` when given); accumulates the weight gradient into fp32 ``dw`` when given. ``dw``
+    ``[examples, D]``: the rows are that many examples of equal length, one after the other."""
     T, D = x.shape
+    n, pitch = _per_example(dw)
     dx = torch.empty_like(x) if out is None else out
-    ws = _rms_workspace(x.device, D) if dw is not None else None
+    ws_rows = _RMS_WS_ROWS * n
+    ws = None
+    if dw is not None:
+        ws = _rms_workspace(x.device, ws_rows * D) if scratch is None else scratch
+        if ws.numel() < ws_rows * D:
+            raise ValueError("scratch is too small")
     if dres is not None and dres.stride(0) != dx.stride(0):
         raise ValueError("dres must have the row pitch of the output")
     _chk(_L().opk_rmsnorm_bwd_ld(_p(dy), dy.stride(0), _p(x), x.stride(0), _p(w), _p(rstd), _p(dres), _p(dx), dx.stride(0),
-                                 _p(dw), _p(ws), _RMS_WS_ROWS, T, D, w_offset, _s(x)), "rmsnorm_bwd")
+                                 _p(dw), _p(ws), ws_rows, T // n, D, w_offset, n, pitch, _s(x)), "rmsnorm_bwd")
     return dx
 
 
@@ -94,7 +111,10 @@ def layernorm_fwd(x, w, b, eps: float = 1e-5, out=None):
 def layernorm_bwd(dy, x, w, mean, rstd, dres=None, dw=None, db=None, out=None):
     T, D = x.shape
     dx = torch.empty_like(x) if out is None else out
-    _chk(_L().opk_layernorm_bwd(_p(dy), _p(x), _p(w), _p(mean), _p(rstd), _p(dres), _p(dx), _p(dw), _p(db), T, D,
+    n, pitch = _per_example(dw)
+    if dw is not None and db is not None and _per_example(db) != (n, pitch):
+        raise ValueError("dw and db must have one layout")
+    _chk(_L().opk_layernorm_bwd(_p(dy), _p(x), _p(w), _p(mean), _p(rstd), _p(dres), _p(dx), _p(dw), _p(db), T // n, D, n, pitch,
                                 _s(x)), "layernorm_bwd")
     return dx
 
@@ -180,27 +200,41 @@ def gelu_bwd(dy, x, out=None):
 
 
 # ------------------------------------------------------------------------------------------------ embedding
-def embedding_fwd(tok, table, pos_table=None, out=None):
+def embedding_fwd(tok, table, pos_table=None, out=None, period: int = 0):
+    """``out[t] = table[tok[t]]`` (``+ pos_table[t]``; with ``period`` rows per sequence ``pos_table[t % period]``)."""
     T, D = tok.numel(), table.shape[1]
     if out is None:
         out = torch.empty(T, D, dtype=_bf16, device=table.device)
-    _chk(_L().opk_embedding_fwd(_p(tok), _p(table), _p(pos_table), _p(out), T, D, table.shape[0], _s(table)), "embedding_fwd")
+    _chk(_L().opk_embedding_fwd(_p(tok), _p(table), _p(pos_table), _p(out), T, D, table.shape[0], period, _s(table)), "embedding_fwd")
     return out
 
 
 class EmbeddingGradWorkspace:
-    """Scratch for the per-example compact embedding gradient (first-occurrence table, fp32 rows)."""
+    """Scratch for the per-example compact embedding gradient (first-occurrence table, fp32 rows) of ``examples`` sequences."""
 
-    def __init__(self, vocab: int, max_tokens: int, dim: int, device):
-        self.first_pos = torch.full((vocab,), 2**31 - 1, dtype=torch.int32, device=device)
-        self.rep = torch.empty(max_tokens, dtype=torch.int32, device=device)
-        self.gc = torch.empty(max_tokens, dim, dtype=torch.float32, device=device)
+    def __init__(self, vocab: int, max_tokens: int, dim: int, device, examples: int = 1):
+        self.vocab, self.max_tokens = vocab, max_tokens
+        self.first_pos = torch.full((examples * vocab,), 2**31 - 1, dtype=torch.int32, device=device)
+        self.rep = torch.empty(examples * max_tokens, dtype=torch.int32, device=device)
+        self.gc = torch.empty(examples * max_tokens, dim, dtype=torch.float32, device=device)
+
+    def examples(self, j: int, n: int) -> "EmbeddingGradWorkspace":
+        """The scratch of examples ``j .. j+n-1`` as a workspace of its own (views)."""
+        part = object.__new__(EmbeddingGradWorkspace)
+        part.vocab, part.max_tokens = self.vocab, self.max_tokens
+        part.first_pos = self.first_pos[j * self.vocab : (j + n) * self.vocab]
+        part.rep = self.rep[j * self.max_tokens : (j + n) * self.max_tokens]
+        part.gc = self.gc[j * self.max_tokens : (j + n) * self.max_tokens]
+        return part
 
 
-def embedding_bwd_compact(tok, dx, ws: EmbeddingGradWorkspace, sumsq):
+def embedding_bwd_compact(tok, dx, ws: EmbeddingGradWorkspace, sumsq, examples: int = 1):
+    """``examples`` sequences of ``ws.max_tokens`` tokens one after the other (one sequence may be shorter)."""
     T, D = dx.shape
-    _chk(_L().opk_embedding_bwd_compact(_p(tok), _p(dx), _p(ws.first_pos), _p(ws.rep), _p(ws.gc), _p(sumsq), T, D,
-                                        ws.first_pos.numel(), _s(dx)), "embedding_bwd_compact")
+    if examples > 1 and (T != examples * ws.max_tokens or ws.first_pos.numel() < examples * ws.vocab):
+        raise ValueError("the workspace holds sequences of another number or length")
+    _chk(_L().opk_embedding_bwd_compact(_p(tok), _p(dx), _p(ws.first_pos), _p(ws.rep), _p(ws.gc), _p(sumsq), T // examples, D,
+                                        ws.vocab, examples, _s(dx)), "embedding_bwd_compact")
 
 
 def embedding_accumulate(tok, ws: EmbeddingGradWorkspace, scale, acc, T: int, shared: bool = False):
@@ -233,8 +267,10 @@ def rmsnorm_dw_per_example(dy, x, rstd, batch: int):
 
 def loss_coef(labels, nll, coef, loss, ntok=None, weight=None):
     """Mean-over-supervised-tokens loss of one example and the per-token coefficients of its gradient:
-    ``coef[t] = (labels[t] >= 0) / max(1, n_supervised)`` (times ``weight``), ``loss = sum(nll * coef)``."""
-    _chk(_L().opk_loss_coef(_p(labels), _p(nll), _p(weight), _p(coef), _p(loss), _p(ntok), labels.numel(), _s(nll)), "loss_coef")
+    ``coef[t] = (labels[t] >= 0) / max(1, n_supervised)`` (times ``weight``), ``loss = sum(nll * coef)``. ``loss`` of several
+    elements: that many examples of equal length, one after the other."""
+    n = loss.numel()
+    _chk(_L().opk_loss_coef(_p(labels), _p(nll), _p(weight), _p(coef), _p(loss), _p(ntok), labels.numel() // n, n, _s(nll)), "loss_coef")
 
 
 def cross_entropy_fwd(logits, labels, scale: float = 1.0, softcap: float = 0.0):
@@ -256,32 +292,40 @@ def cross_entropy_bwd(logits, labels, lse, coef, scale: float = 1.0, softcap: fl
 
 # ------------------------------------------------------------------------------------------------ DP primitives
 def sumsq_(x, out, round_bf16: bool = False):
-    """``out (float64 scalar) += sum(x**2)``."""
-    _chk(_L().opk_sumsq(_p(x), int(x.dtype == torch.float32), int(round_bf16), x.numel(), _p(out), _s(x)), "sumsq")
+    """``out (float64) += sum(x**2)``: one sum, or with ``out`` of several elements one for each ``x[j]`` (contiguous)."""
+    n = out.numel()
+    _chk(_L().opk_sumsq(_p(x), int(x.dtype == torch.float32), int(round_bf16), x.numel() // n, _p(out), n,
+                        x.stride(0) if n > 1 else 0, _s(x)), "sumsq")
 
 
 def scatter_rows_cast_sumsq(src, dst_base, offsets, sumsq, widths=None):
     """fp32 rows ``src[r]`` (their first ``widths[r]`` columns, int32, when given) -> bf16 at ``dst_base + offsets[r]``;
-    ``sumsq += sum(stored**2)``."""
-    R, D = src.shape
-    _chk(_L().opk_scatter_rows_cast_sumsq(_p(src), _p(dst_base), _p(offsets), _p(widths), R, D, _p(sumsq), _s(src)),
-         "scatter_rows_cast_sumsq")
+    ``sumsq += sum(stored**2)``. ``src [examples, R, D]`` and ``dst_base [examples, n]``: one destination and sum each."""
+    R, D = src.shape[-2:]
+    n = src.shape[0] if src.dim() == 3 else 1
+    _chk(_L().opk_scatter_rows_cast_sumsq(_p(src), _p(dst_base), _p(offsets), _p(widths), R, D, _p(sumsq), n,
+                                          dst_base.stride(0) if n > 1 else 0, _s(src)), "scatter_rows_cast_sumsq")
 
 
 def colsum_(dy, out):
+    """``out += dy.sum(0)``; ``out [examples, N]``: the rows are that many examples of equal length, one after the other."""
     T, N = dy.shape
-    _chk(_L().opk_colsum(_p(dy), _p(out), T, N, dy.stride(0), _s(dy)), "colsum")
+    n, pitch = _per_example(out)
+    _chk(_L().opk_colsum(_p(dy), _p(out), T // n, N, dy.stride(0), n, pitch, _s(dy)), "colsum")
 
 
 def embedding_add_rows(tok, ws, dense, T: int):
-    _chk(_L().opk_embedding_add_rows(_p(tok), _p(ws.rep), _p(ws.gc), _p(dense), T, dense.shape[1], _s(dense)),
-         "embedding_add_rows")
+    """``dense[tok[t]] += gc[t]``; ``dense [examples, V, D]``: ``T`` tokens of each example into a matrix of its own."""
+    n = dense.shape[0] if dense.dim() == 3 else 1
+    _chk(_L().opk_embedding_add_rows(_p(tok), _p(ws.rep), _p(ws.gc), _p(dense), T, dense.shape[-1], n,
+                                     dense.stride(0) if n > 1 else 0, _s(dense)), "embedding_add_rows")
 
 
 def clip_scale(sumsq, clip: float, *, scale_out, norm_out=None, counters=None, auto: bool = False, gamma: float = 0.01,
                n_leaves: int = 1, widest_leaf: int = 1, reset: bool = True):
+    """``sumsq`` of several elements: one factor (and norm) for each."""
     _chk(_L().opk_clip_scale(_p(sumsq), clip, int(auto), gamma, n_leaves, widest_leaf, _p(scale_out), _p(norm_out),
-                             _p(counters), int(reset), _s(sumsq)), "clip_scale")
+                             _p(counters), int(reset), sumsq.numel(), _s(sumsq)), "clip_scale")
 
 
 def clip_accumulate(g, scale, acc, overwrite: bool = False):

@@ -32,6 +32,14 @@ from . import comm
 
 _bf16 = torch.bfloat16
 
+# Examples of an accumulation group go through the model together up to so many hidden values (rows * d_model): what a pass over
+# few rows waits for is the chain of launches, first loads and epilogues, the same for one example as for several. Steps of eight
+# examples, groups of eight, ms with 1, 2, 4 and 8 examples in a pass: GPT-2-small T = 128 16.4, 9.0, 5.6, 3.9; T = 1024 24.5, 16.3,
+# 13.5, 12.2 (6.3 M values); Llama-3.2-1B with four layers, T = 317 21.2, 15.9, 13.7, 13.2. Four examples, groups of four: 1B T = 1024
+# 17.1, 15.5, 14.9 (8.4 M), T = 1500 22.6, 22.1, 22.3; 8B with two layers T = 317 19.4, 17.2, 17.0, T = 1024 29.9, 29.7 (8.4 M), 30.2.
+# Beyond, the products fill the chip by themselves and only the workspaces grow.
+_JOIN_VALUES = 1 << 23
+
 
 @dataclass
 class EngineConfig:
@@ -160,14 +168,15 @@ class ShardedDPEngine:
         self.runtime = DecoderRuntime(model_cfg, self.params, layout=self.layout, attn_impl=cfg.attn_impl, n_slots=self.group,
                                       ep=self.ep, canaries=self.canaries)
         self._side = torch.cuda.Stream(device=device)
-        self._warm: dict[int, bool] = {}
+        self._warm: dict[tuple, bool] = {}
+        self._join_limit: dict[int, int] = {}
         self.step_count = 0
         self.phi = 0.0
         from ..engine.random import fold_in, key
 
         self._noise_key = key(cfg.seed)
         self._fold_in = fold_in
-        self._graphs: dict[int, tuple] = {}
+        self._graphs: dict[tuple, tuple] = {}
         self._losses = None
         self.graph_kernel_launches = 0   # native launches replayed through CUDA graphs (not seen by the ctypes counter)
         if self.world > 1:
@@ -303,11 +312,96 @@ class ShardedDPEngine:
             rt.clip_factor(cfg.clip_norm, auto=cfg.auto_clip, gamma=cfg.auto_gamma, slot=slot)
         ws["loss_sum"].add_(st.loss.reshape(1))
         if slot == 0:
-            ws["tok_keep"].copy_(ws["toks"][0])      # slot 0's tokens are replaced before its deferred pass runs
+            ws["tok_keep"][0].copy_(ws["toks"][0])   # slot 0's tokens are replaced before its deferred pass runs
 
     @staticmethod
     def _group_toks(ws, n: int):
-        return [ws["tok_keep"], *ws["toks"][1:n]]
+        return [ws["tok_keep"][0], *ws["toks"][1:n]]
+
+    def _joined(self, T: int) -> int:
+        """How many examples of ``T`` tokens go through the model in one pass (at least 1). Only on one rank: with several, an
+        example's passes carry the exchange with the other ranks."""
+        if self.world > 1 or not self.runtime.can_join():
+            return 1
+        most = self._join_limit.get(T, self.group)
+        return max(1, min(most, _JOIN_VALUES // (T * self.model_cfg.d_model)))
+
+    def _step_workspace(self, T: int) -> tuple[int, dict]:
+        """Examples per pass for this length and their workspace: one by one where several do not fit the memory."""
+        n = self._joined(T)
+        try:
+            return n, self.runtime.workspace(T, n)
+        except torch.cuda.OutOfMemoryError:
+            if n == 1:
+                raise
+        self._join_limit[T] = 1
+        torch.cuda.empty_cache()
+        return 1, self.runtime.workspace(T)
+
+    def _joined_body(self, ws, n: int, slot: int, drain_prev: bool, first: bool) -> None:
+        """``_example_body`` for the ``n`` examples in slots ``slot ..``: one pass through the model."""
+        rt, cfg = self.runtime, self.cfg
+        part, main = self.runtime.part(ws, n), torch.cuda.current_stream(self.device)
+        hook = None
+        if drain_prev:
+            self._side.wait_stream(main)
+            with torch.cuda.stream(self._side):
+                self._accumulate(ws, self.group, ws["kept"], overwrite=first)
+            hook = lambda: main.wait_stream(self._side)
+        toks = ws["tok_all"][slot : slot + n]
+        st = rt.example_grad(toks.view(-1), part["labels"], ws=part, slot=slot, before_wgrad=hook)
+        rt.clip_factor(cfg.clip_norm, auto=cfg.auto_clip, gamma=cfg.auto_gamma, slot=slot, n=n)
+        ws["loss_sum"].add_(st.loss.sum())
+        ws["tok_keep"][slot : slot + n].copy_(toks)      # the slots' tokens are replaced before their deferred pass runs
+
+    def _run_joined(self, ws, tok_host: torch.Tensor, labels_host: torch.Tensor, index: int) -> None:
+        """Examples ``index ..`` of the step (``tok_host`` ``[n, T]``), as many as go through the model together."""
+        n, T = tok_host.shape
+        slot = index % self.group
+        drain = index > 0 and slot == 0
+        first = drain and self._fuse_last_group and not self._have_sums
+        if drain:
+            self._have_sums = True
+        ws["tok_all"][slot : slot + n].copy_(tok_host, non_blocking=True)
+        self.runtime.part(ws, n)["labels"].view(n, T).copy_(labels_host, non_blocking=True)
+        if not self.cfg.use_cuda_graph:
+            self._joined_body(ws, n, slot, drain, first)
+            return
+        key = ("joined", T, slot, n, drain, first)
+        self._replay(key, ("joined", T) if index == 0 else None, ws, lambda: self._joined_body(ws, n, slot, False, False),
+                     lambda: self._joined_body(ws, n, slot, drain, first))
+
+    def _replay(self, key: tuple, warm_key, ws, warm_up, body) -> None:
+        """Runs ``body`` as the CUDA graph ``key``, captured on first use. ``warm_up`` runs eagerly before the first capture of
+        ``warm_key`` (lazy workspaces), with the step's state restored; ``None``: an earlier part of the step has done so."""
+        entry = self._graphs.get(key)
+        if entry is None:
+            from ..ops import _lib
+
+            if warm_key is not None and not self._warm.get(warm_key):
+                # eager warm-up (lazy workspaces, library autotuning) on a side stream, state restored afterwards
+                saved = ws["loss_sum"].clone()
+                s = torch.cuda.Stream(device=self.device)
+                s.wait_stream(torch.cuda.current_stream(self.device))
+                with torch.cuda.stream(s):
+                    warm_up()
+                torch.cuda.current_stream(self.device).wait_stream(s)
+                torch.cuda.synchronize(self.device)
+                ws["loss_sum"].copy_(saved)
+                self.runtime.clip_count.zero_()
+                if self.ep is not None:
+                    # warm-ups only ever happen on the first example of a step, where the expert sums are still zero
+                    self.ep.acc.zero_()
+                self._warm[warm_key] = True
+            g = torch.cuda.CUDAGraph()
+            before = _lib.LAUNCHES[0]
+            with torch.cuda.graph(g):
+                body()
+            entry = (g, _lib.LAUNCHES[0] - before)
+            self._graphs[key] = entry
+            # capture does not execute: fall through to the first replay
+        entry[0].replay()
+        self.graph_kernel_launches += entry[1]
 
     def _run_example(self, tok_host: torch.Tensor, labels_host: torch.Tensor, index: int) -> None:
         T = tok_host.numel()
@@ -326,35 +420,8 @@ class ShardedDPEngine:
         if not self.cfg.use_cuda_graph:
             self._example_body(ws, slot, drain, refresh, first)
             return
-        key = (T, slot, drain, refresh, first)
-        entry = self._graphs.get(key)
-        if entry is None:
-            from ..ops import _lib
-
-            if not self._warm.get((T, refresh)):
-                # eager warm-up (lazy workspaces, library autotuning) on a side stream, state restored afterwards
-                saved = ws["loss_sum"].clone()
-                s = torch.cuda.Stream(device=self.device)
-                s.wait_stream(torch.cuda.current_stream(self.device))
-                with torch.cuda.stream(s):
-                    self._example_body(ws, slot, False, refresh)
-                torch.cuda.current_stream(self.device).wait_stream(s)
-                torch.cuda.synchronize(self.device)
-                ws["loss_sum"].copy_(saved)
-                self.runtime.clip_count.zero_()
-                if self.ep is not None:
-                    # warm-ups only ever happen on the first example of a step, where the expert sums are still zero
-                    self.ep.acc.zero_()
-                self._warm[(T, refresh)] = True
-            g = torch.cuda.CUDAGraph()
-            before = _lib.LAUNCHES[0]
-            with torch.cuda.graph(g):
-                self._example_body(ws, slot, drain, refresh, first)
-            entry = (g, _lib.LAUNCHES[0] - before)
-            self._graphs[key] = entry
-            # capture does not execute: fall through to the first replay
-        entry[0].replay()
-        self.graph_kernel_launches += entry[1]
+        self._replay((T, slot, drain, refresh, first), (T, refresh), ws, lambda: self._example_body(ws, slot, False, refresh),
+                     lambda: self._example_body(ws, slot, drain, refresh, first))
 
     # ------------------------------------------------------------------ optimizer step
     def _noise_sigma(self) -> float:
@@ -376,23 +443,31 @@ class ShardedDPEngine:
             dist.barrier()
         if self._last_group:
             self._settle_sums()       # left over from an update that was not applied: the gradient slots are refilled now
-        ws = self.runtime.workspace(tokens.shape[1])
+        joined, ws = self._step_workspace(tokens.shape[1])
         if "loss_sum" not in ws:
             ws["loss_sum"] = torch.zeros(1, dtype=torch.float32, device=self.device)
-        if "tok_keep" not in ws:
-            ws["tok_keep"] = torch.zeros_like(ws["toks"][0])
+            ws["tok_keep"] = torch.zeros_like(ws["tok_all"])
+            ws["kept"] = list(ws["tok_keep"].unbind(0))
         ws["loss_sum"].zero_()
         with nvtx_range("opake::examples"):
-            for i in range(B_local):
-                self._run_example(tokens[i], labels[i], i)
+            if joined > 1:
+                for start in range(0, B_local, self.group):          # one accumulation group after the other, each in joined passes
+                    stop = min(start + self.group, B_local)
+                    for i in range(start, stop, joined):
+                        j = min(i + joined, stop)
+                        self._run_joined(ws, tokens[i:j], labels[i:j], i)
+            else:
+                for i in range(B_local):
+                    self._run_example(tokens[i], labels[i], i)
         # the last group (complete or not) has not been added yet: every earlier one was added at the start of the
         # example that followed it
         n_last = B_local % self.group or min(self.group, B_local)
+        toks = ws["kept"][:n_last] if joined > 1 else self._group_toks(ws, n_last)
         if n_last and self._fuse_last_group:
-            self.runtime.accumulate_embeddings(self._acc, ws, n_last, toks=self._group_toks(ws, n_last))
+            self.runtime.accumulate_embeddings(self._acc, ws, n_last, toks=toks)
             self._last_group = n_last
         elif n_last:
-            self._accumulate(ws, n_last, self._group_toks(ws, n_last))
+            self._accumulate(ws, n_last, toks)
         loss_sum = ws["loss_sum"].clone()
         with nvtx_range("opake::dp_step"):
             self.apply_update()
