@@ -19,6 +19,8 @@ OUT = Path(__file__).resolve().parent / "_C"
 KERNEL_LIB = OUT / "libopake_kernels.so"
 # same sources with -DOPK_DEBUG_BOUNDS: data-dependent indices are checked, a bad one is recorded and its access skipped
 KERNEL_LIB_DEBUG = OUT / "libopake_kernels_debug.so"
+# autograd nodes of the operators of ops/nodes.py: the one library here that is compiled against torch's headers
+NODES_LIB = OUT / ("_opake_nodes" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 ACCOUNTING_LIB = OUT / ("_opake_accounting" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC_FLAGS = [
@@ -102,9 +104,31 @@ def build_accounting(force: bool = False) -> Path:
     return ACCOUNTING_LIB
 
 
+def build_nodes(force: bool = False) -> Path:
+    """Compile the autograd nodes of the dispatcher operators (host code on torch's C++ API)."""
+    src = CSRC / "host" / "nodes.cpp"
+    if not force and _newer(NODES_LIB, [src]):
+        return NODES_LIB
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    OUT.mkdir(parents=True, exist_ok=True)
+    cmd = [
+        os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=_opake_nodes",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in include_paths()),
+        f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(NODES_LIB), *(f"-L{p}" for p in library_paths()),
+        "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10",
+    ]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"build of the autograd nodes failed:\n{r.stdout}")
+    return NODES_LIB
+
+
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_kernels(force=force, verbose=verbose)
     build_kernels(force=force, debug_bounds=True)
+    build_nodes(force=force)
     build_accounting(force=force)
 
 

@@ -8,7 +8,7 @@ finalize kernel merges the tiles, and the backward epilogue recomputes the logit
 ``coef * (softmax - onehot)`` in bf16, from which dH and dW are two more GEMMs. Up to ``KEEP_BYTES`` of logits are left
 behind by the forward epilogue for one backward pass instead (same bits, a pass over memory in place of the product).
 
-Both directions are ``torch.autograd.Function`` objects with ``vmap`` rules so that ``vmap(grad(loss))`` works: a
+Both directions are dispatcher operators (``ops/nodes.py``) with ``vmap`` rules so that ``vmap(grad(loss))`` works: a
 batch of examples sharing one weight is flattened into rows for the forward and dH; the per-example weight gradient
 is one batched GEMM (packages/opake-patches/src/opake/api/patches/kernels/linear_cross_entropy.py:772-779 allocates
 the same ``(B, V, D)`` result).
@@ -16,6 +16,8 @@ the same ``(B, V, D)`` result).
 from __future__ import annotations
 
 import torch
+
+from .nodes import Operator, front
 
 IGNORE_INDEX = -100
 
@@ -61,7 +63,7 @@ def _native_fwd(hidden, weight, labels, logit_scale, softcap, keep):
     pmax = torch.empty(T, tiles, dtype=torch.float32, device=hidden.device)
     psum = torch.empty_like(pmax)
     tgt = torch.empty(T, dtype=torch.float32, device=hidden.device)
-    lab = labels.to(torch.int32).contiguous()
+    lab = labels.to(torch.int32, copy=True).contiguous()      # kept for the backward pass: never the caller's buffer
     n = G.lce_logits_floats(T, V)
     try:
         keep = keep and 4 * n <= KEEP_BYTES and G.lce_keeps_logits(T, V, hidden.shape[1], softcap)
@@ -86,86 +88,60 @@ def _native_dlogits(hidden, weight, lab, lse, z, coef, logit_scale, softcap):
     return dlog
 
 
-class _LinearCEBackward(torch.autograd.Function):
-    """Backward of the fused loss as its own Function so that it can carry a vmap rule (per-example dW)."""
-
-    @staticmethod
-    def forward(grad_nll, hidden, weight, lab, lse, z, logit_scale, softcap):
-        from . import gemm as G
-        coef = (grad_nll.to(torch.float32) * (lab >= 0)).contiguous()
-        dlog = _native_dlogits(hidden, weight, lab, lse, z, coef, logit_scale, softcap)
-        # dlog is the gradient with respect to logit_scale * (hidden @ weight.T)
-        d_hidden = G.gemm(dlog, weight, b_mn=True, alpha=logit_scale)
-        d_weight = G.linear_wgrad(dlog, hidden)
-        if logit_scale != 1.0:
-            d_weight = d_weight * logit_scale
-        return d_hidden, d_weight
-
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        ctx.set_materialize_grads(False)
-
-    @staticmethod
-    def backward(ctx, *grads):
-        raise NotImplementedError("second-order differentiation of the fused linear cross-entropy is not supported")
-
-    @staticmethod
-    def vmap(info, in_dims, grad_nll, hidden, weight, lab, lse, z, logit_scale, softcap):
-        from . import gemm as G
-        if in_dims[2] is not None:
-            raise NotImplementedError("fused linear cross-entropy under vmap needs one shared weight")
-        B = info.batch_size
-
-        def front(x, d):
-            return x.movedim(d, 0) if d is not None else x.unsqueeze(0).expand(B, *x.shape)
-
-        g, h, lb, ls = (front(x, d) for x, d in zip((grad_nll, hidden, lab, lse), (in_dims[0], in_dims[1], in_dims[3], in_dims[4])))
-        T, D = h.shape[1], h.shape[2]
-        hf = h.reshape(B * T, D).contiguous()
-        labf = lb.reshape(B * T).contiguous()
-        coef = (g.to(torch.float32).reshape(B * T) * (labf >= 0)).contiguous()
-        # the stored logits have the rows of the whole batch when the forward pass ran under this vmap, which shows in lse; with
-        # a vmap over cotangents alone they are one example's
-        zf = z if in_dims[4] is not None and in_dims[5] is None else z.new_empty(0)
-        dlog = _native_dlogits(hf, weight, labf, ls.reshape(B * T).contiguous(), zf, coef, logit_scale, softcap)
-        d_hidden = G.gemm(dlog, weight, b_mn=True, alpha=logit_scale).view(B, T, D)
-        V = weight.shape[0]
-        d_weight = torch.empty(B, V, D, dtype=torch.bfloat16, device=hidden.device)
-        G.gemm(dlog.view(B, T, -1), hf.view(B, T, D), a_mn=True, b_mn=True, out=d_weight)
-        if logit_scale != 1.0:
-            d_weight = d_weight * logit_scale
-        return (d_hidden, d_weight), (0, 0)
+def _linear_ce_bwd(grad_nll, hidden, weight, lab, lse, z, logit_scale, softcap):
+    from . import gemm as G
+    coef = (grad_nll.to(torch.float32) * (lab >= 0)).contiguous()
+    dlog = _native_dlogits(hidden, weight, lab, lse, z, coef, logit_scale, softcap)
+    # dlog is the gradient with respect to logit_scale * (hidden @ weight.T)
+    d_hidden = G.gemm(dlog, weight, b_mn=True, alpha=logit_scale)
+    d_weight = G.linear_wgrad(dlog, hidden)
+    if logit_scale != 1.0:
+        d_weight = d_weight * logit_scale
+    return d_hidden, d_weight
 
 
-class _LinearCE(torch.autograd.Function):
-    @staticmethod
-    def forward(hidden, weight, labels, logit_scale, softcap, keep):
-        return _native_fwd(hidden.contiguous(), weight, labels, logit_scale, softcap, keep)
+def _linear_ce_bwd_vmap(B, in_dims, grad_nll, hidden, weight, lab, lse, z, logit_scale, softcap):
+    from . import gemm as G
+    if in_dims[2] is not None:
+        raise NotImplementedError("fused linear cross-entropy under vmap needs one shared weight")
+    g, h, lb, ls = (front(x, d, B) for x, d in zip((grad_nll, hidden, lab, lse), (in_dims[0], in_dims[1], in_dims[3], in_dims[4])))
+    T, D = h.shape[1], h.shape[2]
+    hf = h.reshape(B * T, D).contiguous()
+    labf = lb.reshape(B * T).contiguous()
+    coef = (g.to(torch.float32).reshape(B * T) * (labf >= 0)).contiguous()
+    # the stored logits have the rows of the whole batch when the forward pass ran under this vmap, which shows in lse; with
+    # a vmap over cotangents alone they are one example's
+    zf = z if in_dims[4] is not None and in_dims[5] is None else z.new_empty(0)
+    dlog = _native_dlogits(hf, weight, labf, ls.reshape(B * T).contiguous(), zf, coef, logit_scale, softcap)
+    d_hidden = G.gemm(dlog, weight, b_mn=True, alpha=logit_scale).view(B, T, D)
+    V = weight.shape[0]
+    d_weight = torch.empty(B, V, D, dtype=torch.bfloat16, device=hidden.device)
+    G.gemm(dlog.view(B, T, -1), hf.view(B, T, D), a_mn=True, b_mn=True, out=d_weight)
+    if logit_scale != 1.0:
+        d_weight = d_weight * logit_scale
+    return (d_hidden, d_weight), (0, 0)
 
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        hidden, weight, _labels, logit_scale, softcap, _keep = inputs
-        _nll, lse, lab, z = output
-        ctx.save_for_backward(hidden, weight, lab, lse, z)
-        ctx.mark_non_differentiable(lse, lab, z)
-        ctx.logit_scale, ctx.softcap = logit_scale, softcap
 
-    @staticmethod
-    def backward(ctx, g_nll, _g_lse, _g_lab, _g_z):
-        hidden, weight, lab, lse, z = ctx.saved_tensors
-        d_hidden, d_weight = _LinearCEBackward.apply(g_nll, hidden, weight, lab, lse, z, ctx.logit_scale, ctx.softcap)
-        return d_hidden, d_weight, None, None, None, None
+def _linear_ce(hidden, weight, labels, logit_scale, softcap, keep):
+    return _native_fwd(hidden.contiguous(), weight, labels, logit_scale, softcap, keep)
 
-    @staticmethod
-    def vmap(info, in_dims, hidden, weight, labels, logit_scale, softcap, keep):
-        if in_dims[1] is not None:
-            raise NotImplementedError("fused linear cross-entropy under vmap needs one shared weight")
-        B = info.batch_size
-        h = hidden.movedim(in_dims[0], 0) if in_dims[0] is not None else hidden.unsqueeze(0).expand(B, *hidden.shape)
-        lb = labels.movedim(in_dims[2], 0) if in_dims[2] is not None else labels.unsqueeze(0).expand(B, *labels.shape)
-        T, D = h.shape[1], h.shape[2]
-        nll, lse, lab, z = _native_fwd(h.reshape(B * T, D).contiguous(), weight, lb.reshape(B * T), logit_scale, softcap, keep)
-        return (nll.view(B, T), lse.view(B, T), lab.view(B, T), z), (0, 0, 0, None)
+
+def _linear_ce_vmap(B, in_dims, hidden, weight, labels, logit_scale, softcap, keep):
+    if in_dims[1] is not None:
+        raise NotImplementedError("fused linear cross-entropy under vmap needs one shared weight")
+    h, lb = front(hidden, in_dims[0], B), front(labels, in_dims[2], B)
+    T, D = h.shape[1], h.shape[2]
+    nll, lse, lab, z = _native_fwd(h.reshape(B * T, D).contiguous(), weight, lb.reshape(B * T), logit_scale, softcap, keep)
+    return (nll.view(B, T), lse.view(B, T), lab.view(B, T), z), (0, 0, 0, None)
+
+
+# the backward pass is an operator of its own so that it can carry a vmap rule (per-example dW)
+_LinearCEBackward = Operator("linear_ce_bwd", "(Tensor grad_nll, Tensor hidden, Tensor weight, Tensor lab, Tensor lse, Tensor z, "
+                             "float logit_scale, float softcap) -> (Tensor, Tensor)", _linear_ce_bwd, _linear_ce_bwd_vmap)
+_LinearCEBackward.not_differentiable("second-order differentiation of the fused linear cross-entropy is not supported")
+_LinearCE = Operator("linear_ce", "(Tensor hidden, Tensor weight, Tensor labels, float logit_scale, float softcap, bool keep) -> "
+                     "(Tensor, Tensor, Tensor, Tensor)", _linear_ce, _linear_ce_vmap)
+_LinearCE.differentiated_by(_LinearCEBackward, "g0 i0 i1 o2 o1 o3 i3 i4", [0, 1, None, None, None, None], [True, False, False, False])
 
 
 def linear_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor, *, logit_scale: float = 1.0,
@@ -180,7 +156,7 @@ def linear_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, labels: tor
     if hidden.dim() != 2:
         raise ValueError("hidden must be [T, D]; flatten leading dimensions first")
     if not force_portable and native_available(hidden, weight):
-        nll = _LinearCE.apply(hidden, weight, labels, float(logit_scale), float(logit_softcapping), _keep_logits(hidden, weight))[0]
+        nll = _LinearCE(hidden, weight, labels, float(logit_scale), float(logit_softcapping), _keep_logits(hidden, weight))[0]
     else:
         nll = _chunked_nll(hidden, weight, labels, float(logit_scale), float(logit_softcapping))
     if use_token_scaling:

@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import torch
 
-from .functions import _run
+from ...ops.nodes import Operator, front
 
 __all__ = ["lora_linear", "lora_qkv", "lora_mlp", "lora_grad_sq_norms"]
 
@@ -59,80 +59,55 @@ def _adapted_nn(dy, W, dyB, A, s, dx=None):
     return (base if dx is None else dx + base) + s * _mm_nn(dyB, A)
 
 
-class _LoRABwd(torch.autograd.Function):
-    @staticmethod
-    def forward(dy, x, xa, W, A, B, s):
-        # dy [M, out], x [M, in], xa [M, r]
-        dyB = _mm_nn(dy, B)                                  # [M, r]
-        dx = _adapted_nn(dy, W, dyB, A, s)                   # [M, in]
-        dA = s * (dyB.t() @ x)                               # [r, in]
-        dB = s * (dy.t() @ xa)                               # [out, r]
-        return dx, dA, dB
-
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        pass
-
-    @staticmethod
-    def backward(ctx, *g):
-        raise NotImplementedError("double backward through the fused LoRA linear is not supported")
-
-    @staticmethod
-    def vmap(info, in_dims, dy, x, xa, W, A, B, s):
-        if any(d is not None for d in in_dims[3:6]):
-            raise NotImplementedError("per-example LoRA weights are not supported")
-        n = info.batch_size
-        dy, x, xa = (t.movedim(d, 0) if d is not None else t.unsqueeze(0).expand(n, *t.shape) for t, d in zip((dy, x, xa), in_dims[:3]))
-        M = dy.shape[1]
-        dyf = dy.reshape(n * M, -1)
-        dyB = _mm_nn(dyf, B)
-        dx = _adapted_nn(dyf, W, dyB, A, s).view(n, M, -1)
-        dA = s * torch.bmm(dyB.view(n, M, -1).transpose(1, 2), x)        # [n, r, in]
-        dB = s * torch.bmm(dy.transpose(1, 2), xa)                       # [n, out, r]
-        return (dx, dA, dB), (0, 0, 0)
+def _lora_bwd(dy, x, xa, W, A, B, s):
+    # dy [M, out], x [M, in], xa [M, r]
+    dyB = _mm_nn(dy, B)                                  # [M, r]
+    dx = _adapted_nn(dy, W, dyB, A, s)                   # [M, in]
+    dA = s * (dyB.t() @ x)                               # [r, in]
+    dB = s * (dy.t() @ xa)                               # [out, r]
+    return dx, dA, dB
 
 
-class _LoRA(torch.autograd.Function):
-    @staticmethod
-    def forward(x, W, A, B, s):
-        xa = _mm(x, A)                                       # [M, r]
-        return _adapted(x, W, xa, B, s), xa
+def _lora_bwd_vmap(n, in_dims, dy, x, xa, W, A, B, s):
+    if any(d is not None for d in in_dims[3:6]):
+        raise NotImplementedError("per-example LoRA weights are not supported")
+    dy, x, xa = (front(t, d, n) for t, d in zip((dy, x, xa), in_dims[:3]))
+    M = dy.shape[1]
+    dyf = dy.reshape(n * M, -1)
+    dyB = _mm_nn(dyf, B)
+    dx = _adapted_nn(dyf, W, dyB, A, s).view(n, M, -1)
+    dA = s * torch.bmm(dyB.view(n, M, -1).transpose(1, 2), x)        # [n, r, in]
+    dB = s * torch.bmm(dy.transpose(1, 2), xa)                       # [n, out, r]
+    return (dx, dA, dB), (0, 0, 0)
 
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        x, W, A, B, s = inputs
-        ctx.save_for_backward(x, output[1], W, A, B)
-        ctx.mark_non_differentiable(output[1])
-        ctx.s = s
 
-    @staticmethod
-    def backward(ctx, dy, _dxa):
-        x, xa, W, A, B = ctx.saved_tensors
-        dx, dA, dB = _run(_LoRABwd, dy.contiguous(), x, xa, W, A, B, ctx.s)
-        return dx, None, dA, dB, None
+def _lora(x, W, A, B, s):
+    xa = _mm(x, A)                                       # [M, r]
+    return _adapted(x, W, xa, B, s), xa
 
-    @staticmethod
-    def vmap(info, in_dims, x, W, A, B, s):
-        if any(d is not None for d in in_dims[1:4]):
-            raise NotImplementedError("per-example LoRA weights are not supported")
-        n = info.batch_size
-        x = x.movedim(in_dims[0], 0) if in_dims[0] is not None else x.unsqueeze(0).expand(n, *x.shape)
-        M = x.shape[1]
-        y, xa = _run(_LoRA, x.reshape(n * M, -1), W, A, B, s)
-        return (y.view(n, M, -1), xa.view(n, M, -1)), (0, 0)
+
+def _lora_vmap(n, in_dims, x, W, A, B, s):
+    if any(d is not None for d in in_dims[1:4]):
+        raise NotImplementedError("per-example LoRA weights are not supported")
+    x = front(x, in_dims[0], n)
+    M = x.shape[1]
+    y, xa = _LoRA(x.reshape(n * M, -1), W, A, B, s)
+    return (y.view(n, M, -1), xa.view(n, M, -1)), (0, 0)
+
+
+_LoRABwd = Operator("lora_bwd", "(Tensor dy, Tensor x, Tensor xa, Tensor W, Tensor A, Tensor B, float s) -> (Tensor, Tensor, Tensor)",
+                    _lora_bwd, _lora_bwd_vmap).not_differentiable("double backward through the fused LoRA linear is not supported")
+_LoRA = Operator("lora", "(Tensor x, Tensor W, Tensor A, Tensor B, float s) -> (Tensor, Tensor)", _lora, _lora_vmap)
+_LoRA.differentiated_by(_LoRABwd, "g0 i0 o1 i1 i2 i3 i4", [0, None, 1, 2, None], [True, False])
 
 
 def lora_linear(x, weight, lora_a, lora_b, scaling: float, bias=None):
     """``x [..., in]`` -> ``[..., out]``."""
     lead = x.shape[:-1]
-    y = _LoRA.apply(x.reshape(-1, x.shape[-1]), weight, lora_a, lora_b, float(scaling))[0]
+    y = _LoRA(x.reshape(-1, x.shape[-1]), weight, lora_a, lora_b, float(scaling))[0]
     if bias is not None:
         y = y + bias
     return y.view(*lead, -1)
-
-
-def _front(t, d, n):
-    return t.movedim(d, 0) if d is not None else t.unsqueeze(0).expand(n, *t.shape)
 
 
 def _adapter_grads(dy, x, xa, A, B, s, n=None):
@@ -147,85 +122,59 @@ def _adapter_grads(dy, x, xa, A, B, s, n=None):
     return dyB, dA, dB
 
 
-class _LoRAQKVBwd(torch.autograd.Function):
+def _lora_qkv_grads(n, dq, dk, dv, x, xaq, xak, xav, Wq, Aq, Bq, Wk, Ak, Bk, Wv, Av, Bv, sq, sk, sv):
     """Backward of three adapted projections of ONE input: the input gradient is a single accumulated chain, the six
     adapter gradients are the only per-example tensors under vmap (``Opake_LoRA_QKV``, lora.py:499 of the reference)."""
-
-    @staticmethod
-    def forward(dq, dk, dv, x, xaq, xak, xav, Wq, Aq, Bq, Wk, Ak, Bk, Wv, Av, Bv, sq, sk, sv):
-        return _LoRAQKVBwd._run(None, dq, dk, dv, x, xaq, xak, xav, Wq, Aq, Bq, Wk, Ak, Bk, Wv, Av, Bv, sq, sk, sv)
-
-    @staticmethod
-    def _run(n, dq, dk, dv, x, xaq, xak, xav, Wq, Aq, Bq, Wk, Ak, Bk, Wv, Av, Bv, sq, sk, sv):
-        dx, grads = None, []
-        for dy, xa, W, A, B, s in ((dq, xaq, Wq, Aq, Bq, sq), (dk, xak, Wk, Ak, Bk, sk), (dv, xav, Wv, Av, Bv, sv)):
-            dyB, dA, dB = _adapter_grads(dy, x, xa, A, B, s, n)
-            part = _adapted_nn(dy, W, dyB, A, s)
-            dx = part if dx is None else dx + part
-            grads += [dA, dB]
-        return (dx, *grads)
-
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        pass
-
-    @staticmethod
-    def backward(ctx, *g):
-        raise NotImplementedError("double backward through the fused LoRA projections is not supported")
-
-    @staticmethod
-    def vmap(info, in_dims, dq, dk, dv, x, xaq, xak, xav, *rest):
-        if any(d is not None for d in in_dims[7:16]):
-            raise NotImplementedError("per-example LoRA weights are not supported")
-        n = info.batch_size
-        acts = [_front(t, d, n) for t, d in zip((dq, dk, dv, x, xaq, xak, xav), in_dims[:7])]
-        M = acts[0].shape[1]
-        flat = [t.reshape(n * M, -1) for t in acts]
-        out = _LoRAQKVBwd._run(n, *flat, *rest)
-        return (out[0].view(n, M, -1), *out[1:]), (0,) * 7
+    dx, grads = None, []
+    for dy, xa, W, A, B, s in ((dq, xaq, Wq, Aq, Bq, sq), (dk, xak, Wk, Ak, Bk, sk), (dv, xav, Wv, Av, Bv, sv)):
+        dyB, dA, dB = _adapter_grads(dy, x, xa, A, B, s, n)
+        part = _adapted_nn(dy, W, dyB, A, s)
+        dx = part if dx is None else dx + part
+        grads += [dA, dB]
+    return (dx, *grads)
 
 
-class _LoRAQKV(torch.autograd.Function):
-    @staticmethod
-    def forward(x, Wq, Aq, Bq, Wk, Ak, Bk, Wv, Av, Bv, sq, sk, sv):
-        outs, xas = [], []
-        for W, A, B, s in ((Wq, Aq, Bq, sq), (Wk, Ak, Bk, sk), (Wv, Av, Bv, sv)):
-            xa = _mm(x, A)
-            outs.append(_adapted(x, W, xa, B, s))
-            xas.append(xa)
-        return (*outs, *xas)
+def _lora_qkv_bwd_vmap(n, in_dims, *args):
+    if any(d is not None for d in in_dims[7:16]):
+        raise NotImplementedError("per-example LoRA weights are not supported")
+    acts = [front(t, d, n) for t, d in zip(args[:7], in_dims[:7])]
+    M = acts[0].shape[1]
+    out = _lora_qkv_grads(n, *[t.reshape(n * M, -1) for t in acts], *args[7:])
+    return (out[0].view(n, M, -1), *out[1:]), (0,) * 7
 
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        x, Wq, Aq, Bq, Wk, Ak, Bk, Wv, Av, Bv, sq, sk, sv = inputs
-        ctx.save_for_backward(x, *output[3:], Wq, Aq, Bq, Wk, Ak, Bk, Wv, Av, Bv)
-        ctx.mark_non_differentiable(*output[3:])
-        ctx.s = (sq, sk, sv)
 
-    @staticmethod
-    def backward(ctx, dq, dk, dv, *_):
-        x, xaq, xak, xav, *w = ctx.saved_tensors
-        dx, dAq, dBq, dAk, dBk, dAv, dBv = _run(_LoRAQKVBwd, dq.contiguous(), dk.contiguous(), dv.contiguous(), x, xaq, xak, xav,
-                                                             *w, *ctx.s)
-        return dx, None, dAq, dBq, None, dAk, dBk, None, dAv, dBv, None, None, None
+def _lora_qkv(x, Wq, Aq, Bq, Wk, Ak, Bk, Wv, Av, Bv, sq, sk, sv):
+    outs, xas = [], []
+    for W, A, B, s in ((Wq, Aq, Bq, sq), (Wk, Ak, Bk, sk), (Wv, Av, Bv, sv)):
+        xa = _mm(x, A)
+        outs.append(_adapted(x, W, xa, B, s))
+        xas.append(xa)
+    return (*outs, *xas)
 
-    @staticmethod
-    def vmap(info, in_dims, x, *rest):
-        if any(d is not None for d in in_dims[1:10]):
-            raise NotImplementedError("per-example LoRA weights are not supported")
-        n = info.batch_size
-        x = _front(x, in_dims[0], n)
-        M = x.shape[1]
-        out = _run(_LoRAQKV, x.reshape(n * M, -1), *rest)
-        return tuple(t.view(n, M, -1) for t in out), (0,) * 6
+
+def _lora_qkv_vmap(n, in_dims, x, *rest):
+    if any(d is not None for d in in_dims[1:10]):
+        raise NotImplementedError("per-example LoRA weights are not supported")
+    x = front(x, in_dims[0], n)
+    M = x.shape[1]
+    return tuple(t.view(n, M, -1) for t in _LoRAQKV(x.reshape(n * M, -1), *rest)), (0,) * 6
+
+
+_QKV_WEIGHTS = "Tensor Wq, Tensor Aq, Tensor Bq, Tensor Wk, Tensor Ak, Tensor Bk, Tensor Wv, Tensor Av, Tensor Bv, float sq, float sk, float sv"
+_LoRAQKVBwd = Operator("lora_qkv_bwd", "(Tensor dq, Tensor dk, Tensor dv, Tensor x, Tensor xaq, Tensor xak, Tensor xav, " + _QKV_WEIGHTS
+                       + ") -> (" + ", ".join(["Tensor"] * 7) + ")", lambda *args: _lora_qkv_grads(None, *args), _lora_qkv_bwd_vmap)
+_LoRAQKVBwd.not_differentiable("double backward through the fused LoRA projections is not supported")
+_LoRAQKV = Operator("lora_qkv", "(Tensor x, " + _QKV_WEIGHTS + ") -> (" + ", ".join(["Tensor"] * 6) + ")", _lora_qkv, _lora_qkv_vmap)
+_LoRAQKV.differentiated_by(_LoRAQKVBwd, "g0 g1 g2 i0 o3 o4 o5 " + " ".join(f"i{j}" for j in range(1, 13)),
+                           [0, None, 1, 2, None, 3, 4, None, 5, 6, None, None, None], [True] * 3 + [False] * 3)
 
 
 def lora_qkv(x, q, k, v):
     """Three adapted projections of the same input in one autograd node; each of ``q, k, v`` is
     ``(weight, A, B, scaling, bias)``. The input is saved once and its gradient accumulated in one chain."""
     lead = x.shape[:-1]
-    out = _LoRAQKV.apply(x.reshape(-1, x.shape[-1]), q[0], q[1], q[2], k[0], k[1], k[2], v[0], v[1], v[2],
-                         float(q[3]), float(k[3]), float(v[3]))[:3]
+    out = _LoRAQKV(x.reshape(-1, x.shape[-1]), q[0], q[1], q[2], k[0], k[1], k[2], v[0], v[1], v[2],
+                   float(q[3]), float(k[3]), float(v[3]))[:3]
     res = []
     for y, p in zip(out, (q, k, v)):
         if len(p) > 4 and p[4] is not None:
@@ -265,75 +214,52 @@ def _act_bwd(dh, g, u, act: str):
     return (dhf * uf * da).to(g.dtype), (dhf * a).to(g.dtype)
 
 
-class _LoRAMLPBwd(torch.autograd.Function):
+def _lora_mlp_grads(n, dy, x, g, u, xag, xau, had, Wg, Ag, Bg, Wu, Au, Bu, Wd, Ad, Bd, sg, su, sd, act):
     """Backward of the adapted gated MLP (``Opake_LoRA_MLP``, lora.py:1063 of the reference): the activation is
     recomputed from the saved pre-activations, the three adapted projections are differentiated by hand."""
-
-    @staticmethod
-    def forward(dy, x, g, u, xag, xau, had, Wg, Ag, Bg, Wu, Au, Bu, Wd, Ad, Bd, sg, su, sd, act):
-        return _LoRAMLPBwd._run(None, dy, x, g, u, xag, xau, had, Wg, Ag, Bg, Wu, Au, Bu, Wd, Ad, Bd, sg, su, sd, act)
-
-    @staticmethod
-    def _run(n, dy, x, g, u, xag, xau, had, Wg, Ag, Bg, Wu, Au, Bu, Wd, Ad, Bd, sg, su, sd, act):
-        h = _act_fwd(g, u, act)
-        dyB, dAd, dBd = _adapter_grads(dy, h, had, Ad, Bd, sd, n)
-        dh = _adapted_nn(dy, Wd, dyB, Ad, sd)
-        dg, du = _act_bwd(dh, g, u, act)
-        dgB, dAg, dBg = _adapter_grads(dg, x, xag, Ag, Bg, sg, n)
-        duB, dAu, dBu = _adapter_grads(du, x, xau, Au, Bu, su, n)
-        dx = _adapted_nn(du, Wu, duB, Au, su, _adapted_nn(dg, Wg, dgB, Ag, sg))
-        return dx, dAg, dBg, dAu, dBu, dAd, dBd
-
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        pass
-
-    @staticmethod
-    def backward(ctx, *g):
-        raise NotImplementedError("double backward through the fused LoRA MLP is not supported")
-
-    @staticmethod
-    def vmap(info, in_dims, dy, x, g, u, xag, xau, had, *rest):
-        if any(d is not None for d in in_dims[7:16]):
-            raise NotImplementedError("per-example LoRA weights are not supported")
-        n = info.batch_size
-        acts = [_front(t, d, n) for t, d in zip((dy, x, g, u, xag, xau, had), in_dims[:7])]
-        M = acts[0].shape[1]
-        out = _LoRAMLPBwd._run(n, *[t.reshape(n * M, -1) for t in acts], *rest)
-        return (out[0].view(n, M, -1), *out[1:]), (0,) * 7
+    h = _act_fwd(g, u, act)
+    dyB, dAd, dBd = _adapter_grads(dy, h, had, Ad, Bd, sd, n)
+    dh = _adapted_nn(dy, Wd, dyB, Ad, sd)
+    dg, du = _act_bwd(dh, g, u, act)
+    dgB, dAg, dBg = _adapter_grads(dg, x, xag, Ag, Bg, sg, n)
+    duB, dAu, dBu = _adapter_grads(du, x, xau, Au, Bu, su, n)
+    dx = _adapted_nn(du, Wu, duB, Au, su, _adapted_nn(dg, Wg, dgB, Ag, sg))
+    return dx, dAg, dBg, dAu, dBu, dAd, dBd
 
 
-class _LoRAMLP(torch.autograd.Function):
-    @staticmethod
-    def forward(x, Wg, Ag, Bg, Wu, Au, Bu, Wd, Ad, Bd, sg, su, sd, act):
-        xag, xau = _mm(x, Ag), _mm(x, Au)
-        g, u = _adapted(x, Wg, xag, Bg, sg), _adapted(x, Wu, xau, Bu, su)
-        h = _act_fwd(g, u, act)
-        had = _mm(h, Ad)
-        return _adapted(h, Wd, had, Bd, sd), g, u, xag, xau, had
+def _lora_mlp_bwd_vmap(n, in_dims, *args):
+    if any(d is not None for d in in_dims[7:16]):
+        raise NotImplementedError("per-example LoRA weights are not supported")
+    acts = [front(t, d, n) for t, d in zip(args[:7], in_dims[:7])]
+    M = acts[0].shape[1]
+    out = _lora_mlp_grads(n, *[t.reshape(n * M, -1) for t in acts], *args[7:])
+    return (out[0].view(n, M, -1), *out[1:]), (0,) * 7
 
-    @staticmethod
-    def setup_context(ctx, inputs, output):
-        x, Wg, Ag, Bg, Wu, Au, Bu, Wd, Ad, Bd, sg, su, sd, act = inputs
-        ctx.save_for_backward(x, *output[1:], Wg, Ag, Bg, Wu, Au, Bu, Wd, Ad, Bd)
-        ctx.mark_non_differentiable(*output[1:])
-        ctx.consts = (sg, su, sd, act)
 
-    @staticmethod
-    def backward(ctx, dy, *_):
-        x, g, u, xag, xau, had, *w = ctx.saved_tensors
-        dx, dAg, dBg, dAu, dBu, dAd, dBd = _run(_LoRAMLPBwd, dy.contiguous(), x, g, u, xag, xau, had, *w, *ctx.consts)
-        return dx, None, dAg, dBg, None, dAu, dBu, None, dAd, dBd, None, None, None, None
+def _lora_mlp(x, Wg, Ag, Bg, Wu, Au, Bu, Wd, Ad, Bd, sg, su, sd, act):
+    xag, xau = _mm(x, Ag), _mm(x, Au)
+    g, u = _adapted(x, Wg, xag, Bg, sg), _adapted(x, Wu, xau, Bu, su)
+    h = _act_fwd(g, u, act)
+    had = _mm(h, Ad)
+    return _adapted(h, Wd, had, Bd, sd), g, u, xag, xau, had
 
-    @staticmethod
-    def vmap(info, in_dims, x, *rest):
-        if any(d is not None for d in in_dims[1:10]):
-            raise NotImplementedError("per-example LoRA weights are not supported")
-        n = info.batch_size
-        x = _front(x, in_dims[0], n)
-        M = x.shape[1]
-        out = _run(_LoRAMLP, x.reshape(n * M, -1), *rest)
-        return tuple(t.view(n, M, -1) for t in out), (0,) * 6
+
+def _lora_mlp_vmap(n, in_dims, x, *rest):
+    if any(d is not None for d in in_dims[1:10]):
+        raise NotImplementedError("per-example LoRA weights are not supported")
+    x = front(x, in_dims[0], n)
+    M = x.shape[1]
+    return tuple(t.view(n, M, -1) for t in _LoRAMLP(x.reshape(n * M, -1), *rest)), (0,) * 6
+
+
+_MLP_WEIGHTS = ("Tensor Wg, Tensor Ag, Tensor Bg, Tensor Wu, Tensor Au, Tensor Bu, Tensor Wd, Tensor Ad, Tensor Bd, float sg, float su, "
+                "float sd, str act")
+_LoRAMLPBwd = Operator("lora_mlp_bwd", "(Tensor dy, Tensor x, Tensor g, Tensor u, Tensor xag, Tensor xau, Tensor had, " + _MLP_WEIGHTS
+                       + ") -> (" + ", ".join(["Tensor"] * 7) + ")", lambda *args: _lora_mlp_grads(None, *args), _lora_mlp_bwd_vmap)
+_LoRAMLPBwd.not_differentiable("double backward through the fused LoRA MLP is not supported")
+_LoRAMLP = Operator("lora_mlp", "(Tensor x, " + _MLP_WEIGHTS + ") -> (" + ", ".join(["Tensor"] * 6) + ")", _lora_mlp, _lora_mlp_vmap)
+_LoRAMLP.differentiated_by(_LoRAMLPBwd, "g0 i0 o1 o2 o3 o4 o5 " + " ".join(f"i{j}" for j in range(1, 14)),
+                           [0, None, 1, 2, None, 3, 4, None, 5, 6, None, None, None, None], [True] + [False] * 5)
 
 
 def lora_mlp(x, gate, up, down, act: str = "silu"):
@@ -345,8 +271,8 @@ def lora_mlp(x, gate, up, down, act: str = "silu"):
         h = opake_swiglu(g, u) if act == "silu" else opake_geglu(g, u)
         return lora_linear(h, *down)
     lead = x.shape[:-1]
-    y = _LoRAMLP.apply(x.reshape(-1, x.shape[-1]), gate[0], gate[1], gate[2], up[0], up[1], up[2], down[0], down[1], down[2],
-                       float(gate[3]), float(up[3]), float(down[3]), "silu" if act == "silu" else "gelu_tanh")[0]
+    y = _LoRAMLP(x.reshape(-1, x.shape[-1]), gate[0], gate[1], gate[2], up[0], up[1], up[2], down[0], down[1], down[2],
+                 float(gate[3]), float(up[3]), float(down[3]), "silu" if act == "silu" else "gelu_tanh")[0]
     return y.view(*lead, -1)
 
 
