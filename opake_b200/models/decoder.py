@@ -253,18 +253,19 @@ class DecoderRuntime:
         return s
 
     # ------------------------------------------------------------------ second stream for weight gradients
-    def _wgrad(self, dy, x, out, sumsq=None, main: bool = False) -> None:
-        """``out = dy^T x`` (+ squared norm) ordered after everything issued so far, on the weight-gradient stream (``main``: on
-        the current one). ``out [n, N, K]``: the rows are ``n`` sequences, each with a gradient (and norm) of its own."""
+    def _wgrad(self, dy, x, out, sumsq=None, bias=None) -> None:
+        """``out = dy^T x`` (+ squared norm; + ``bias += column sums of dy``) ordered after everything issued so far, on the
+        weight-gradient stream. ``out [n, N, K]``: the rows are ``n`` sequences, each with a gradient (and norm) of its own."""
+        rows = dy
         if out.dim() == 3:
             dy, x = dy.unflatten(0, (out.shape[0], -1)), x.unflatten(0, (out.shape[0], -1))
-        side = None if main else self._wstream
-        if side is None:
+
+        def run():
             G.linear_wgrad(dy, x, out=out, sumsq=sumsq)
-            return
-        side.wait_stream(torch.cuda.current_stream(self.device))
-        with torch.cuda.stream(side):
-            G.linear_wgrad(dy, x, out=out, sumsq=sumsq)
+            if bias is not None:
+                K.colsum_(rows, bias)
+
+        self._wgrad_call(run)
 
     def _grads(self, slot: int, n: int) -> tuple[dict, torch.Tensor]:
         """Gradient views and squared norms of slots ``slot .. slot+n-1``; several slots: stacked, ``[n, *shape]``."""
@@ -504,20 +505,15 @@ class DecoderRuntime:
                 dxn2 = G.gemm(dgu, w[p + "wgu"], b_mn=True, out=ws["dx2"])
                 self._wgrad_join()            # the norm backward below overwrites dx in place
             else:
-                self._wgrad(dx, a["act"], g[p + "wproj"], sumsq, main=True)
-                if cfg.bias:
-                    K.colsum_(dx, self._vec(ws, p + "bproj"))
+                self._wgrad(dx, a["act"], g[p + "wproj"], sumsq, self._vec(ws, p + "bproj") if cfg.bias else None)
                 dact = G.gemm(dx, w[p + "wproj"], b_mn=True, out=ws["dact"])
                 dfc = K.gelu_bwd(dact, a["fc"], out=ws["dwide"])
-                self._wgrad(dfc, a["xn2"], g[p + "wfc"], sumsq, main=True)
-                if cfg.bias:
-                    K.colsum_(dfc, self._vec(ws, p + "bfc"))
+                self._wgrad(dfc, a["xn2"], g[p + "wfc"], sumsq, self._vec(ws, p + "bfc") if cfg.bias else None)
                 dxn2 = G.gemm(dfc, w[p + "wfc"], b_mn=True, out=ws["dx2"])
+                self._wgrad_join()            # the norm backward below overwrites dx in place
             dx_mid = self._norm_bwd(ws, dxn2, a["x_mid"], p + "norm2", st2, dx, ws["dx"])  # in place over dres
             # ---- attention
-            self._wgrad(dx_mid, a["attn"], g[p + "wo"], sumsq)
-            if cfg.bias:
-                K.colsum_(dx_mid, self._vec(ws, p + "bo"))
+            self._wgrad(dx_mid, a["attn"], g[p + "wo"], sumsq, self._vec(ws, p + "bo") if cfg.bias else None)
             dattn = G.gemm(dx_mid, w[p + "wo"], b_mn=True, out=ws["dattn"])
             dqkv = ws["dqkv"]
             A.attention_bwd(dattn, a["qkv"], a["attn"], actx, H, KV, hd, dqkv)
@@ -541,9 +537,7 @@ class DecoderRuntime:
                               dw=self._vec(ws, p + "q_norm.weight"), scratch=self._scratch(ws), out=dqkv[:, :nq])
                 K.rmsnorm_bwd(dqkv[:, nq : nq + nk], a["qk_raw"][:, nq:], w[p + "k_norm.weight"], stq[1],
                               dw=self._vec(ws, p + "k_norm.weight"), scratch=self._scratch(ws), out=dqkv[:, nq : nq + nk])
-            self._wgrad(dqkv, a["xn"], g[p + "wqkv"], sumsq)
-            if cfg.bias or cfg.qkv_bias:
-                K.colsum_(dqkv, self._vec(ws, p + "bqkv"))
+            self._wgrad(dqkv, a["xn"], g[p + "wqkv"], sumsq, self._vec(ws, p + "bqkv") if cfg.bias or cfg.qkv_bias else None)
             dxn = G.gemm(dqkv, w[p + "wqkv"], b_mn=True, out=ws["dx2"])
             self._wgrad_join()                # dx_mid (read by the wo gradient) is overwritten in place below
             dx = self._norm_bwd(ws, dxn, a["x"], p + "norm1", st1, dx_mid, ws["dx"])
