@@ -133,23 +133,29 @@ __global__ void __launch_bounds__(256) moe_route_bwd_kernel(const float* __restr
 // that expert), then every warp walks its chunk in order, 32 entries at a time, lanes with the same expert finding
 // each other with match.any. Segments are padded to multiples of 128 rows and are at least 128 rows long (an expert
 // without tokens still owns one all-zero tile, so its weight gradient is produced as exact zeros by the GEMM).
-__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, int n_entries, int E, int r_cap,
+//
+// With several examples (of equal numbers of entries, one after the other) the sort key is (expert, example): an expert's rows
+// are still one segment, the range of the forward and input-gradient products, in which every example's rows are padded to a
+// multiple of 64 (at least 64): whole blocks of the reduction, so that group_k[example][expert] gives the range of the example's
+// own weight gradient. The rows of an example meet the same blocks in the same order as in a plan of its own.
+__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, int n_entries, int E, int examples, int r_cap,
                                                         int* __restrict__ dest, int* __restrict__ src_entry,
                                                         int* __restrict__ tile_group, int* __restrict__ group_k,
                                                         int* __restrict__ counts_out) {
-  __shared__ int hist[32][MAX_E];     // [warp][expert]; becomes the next free row of (warp, expert)
+  __shared__ int hist[32][MAX_E];     // [warp][key]; becomes the next free row of (warp, key); keys = expert * examples + example
   __shared__ int counts[MAX_E];
   __shared__ int offs[MAX_E + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int keys = E * examples, per_example = n_entries / examples;
   for (int i = threadIdx.x; i < 32 * MAX_E; i += blockDim.x) (&hist[0][0])[i] = 0;
   __syncthreads();
   const int chunk = ((n_entries + 31) / 32 + 31) / 32 * 32;   // entries per warp, a multiple of 32
   const int c0 = warp * chunk, c1 = min(c0 + chunk, n_entries);
   // an expert id outside [0, E) is dropped from the plan (its dest stays -1): never an index past the histograms
   for (int n = c0 + lane; n < c1; n += 32)
-    if (OPK_IDX_OK(idx[n], E) && (unsigned)idx[n] < (unsigned)E) atomicAdd(&hist[warp][idx[n]], 1);
+    if (OPK_IDX_OK(idx[n], E) && (unsigned)idx[n] < (unsigned)E) atomicAdd(&hist[warp][idx[n] * examples + n / per_example], 1);
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+  for (int e = threadIdx.x; e < keys; e += blockDim.x) {
     int run = 0;
     for (int w = 0; w < 32; ++w) {
       const int c = hist[w][e];
@@ -162,29 +168,35 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
   if (threadIdx.x == 0) {
     int off = 0;
     for (int e = 0; e < E; ++e) {
-      offs[e] = off;
-      const int padded = counts[e] == 0 ? 128 : (counts[e] + 127) / 128 * 128;
-      group_k[2 * e] = off;
-      group_k[2 * e + 1] = padded / 64;
-      off += padded;
-      if (counts_out) counts_out[e] = counts[e];
+      int all = 0;
+      for (int j = 0; j < examples; ++j) {
+        const int key = e * examples + j, c = counts[key], unit = examples == 1 ? 128 : 64;
+        const int padded = c == 0 ? unit : (c + unit - 1) / unit * unit;
+        offs[key] = off;
+        group_k[2 * (j * E + e)] = off;
+        group_k[2 * (j * E + e) + 1] = padded / 64;
+        off += padded;
+        all += c;
+      }
+      off = (off + 127) / 128 * 128;
+      if (counts_out) counts_out[e] = all;
     }
-    offs[E] = off;
+    offs[keys] = off;
   }
   __syncthreads();
-  const int total = offs[E];
+  const int total = offs[keys];
   // tile -> expert table, padding rows of every segment, everything past the last segment
-  for (int e = warp; e < E; e += 32) {
-    for (int tl = offs[e] / 128 + lane; tl < offs[e + 1] / 128; tl += 32) tile_group[tl] = e;
+  for (int e = warp; e < E; e += 32)
+    for (int tl = offs[e * examples] / 128 + lane; tl < (offs[(e + 1) * examples]) / 128; tl += 32) tile_group[tl] = e;
+  for (int e = warp; e < keys; e += 32)
     for (int r = offs[e] + counts[e] + lane; r < offs[e + 1]; r += 32) src_entry[r] = -1;
-  }
   for (int tl = total / 128 + threadIdx.x; tl < r_cap / 128; tl += blockDim.x) tile_group[tl] = -1;
   for (int r = total + threadIdx.x; r < r_cap; r += blockDim.x) src_entry[r] = -1;
   for (int base = c0; base < c1; base += 32) {
     const int n = base + lane;
     const bool valid = n < c1 && (unsigned)idx[n < c1 ? n : c0] < (unsigned)E;
     if (n < c1 && !valid) dest[n] = -1;
-    const int e = valid ? idx[n] : -1 - lane;                 // invalid lanes match nobody
+    const int e = valid ? idx[n] * examples + n / per_example : -1 - lane;      // invalid lanes match nobody
     const unsigned m = __match_any_sync(0xffffffffu, e);
     if (valid) {
       const int row = offs[e] + hist[warp][e] + __popc(m & ((1u << lane) - 1u));
@@ -311,12 +323,18 @@ extern "C" int opk_moe_route_bwd(const float* probs, const int32_t* idx, const f
   return (int)cudaGetLastError();
 }
 
-extern "C" int opk_moe_rows_capacity(int n_entries, int E) { return (n_entries + 127) / 128 * 128 + E * 128; }
+extern "C" int opk_moe_rows_capacity(int n_entries, int E, int examples) {
+  if (examples <= 1) return (n_entries + 127) / 128 * 128 + E * 128;
+  return (n_entries + E * 64 * (examples + 1) + 127) / 128 * 128;      // 64 rows of padding per part and per expert
+}
 
-extern "C" int opk_moe_plan(const int32_t* idx, int n_entries, int E, int r_cap, int32_t* dest, int32_t* src_entry,
+extern "C" int opk_moe_plan(const int32_t* idx, int n_entries, int E, int examples, int r_cap, int32_t* dest, int32_t* src_entry,
                             int32_t* tile_group, int32_t* group_k, int32_t* counts, void* stream) {
-  if (E > MAX_E || r_cap % 128 || r_cap < opk_moe_rows_capacity(n_entries, E)) return -1;
-  moe_plan_kernel<<<1, 1024, 0, ST(stream)>>>(idx, n_entries, E, r_cap, dest, src_entry, tile_group, group_k, counts);
+  if (E < 1 || examples < 1 || E > MAX_E / examples || n_entries % examples || r_cap % 128 ||
+      r_cap < opk_moe_rows_capacity(n_entries, E, examples))
+    return -1;
+  if (n_entries == 0 && examples > 1) return -1;
+  moe_plan_kernel<<<1, 1024, 0, ST(stream)>>>(idx, n_entries, E, examples, r_cap, dest, src_entry, tile_group, group_k, counts);
   return (int)cudaGetLastError();
 }
 

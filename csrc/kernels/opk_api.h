@@ -252,10 +252,11 @@ int opk_moe_route(const void* logits, int64_t ld, int T, int E, int k, int norm_
 int opk_moe_route_bwd(const float* probs, const int32_t* idx, const float* dwts, int T, int E, int k, int norm_topk,
                       void* dlogits, int64_t ld, void* stream);
 // Worst-case number of rows of the expert-sorted buffers for n_entries = T*k routed entries.
-int opk_moe_rows_capacity(int n_entries, int E);
+int opk_moe_rows_capacity(int n_entries, int E, int examples);
 // Stable sort of the entries by expert into 128-row aligned segments. dest[n] = row of entry n; src_entry[row] = entry
-// or -1 (padding); tile_group[r_cap/128] and group_k[E][2] are the tables of the grouped GEMM modes; counts[E] optional.
-int opk_moe_plan(const int32_t* idx, int n_entries, int E, int r_cap, int32_t* dest, int32_t* src_entry, int32_t* tile_group,
+// or -1 (padding); tile_group[r_cap/128] and group_k[examples][E][2] are the tables of the grouped GEMM modes; counts[E] optional.
+// The entries are those of `examples` examples of equal size, one after the other (E * examples <= 256).
+int opk_moe_plan(const int32_t* idx, int n_entries, int E, int examples, int r_cap, int32_t* dest, int32_t* src_entry, int32_t* tile_group,
                  int32_t* group_k, int32_t* counts, void* stream);
 // out[row] = entry_scale[n] * x[n / k] for n = src_entry[row] (zeros when n < 0); bf16 rows of D elements.
 int opk_moe_gather(const void* x, int64_t ldx, const int32_t* src_entry, int k, const float* entry_scale, int R, int D, void* out,

@@ -104,9 +104,10 @@ class DecoderRuntime:
         return self.gs[0]
 
     def can_join(self) -> bool:
-        """Whether several sequences can go through the model in one pass: dense blocks, native attention, slots in one buffer."""
+        """Whether several sequences can go through the model in one pass: experts of its own, native attention, slots in one
+        buffer."""
         impl = A.resolve_impl(self.cfg.head_dim) if self.attn_impl == "auto" else self.attn_impl
-        return self.G_all is not None and not self.cfg.n_experts and impl == "flash" and self.device.type == "cuda"
+        return self.G_all is not None and self.ep is None and impl == "flash" and self.device.type == "cuda"
 
     @property
     def sumsq(self):
@@ -153,7 +154,7 @@ class DecoderRuntime:
             if cfg.n_experts and self.ep is not None:
                 pass        # token rows, pre-activations and routing state live in the expert-parallel layers
             elif cfg.n_experts:
-                plan = K.MoePlan(T, cfg.n_experts, cfg.top_k, dev)
+                plan = K.MoePlan(T, cfg.n_experts, cfg.top_k, dev, examples=n)
                 I = cfg.expert_ffn
                 a.update(plan=plan, rlogits=e(T, cfg.n_experts), xs=e(plan.R, d), gu=e(plan.R, 2 * I), act=e(plan.R, I),
                          ye=e(plan.R, d))
@@ -205,7 +206,16 @@ class DecoderRuntime:
             return out
         out = self._parts[(ws["key"], n)] = dict(ws, n=n)
         rows = n * ws["key"][0]
-        out["layers"] = [{k: v[:rows] for k, v in a.items()} for a in ws["layers"]]
+        layers, plans = [], [a["plan"].part(n) for a in ws["layers"] if "plan" in a]
+        for li, a in enumerate(ws["layers"]):
+            cut = {k: v[: plans[li].R if k in ("xs", "gu", "act", "ye") and plans else rows] for k, v in a.items() if k != "plan"}
+            layers.append(dict(cut, plan=plans[li]) if plans else cut)
+        out["layers"] = layers
+        if plans:
+            for k in ("dye", "dgu", "dxs"):
+                out[k] = ws[k][: plans[0].R]
+            for k in ("dwts", "drl"):
+                out[k] = ws[k][:rows]
         for k in ("x_last", "xf", "pmax", "psum", "tgt", "dlogits", "dx", "dx2", "dact", "dqkv", "dwide", "dattn", "labels", "coef"):
             out[k] = ws[k][:rows]
         for k in ("vec", "loss", "ntok"):
@@ -264,6 +274,15 @@ class DecoderRuntime:
             G.linear_wgrad(dy, x, out=out, sumsq=sumsq)
             if bias is not None:
                 K.colsum_(rows, bias)
+
+        self._wgrad_call(run)
+
+    def _wgrad_experts(self, dy, x, out, plan, sumsq) -> None:
+        def run():
+            for j in range(plan.examples):
+                one = plan.examples == 1
+                G.gemm(dy, x, a_mn=True, b_mn=True, out=out if one else out[j], epilogue=G.EPI_SUMSQ, sumsq=sumsq[j : j + 1],
+                       group_k=plan.group_k if one else plan.group_k[j], sumsq_shared=True)
 
         self._wgrad_call(run)
 
@@ -480,17 +499,16 @@ class DecoderRuntime:
                 plan = a["plan"]
                 K.moe_combine_bwd(dx, a["ye"], plan, ws["dwts"])
                 K.moe_gather(dx, plan, ws["dye"], entry_scale=plan.wts)
-                # expert weight gradients: one grouped GEMM per matrix, reduction range of expert e = its row segment
-                self._wgrad_call(lambda: G.gemm(ws["dye"], a["act"], a_mn=True, b_mn=True, out=g[p + "experts.wd"],
-                                                epilogue=G.EPI_SUMSQ, sumsq=sumsq, group_k=plan.group_k, sumsq_shared=True))
+                # expert weight gradients: one grouped GEMM per matrix and example, reduction range of expert e = the example's
+                # rows in its segment
+                self._wgrad_experts(ws["dye"], a["act"], g[p + "experts.wd"], plan, sumsq)
                 G.swiglu_dgrad(ws["dye"], w[p + "experts.wd"], a["gu"], out=ws["dgu"], tile_group=plan.tile_group)
-                self._wgrad_call(lambda: G.gemm(ws["dgu"], a["xs"], a_mn=True, b_mn=True, out=g[p + "experts.wgu"],
-                                                epilogue=G.EPI_SUMSQ, sumsq=sumsq, group_k=plan.group_k, sumsq_shared=True))
+                self._wgrad_experts(ws["dgu"], a["xs"], g[p + "experts.wgu"], plan, sumsq)
                 G.gemm(ws["dgu"], w[p + "experts.wgu"], b_mn=True, out=ws["dxs"], tile_group=plan.tile_group)
                 dxn2 = K.moe_combine(ws["dxs"], plan, ws["dx2"])
                 # router: d weights -> d logits -> router weight gradient and the second path into dxn2
                 K.moe_route_bwd(plan, ws["dwts"], ws["drl"], cfg.norm_topk_prob)
-                G.linear_wgrad(ws["drl"], a["xn2"], out=g[p + "router"], sumsq=sumsq)
+                self._wgrad(ws["drl"], a["xn2"], g[p + "router"], sumsq)
                 G.gemm(ws["drl"], w[p + "router"], b_mn=True, out=dxn2, residual=dxn2)
                 self._wgrad_join()            # dye / dgu are rewritten by the next layer, dx by the norm backward below
             elif cfg.act in ("swiglu", "geglu"):

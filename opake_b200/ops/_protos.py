@@ -79,8 +79,8 @@ PROTOTYPES: dict = {
     "opk_sumsq": (I, [P, I, I, L, P, I, L, P]),
     "opk_moe_route": (I, [P, L, I, I, I, I, P, P, P, P]),
     "opk_moe_route_bwd": (I, [P, P, P, I, I, I, I, P, L, P]),
-    "opk_moe_rows_capacity": (I, [I, I]),
-    "opk_moe_plan": (I, [P, I, I, I, P, P, P, P, P, P]),
+    "opk_moe_rows_capacity": (I, [I, I, I]),
+    "opk_moe_plan": (I, [P, I, I, I, I, P, P, P, P, P, P]),
     "opk_moe_gather": (I, [P, L, P, I, P, I, I, P, P]),
     "opk_moe_combine": (I, [P, P, P, I, P, I, I, P, P]),
     "opk_moe_combine_bwd": (I, [P, P, P, I, I, I, P, P]),

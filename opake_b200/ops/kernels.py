@@ -416,12 +416,15 @@ def dp_step(*, grad_src: list[int], shard_begin: int, shard_len: int, inv_batch:
 
 # ------------------------------------------------------------------------------------------------ mixture of experts
 class MoePlan:
-    """Device-side routing state of one MoE layer invocation (buffers are reused across examples)."""
+    """Device-side routing state of one MoE layer invocation (buffers are reused across examples). ``T`` tokens are those of
+    ``examples`` sequences of equal length, one after the other; ``group_k [E, 2]``, or ``[examples, E, 2]`` for several."""
 
-    def __init__(self, T: int, E: int, k: int, device):
-        self.T, self.E, self.k = T, E, k
+    def __init__(self, T: int, E: int, k: int, device, examples: int = 1):
+        if examples > 1 and (T % examples or E * examples > 256):
+            raise ValueError("examples of equal length, and at most 256 pairs of expert and example")
+        self.T, self.E, self.k, self.examples = T, E, k, examples
         self.n = T * k
-        self.R = _L().opk_moe_rows_capacity(self.n, E)
+        self.R = _L().opk_moe_rows_capacity(self.n, E, examples)
         i32 = dict(dtype=torch.int32, device=device)
         self.idx = torch.empty(T, k, **i32)
         self.wts = torch.empty(T, k, dtype=torch.float32, device=device)
@@ -429,14 +432,25 @@ class MoePlan:
         self.dest = torch.empty(T, k, **i32)
         self.src_entry = torch.empty(self.R, **i32)
         self.tile_group = torch.empty(self.R // 128, **i32)
-        self.group_k = torch.empty(E, 2, **i32)
+        self.group_k = torch.empty(*(() if examples == 1 else (examples,)), E, 2, **i32)
         self.counts = torch.empty(E, **i32)
+
+    def part(self, examples: int) -> "MoePlan":
+        """Plan for the first ``examples`` sequences, in the same buffers."""
+        p = object.__new__(MoePlan)
+        p.T, p.E, p.k, p.examples = self.T // self.examples * examples, self.E, self.k, examples
+        p.n = p.T * p.k
+        p.R = _L().opk_moe_rows_capacity(p.n, p.E, examples)
+        p.idx, p.wts, p.probs, p.dest = (t[: p.T] for t in (self.idx, self.wts, self.probs, self.dest))
+        p.src_entry, p.tile_group, p.counts = self.src_entry[: p.R], self.tile_group[: p.R // 128], self.counts
+        p.group_k = self.group_k[0] if examples == 1 else self.group_k[:examples]
+        return p
 
     def build(self, idx: torch.Tensor) -> "MoePlan":
         """Row plan for expert ids chosen by the caller (``[T, k]`` int32). Ids outside ``[0, E)`` are dropped: their
         ``dest`` entry becomes -1 and the combine kernels skip them."""
         self.idx.copy_(idx.reshape(self.T, self.k))
-        _chk(_L().opk_moe_plan(_p(self.idx), self.n, self.E, self.R, _p(self.dest), _p(self.src_entry), _p(self.tile_group),
+        _chk(_L().opk_moe_plan(_p(self.idx), self.n, self.E, self.examples, self.R, _p(self.dest), _p(self.src_entry), _p(self.tile_group),
                                _p(self.group_k), _p(self.counts), _s(self.idx)), "moe_plan")
         return self
 
@@ -445,7 +459,7 @@ def moe_route(logits, plan: MoePlan, norm_topk: bool = False):
     T, E = logits.shape
     _chk(_L().opk_moe_route(_p(logits), logits.stride(0), T, E, plan.k, int(norm_topk), _p(plan.idx), _p(plan.wts), _p(plan.probs),
                             _s(logits)), "moe_route")
-    _chk(_L().opk_moe_plan(_p(plan.idx), plan.n, E, plan.R, _p(plan.dest), _p(plan.src_entry), _p(plan.tile_group), _p(plan.group_k),
+    _chk(_L().opk_moe_plan(_p(plan.idx), plan.n, E, plan.examples, plan.R, _p(plan.dest), _p(plan.src_entry), _p(plan.tile_group), _p(plan.group_k),
                            _p(plan.counts), _s(logits)), "moe_plan")
     return plan
 

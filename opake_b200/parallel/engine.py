@@ -324,7 +324,10 @@ class ShardedDPEngine:
         if self.world > 1 or not self.runtime.can_join():
             return 1
         most = self._join_limit.get(T, self.group)
-        return max(1, min(most, _JOIN_VALUES // (T * self.model_cfg.d_model)))
+        n = min(most, _JOIN_VALUES // (T * self.model_cfg.d_model))
+        if self.model_cfg.n_experts:
+            n = min(n, 256 // self.model_cfg.n_experts)      # pairs of expert and example that a routing plan holds
+        return max(1, n)
 
     def _step_workspace(self, T: int) -> tuple[int, dict]:
         """Examples per pass for this length and their workspace: one by one where several do not fit the memory."""

@@ -37,11 +37,11 @@ def _model(name):
     from opake_b200.models.config import gpt2_small, tiny_llama
 
     return {"llama": tiny_llama(), "tied": tiny_llama(tie_embeddings=True, qk_norm="head"), "wide norm": tiny_llama(qk_norm=True, qkv_bias=True),
-            "geglu": tiny_llama(act="geglu"),
+            "geglu": tiny_llama(act="geglu"), "experts": tiny_llama(n_experts=8, top_k=2, expert_ffn=64, qk_norm=True),
             "gpt2": replace(gpt2_small(), vocab_size=515, d_model=192, n_layers=2, n_heads=3, n_kv_heads=3, ffn=768, max_seq=320)}[name]
 
 
-@pytest.mark.parametrize("name", ["llama", "tied", "wide norm", "geglu", "gpt2"])
+@pytest.mark.parametrize("name", ["llama", "tied", "wide norm", "geglu", "gpt2", "experts"])
 @pytest.mark.parametrize("T,graph", [(33, True), (128, False), (300, True)])
 def test_steps_equal_those_of_single_examples(cuda, name, T, graph, monkeypatch):
     """Groups of three, joined in twos, whole and partial: losses, norms, gradients and updates. RMSNorm models to the bit;
@@ -94,3 +94,33 @@ def test_norms_of_several_gradients_in_one_launch(cuda, batch, N):
         one = torch.zeros(1, dtype=torch.float64, device=cuda)
         assert torch.equal(G.linear_wgrad(dy[j], x[j], sumsq=one), out[j])
         assert abs(one.item() - sums[j].item()) <= 1e-12 * one.item()
+
+
+@pytest.mark.parametrize("E,k,examples,T", [(8, 2, 2, 33), (64, 8, 4, 200), (3, 1, 3, 1), (128, 4, 2, 65)])
+def test_routing_plan_of_several_examples(cuda, E, k, examples, T):
+    """Rows sorted by expert, then example, in order; parts of whole 64-row blocks (empty ones too), segments of whole tiles; a
+    plan for the first example alone in the same buffers."""
+    from opake_b200.ops import kernels as K
+
+    plan = K.MoePlan(examples * T, E, k, cuda, examples=examples)
+    idx = torch.randint(0, max(1, E - 1), (examples * T, k), dtype=torch.int32)          # the last expert gets nothing
+    idx[::7, 0] = E                                                                       # dropped
+    for n in (examples, 1):
+        p = plan.part(n) if n < examples else plan
+        p.build(idx[: n * T].to(cuda))
+        unit, off, flat = (64 if n > 1 else 128), 0, idx[: n * T].reshape(-1).tolist()
+        src, dest = torch.full((p.R,), -1), torch.full((len(flat),), -1)
+        gk, tiles = torch.zeros(n, E, 2), torch.full((p.R // 128,), -1)
+        for e in range(E):
+            start = off
+            for j in range(n):
+                rows = [i for i in range(j * T * k, (j + 1) * T * k) if flat[i] == e]
+                for r, i in enumerate(rows):
+                    src[off + r], dest[i] = i, off + r
+                padded = max(unit, -(-len(rows) // unit) * unit)
+                gk[j, e] = torch.tensor([off, padded // 64])
+                off += padded
+            off = -(-off // 128) * 128
+            tiles[start // 128 : off // 128] = e
+        assert torch.equal(p.src_entry.cpu().long(), src) and torch.equal(p.dest.cpu().long().reshape(-1), dest)
+        assert torch.equal(p.group_k.cpu().float().reshape(n, E, 2), gk) and torch.equal(p.tile_group.cpu().long(), tiles)
