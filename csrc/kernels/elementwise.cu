@@ -65,18 +65,21 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __
                                                          const __nv_bfloat16* __restrict__ w,
                                                          __nv_bfloat16* __restrict__ sum_out,
                                                          __nv_bfloat16* __restrict__ y, float* __restrict__ rstd,
-                                                         int D, float eps, float w_off, long long ldx, long long ldy) {
+                                                         int D, float eps, float w_off, long long ldx, long long ldy,
+                                                         long long ld_sum) {
   opk::pdl_trigger();
   __shared__ float sh[32];
   const long long row = blockIdx.x;
   const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * ldx);
   const bf16x8* rr = ADD ? reinterpret_cast<const bf16x8*>(r + row * D) : nullptr;
-  bf16x8* sr = ADD ? reinterpret_cast<bf16x8*>(sum_out + row * D) : nullptr;
+  bf16x8* sr = sum_out ? reinterpret_cast<bf16x8*>(sum_out + row * ld_sum) : nullptr;     // without ADD: a copy of x
   const int nv = D >> 3;
   float ss = 0.f;
   for (int i = threadIdx.x; i < nv; i += NT) {
     float f[8];
-    unpack8(xr[i], f);
+    const bf16x8 in = xr[i];
+    unpack8(in, f);
+    if (!ADD && sr) sr[i] = in;
     if (ADD) {
       float g[8];
       unpack8(rr[i], g);
@@ -108,11 +111,15 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __
 // One warp per row, the row held in registers (VPL vectors of 8 per lane): one pass over memory, no block barrier.
 // (Without the opaque barrier below the compiler keeps the row UNPACKED across the reduction, 255 registers per thread at
 // 16 vectors per lane: one CTA per SM and 12 % of the warp slots in use. Packed, the row is 64 registers.)
+//
+// `copy` (optional) receives the row as it was read, for a norm in place whose input the backward pass needs (query and key columns
+// of a fused projection: 4096 x 4096 values took 107 us in a strided copy of their own, 428 us of a 22.6 ms OLMoE step).
 template <int VPL>
 __global__ void __launch_bounds__(256, VPL >= 16 ? 2 : 4) rmsnorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ w,
                                                                __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int T,
-                                                               float eps, float w_off, long long ldx, long long ldy) {
+                                                               float eps, float w_off, long long ldx, long long ldy,
+                                                               __nv_bfloat16* __restrict__ copy, long long ld_copy) {
   opk::pdl_trigger();
   constexpr int D = VPL * 32 * 8;
   const int lane = threadIdx.x & 31;
@@ -122,6 +129,11 @@ __global__ void __launch_bounds__(256, VPL >= 16 ? 2 : 4) rmsnorm_fwd_warp_kerne
   bf16x8 v[VPL];
 #pragma unroll
   for (int i = 0; i < VPL; ++i) v[i] = xr[lane + 32 * i];
+  if (copy) {
+    bf16x8* cr = reinterpret_cast<bf16x8*>(copy + row * ld_copy);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) cr[lane + 32 * i] = v[i];
+  }
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
@@ -1252,24 +1264,25 @@ inline int grid_for(long long n, int block, int cap_blocks = 148 * 16) {
 #define BFM(p) reinterpret_cast<__nv_bfloat16*>(p)
 
 extern "C" int opk_rmsnorm_fwd_ld(const void* x, int64_t ldx, const void* w, void* y, int64_t ldy, float* rstd, int T, int D,
-                                  float eps, float w_offset, void* stream) {
+                                  float eps, float w_offset, void* copy, int64_t ld_copy, void* stream) {
   if (T <= 0) return 0;
   if (D % 8 || ldx % 8 || ldy % 8 || ldx < D || ldy < D) return -1;
+  if (copy && (ld_copy % 8 || ld_copy < D || (reinterpret_cast<uintptr_t>(copy) & 15))) return -1;
   const int warp_grid = (T + 7) / 8;
   if (D == 4096)
-    rmsnorm_fwd_warp_kernel<16><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy);
+    rmsnorm_fwd_warp_kernel<16><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy, BFM(copy), ld_copy);
   else if (D == 2048)
-    rmsnorm_fwd_warp_kernel<8><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy);
+    rmsnorm_fwd_warp_kernel<8><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy, BFM(copy), ld_copy);
   else if (D == 1024)
-    rmsnorm_fwd_warp_kernel<4><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy);
+    rmsnorm_fwd_warp_kernel<4><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy, BFM(copy), ld_copy);
   else
-    rmsnorm_fwd_kernel<false><<<T, NT, 0, ST(stream)>>>(BF(x), nullptr, BF(w), nullptr, BFM(y), rstd, D, eps, w_offset, ldx, ldy);
+    rmsnorm_fwd_kernel<false><<<T, NT, 0, ST(stream)>>>(BF(x), nullptr, BF(w), BFM(copy), BFM(y), rstd, D, eps, w_offset, ldx, ldy, ld_copy);
   OPK_LAUNCH_CHECK();
   return 0;
 }
 extern "C" int opk_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int T, int D, float eps,
                                float w_offset, void* stream) {
-  return opk_rmsnorm_fwd_ld(x, D, w, y, D, rstd, T, D, eps, w_offset, stream);
+  return opk_rmsnorm_fwd_ld(x, D, w, y, D, rstd, T, D, eps, w_offset, nullptr, 0, stream);
 }
 extern "C" int opk_add_rmsnorm_fwd(const void* x, const void* r, const void* w, void* sum_out, void* y, float* rstd,
                                    int T, int D, float eps, float w_offset, void* stream) {
@@ -1282,7 +1295,7 @@ extern "C" int opk_add_rmsnorm_fwd(const void* x, const void* r, const void* w, 
   else if (D <= 8192)
     add_rmsnorm_fwd_kernel<4><<<T, NT, 0, ST(stream)>>>(BF(x), BF(r), BF(w), BFM(sum_out), BFM(y), rstd, D, eps, w_offset);
   else
-    rmsnorm_fwd_kernel<true><<<T, NT, 0, ST(stream)>>>(BF(x), BF(r), BF(w), BFM(sum_out), BFM(y), rstd, D, eps, w_offset, D, D);
+    rmsnorm_fwd_kernel<true><<<T, NT, 0, ST(stream)>>>(BF(x), BF(r), BF(w), BFM(sum_out), BFM(y), rstd, D, eps, w_offset, D, D, D);
   OPK_LAUNCH_CHECK();
   return 0;
 }

@@ -72,9 +72,9 @@ const char* opk_last_error(void);
 int opk_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, int T, int D, float eps, float w_offset,
                     void* stream);
 // The same with row pitches (elements): normalises a column slice of a wider matrix, e.g. the query part of a fused
-// QKV activation. x and y may alias.
+// QKV activation. x and y may alias; copy (optional) receives x.
 int opk_rmsnorm_fwd_ld(const void* x, int64_t ldx, const void* w, void* y, int64_t ldy, float* rstd, int T, int D, float eps,
-                       float w_offset, void* stream);
+                       float w_offset, void* copy, int64_t ld_copy, void* stream);
 // `batch` examples of T rows one after the other, each with a weight gradient of its own (dw_stride floats apart).
 int opk_rmsnorm_bwd_ld(const void* dy, int64_t ld_dy, const void* x, int64_t ldx, const void* w, const float* rstd,
                        const void* dres, void* dx_out, int64_t ld_dx, float* dw, float* workspace, int ws_rows, int T, int D,

@@ -383,9 +383,9 @@ class DecoderRuntime:
                 stq = (rq, rk)
             elif cfg.qk_norm:
                 nq, nk = H * hd, KV * hd
-                a["qk_raw"].copy_(a["qkv"][:, : nq + nk])
-                _, rq = K.rmsnorm_fwd(a["qk_raw"][:, :nq], w[p + "q_norm.weight"], cfg.norm_eps, out=a["qkv"][:, :nq])
-                _, rk = K.rmsnorm_fwd(a["qk_raw"][:, nq:], w[p + "k_norm.weight"], cfg.norm_eps, out=a["qkv"][:, nq : nq + nk])
+                q, k = a["qkv"][:, :nq], a["qkv"][:, nq : nq + nk]                    # in place; the backward pass reads the copies
+                _, rq = K.rmsnorm_fwd(q, w[p + "q_norm.weight"], cfg.norm_eps, out=q, copy=a["qk_raw"][:, :nq])
+                _, rk = K.rmsnorm_fwd(k, w[p + "k_norm.weight"], cfg.norm_eps, out=k, copy=a["qk_raw"][:, nq:])
                 stq = (rq, rk)
             if cfg.pos == "rope":
                 K.rope_(a["qkv"], self._rope_table(seq), H + KV, hd, period=period)

@@ -53,7 +53,7 @@ PROTOTYPES: dict = {
     "opk_lce_logits_floats": (L, [I, I]),
     "opk_lce_grad": (I, [P, P, P, P, P, L, I, I, F, P]),
     "opk_rmsnorm_fwd": (I, [P, P, P, P, I, I, F, F, P]),
-    "opk_rmsnorm_fwd_ld": (I, [P, L, P, P, L, P, I, I, F, F, P]),
+    "opk_rmsnorm_fwd_ld": (I, [P, L, P, P, L, P, I, I, F, F, P, L, P]),
     "opk_rmsnorm_bwd_ld": (I, [P, L, P, L, P, P, P, P, L, P, P, I, I, I, F, I, L, P]),
     "opk_add_rmsnorm_fwd": (I, [P, P, P, P, P, P, I, I, F, F, P]),
     "opk_rmsnorm_bwd": (I, [P, P, P, P, P, P, P, P, I, I, I, F, P]),

@@ -36,13 +36,14 @@ def _chk(code: int, name: str) -> None:
 
 
 # ------------------------------------------------------------------------------------------------ norms
-def rmsnorm_fwd(x, w, eps: float = 1e-6, w_offset: float = 0.0, out=None):
-    """``x`` and ``out`` may be column slices of wider row-major matrices (row pitch = ``stride(0)``)."""
+def rmsnorm_fwd(x, w, eps: float = 1e-6, w_offset: float = 0.0, out=None, copy=None):
+    """``x``, ``out`` and ``copy`` may be column slices of wider row-major matrices (row pitch = ``stride(0)``). ``out`` may be
+    ``x``; ``copy`` receives ``x``."""
     T, D = x.shape
     y = torch.empty_like(x) if out is None else out
     rstd = torch.empty(T, dtype=torch.float32, device=x.device)
-    _chk(_L().opk_rmsnorm_fwd_ld(_p(x), x.stride(0), _p(w), _p(y), y.stride(0), _p(rstd), T, D, eps, w_offset, _s(x)),
-         "rmsnorm_fwd")
+    _chk(_L().opk_rmsnorm_fwd_ld(_p(x), x.stride(0), _p(w), _p(y), y.stride(0), _p(rstd), T, D, eps, w_offset, _p(copy),
+                                   0 if copy is None else copy.stride(0), _s(x)), "rmsnorm_fwd")
     return y, rstd
 
 

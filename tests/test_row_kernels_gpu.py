@@ -230,3 +230,18 @@ def test_cross_entropy_of_padded_rows(cuda):
         nll2, lse2 = K.cross_entropy_fwd(zc, lab)
         d2 = K.cross_entropy_bwd(zc, lab, lse2, c)
         assert torch.allclose(nll, nll2, rtol=1e-6, atol=1e-6) and torch.allclose(d, d2, rtol=1e-5, atol=1e-7)
+
+
+@pytest.mark.parametrize("T,D", [(5, 64), (9, 1024), (33, 2048), (7, 4096), (3, 8200)])
+def test_rmsnorm_in_place_leaves_a_copy_of_its_input(cuda, T, D):
+    from opake_b200.ops import kernels as K
+
+    wide = torch.randn(T, 2 * D + 16, device=cuda).to(torch.bfloat16)
+    w = torch.randn(D, device=cuda).to(torch.bfloat16)
+    want, rstd = K.rmsnorm_fwd(wide[:, 8 : D + 8].contiguous(), w)
+    before, copies = wide.clone(), torch.zeros(T, D + 8, device=cuda, dtype=torch.bfloat16)
+    x = wide[:, 8 : D + 8]
+    _, again = K.rmsnorm_fwd(x, w, out=x, copy=copies[:, 8:])
+    assert torch.equal(copies[:, 8:], before[:, 8 : D + 8]) and not copies[:, :8].any()
+    assert torch.equal(x, want) and torch.equal(again, rstd)
+    assert torch.equal(wide[:, :8], before[:, :8]) and torch.equal(wide[:, D + 8 :], before[:, D + 8 :])
