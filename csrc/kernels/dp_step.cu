@@ -84,12 +84,13 @@ __global__ void clip_scale_kernel(double* sumsq, float clip, int mode_auto, floa
 
 struct alignas(16) bf16x8 { __nv_bfloat162 h[4]; };
 
+// a value that rounded *up* into (or within) the subnormal range would break the bound: flush it
+__device__ __forceinline__ float flush_rounded_up(float stored, float scaled) {
+  return fabsf(stored) <= 1.1754943508222875e-38f && fabsf(stored) > fabsf(scaled) ? 0.f : stored;
+}
 __device__ __forceinline__ float clip_store(float g, float s) {
   const float scaled = g * s;
-  float stored = __bfloat162float(__float2bfloat16(scaled));
-  // a value that rounded *up* into (or within) the subnormal range would break the bound: flush it
-  if (fabsf(stored) <= 1.1754943508222875e-38f && fabsf(stored) > fabsf(scaled)) stored = 0.f;
-  return stored;
+  return flush_rounded_up(__bfloat162float(__float2bfloat16(scaled)), scaled);
 }
 
 __global__ void __launch_bounds__(256) clip_accumulate_kernel(const bf16x8* __restrict__ g, const float* __restrict__ scale,
@@ -178,22 +179,47 @@ struct PeerTable {
   __nv_bfloat16* param[MAX_PEERS];
 };
 
-// One parameter update given the averaged, noised gradient. Returns the new parameter value.
+// Two lanes of fp32 arithmetic per instruction: same rounding as the scalar forms, half the issue slots.
+__device__ __forceinline__ float2 pair(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
+// Two parameter updates given the averaged, noised gradients. Returns the new parameter values.
 template <bool ADAM>
-__device__ __forceinline__ float dp_update(const OpkDpStepArgs& a, float inv_bc1, float inv_bc2, float grad, float p_old,
-                                           float& m, float& v) {
-  float upd;
+__device__ __forceinline__ float2 dp_update(const OpkDpStepArgs& a, float inv_bc1, float inv_bc2, float2 grad, float2 p_old,
+                                            float2& m, float2& v) {
+  float2 upd;
   if (!ADAM) {
-    upd = grad + a.weight_decay * p_old;
+    upd = fma2(pair(a.weight_decay), p_old, grad);
   } else {
-    m = a.beta1 * m + (1.f - a.beta1) * grad;
-    v = a.beta2 * v + (1.f - a.beta2) * grad * grad;
-    const float mh = m * inv_bc1, vh = v * inv_bc2;
-    const float d = vh - a.phi_hat;            // noise bias correction: subtract the noise's share of v-hat
-    const float den = sqrtf(d > 0.f ? d : vh) + a.eps;
-    upd = __fdividef(mh, den) + a.weight_decay * p_old;
+    m = fma2(pair(a.beta1), m, mul2(pair(1.f - a.beta1), grad));
+    v = fma2(pair(a.beta2), v, mul2(mul2(pair(1.f - a.beta2), grad), grad));
+    const float2 mh = mul2(m, pair(inv_bc1)), vh = mul2(v, pair(inv_bc2));
+    const float2 d = add2(vh, pair(-a.phi_hat));            // noise bias correction: subtract the noise's share of v-hat
+    const float2 den = add2(make_float2(sqrtf(d.x > 0.f ? d.x : vh.x), sqrtf(d.y > 0.f ? d.y : vh.y)), pair(a.eps));
+    upd = fma2(pair(a.weight_decay), p_old, make_float2(__fdividef(mh.x, den.x), __fdividef(mh.y, den.y)));
   }
-  return p_old - a.lr * upd;
+  return fma2(pair(-a.lr), upd, p_old);
 }
 
 // Correlated-noise transforms of the iid draw z (DP-FTRL), applied element-wise on the shard:
@@ -203,39 +229,97 @@ __device__ __forceinline__ float dp_update(const OpkDpStepArgs& a, float inv_bc1
 //                  new output overwrites the oldest slot, (pos + nlag - 1) mod nlag, which the host makes the next pos
 enum { CORR_NONE = 0, CORR_BLT = 1, CORR_TOEPLITZ = 2 };
 
-template <int CORR>
-__device__ __forceinline__ void correlate_quad(const OpkDpStepArgs& a, long long i0, float (&z)[4]) {
-  if (CORR == CORR_BLT) {
-    float rd[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int k = 0; k < a.blt_nbuf; ++k) {
-      const float4 st = *reinterpret_cast<const float4*>(a.blt_state + (long long)k * a.shard_len + i0);
-      const float sc = a.blt_scale[k];
-      rd[0] += sc * st.x; rd[1] += sc * st.y; rd[2] += sc * st.z; rd[3] += sc * st.w;
-    }
+// VEC consecutive elements of a streamed array: one 32-byte access (8 floats), or 16 bytes where the alignment allows no more.
+// Everything is touched once: streaming loads and stores.
+template <int VEC>
+__device__ __forceinline__ void ld_stream(const float* p, float (&o)[VEC]) {
+  static_assert(VEC == 4 || VEC == 8);
+  if constexpr (VEC == 8)
+    asm volatile("ld.global.cs.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+                 : "l"(p));
+  else
+    asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]) : "l"(p));
+}
+template <int VEC>
+__device__ __forceinline__ void st_stream(float* p, const float (&o)[VEC]) {
+  if constexpr (VEC == 8)
+    asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(o[0]), "f"(o[1]), "f"(o[2]), "f"(o[3]),
+                 "f"(o[4]), "f"(o[5]), "f"(o[6]), "f"(o[7]));
+  else
+    asm volatile("st.global.cs.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(o[0]), "f"(o[1]), "f"(o[2]), "f"(o[3]));
+}
+template <int VEC>
+__device__ __forceinline__ void ld_stream(const __nv_bfloat16* p, uint32_t (&o)[VEC / 2]) {
+  if constexpr (VEC == 8)
+    asm volatile("ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]) : "l"(p));
+  else
+    asm volatile("ld.global.cs.v2.u32 {%0, %1}, [%2];" : "=r"(o[0]), "=r"(o[1]) : "l"(p));
+}
+__device__ __forceinline__ float2 unpack2(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
+
+// The rows of correlation state that a vector needs first are loaded with everything else (four rows: BLT with up to four buffers
+// needs no other access before its stores; two next to eight gradient buffers, which leave no registers for more).
+template <int CORR, int VEC, int ROWS>
+struct CorrIn {
+  float row[ROWS][VEC];
+};
+template <int VEC, int ROWS>
+struct CorrIn<CORR_NONE, VEC, ROWS> {};
+
+__device__ __forceinline__ int toep_slot(const OpkDpStepArgs& a, int k) {      // ring slot of lag k + 1
+  const int slot = a.toep_pos + k;
+  return slot >= a.toep_nlag ? slot - a.toep_nlag : slot;
+}
+template <int CORR, int VEC, int ROWS>
+__device__ __forceinline__ void load_corr(const OpkDpStepArgs& a, long long i0, int first, CorrIn<CORR, VEC, ROWS>& in) {
+  if constexpr (CORR == CORR_BLT) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) z[j] -= rd[j];
-    for (int k = 0; k < a.blt_nbuf; ++k) {
-      float4* sp = reinterpret_cast<float4*>(a.blt_state + (long long)k * a.shard_len + i0);
-      float4 st = *sp;
-      const float dc = a.blt_decay[k];
-      st.x = dc * st.x + z[0]; st.y = dc * st.y + z[1]; st.z = dc * st.z + z[2]; st.w = dc * st.w + z[3];
-      *sp = st;
-    }
-  } else if (CORR == CORR_TOEPLITZ) {
-    float rd[4] = {0.f, 0.f, 0.f, 0.f};
-    int slot = a.toep_pos;
-    for (int k = 1; k <= a.toep_nlag; ++k) {
-      const float4 st = __ldcs(reinterpret_cast<const float4*>(a.toep_state + (long long)slot * a.shard_len + i0));
-      const float c = a.toep_coef[k];
-      rd[0] += c * st.x; rd[1] += c * st.y; rd[2] += c * st.z; rd[3] += c * st.w;
-      if (++slot == a.toep_nlag) slot = 0;
-    }
-    const float inv_c0 = 1.f / a.toep_coef[0];
+    for (int k = 0; k < ROWS; ++k)
+      if (first + k < a.blt_nbuf) ld_stream<VEC>(a.blt_state + (long long)(first + k) * a.shard_len + i0, in.row[k]);
+  } else if constexpr (CORR == CORR_TOEPLITZ) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) z[j] = (z[j] - rd[j]) * inv_c0;
-    if (a.toep_nlag > 0) {
-      const int oldest = a.toep_pos == 0 ? a.toep_nlag - 1 : a.toep_pos - 1;
-      __stcs(reinterpret_cast<float4*>(a.toep_state + (long long)oldest * a.shard_len + i0), make_float4(z[0], z[1], z[2], z[3]));
+    for (int k = 0; k < ROWS; ++k)
+      if (first + k < a.toep_nlag) ld_stream<VEC>(a.toep_state + (long long)toep_slot(a, first + k) * a.shard_len + i0, in.row[k]);
+  }
+}
+template <int CORR, int VEC, int ROWS>
+__device__ __forceinline__ void correlate(const OpkDpStepArgs& a, long long i0, CorrIn<CORR, VEC, ROWS>& in, float (&z)[VEC]) {
+  if constexpr (CORR != CORR_NONE) {
+    const int rows = CORR == CORR_BLT ? a.blt_nbuf : a.toep_nlag;
+    float rd[VEC];
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) rd[j] = 0.f;
+    for (int first = 0; first < rows; first += ROWS) {
+      if (first) load_corr<CORR, VEC, ROWS>(a, i0, first, in);
+#pragma unroll
+      for (int k = 0; k < ROWS; ++k)
+        if (first + k < rows) {
+          const float c = CORR == CORR_BLT ? a.blt_scale[first + k] : a.toep_coef[first + k + 1];
+#pragma unroll
+          for (int j = 0; j < VEC; ++j) rd[j] += c * in.row[k][j];
+        }
+    }
+    if constexpr (CORR == CORR_BLT) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) z[j] -= rd[j];
+      for (int first = 0; first < rows; first += ROWS) {
+        if (rows > ROWS) load_corr<CORR, VEC, ROWS>(a, i0, first, in);
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k)
+          if (first + k < rows) {
+            const float dc = a.blt_decay[first + k];
+            float st[VEC];
+#pragma unroll
+            for (int j = 0; j < VEC; ++j) st[j] = dc * in.row[k][j] + z[j];
+            st_stream<VEC>(a.blt_state + (long long)(first + k) * a.shard_len + i0, st);
+          }
+      }
+    } else {
+      const float inv_c0 = 1.f / a.toep_coef[0];
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) z[j] = (z[j] - rd[j]) * inv_c0;
+      if (rows > 0) st_stream<VEC>(a.toep_state + (long long)(a.toep_pos == 0 ? rows - 1 : a.toep_pos - 1) * a.shard_len + i0, z);
     }
   }
 }
@@ -262,148 +346,204 @@ __device__ __forceinline__ float correlate_one(const OpkDpStepArgs& a, long long
   return z;
 }
 
-// Everything a full quad needs from memory, fetched before any arithmetic so that two quads per thread keep eight to
-// ten 16-byte loads in flight.
-template <int NG>
-struct QuadIn {
-  float4 g, m, v, mw;
-  uint2 pw;
-  uint2 gr[NG > 0 ? NG : 1];
+// Everything a vector of elements needs from memory, fetched before any arithmetic.
+template <int NG, int CORR, int VEC>
+struct VecIn {
+  float g[VEC], m[VEC], v[VEC], mw[VEC];
+  uint32_t pw[VEC / 2], gr[NG > 0 ? NG : 1][VEC / 2];
+  CorrIn<CORR, VEC, (NG > 2 && CORR == CORR_BLT ? 2 : 4)> corr;
 };
-// NG > 0 (the most buffers the variant takes: 2, or all 8): the last group of per-example gradients is clipped and added here instead of in a pass of its own. A separate
-// pass reads and writes the fp32 sums once more and the step reads them again: 12 bytes per parameter (with the zeroing of
-// the sums, which a first group that overwrites them makes unnecessary), 2.8 ms of a 58 ms step at 1.49e9 parameters.
+// NG > 0 (the most buffers the variant takes: 2, or all 8): the last group of per-example gradients is clipped and added here
+// instead of in a pass of its own. A separate pass reads and writes the fp32 sums once more and the step reads them again: 12 bytes
+// per parameter (with the zeroing of the sums, which a first group that overwrites them makes unnecessary), 2.8 ms of a 58 ms step
+// at 1.49e9 parameters.
 struct StepGroup {
   const __nv_bfloat16* g[OPK_ACC_GROUP_MAX];
   const float* scale[OPK_ACC_GROUP_MAX];
   int n, skip_sum;
   long long len;
 };
-template <int NG>
-__device__ __forceinline__ void add_group(const StepGroup& grp, const float (&s)[NG > 0 ? NG : 1], const QuadIn<NG>& q, float (&gr)[4]) {
-  float f[4] = {0.f, 0.f, 0.f, 0.f};
+template <int NG, int CORR, int VEC>
+__device__ __forceinline__ void add_group(const StepGroup& grp, const float (&s)[NG > 0 ? NG : 1], const VecIn<NG, CORR, VEC>& q,
+                                          float (&gr)[VEC]) {
+  float2 f[VEC / 2];
+#pragma unroll
+  for (int k = 0; k < VEC / 2; ++k) f[k] = pair(0.f);
 #pragma unroll
   for (int j = 0; j < NG; ++j)
     if (j < grp.n) {                    // examples in slot order, as in the separate pass
-      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.gr[j].x));
-      const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.gr[j].y));
-      f[0] += clip_store(lo.x, s[j]); f[1] += clip_store(lo.y, s[j]);
-      f[2] += clip_store(hi.x, s[j]); f[3] += clip_store(hi.y, s[j]);
+      float2 scaled[VEC / 2], stored[VEC / 2];
+      float least = INFINITY;
+#pragma unroll
+      for (int k = 0; k < VEC / 2; ++k) {
+        scaled[k] = mul2(unpack2(q.gr[j][k]), pair(s[j]));
+        stored[k] = __bfloat1622float2(__floats2bfloat162_rn(scaled[k].x, scaled[k].y));
+        least = fminf(least, fminf(fabsf(scaled[k].x), fabsf(scaled[k].y)));
+      }
+      if (least < 1.1754943508222875e-38f) {      // clip_store: only a subnormal product may have to be flushed
+#pragma unroll
+        for (int k = 0; k < VEC / 2; ++k) {
+          stored[k].x = flush_rounded_up(stored[k].x, scaled[k].x);
+          stored[k].y = flush_rounded_up(stored[k].y, scaled[k].y);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < VEC / 2; ++k) f[k] = add2(f[k], stored[k]);
     }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) gr[k] += f[k];
+  for (int k = 0; k < VEC / 2; ++k) {
+    gr[2 * k] += f[k].x;
+    gr[2 * k + 1] += f[k].y;
+  }
 }
-template <bool ADAM, bool MASTER, int NG>
-__device__ __forceinline__ void load_quad(const OpkDpStepArgs& a, const PeerTable& pt, const StepGroup& grp, long long i0, long long e0,
-                                          QuadIn<NG>& q) {
-  // reduce-scatter: sum the owned quad over every rank's buffer (peer reads travel over NVLink)
-  if (NG == 0 || !grp.skip_sum || e0 >= grp.len) q.g = __ldcs(reinterpret_cast<const float4*>(pt.grad[0] + e0));
-  else q.g = make_float4(0.f, 0.f, 0.f, 0.f);
+template <bool ADAM, bool MASTER, int CORR, int NG, int VEC>
+__device__ __forceinline__ void load_vec(const OpkDpStepArgs& a, const PeerTable& pt, const StepGroup& grp, long long i0, long long e0,
+                                         VecIn<NG, CORR, VEC>& q) {
+  // reduce-scatter: sum the owned elements over every rank's buffer (peer reads travel over NVLink)
+  if (NG == 0 || !grp.skip_sum || e0 >= grp.len) {
+    ld_stream<VEC>(pt.grad[0] + e0, q.g);
+  } else {
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) q.g[j] = 0.f;
+  }
   for (int r = 1; r < a.n_src; ++r) {
-    const float4 t = __ldcs(reinterpret_cast<const float4*>(pt.grad[r] + e0));
-    q.g.x += t.x; q.g.y += t.y; q.g.z += t.z; q.g.w += t.w;
+    float t[VEC];
+    ld_stream<VEC>(pt.grad[r] + e0, t);
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) q.g[j] += t[j];
   }
   if (NG > 0 && e0 < grp.len) {
 #pragma unroll
     for (int j = 0; j < NG; ++j)
-      if (j < grp.n) q.gr[j] = __ldcs(reinterpret_cast<const uint2*>(grp.g[j] + e0));
+      if (j < grp.n) ld_stream<VEC>(grp.g[j] + e0, q.gr[j]);
   }
-  if (MASTER) q.mw = __ldcs(reinterpret_cast<const float4*>(a.master + i0));
-  else q.pw = __ldcs(reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(a.param_src) + e0));
+  if (MASTER) ld_stream<VEC>(a.master + i0, q.mw);
+  else ld_stream<VEC>(reinterpret_cast<const __nv_bfloat16*>(a.param_src) + e0, q.pw);
   if (ADAM) {
-    q.m = __ldcs(reinterpret_cast<const float4*>(a.m + i0));
-    q.v = __ldcs(reinterpret_cast<const float4*>(a.v + i0));
-  }
-}
-template <bool ADAM, bool MASTER, int CORR, int NG>
-__device__ __forceinline__ void finish_quad(const OpkDpStepArgs& a, const PeerTable& pt, const StepGroup& grp,
-                                            const float (&gs)[NG > 0 ? NG : 1], float inv_bc1, float inv_bc2, long long i0,
-                                            long long e0, const QuadIn<NG>& q) {
-  float z[4] = {0.f, 0.f, 0.f, 0.f};
-  if (a.sigma != 0.f) normal4((uint64_t)e0 >> 2, a.seed, a.stream_id, a.step, z);
-  correlate_quad<CORR>(a, i0, z);
-  float po[4];
-  if (MASTER) {
-    po[0] = q.mw.x; po[1] = q.mw.y; po[2] = q.mw.z; po[3] = q.mw.w;
+    ld_stream<VEC>(a.m + i0, q.m);
+    ld_stream<VEC>(a.v + i0, q.v);
   } else {
-    const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.pw.x));
-    const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.pw.y));
-    po[0] = lo.x; po[1] = lo.y; po[2] = hi.x; po[3] = hi.y;
-  }
-  float gr[4] = {q.g.x, q.g.y, q.g.z, q.g.w};
-  if (NG > 0 && e0 < grp.len) add_group<NG>(grp, gs, q, gr);
-  float mm[4] = {q.m.x, q.m.y, q.m.z, q.m.w}, vv[4] = {q.v.x, q.v.y, q.v.z, q.v.w};
-  float pn[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    pn[j] = dp_update<ADAM>(a, inv_bc1, inv_bc2, gr[j] * a.inv_batch + a.sigma * z[j], po[j], mm[j], vv[j]);
-  if (ADAM) {
-    __stcs(reinterpret_cast<float4*>(a.m + i0), make_float4(mm[0], mm[1], mm[2], mm[3]));
-    __stcs(reinterpret_cast<float4*>(a.v + i0), make_float4(vv[0], vv[1], vv[2], vv[3]));
+    for (int j = 0; j < VEC; ++j) q.m[j] = q.v[j] = 0.f;
   }
-  if (MASTER) __stcs(reinterpret_cast<float4*>(a.master + i0), make_float4(pn[0], pn[1], pn[2], pn[3]));
-  // all-gather: write the updated bf16 quad into every destination parameter buffer
-  uint2 o;
-  __nv_bfloat162 lo = __floats2bfloat162_rn(pn[0], pn[1]), hi = __floats2bfloat162_rn(pn[2], pn[3]);
-  o.x = *reinterpret_cast<uint32_t*>(&lo);
-  o.y = *reinterpret_cast<uint32_t*>(&hi);
-  for (int r = 0; r < a.n_dst; ++r) *reinterpret_cast<uint2*>(pt.param[r] + e0) = o;
-  if (a.zero_grad) *reinterpret_cast<float4*>(const_cast<float*>(pt.grad[0]) + e0) = make_float4(0.f, 0.f, 0.f, 0.f);
+  load_corr(a, i0, 0, q.corr);
+}
+template <bool ADAM, bool MASTER, int CORR, int NG, int VEC>
+__device__ __forceinline__ void finish_vec(const OpkDpStepArgs& a, const opk::PhiloxKeys& key, const PeerTable& pt, const StepGroup& grp,
+                                           const float (&gs)[NG > 0 ? NG : 1], float inv_bc1, float inv_bc2, long long i0, long long e0,
+                                           VecIn<NG, CORR, VEC>& q) {
+  float z[VEC];
+#pragma unroll
+  for (int h = 0; h < VEC; h += 4) {
+    float n[4] = {0.f, 0.f, 0.f, 0.f};
+    if (a.sigma != 0.f) normal4((uint64_t)(e0 + h) >> 2, key, a.stream_id, a.step, n);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) z[h + j] = n[j];
+  }
+  correlate(a, i0, q.corr, z);
+  if (NG > 0 && e0 < grp.len) add_group<NG, CORR, VEC>(grp, gs, q, q.g);
+  float pn[VEC];
+#pragma unroll
+  for (int j = 0; j < VEC; j += 2) {
+    const float2 po = MASTER ? make_float2(q.mw[j], q.mw[j + 1]) : unpack2(q.pw[j / 2]);
+    const float2 grad = fma2(make_float2(q.g[j], q.g[j + 1]), pair(a.inv_batch), mul2(pair(a.sigma), make_float2(z[j], z[j + 1])));
+    float2 m = make_float2(q.m[j], q.m[j + 1]), v = make_float2(q.v[j], q.v[j + 1]);
+    const float2 p = dp_update<ADAM>(a, inv_bc1, inv_bc2, grad, po, m, v);
+    q.m[j] = m.x; q.m[j + 1] = m.y;
+    q.v[j] = v.x; q.v[j + 1] = v.y;
+    pn[j] = p.x; pn[j + 1] = p.y;
+  }
+  if (ADAM) {
+    st_stream<VEC>(a.m + i0, q.m);
+    st_stream<VEC>(a.v + i0, q.v);
+  }
+  if (MASTER) st_stream<VEC>(a.master + i0, pn);
+  // all-gather: write the updated bf16 values into every destination parameter buffer
+  uint32_t o[VEC / 2];
+#pragma unroll
+  for (int j = 0; j < VEC / 2; ++j) {
+    const __nv_bfloat162 both = __floats2bfloat162_rn(pn[2 * j], pn[2 * j + 1]);
+    o[j] = *reinterpret_cast<const uint32_t*>(&both);
+  }
+  for (int r = 0; r < a.n_dst; ++r) {
+    if constexpr (VEC == 8) *reinterpret_cast<uint4*>(pt.param[r] + e0) = make_uint4(o[0], o[1], o[2], o[3]);
+    else *reinterpret_cast<uint2*>(pt.param[r] + e0) = make_uint2(o[0], o[1]);
+  }
+  if (a.zero_grad) {
+    float none[VEC];
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) none[j] = 0.f;
+    st_stream<VEC>(const_cast<float*>(pt.grad[0]) + e0, none);
+  }
 }
 
-template <bool ADAM, bool MASTER, int CORR, int NG>
-__global__ void __launch_bounds__(256) dp_step_kernel(const OpkDpStepArgs a, const PeerTable pt, const StepGroup grp) {
-  // Each thread owns aligned quads of the shard, two per iteration; shard_begin is a multiple of 4 and a ragged last
-  // quad takes the scalar path. Everything is touched exactly once: streaming loads and stores.
-  const long long nfull = a.shard_len >> 2;                // whole quads
+// CTAs per SM that the registers must allow: what the variant fits without spilling.
+constexpr int step_min_ctas(bool adam, bool master, int corr, int ng, int vec) {
+  return vec == 8 || ng > 2 || corr != CORR_NONE || (adam && master && ng > 0) ? 2 : adam ? 3 : 4;
+}
+template <bool ADAM, bool MASTER, int CORR, int NG, int VEC>
+__global__ void __launch_bounds__(256, step_min_ctas(ADAM, MASTER, CORR, NG, VEC))
+dp_step_kernel(const OpkDpStepArgs a, const opk::PhiloxKeys key, const PeerTable pt, const StepGroup grp) {
+  // Each thread owns aligned vectors of the shard: eight elements an iteration, or two times four; a ragged end takes the scalar
+  // path.
+  //
+  // What bounds it: memory, 28 bytes per parameter with two gradient buffers, and next to it the issue slots: 118 instructions per
+  // parameter kept 72 % of them busy at full clock, and a step under the power cap runs at two thirds of that. Eight elements per
+  // thread halve the accesses and their addresses, the round keys come from the constant bank, fp32 arithmetic goes two lanes an
+  // instruction and only subnormal products are looked at for the flush. AdamW with two buffers, 1.49e9 parameters, right after
+  // large products: 8.56 -> 7.41 ms (5.6 TB/s); without buffers 6.77 -> 5.88. Correlation state is read with everything else, not
+  // row by row behind the noise: 2^28 elements, three Toeplitz rows 2.61 -> 1.83 ms (6.4 TB/s), four BLT buffers 3.00 -> 2.75.
+  // Loading the next vector before this one is finished changed nothing without state (7.2 ms) and spills with it.
+  const long long nfull = a.shard_len / VEC;
   const float inv_bc1 = 1.f / a.bc1, inv_bc2 = 1.f / a.bc2;
   float gs[NG > 0 ? NG : 1];
 #pragma unroll
   for (int j = 0; j < NG; ++j) gs[j] = j < grp.n ? *grp.scale[j] : 0.f;
   const long long stride = (long long)gridDim.x * 256;
   long long q = blockIdx.x * 256ll + threadIdx.x;
-  for (; q + stride < nfull; q += 2 * stride) {
-    const long long ia = q << 2, ib = (q + stride) << 2;
-    QuadIn<NG> qa, qb;
-    qa.m = qa.v = qb.m = qb.v = make_float4(0.f, 0.f, 0.f, 0.f);
-    load_quad<ADAM, MASTER, NG>(a, pt, grp, ia, a.shard_begin + ia, qa);
-    load_quad<ADAM, MASTER, NG>(a, pt, grp, ib, a.shard_begin + ib, qb);
-    finish_quad<ADAM, MASTER, CORR, NG>(a, pt, grp, gs, inv_bc1, inv_bc2, ia, a.shard_begin + ia, qa);
-    finish_quad<ADAM, MASTER, CORR, NG>(a, pt, grp, gs, inv_bc1, inv_bc2, ib, a.shard_begin + ib, qb);
-  }
-  if (q < nfull) {
-    const long long ia = q << 2;
-    QuadIn<NG> qa;
-    qa.m = qa.v = make_float4(0.f, 0.f, 0.f, 0.f);
-    load_quad<ADAM, MASTER, NG>(a, pt, grp, ia, a.shard_begin + ia, qa);
-    finish_quad<ADAM, MASTER, CORR, NG>(a, pt, grp, gs, inv_bc1, inv_bc2, ia, a.shard_begin + ia, qa);
-  }
-  // ragged tail (fewer than 4 elements): one thread
-  const int cnt = (int)(a.shard_len & 3);
-  if (cnt && blockIdx.x == 0 && threadIdx.x == 0) {
-    const long long i0 = nfull << 2, e0 = a.shard_begin + i0;
-    float z[4] = {0.f, 0.f, 0.f, 0.f};
-    if (a.sigma != 0.f) normal4((uint64_t)e0 >> 2, a.seed, a.stream_id, a.step, z);
-    for (int j = 0; j < cnt; ++j) {
-      const long long i = i0 + j;
-      float g = 0.f;
-      const bool in_group = NG > 0 && e0 + j < grp.len;
-      for (int r = 0; r < a.n_src; ++r)
-        if (!(in_group && grp.skip_sum)) g += pt.grad[r][e0 + j];
-      if (in_group) {
-        float f = 0.f;
-        for (int k = 0; k < grp.n; ++k) f += clip_store(__bfloat162float(grp.g[k][e0 + j]), *grp.scale[k]);
-        g += f;
-      }
-      const float noise = correlate_one<CORR>(a, i, z[j]);
-      const float p_old = MASTER ? a.master[i] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.param_src)[e0 + j]);
-      float m = ADAM ? a.m[i] : 0.f, v = ADAM ? a.v[i] : 0.f;
-      const float p_new = dp_update<ADAM>(a, inv_bc1, inv_bc2, g * a.inv_batch + a.sigma * noise, p_old, m, v);
-      if (ADAM) { a.m[i] = m; a.v[i] = v; }
-      if (MASTER) a.master[i] = p_new;
-      for (int r = 0; r < a.n_dst; ++r) pt.param[r][e0 + j] = __float2bfloat16(p_new);
-      if (a.zero_grad) const_cast<float*>(pt.grad[0])[e0 + j] = 0.f;
+  if constexpr (VEC == 4) {
+#pragma unroll 1
+    for (; q + stride < nfull; q += 2 * stride) {
+      const long long q2 = q + stride;
+      VecIn<NG, CORR, VEC> in, in2;
+      load_vec<ADAM, MASTER, CORR, NG, VEC>(a, pt, grp, q * VEC, a.shard_begin + q * VEC, in);
+      load_vec<ADAM, MASTER, CORR, NG, VEC>(a, pt, grp, q2 * VEC, a.shard_begin + q2 * VEC, in2);
+      finish_vec<ADAM, MASTER, CORR, NG, VEC>(a, key, pt, grp, gs, inv_bc1, inv_bc2, q * VEC, a.shard_begin + q * VEC, in);
+      finish_vec<ADAM, MASTER, CORR, NG, VEC>(a, key, pt, grp, gs, inv_bc1, inv_bc2, q2 * VEC, a.shard_begin + q2 * VEC, in2);
     }
+  }
+#pragma unroll 1
+  for (; q < nfull; q += stride) {
+    VecIn<NG, CORR, VEC> in;
+    load_vec<ADAM, MASTER, CORR, NG, VEC>(a, pt, grp, q * VEC, a.shard_begin + q * VEC, in);
+    finish_vec<ADAM, MASTER, CORR, NG, VEC>(a, key, pt, grp, gs, inv_bc1, inv_bc2, q * VEC, a.shard_begin + q * VEC, in);
+  }
+  // ragged end: one thread per element
+  const long long i = nfull * VEC + threadIdx.x;
+  if (blockIdx.x == 0 && i < a.shard_len) {
+    const long long e = a.shard_begin + i;
+    float z4[4] = {0.f, 0.f, 0.f, 0.f};
+    if (a.sigma != 0.f) normal4((uint64_t)e >> 2, key, a.stream_id, a.step, z4);
+    const int lane = (int)(e & 3);
+    const float z = lane == 0 ? z4[0] : lane == 1 ? z4[1] : lane == 2 ? z4[2] : z4[3];
+    float g = 0.f;
+    const bool in_group = NG > 0 && e < grp.len;
+    for (int r = 0; r < a.n_src; ++r)
+      if (!(in_group && grp.skip_sum)) g += pt.grad[r][e];
+    if (in_group) {
+      float f = 0.f;
+      for (int k = 0; k < grp.n; ++k) f += clip_store(__bfloat162float(grp.g[k][e]), *grp.scale[k]);
+      g += f;
+    }
+    const float noise = correlate_one<CORR>(a, i, z);
+    const float p_old = MASTER ? a.master[i] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(a.param_src)[e]);
+    float2 m = pair(ADAM ? a.m[i] : 0.f), v = pair(ADAM ? a.v[i] : 0.f);
+    const float grad = fmaf(g, a.inv_batch, a.sigma * noise);
+    const float p_new = dp_update<ADAM>(a, inv_bc1, inv_bc2, pair(grad), pair(p_old), m, v).x;
+    if (ADAM) { a.m[i] = m.x; a.v[i] = v.x; }
+    if (MASTER) a.master[i] = p_new;
+    for (int r = 0; r < a.n_dst; ++r) pt.param[r][e] = __float2bfloat16(p_new);
+    if (a.zero_grad) const_cast<float*>(pt.grad[0])[e] = 0.f;
   }
 }
 
@@ -582,18 +722,34 @@ extern "C" int opk_clip_accumulate(const void* g, const float* scale, float* acc
   return opk_clip_accumulate2(g, scale, acc, n, 0, stream);
 }
 
-// One round of resident CTAs walks the shard: every CTA gets the same share. (A fixed 8 CTAs per SM ran as 2.7 rounds of the
-// variants that fit three at a time: 8.1 ms at 1.49e9 parameters.) Eight per SM where that is the faster grid (2^26 elements, one
-// round -> eight per SM): SGD 150 -> 142 us, with two gradient buffers 208 -> 199; AdamW with master weights, without buffers and
-// correlation, on large shards 351 -> 337 us (2^20 elements: 5.6 -> 6.6; with buffers 381 -> 397; correlated noise 627 -> 660).
-template <bool ADAM, bool MASTER, int CORR, int NG>
-void launch_dp_step(long long nq, cudaStream_t st, const OpkDpStepArgs& args, const PeerTable& pt, const StepGroup& grp) {
-  auto kernel = dp_step_kernel<ADAM, MASTER, CORR, NG>;
+// Up to 2^23 elements one round of resident CTAs walks the shard, so that every CTA gets the same share (2^20 elements, one round ->
+// eight CTAs per SM: SGD 3.3 -> 3.6 us, AdamW 4.8 -> 5.1, with two buffers 6.1 -> 6.6). On larger shards eight per SM, which start
+// and end at different times, except for AdamW that adds a group without correlated noise (2^26 elements: AdamW 275 -> 249 us, with
+// master weights 336 -> 312, four BLT rows 608 -> 584, three Toeplitz rows 437 -> 412, SGD 106 -> 102; with two buffers 286 -> 289).
+template <bool ADAM, bool MASTER, int CORR, int NG, int VEC>
+void launch_dp_step(cudaStream_t st, const OpkDpStepArgs& args, const PeerTable& pt, const StepGroup& grp) {
+  auto kernel = dp_step_kernel<ADAM, MASTER, CORR, NG, VEC>;
   int per_sm = 8, dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool eight = !ADAM || (MASTER && CORR == CORR_NONE && NG == 0 && nq > (1ll << 21));
+  const bool eight = args.shard_len > (1ll << 23) && (!ADAM || NG == 0 || CORR != CORR_NONE);
   if (!eight && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0) != cudaSuccess || per_sm < 1)) per_sm = 2;
-  kernel<<<grid_for((nq + 1) / 2, 256, sms * per_sm), 256, 0, st>>>(args, pt, grp);
+  kernel<<<grid_for((args.shard_len + VEC - 1) / VEC, 256, sms * per_sm), 256, 0, st>>>(args, opk::philox_keys(args.seed), pt, grp);
+}
+// Whether every array of the step can be read eight elements at a time: 32-byte fp32 and 16-byte bf16 vectors that start with the
+// shard, whole vectors in the group's buffers and in every row of correlation state.
+bool eight_at_a_time(const OpkDpStepArgs& a, const PeerTable& pt, const StepGroup& grp) {
+  auto off = [](const void* p) { return reinterpret_cast<uintptr_t>(p) & 31; };
+  if ((a.shard_begin & 7) || (grp.len & 7)) return false;
+  for (int r = 0; r < a.n_src; ++r)
+    if (off(pt.grad[r])) return false;
+  for (int r = 0; r < a.n_dst; ++r)
+    if (off(pt.param[r]) & 15) return false;
+  for (int j = 0; j < grp.n; ++j)
+    if (off(grp.g[j]) & 15) return false;
+  if ((off(a.param_src) & 15) || off(a.m) || off(a.v) || off(a.master)) return false;
+  if (a.blt_nbuf > 0 && (off(a.blt_state) || (a.blt_nbuf > 1 && (a.shard_len & 7)))) return false;
+  if (a.toep_nlag > 0 && (off(a.toep_state) || (a.toep_nlag > 1 && (a.shard_len & 7)))) return false;
+  return true;
 }
 
 // grad_src / param_dst are HOST arrays of device pointers here (copied into the kernel's parameter space).
@@ -615,7 +771,6 @@ extern "C" int opk_dp_step(const OpkDpStepArgs* args, void* stream) {
       (reinterpret_cast<uintptr_t>(args->master) & 15))
     return -2;
   if (args->toep_nlag > 0 && (!args->toep_state || !args->toep_coef || args->toep_pos < 0 || args->toep_pos >= args->toep_nlag)) return -3;
-  const long long nq = (args->shard_len + 3) >> 2;
   cudaStream_t st = ST(stream);
   const int corr = args->blt_nbuf > 0 ? CORR_BLT : (args->toep_coef ? CORR_TOEPLITZ : CORR_NONE);
   const bool adam = !args->sgd_mode, master = args->master != nullptr;
@@ -636,14 +791,19 @@ extern "C" int opk_dp_step(const OpkDpStepArgs* args, void* stream) {
     grp.len = args->group_len;
   }
   // One variant for groups of at most two and one for all others, because registers set how many CTAs an SM holds: with two
-  // buffers 1,251 us against 1,533 on the variant for eight (2^28 elements, AdamW), with one 1,165 against 1,457. From three
-  // buffers on only the wide one fits: 1,629 us for three (4.9 TB/s), 2,002 for eight (5.4 TB/s). Accumulation pass, step without
-  // a group and zeroing take 1,880 us together for two buffers, 1,907 for three, 2,356 for eight.
+  // buffers 287 us against 300 on the variant for eight (2^26 elements, AdamW), with one 270 against 284. From three buffers on
+  // only the wide one fits: 316 us for three, 404 for eight (6.6 TB/s).
+  const bool wide = eight_at_a_time(*args, pt, grp);
+#define OPK_DP_STEP_VEC(A, M, C, N)                                                  \
+  do {                                                                               \
+    if (wide) launch_dp_step<A, M, C, N, 8>(st, *args, pt, grp);                     \
+    else launch_dp_step<A, M, C, N, 4>(st, *args, pt, grp);                          \
+  } while (0)
 #define OPK_DP_STEP_LAUNCH(A, M, C)                                                  \
   do {                                                                               \
-    if (!group) launch_dp_step<A, M, C, 0>(nq, st, *args, pt, grp);   \
-    else if (grp.n <= 2) launch_dp_step<A, M, C, 2>(nq, st, *args, pt, grp); \
-    else launch_dp_step<A, M, C, OPK_ACC_GROUP_MAX>(nq, st, *args, pt, grp); \
+    if (!group) OPK_DP_STEP_VEC(A, M, C, 0);                                         \
+    else if (grp.n <= 2) OPK_DP_STEP_VEC(A, M, C, 2);                                \
+    else OPK_DP_STEP_VEC(A, M, C, OPK_ACC_GROUP_MAX);                                \
   } while (0)
 #define OPK_DP_STEP_CORR(A, M)                                      \
   do {                                                              \
@@ -657,6 +817,7 @@ extern "C" int opk_dp_step(const OpkDpStepArgs* args, void* stream) {
   else OPK_DP_STEP_CORR(false, false);
 #undef OPK_DP_STEP_CORR
 #undef OPK_DP_STEP_LAUNCH
+#undef OPK_DP_STEP_VEC
   OPK_LAUNCH_CHECK();
   return 0;
 }

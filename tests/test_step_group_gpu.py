@@ -156,3 +156,41 @@ def test_step_after_an_update_that_failed(cuda):
                 assert i == 0
     a, b = engines
     assert torch.equal(a.params, b.params) and torch.equal(a.m, b.m)
+
+
+@pytest.mark.parametrize("n_group,group_len", [(0, 0), (2, 4096), (3, 7000)])
+@pytest.mark.parametrize("noise", ["independent", "blt 2", "blt 6", "toeplitz 1", "toeplitz 5"])
+@pytest.mark.parametrize("sgd,master", [(False, False), (False, True), (True, False)])
+def test_vectors_of_eight_and_of_four_give_the_same_bits(cuda, n_group, group_len, noise, sgd, master):
+    """One shard whose arrays start on 32-byte boundaries against shards that start at 4, 12, ... (16 bytes), ragged at the end."""
+    from opake_b200.ops import kernels as K
+
+    n = 8008                                      # rows of correlation state are whole vectors
+    gs = [torch.randn(n, device=cuda).to(torch.bfloat16) for _ in range(n_group)]
+    scales = [torch.rand(1, device=cuda) for _ in range(n_group)]
+    acc, start = torch.randn(n, device=cuda), torch.randn(n, device=cuda)
+    kind, rows = noise.split()[0], int(noise.split()[-1]) if " " in noise else 0
+    state = torch.randn(rows, n, device=cuda)
+    coef = torch.rand(rows + 1, device=cuda) + 0.5
+    out = []
+    for cuts in ([0, n], [0, 4, 12, 4100, n]):
+        p = start.to(torch.bfloat16)
+        full = dict(m=torch.full((n,), 0.01, device=cuda), v=torch.full((n,), 0.02, device=cuda), master=start.clone(), state=state.clone())
+        for a, b in zip(cuts, cuts[1:]):
+            part = {k: t[..., a:b].clone() for k, t in full.items()}          # own allocations: the shard's state starts aligned
+            if len(cuts) > 2:                                                 # ... and here 16 bytes after such a boundary
+                part = {k: torch.empty(t.numel() + 4, device=cuda)[4:].view(t.shape).copy_(t) for k, t in part.items()}
+            corr = {}
+            if kind == "blt":
+                corr = dict(blt_state=part["state"], blt_decay=coef[1:] / 2, blt_scale=coef[1:] / 8)
+            elif kind == "toeplitz":
+                corr = dict(toep_state=part["state"], toep_coef=coef, toep_pos=rows - 1)
+            K.dp_step(grad_src=[acc.data_ptr()], shard_begin=a, shard_len=b - a, inv_batch=0.25, sigma=0.01, seed=3, step=1,
+                      m=None if sgd else part["m"], v=None if sgd else part["v"], master=part["master"] if master else None,
+                      param_dst=[p.data_ptr()], param_src=p, lr=0.1, beta1=0.9, beta2=0.99, eps=1e-8, weight_decay=0.01, bc1=0.1,
+                      bc2=0.01, phi_hat=1e-5, device=cuda, sgd_mode=sgd, group=gs, group_scales=scales, group_len=group_len, **corr)
+            for k, t in full.items():
+                t[..., a:b] = part[k]
+        out.append((p, *full.values()))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
