@@ -1,5 +1,5 @@
-// Two-CTA (cta_group::2) variant of the bf16 GEMM: a cluster of two CTAs on a pair of SMs computes one 256 x 256
-// output tile per step. Each CTA stages its own 128 rows of A and its own 128 columns of B (32 KB per pipeline stage
+// Two-CTA (cta_group::2) variant of the bf16 GEMM: a cluster of two CTAs on a pair of SMs computes one 256 x 256 (G2_HALF: 256 x
+// 128) output tile per step. Each CTA stages its own 128 rows of A and its own 128 columns of B (32 KB per pipeline stage
 // instead of 48 KB for a 128 x 256 tile), the even CTA of the pair issues tcgen05.mma.cta_group::2 instructions that
 // read both CTAs' shared memory, and each CTA ends up with the accumulator of its own 128 rows (all 256 columns) in
 // its own TMEM. Per tensor-core cycle this halves the shared-memory and TMA traffic of the B operand, which is what
@@ -61,23 +61,26 @@ __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
                : "memory");
 }
 
+template <int COLS>
 struct Gemm2Cfg {
   static constexpr int BM = 128;            // rows per CTA (256 per pair)
-  static constexpr int BN = 256;            // columns per pair; each CTA stages BN / 2 of them
+  static constexpr int BN = COLS;           // columns per pair (256 or 128); each CTA stages BN / 2 of them
   static constexpr int BK = 64;
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = (BN / 2) * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;          // 32 KB
-  static constexpr int STAGES = 6;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;          // 32 KB, 24 KB
+  static constexpr int STAGES = BN == 256 ? 6 : 8;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256 + 8 * kEpiScratch + 8 * 8 * 8;
   static constexpr int TMEM_COLS = 2 * BN;                        // two accumulator buffers
 };
 
 constexpr int kStageWarps = 8;     // copier warps per CTA of the staged variant
-enum Gemm2Variant : int { G2_PLAIN = 0, G2_STAGE = 1, G2_WIDE = 2 };      // G2_WIDE: eight epilogue warps (see wide_epilogue)
+// G2_WIDE: eight epilogue warps (see wide_epilogue); G2_HALF: the same with tiles of 128 columns (see choose_tile).
+enum Gemm2Variant : int { G2_PLAIN = 0, G2_STAGE = 1, G2_WIDE = 2, G2_HALF = 3 };
+__host__ __device__ constexpr int gemm2_cols(int variant) { return variant == G2_HALF ? 128 : 256; }
 // The staged variant keeps four epilogue warps: with eight next to its copier warps a thread would have 112 registers.
 __host__ __device__ constexpr int gemm2_epi_warps(int epi, int variant) {
-  return variant == G2_STAGE ? 4 : variant == G2_WIDE ? 8 : gemm_epi_warps(epi);
+  return variant == G2_STAGE ? 4 : variant == G2_WIDE || variant == G2_HALF ? 8 : gemm_epi_warps(epi);
 }
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
@@ -90,7 +93,7 @@ template <bool A_MN, bool B_MN, int EPI, int VARIANT = G2_PLAIN>
 __global__ void __cluster_dims__(2, 1, 1)
 __launch_bounds__(64 + 32 * gemm2_epi_warps(EPI, VARIANT) + (VARIANT == G2_STAGE ? 32 * kStageWarps : 0), 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
-  using Cfg = Gemm2Cfg;
+  using Cfg = Gemm2Cfg<gemm2_cols(VARIANT)>;
   constexpr bool STAGE = VARIANT == G2_STAGE;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];

@@ -95,7 +95,7 @@ bool pair_mode() { return g_pair_mode == 1; }
 
 template <bool A_MN, bool B_MN, int EPI, int VARIANT = opk::G2_PLAIN>
 int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmParams& p, int max_ctas, cudaStream_t st) {
-  using Cfg = opk::Gemm2Cfg;
+  using Cfg = opk::Gemm2Cfg<opk::gemm2_cols(VARIANT)>;
   auto kern = opk::gemm2_bf16_kernel<A_MN, B_MN, EPI, VARIANT>;
   constexpr int kThreads = 64 + 32 * opk::gemm2_epi_warps(EPI, VARIANT) + (VARIANT == opk::G2_STAGE ? 32 * opk::kStageWarps : 0);
   static bool attr_done = false;
@@ -132,9 +132,11 @@ int launch_narrow(const CUtensorMap& ta, const CUtensorMap& tb, const opk::GemmP
   return 0;
 }
 
-// Tile width of the narrow kernel for this product; 0: one of the persistent kernels. Never EPI_SUMSQ: a norm's fp32 partial
+constexpr int kHalfPair = 1;      // choose_tile: pairs of CTAs on tiles of 256 x 128
+
+// Tile width of the narrow kernel for this product, kHalfPair, or 0: one of the persistent kernels. Never EPI_SUMSQ: a norm's fp32 partial
 // sums follow the tiles, and the clip factor of an example must not depend on which kernel its length favours.
-int choose_narrow(const OpkGemmArgs* a, int bn, bool pair) {
+int choose_tile(const OpkGemmArgs* a, int bn, bool pair) {
   if (!pair_mode() || a->tile_group || a->group_k || a->stage_dst || a->max_ctas > 0) return 0;
   const int key = (a->a_mn ? 1 : 0) | (a->b_mn ? 2 : 0);
   const bool ok = a->epilogue == opk::EPI_STORE ? key != 1
@@ -147,6 +149,7 @@ int choose_narrow(const OpkGemmArgs* a, int bn, bool pair) {
   // 16 .. 128256): a fixed part and a slope per 64-element block of the reduction and round of tiles.
   //   tile            fixed   slope   measured at M x N x K (persistent kernel -> narrow kernel, us)
   //   256 x 256 pair   6600     280
+  //   256 x 128 pair   6600     205
   //   128 x 256        5200     315   2048 x 2048 x 2048: 16.9 -> 16.3; 1024 x 3072 x 768: 10.3 -> 9.5
   //   128 x 128        4200     235   1024 x 2304 x 768: 10.2 -> 7.6
   //   128 x 64         3500     225   1024 x 768 x 768: 10.0 -> 6.3
@@ -163,6 +166,15 @@ int choose_narrow(const OpkGemmArgs* a, int bn, bool pair) {
     const long long round = w == 256 ? 4500 : w == 128 ? 1500 : 800;          // epilogue of every further round
     const long long c = fixed + per * kb * slope + (per - 1) * round;
     if (c < cost) { cost = c; best = w; }
+  }
+  // Pairs on tiles of 256 x 128: 24 KB per block and SM for the work of a 128 x 128 tile (32 KB) where 256-wide tiles leave pairs
+  // idle. From long reductions on, for the layouts of forward products and input gradients (us, before -> with it): 634 x 2048 over
+  // 8192 34.2 -> 31.4, over 16384 64.4 -> 56.6, over 128256 477 -> 396; 1021 x 2048 x 50304 197 -> 180; 2048 x 768 x 50257 (two
+  // examples' logit gradients) 230 -> 187; 3000 x 768 x 3072 20 -> 17. Short reductions stay with one CTA (2048 x 2048 over 634 rows
+  // 11.3, in pairs 12.3) and so does what 64-wide tiles finish in one round (256 x 768 x 50257 175, in pairs 177).
+  if (pair && a->epilogue == opk::EPI_STORE && key != 3 && best != 64) {
+    const long long per = ceil_div(ceil_div(a->M, 256) * ceil_div(a->N, 128) * a->batch, sms / 2);
+    if (6600 + per * kb * 205 + (per - 1) * 1200 < cost) best = kHalfPair;
   }
   return best;
 }
@@ -236,7 +248,9 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   if (!a || a->M <= 0 || a->N <= 0 || a->K <= 0 || a->batch <= 0) { set_err("opk_gemm: bad sizes"); return -1; }
   const int bn = pick_bn(a->N, a->epilogue);
   const bool pair = bn == 256 && !a->tile_group && !a->group_k && a->M >= 256 && pair_mode();
-  const int narrow = choose_narrow(a, bn, pair);
+  const int tile = choose_tile(a, bn, pair);
+  const bool half = tile == kHalfPair;
+  const int narrow = half ? 0 : tile;
   CUtensorMap ta, tb;
   // A: K-major -> {K, M, batch} box {64, 128}; MN-major -> {M, K, batch} box {64, 64}
   if (a->tile_group && (a->batch != 1 || a->n_groups <= 0)) { set_err("opk_gemm: tile_group needs batch == 1 and n_groups"); return -1; }
@@ -266,7 +280,7 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   } else if (a->b_mn) {
     if (!make_map(&tb, a->B, a->N, a->K, bbatch, a->ldb, a->strideB, 64)) return -2;
   } else {
-    if (!make_map(&tb, a->B, a->K, a->N, bbatch, a->ldb, a->strideB, narrow ? narrow : pair ? 128 : bn)) return -2;
+    if (!make_map(&tb, a->B, a->K, a->N, bbatch, a->ldb, a->strideB, narrow ? narrow : half ? 64 : pair ? 128 : bn)) return -2;
   }
   if (a->stepwise && (a->epilogue != opk::EPI_STORE || a->bias)) { set_err("opk_gemm: stepwise rounding takes a plain store without a bias"); return -1; }
   opk::GemmParams p;
@@ -315,6 +329,9 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
   if (pair) {
     switch (a->epilogue) {
       case opk::EPI_STORE:
+        if (half)
+          return key == 0 ? launch2<false, false, opk::EPI_STORE, opk::G2_HALF>(ta, tb, p, mc, st)
+                          : launch2<false, true, opk::EPI_STORE, opk::G2_HALF>(ta, tb, p, mc, st);
         if (wide_epilogue(a)) {
           if (key == 0) return launch2<false, false, opk::EPI_STORE, opk::G2_WIDE>(ta, tb, p, mc, st);
           if (key == 2) return launch2<false, true, opk::EPI_STORE, opk::G2_WIDE>(ta, tb, p, mc, st);

@@ -67,3 +67,30 @@ def test_functional_gradients_do_not_depend_on_the_micro_batch(cuda, T, D, V):
     for lo, hi in ((0, 1), (1, 4), (4, 8)):
         ph, pw = f(h[lo:hi], w, lab[lo:hi])
         assert torch.equal(ph, dh[lo:hi]) and torch.equal(pw, dw[lo:hi])
+
+
+@pytest.mark.parametrize("M,N,K", [(634, 2048, 8192), (600, 1992, 8200), (2048, 768, 6408), (3000, 760, 3072), (1021, 2048, 12296)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_pair_tiles_of_128_columns(cuda, M, N, K, b_mn):
+    """Sizes that leave 256-wide pairs idle over a long reduction, with and without bias and residual: the bits of the single-CTA
+    kernel (every product adds in one order), and those within the rounding of bf16 of the exact sum."""
+    from opake_b200.ops import gemm as G
+
+    a = torch.randn(M, K, device=cuda).to(torch.bfloat16)
+    b = (torch.randn(K, N, device=cuda) if b_mn else torch.randn(N, K, device=cuda)).to(torch.bfloat16)
+    r, bias = torch.randn(M, N, device=cuda).to(torch.bfloat16), torch.randn(N, device=cuda).to(torch.bfloat16)
+    for kw in ({}, {"bias": bias, "residual": r}):
+        out = torch.empty(M, N + 8, device=cuda, dtype=torch.bfloat16)[:, :N] if not kw else torch.empty(M, N, device=cuda, dtype=torch.bfloat16)
+        G.gemm(a, b, b_mn=b_mn, out=out, **kw)
+        before = G.pair_mode()
+        try:
+            G.set_pair_mode(False)
+            single = G.gemm(a, b, b_mn=b_mn, out=torch.empty(M, N, device=cuda, dtype=torch.bfloat16), **kw)
+        finally:
+            G.set_pair_mode(before)
+        assert torch.equal(out, single)
+    exact = a.double() @ (b.double() if b_mn else b.double().t())
+    got = G.gemm(a, b, b_mn=b_mn).double()
+    bound = a.double().abs() @ (b.double().abs() if b_mn else b.double().abs().t())
+    # one rounding to bf16 and K fp32 additions, each at most 2^-24 of the absolute sum
+    assert ((got - exact).abs() <= exact.abs() * 2.0 ** -8 + bound * K * 2.0 ** -24).all()
