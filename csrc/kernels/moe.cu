@@ -8,6 +8,7 @@
 // (buffers are sized for the worst case R = T*k + E*128 rows).
 // The reference routes with eager PyTorch ops and calls torch._grouped_mm
 // (packages/opake-patches/src/opake/api/patches/kernels/fused_moe.py:159-335, moe.py:570-627).
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -127,10 +128,10 @@ __global__ void __launch_bounds__(256) moe_route_bwd_kernel(const float* __restr
 }
 
 // ------------------------------------------------------------------------------------------------ plan
-// Single CTA, one pass over the entries. Stable counting sort by expert: entry n = t*k + slot goes to row off[e] +
-// (number of earlier entries with the same expert). Warp w owns the contiguous chunk w of the entry list: per-warp
-// histograms in shared memory, per expert an exclusive prefix over the warps (the rank of the warp's first entry of
-// that expert), then every warp walks its chunk in order, 32 entries at a time, lanes with the same expert finding
+// One CTA, or a cluster of eight for many entries; one pass over the entries. Stable counting sort by expert: entry n = t*k +
+// slot goes to row off[e] + (number of earlier entries with the same expert). Warp w owns the contiguous chunk w of the entry
+// list: per-warp histograms in shared memory, per expert an exclusive prefix over the warps, and over the CTAs of the cluster
+// through distributed shared memory (the rank of the warp's first entry of that expert), then every warp walks its chunk in order, 32 entries at a time, lanes with the same expert finding
 // each other with match.any. Segments are padded to multiples of 128 rows and are at least 128 rows long (an expert
 // without tokens still owns one all-zero tile, so its weight gradient is produced as exact zeros by the GEMM).
 //
@@ -138,6 +139,12 @@ __global__ void __launch_bounds__(256) moe_route_bwd_kernel(const float* __restr
 // are still one segment, the range of the forward and input-gradient products, in which every example's rows are padded to a
 // multiple of 64 (at least 64): whole blocks of the reduction, so that group_k[example][expert] gives the range of the example's
 // own weight gradient. The rows of an example meet the same blocks in the same order as in a plan of its own.
+//
+// What bounds it: latency, it stands alone in the chain between router and products. Expert ids are loaded eight at a time (a load per
+// step of 32 entries waited for memory each time), segments are placed by a scan over the experts instead of one thread, and the
+// matching of equal experts, the longest part on one SM, is spread over eight: 64 experts, 32768 entries 60 -> 13 us, 16384 38 -> 10,
+// 1024 21 -> 7.
+template <bool CLUSTER>
 __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, int n_entries, int E, int examples, int r_cap,
                                                         int* __restrict__ dest, int* __restrict__ src_entry,
                                                         int* __restrict__ tile_group, int* __restrict__ group_k,
@@ -145,15 +152,28 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
   __shared__ int hist[32][MAX_E];     // [warp][key]; becomes the next free row of (warp, key); keys = expert * examples + example
   __shared__ int counts[MAX_E];
   __shared__ int offs[MAX_E + 1];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ int local[MAX_E];        // this CTA's entries per key, read by the others of the cluster
+  __shared__ int prior[MAX_E];        // entries per key in the CTAs before this one
+  const int ctas = CLUSTER ? (int)gridDim.x : 1, rank = CLUSTER ? (int)blockIdx.x : 0;               // the grid is one cluster
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gwarp = rank * 32 + warp, warps = ctas * 32;
   const int keys = E * examples, per_example = n_entries / examples;
   for (int i = threadIdx.x; i < 32 * MAX_E; i += blockDim.x) (&hist[0][0])[i] = 0;
   __syncthreads();
-  const int chunk = ((n_entries + 31) / 32 + 31) / 32 * 32;   // entries per warp, a multiple of 32
-  const int c0 = warp * chunk, c1 = min(c0 + chunk, n_entries);
+  const int chunk = ((n_entries + warps - 1) / warps + 31) / 32 * 32;      // entries per warp, a multiple of 32
+  const int c0 = min(gwarp * chunk, n_entries), c1 = min(c0 + chunk, n_entries);
   // an expert id outside [0, E) is dropped from the plan (its dest stays -1): never an index past the histograms
-  for (int n = c0 + lane; n < c1; n += 32)
-    if (OPK_IDX_OK(idx[n], E) && (unsigned)idx[n] < (unsigned)E) atomicAdd(&hist[warp][idx[n] * examples + n / per_example], 1);
+  constexpr int U = 8;                  // ids in flight per lane
+  for (int base = c0; base < c1; base += 32 * U) {
+    int id[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) id[u] = base + 32 * u + lane < c1 ? idx[base + 32 * u + lane] : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int n = base + 32 * u + lane;
+      if (base + 32 * u >= c1) break;
+      if (n < c1 && OPK_IDX_OK(id[u], E) && (unsigned)id[u] < (unsigned)E) atomicAdd(&hist[warp][id[u] * examples + n / per_example], 1);
+    }
+  }
   __syncthreads();
   for (int e = threadIdx.x; e < keys; e += blockDim.x) {
     int run = 0;
@@ -162,50 +182,95 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
       hist[w][e] = run;
       run += c;
     }
-    counts[e] = run;
+    (CLUSTER ? local : counts)[e] = run;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int off = 0;
-    for (int e = 0; e < E; ++e) {
-      int all = 0;
-      for (int j = 0; j < examples; ++j) {
-        const int key = e * examples + j, c = counts[key], unit = examples == 1 ? 128 : 64;
-        const int padded = c == 0 ? unit : (c + unit - 1) / unit * unit;
-        offs[key] = off;
-        group_k[2 * (j * E + e)] = off;
-        group_k[2 * (j * E + e) + 1] = padded / 64;
-        off += padded;
+  if constexpr (CLUSTER) {
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    for (int e = threadIdx.x; e < keys; e += blockDim.x) {
+      int all = 0, before = 0;
+      for (int r = 0; r < ctas; ++r) {
+        const int c = cluster.map_shared_rank(local, r)[e];
+        if (r < rank) before += c;
         all += c;
       }
-      off = (off + 127) / 128 * 128;
-      if (counts_out) counts_out[e] = all;
+      counts[e] = all;
+      prior[e] = before;
     }
-    offs[keys] = off;
+    cluster.sync();                     // nobody leaves, or goes on, before `local` has been read
+  } else {
+    __syncthreads();
+  }
+  // thread e places the parts of expert e behind the segments of the experts before it
+  __shared__ int warp_sum[MAX_E / 32];
+  int off = 0, rows = 0;
+  if (threadIdx.x < MAX_E) {
+    const int e = threadIdx.x, unit = examples == 1 ? 128 : 64;
+    int all = 0;
+    if (e < E) {
+      for (int j = 0; j < examples; ++j) {
+        const int c = counts[e * examples + j];
+        rows += c == 0 ? unit : (c + unit - 1) / unit * unit;
+        all += c;
+      }
+      rows = (rows + 127) / 128 * 128;
+      if (counts_out && rank == 0) counts_out[e] = all;
+    }
+    off = rows;                         // inclusive sum over the experts of this warp
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int before = __shfl_up_sync(0xffffffffu, off, d);
+      if (lane >= d) off += before;
+    }
+    if (lane == 31) warp_sum[warp] = off;
+  }
+  __syncthreads();
+  if (threadIdx.x < E) {
+    const int e = threadIdx.x, unit = examples == 1 ? 128 : 64;
+    for (int w = 0; w < warp; ++w) off += warp_sum[w];
+    if (e == E - 1) offs[keys] = off;
+    off -= rows;
+    for (int j = 0; j < examples; ++j) {
+      const int key = e * examples + j, c = counts[key];
+      const int padded = c == 0 ? unit : (c + unit - 1) / unit * unit;
+      offs[key] = off;
+      if (rank == 0) {
+        group_k[2 * (j * E + e)] = off;
+        group_k[2 * (j * E + e) + 1] = padded / 64;
+      }
+      off += padded;
+    }
   }
   __syncthreads();
   const int total = offs[keys];
   // tile -> expert table, padding rows of every segment, everything past the last segment
-  for (int e = warp; e < E; e += 32)
+  for (int e = gwarp; e < E; e += warps)
     for (int tl = offs[e * examples] / 128 + lane; tl < (offs[(e + 1) * examples]) / 128; tl += 32) tile_group[tl] = e;
-  for (int e = warp; e < keys; e += 32)
+  for (int e = gwarp; e < keys; e += warps)
     for (int r = offs[e] + counts[e] + lane; r < offs[e + 1]; r += 32) src_entry[r] = -1;
-  for (int tl = total / 128 + threadIdx.x; tl < r_cap / 128; tl += blockDim.x) tile_group[tl] = -1;
-  for (int r = total + threadIdx.x; r < r_cap; r += blockDim.x) src_entry[r] = -1;
-  for (int base = c0; base < c1; base += 32) {
-    const int n = base + lane;
-    const bool valid = n < c1 && (unsigned)idx[n < c1 ? n : c0] < (unsigned)E;
-    if (n < c1 && !valid) dest[n] = -1;
-    const int e = valid ? idx[n] * examples + n / per_example : -1 - lane;      // invalid lanes match nobody
-    const unsigned m = __match_any_sync(0xffffffffu, e);
-    if (valid) {
-      const int row = offs[e] + hist[warp][e] + __popc(m & ((1u << lane) - 1u));
-      dest[n] = row;
-      src_entry[row] = n;
+  for (int tl = total / 128 + rank * 1024 + threadIdx.x; tl < r_cap / 128; tl += ctas * 1024) tile_group[tl] = -1;
+  for (int r = total + rank * 1024 + threadIdx.x; r < r_cap; r += ctas * 1024) src_entry[r] = -1;
+  for (int base = c0; base < c1; base += 32 * U) {
+    int id[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) id[u] = base + 32 * u + lane < c1 ? idx[base + 32 * u + lane] : -1;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int n = base + 32 * u + lane;
+      if (base + 32 * u >= c1) break;
+      const bool valid = (unsigned)id[u] < (unsigned)E;
+      if (n < c1 && !valid) dest[n] = -1;
+      const int e = valid ? id[u] * examples + n / per_example : -1 - lane;     // invalid lanes match nobody
+      const unsigned m = __match_any_sync(0xffffffffu, e);
+      if (valid) {
+        const int row = offs[e] + (CLUSTER ? prior[e] : 0) + hist[warp][e] + __popc(m & ((1u << lane) - 1u));
+        dest[n] = row;
+        src_entry[row] = n;
+      }
+      __syncwarp();
+      if (valid && (m >> lane) == 1u) hist[warp][e] += __popc(m);   // highest lane of each match group
+      __syncwarp();
     }
-    __syncwarp();
-    if (valid && (m >> lane) == 1u) hist[warp][e] += __popc(m);   // highest lane of each match group
-    __syncwarp();
   }
 }
 
@@ -271,7 +336,9 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* _
   }
 }
 
-// dw[t][slot] = <dy[t], y[dest[t][slot]]>; one warp per entry.
+// dw[t][slot] = <dy[t], y[dest[t][slot]]>; one warp per entry. The order of the additions is part of the result (16 bytes a lane
+// take 28 us instead of 43 for 32768 entries of 2048 values, but a router gradient that differs in its last bit moves tokens to other
+// experts a step later).
 __global__ void __launch_bounds__(256) moe_combine_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                               const __nv_bfloat16* __restrict__ y,
                                                               const int* __restrict__ dest, int n_entries, int k, int D,
@@ -334,7 +401,25 @@ extern "C" int opk_moe_plan(const int32_t* idx, int n_entries, int E, int exampl
       r_cap < opk_moe_rows_capacity(n_entries, E, examples))
     return -1;
   if (n_entries == 0 && examples > 1) return -1;
-  moe_plan_kernel<<<1, 1024, 0, ST(stream)>>>(idx, n_entries, E, examples, r_cap, dest, src_entry, tile_group, group_k, counts);
+  // From 4096 entries on a cluster (64 experts, us, one CTA -> cluster): 4096 11.1 -> 8.9, 8192 16.6 -> 8.9, 16384 25 -> 10, 32768
+  // 45 -> 13; 2048 takes 8.8 on one CTA.
+  if (n_entries < 4096) {
+    moe_plan_kernel<false><<<1, 1024, 0, ST(stream)>>>(idx, n_entries, E, examples, r_cap, dest, src_entry, tile_group, group_k, counts);
+    return (int)cudaGetLastError();
+  }
+  const int ctas = 8;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(1024);
+  cfg.stream = ST(stream);
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = ctas;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, moe_plan_kernel<true>, idx, n_entries, E, examples, r_cap, dest, src_entry, tile_group, group_k, counts);
+  if (e != cudaSuccess) return (int)e;
   return (int)cudaGetLastError();
 }
 

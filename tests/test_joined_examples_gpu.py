@@ -96,7 +96,8 @@ def test_norms_of_several_gradients_in_one_launch(cuda, batch, N):
         assert abs(one.item() - sums[j].item()) <= 1e-12 * one.item()
 
 
-@pytest.mark.parametrize("E,k,examples,T", [(8, 2, 2, 33), (64, 8, 4, 200), (3, 1, 3, 1), (128, 4, 2, 65)])
+@pytest.mark.parametrize("E,k,examples,T", [(8, 2, 2, 33), (64, 8, 4, 200), (3, 1, 3, 1), (128, 4, 2, 65), (64, 8, 1, 1025),
+                                                (4, 2, 3, 3001)])
 def test_routing_plan_of_several_examples(cuda, E, k, examples, T):
     """Rows sorted by expert, then example, in order; parts of whole 64-row blocks (empty ones too), segments of whole tiles; a
     plan for the first example alone in the same buffers."""

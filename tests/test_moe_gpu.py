@@ -102,3 +102,22 @@ def test_expert_parallel_fused_single_rank(cuda):
     res = ep_fused_check(0, 1, cuda)
     for name in ("out", "dx", "d_router", "acc_wgu", "acc_wd", "norms"):
         assert res[name] < 3e-2, (name, res)
+
+
+@pytest.mark.parametrize("D,offset", [(2, 0), (8, 0), (264, 0), (264, 2), (66, 0), (2048, 0)])
+def test_gradient_of_the_routing_weights(cuda, D, offset):
+    """Dot products of rows with and without 16-byte rows; entries that the plan dropped get zero."""
+    from opake_b200.ops import kernels as K
+
+    T, E, k = 37, 5, 2
+    plan = K.MoePlan(T, E, k, cuda)
+    idx = torch.randint(0, E + 1, (T, k), device=cuda, dtype=torch.int32)            # E: dropped
+    plan.build(idx)
+    y = torch.randn(plan.R * D + offset, device=cuda).to(torch.bfloat16)[offset:].view(plan.R, D)
+    dy = torch.randn(T, D, device=cuda).to(torch.bfloat16)
+    got = torch.full((T, k), 7.0, device=cuda)
+    K.moe_combine_bwd(dy, y, plan, got)
+    rows = y.double()[plan.dest.long().clamp(min=0)]
+    want = (rows * dy.double()[:, None]).sum(-1) * (idx < E)
+    bound = (rows.abs() * dy.double().abs()[:, None]).sum(-1) * (D + 8) * 2.0 ** -24
+    assert ((got.double() - want).abs() <= bound).all()
