@@ -2,8 +2,9 @@
 
 Per optimizer step (logical batch of B sequences, B / W per rank):
 
-1. every rank runs its examples one at a time through ``DecoderRuntime.example_grad`` (tensor-core GEMMs with the
-   per-example norm reduced in the weight-gradient epilogues), clips and adds them into its fp32 sum ``acc``;
+1. every rank runs its examples through ``DecoderRuntime.example_grad`` (tensor-core GEMMs with the per-example norm
+   reduced in the weight-gradient epilogues; on one rank several short examples of an accumulation group in one pass),
+   clips and adds them into its fp32 sum ``acc``;
 2. one fused kernel per rank (``opk_dp_step``) then *reduce-scatters* the sums by reading its shard of every peer's
    ``acc`` over NVLink, normalises by B, adds Philox Gaussian noise indexed by the global element offset (each
    element is owned by exactly one rank, so noise is added exactly once), optionally passes the noise through the
