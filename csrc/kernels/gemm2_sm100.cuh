@@ -75,12 +75,14 @@ struct Gemm2Cfg {
 };
 
 constexpr int kStageWarps = 8;     // copier warps per CTA of the staged variant
-// G2_WIDE: eight epilogue warps (see wide_epilogue); G2_HALF: the same with tiles of 128 columns (see choose_tile).
-enum Gemm2Variant : int { G2_PLAIN = 0, G2_STAGE = 1, G2_WIDE = 2, G2_HALF = 3 };
+// G2_WIDE: eight epilogue warps (see wide_epilogue); G2_HALF: the same with tiles of 128 columns (see choose_tile); G2_TEAMS: eight
+// epilogue warps in two teams of four that take the tiles in turn, so that a warp still covers the whole width of its tile and a
+// norm's fp32 partial sums are those of four warps.
+enum Gemm2Variant : int { G2_PLAIN = 0, G2_STAGE = 1, G2_WIDE = 2, G2_HALF = 3, G2_TEAMS = 4 };
 __host__ __device__ constexpr int gemm2_cols(int variant) { return variant == G2_HALF ? 128 : 256; }
 // The staged variant keeps four epilogue warps: with eight next to its copier warps a thread would have 112 registers.
 __host__ __device__ constexpr int gemm2_epi_warps(int epi, int variant) {
-  return variant == G2_STAGE ? 4 : variant == G2_WIDE || variant == G2_HALF ? 8 : gemm_epi_warps(epi);
+  return variant == G2_STAGE ? 4 : variant >= G2_WIDE ? 8 : gemm_epi_warps(epi);
 }
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
@@ -95,6 +97,7 @@ __launch_bounds__(64 + 32 * gemm2_epi_warps(EPI, VARIANT) + (VARIANT == G2_STAGE
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
   using Cfg = Gemm2Cfg<gemm2_cols(VARIANT)>;
   constexpr bool STAGE = VARIANT == G2_STAGE;
+  constexpr int TEAMS = VARIANT == G2_TEAMS ? 2 : 1;        // each with an accumulator buffer of its own
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -117,7 +120,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 2 * gemm2_epi_warps(EPI, VARIANT));    // the epilogue warps of both CTAs
+      mbar_init(&tempty[b], 2 * gemm2_epi_warps(EPI, VARIANT) / TEAMS);    // the epilogue warps of both CTAs
     }
     *abort_flag = 0;
     fence_barrier_init();
@@ -269,19 +272,20 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs, own 128 rows each)
-    const int quad = warp & 3;
-    constexpr int CSPLIT = gemm2_epi_warps(EPI, VARIANT) / 4;
-    const int c_begin = ((warp - 2) >> 2) * (BN / CSPLIT), c_end = c_begin + BN / CSPLIT;
+    const int quad = warp & 3, quartet = (warp - 2) >> 2;
+    constexpr int CSPLIT = gemm2_epi_warps(EPI, VARIANT) / 4 / TEAMS;
+    const int c_begin = TEAMS == 1 ? quartet * (BN / CSPLIT) : 0, c_end = c_begin + BN / CSPLIT;
     uint8_t* scratch = smem + STAGES * Cfg::STAGE_BYTES + 256 + (warp - 2) * kEpiScratch;
     int it = 0;
     double* sq = sq_slots + (warp - 2) * kSqSums;
     if (EPI == EPI_SUMSQ) epi_zero_sq(sq);
     for (int tile = cluster_id; tile < total; tile += n_clusters, ++it) {
+      const int buf = it & 1;
+      if (TEAMS == 2 && buf != quartet) continue;           // the other team's tile
       const int b = tile / per_batch;
       const int r = tile - b * per_batch;
       int tm, tn;
       tile_coords(r, tiles_m, tiles_n, tm, tn);
-      const int buf = it & 1;
       const uint32_t tph = (it >> 1) & 1;
       if (EPI == EPI_SWIGLU_BWD) prefetch_swiglu_row<BN>(p, tm * 2 * BM + (int)rank * BM + quad * 32 + lane, tn);
       int ok = 1;

@@ -181,14 +181,23 @@ int choose_tile(const OpkGemmArgs* a, int bn, bool pair) {
 
 // Whether the pair kernel takes eight epilogue warps for a plain store. Where the main loop covers the epilogue of the tile before,
 // four are as good and draw less power; eight pay where the epilogue sets the pace (us, four -> eight):
-//   weight gradients over few rows   16384 x 2048 over 317: 28.8 -> 24.3, with norm 35.2 -> 28.7; over 64 25.4 -> 20.4; over 1024
-//                                    51.0 -> 50.4; 128256 x 2048 over 317 189 -> 164 (its 525 MB take 170 us in a copy)
+//   weight gradients over few rows   16384 x 2048 over 317: 28.8 -> 24.3; over 64 25.4 -> 20.4; over 1024 51.0 -> 50.4; 128256 x 2048
+//                                    over 317 189 -> 164 (its 525 MB take 170 us in a copy)
 //   a residual to read               4096 x 768 x 3072 40 -> 33; 2048 x 16384 x 2048 111 -> 103; 1021 x 4096 x 4096 37 -> 33
 //   one round of tiles               the only epilogue is exposed: 2304 x 768 over 1024 16.6 -> 13.1
-// By the tiles of one batch entry: the number of examples in a launch must not choose how a norm is summed.
+// Not for norms: halves of a tile's columns would be halves of their fp32 partial sums (see teams_epilogue).
 bool wide_epilogue(const OpkGemmArgs* a) {
   const long long tiles = (long long)((a->M + 255) / 256) * ((a->N + 255) / 256);
   return a->R || (a->a_mn && a->K <= 512) || tiles <= num_sms() / 2;
+}
+
+// Whether the pair kernel takes two teams of epilogue warps for a weight gradient with its norm: where the epilogue sets the pace, that
+// is over few rows, and a pair has more than one tile. The bits are those of the four warps: how long an example is, and how many
+// share a launch, chooses the faster form and nothing else. (us, four warps -> teams: 16384 x 2048 over 317 rows 35.1 -> 28.1, two examples
+// 65.7 -> 49.7, over 64 rows 33.4 -> 27.8; 128256 x 2048 over 317, two examples 487 -> 381; 3072 x 2048 over 317, two examples 17.4 -> 15.6.)
+bool teams_epilogue(const OpkGemmArgs* a) {
+  const long long tiles = (long long)((a->M + 255) / 256) * ((a->N + 255) / 256) * a->batch;
+  return a->K <= 512 && tiles > num_sms() / 2;
 }
 
 int pick_bn(int N, int epilogue) {
@@ -344,7 +353,7 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
         break;
       case opk::EPI_SUMSQ:
         if (!a->sumsq) { set_err("opk_gemm: sumsq pointer required"); return -1; }
-        if (key == 3 && wide_epilogue(a)) return launch2<true, true, opk::EPI_SUMSQ, opk::G2_WIDE>(ta, tb, p, mc, st);
+        if (key == 3 && teams_epilogue(a)) return launch2<true, true, opk::EPI_SUMSQ, opk::G2_TEAMS>(ta, tb, p, mc, st);
         if (key == 3) return launch2<true, true, opk::EPI_SUMSQ>(ta, tb, p, mc, st);
         break;
       case opk::EPI_SWIGLU:

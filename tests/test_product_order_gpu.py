@@ -94,3 +94,36 @@ def test_pair_tiles_of_128_columns(cuda, M, N, K, b_mn):
     bound = a.double().abs() @ (b.double().abs() if b_mn else b.double().abs().t())
     # one rounding to bf16 and K fp32 additions, each at most 2^-24 of the absolute sum
     assert ((got - exact).abs() <= exact.abs() * 2.0 ** -8 + bound * K * 2.0 ** -24).all()
+
+
+def _norm_by_row_segments(c, width):
+    """Squared norm of ``c [N, K]`` with the fp32 partial sums of the product's epilogue: ``width`` columns of a row one after the other
+    (the squares of bf16 values are exact), 32 rows by halving; the segments in fp64."""
+    N, Kd = c.shape
+    sq = torch.zeros((N + 31) // 32 * 32, (Kd + width - 1) // width * width, device=c.device)
+    sq[:N, :Kd] = c.float() ** 2
+    sq = sq.view(sq.shape[0], -1, width)
+    run = torch.zeros_like(sq[..., 0])
+    for j in range(width):
+        run = run + sq[..., j]
+    run = run.view(-1, 32, run.shape[-1])
+    while run.shape[1] > 1:
+        run = run[:, : run.shape[1] // 2] + run[:, run.shape[1] // 2 :]
+    return run.double().sum().item()
+
+
+@pytest.mark.parametrize("N,K", [(256, 2048), (768, 768), (2304, 768), (2048, 2056), (4104, 2048)])      # one round of tiles, several
+@pytest.mark.parametrize("T", [64, 317, 512, 513, 1024])
+@pytest.mark.parametrize("batch", [1, 3])
+def test_norm_of_a_weight_gradient_is_summed_in_one_way(cuda, N, K, T, batch):
+    """Neither the rows of an example nor the examples of a launch choose the partial sums of its norm."""
+    from opake_b200.ops import gemm as G
+    from opake_b200.ops._lib import raise_if_device_error
+
+    dy, x = _rand((batch, T, N), cuda), _rand((batch, T, K), cuda)
+    sums = torch.zeros(batch, dtype=torch.float64, device=cuda)
+    out = G.linear_wgrad(dy, x, sumsq=sums) if batch > 1 else G.linear_wgrad(dy[0], x[0], sumsq=sums)[None]
+    raise_if_device_error(cuda)
+    for j in range(batch):
+        want = _norm_by_row_segments(out[j], 256)
+        assert abs(sums[j].item() - want) <= 1e-13 * want           # some thousand additions in fp64
