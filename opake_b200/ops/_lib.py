@@ -92,7 +92,14 @@ def stream_ptr(device: torch.device | None = None) -> int:
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
-    return None if t is None else t.data_ptr()
+    """Address of a tensor for a native call. A tensor without memory (fake or meta, while somebody traces) has the address zero,
+    which a kernel must never get; ``NotImplementedError`` is how an operator tells a tracer that it cannot be run on one."""
+    if t is None:
+        return None
+    p = t.data_ptr()
+    if p == 0 and t.numel():
+        raise NotImplementedError("native kernels cannot run on a tensor without memory")
+    return p
 
 
 _ERR: dict[int, torch.Tensor] = {}

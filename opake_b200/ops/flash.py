@@ -6,6 +6,7 @@ import ctypes
 import torch
 
 from . import _lib
+from ._lib import ptr
 
 _P, _I, _L, _F = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_float
 
@@ -28,7 +29,7 @@ def flash_fwd(qkv: torch.Tensor, H: int, KV: int, hd: int, out: torch.Tensor | N
         out = torch.empty(rows, H * hd, dtype=torch.bfloat16, device=qkv.device)
     lse = torch.empty(n_seq * H, T, dtype=torch.float32, device=qkv.device)
     f = _fn("opk_attn_fwd", [_P, _P, _P, _I, _I, _I, _I, _I, _L, _L, _F, _P, _P])
-    rc = f(qkv.data_ptr(), out.data_ptr(), lse.data_ptr(), T, H, KV, hd, n_seq, qkv.stride(0), out.stride(0), hd**-0.5,
+    rc = f(ptr(qkv), ptr(out), ptr(lse), T, H, KV, hd, n_seq, qkv.stride(0), out.stride(0), hd**-0.5,
            _lib.err_word(qkv.device).data_ptr(), _lib.stream_ptr(qkv.device))
     _lib.check(rc, "opk_attn_fwd")
     return out, lse
@@ -43,8 +44,8 @@ def flash_bwd(dout, qkv, out, lse, H: int, KV: int, hd: int, dqkv: torch.Tensor,
     if H > KV and split_heads:
         part = torch.empty(n_seq * 2 * (H // KV) * T * KV * hd, dtype=torch.float32, device=qkv.device)
     f = _fn("opk_attn_bwd", [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _L, _L, _F, _P, _P])
-    rc = f(qkv.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(), dsum.data_ptr(), dqkv.data_ptr(),
-           None if part is None else part.data_ptr(), T, H, KV, hd, n_seq,
+    rc = f(ptr(qkv), ptr(out), ptr(dout), ptr(lse), ptr(dsum), ptr(dqkv),
+           ptr(part), T, H, KV, hd, n_seq,
            qkv.stride(0), out.stride(0), hd**-0.5, _lib.err_word(qkv.device).data_ptr(), _lib.stream_ptr(qkv.device))
     _lib.check(rc, "opk_attn_bwd")
     return dqkv

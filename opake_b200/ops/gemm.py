@@ -14,11 +14,12 @@ EPI_STORE, EPI_SUMSQ, EPI_SWIGLU, EPI_LCE_FWD, EPI_LCE_BWD, EPI_SWIGLU_BWD = ran
 
 
 def _check2d(t: torch.Tensor, name: str) -> None:
+    address = _lib.ptr(t)
     if t.dtype != torch.bfloat16 or not t.is_cuda:
         raise TypeError(f"{name}: expected a CUDA bf16 tensor, got {t.dtype} on {t.device}")
     if t.stride(-1) != 1:
         raise ValueError(f"{name}: last dimension must be contiguous")
-    if t.stride(-2) % 8 != 0 or t.data_ptr() % 16 != 0:
+    if t.stride(-2) % 8 != 0 or address % 16 != 0:
         raise ValueError(f"{name}: row pitch must be a multiple of 8 elements and the base 16-byte aligned")
 
 
@@ -86,8 +87,8 @@ def gemm(
         shape = (batch, M, N) if (batched or group_k is not None) else (M, N)
         out = torch.empty(shape, dtype=torch.bfloat16, device=a.device)
     args = _lib.GemmArgs()
-    args.A, args.B = a.data_ptr(), b.data_ptr()
-    args.C = out.data_ptr() if out is not None else None
+    args.A, args.B = _lib.ptr(a), _lib.ptr(b)
+    args.C = _lib.ptr(out)
     if out is not None:
         _check2d(out, "out")
         args.ldc = out.stride(-2)
@@ -95,7 +96,7 @@ def gemm(
     if residual is not None:
         if residual.shape != out.shape or residual.stride() != out.stride():
             raise ValueError("residual must have the layout of out")
-        args.R = residual.data_ptr()
+        args.R = _lib.ptr(residual)
     args.bias = _lib.ptr(bias)
     args.M, args.N, args.K, args.batch = M, N, K, batch
     args.a_mn, args.b_mn, args.epilogue, args.b_batch_div = int(a_mn), int(b_mn), epilogue, b_batch_div
@@ -105,7 +106,7 @@ def gemm(
     args.alpha, args.softcap = alpha, softcap
     args.sumsq = _lib.ptr(sumsq)
     if act is not None:
-        args.act, args.ld_act = act.data_ptr(), act.stride(-2)
+        args.act, args.ld_act = _lib.ptr(act), act.stride(-2)
     args.labels, args.pmax, args.psum, args.tgt = map(_lib.ptr, (labels, pmax, psum, tgt))
     args.lse, args.coef = _lib.ptr(lse), _lib.ptr(coef)
     if pmax is not None:
@@ -113,20 +114,20 @@ def gemm(
     if z is not None:
         if epilogue != EPI_LCE_FWD or z.dtype != torch.float32 or z.numel() < lce_logits_floats(M, N):
             raise ValueError("z: fp32 buffer of lce_logits_floats() values, filled by the forward cross-entropy epilogue")
-        args.z = z.data_ptr()
+        args.z = _lib.ptr(z)
     args.err = _lib.err_word(a.device).data_ptr()
     args.max_ctas = max_ctas
     if tile_group is not None:      # row-grouped A / C, B batched per group (mixture of experts forward / dgrad)
-        args.tile_group, args.n_groups = tile_group.data_ptr(), b.shape[0]
+        args.tile_group, args.n_groups = _lib.ptr(tile_group), b.shape[0]
         args.strideB = b.stride(0)
     if group_k is not None:         # per-batch reduction ranges over un-batched operands (mixture of experts wgrad)
-        args.group_k = group_k.data_ptr()
+        args.group_k = _lib.ptr(group_k)
     args.sumsq_shared, args.stepwise = int(sumsq_shared), int(stepwise)
     if stage is not None:           # b lives on another GPU: (local scratch [N, K] bf16, int32 band counters)
         scratch, ready = stage
         if scratch.numel() < N * K or scratch.dtype != torch.bfloat16 or ready.dtype != torch.int32 or ready.numel() * 2048 < N:
             raise ValueError("stage: scratch must hold N * K bf16 values and the counters one int32 per 2048 rows of b")
-        args.stage_dst, args.stage_ready = scratch.data_ptr(), ready.data_ptr()
+        args.stage_dst, args.stage_ready = _lib.ptr(scratch), _lib.ptr(ready)
     _lib.check(_lib.lib().opk_gemm(args, _lib.stream_ptr(a.device)), "opk_gemm")
     return out
 
@@ -186,7 +187,7 @@ def lce_grad(z: torch.Tensor, labels: torch.Tensor, lse: torch.Tensor, coef: tor
     _check2d(out, "out")
     if z.numel() < lce_logits_floats(M, N):
         raise ValueError("z holds fewer logits than out has elements")
-    _lib.check(_lib.lib().opk_lce_grad(z.data_ptr(), labels.data_ptr(), lse.data_ptr(), coef.data_ptr(), out.data_ptr(), out.stride(0),
+    _lib.check(_lib.lib().opk_lce_grad(_lib.ptr(z), _lib.ptr(labels), _lib.ptr(lse), _lib.ptr(coef), _lib.ptr(out), out.stride(0),
                                        M, N, softcap, _lib.stream_ptr(out.device)), "opk_lce_grad")
     return out
 

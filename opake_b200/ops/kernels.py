@@ -25,8 +25,7 @@ def _s(t: torch.Tensor) -> int:
     return _lib.stream_ptr(t.device)
 
 
-def _p(t):
-    return None if t is None else t.data_ptr()
+_p = _lib.ptr
 
 
 def _chk(code: int, name: str) -> None:
@@ -340,8 +339,8 @@ def clip_accumulate_group(gs, scales, acc, overwrite: bool = False):
     n = len(gs)
     if not 1 <= n <= 8 or len(scales) != n:
         raise ValueError("a group holds 1 to 8 gradient buffers with one scale each")
-    gp = (ctypes.c_void_p * n)(*[g.data_ptr() for g in gs])
-    sp = (ctypes.c_void_p * n)(*[t.data_ptr() for t in scales])
+    gp = (ctypes.c_void_p * n)(*[_p(g) for g in gs])
+    sp = (ctypes.c_void_p * n)(*[_p(t) for t in scales])
     _chk(_L().opk_clip_accumulate_group(gp, sp, n, _p(acc), gs[0].numel(), int(overwrite), _s(acc)), "clip_accumulate_group")
 
 
@@ -354,8 +353,8 @@ def clip_accumulate_group_push(gs, scales, acc_ptrs: list[int], bounds: list[int
     k = len(gs)
     if not 1 <= k <= 8 or len(scales) != k:
         raise ValueError("a group holds 1 to 8 gradient buffers with one scale each")
-    gp = (ctypes.c_void_p * k)(*[g.data_ptr() for g in gs])
-    sp = (ctypes.c_void_p * k)(*[t.data_ptr() for t in scales])
+    gp = (ctypes.c_void_p * k)(*[_p(g) for g in gs])
+    sp = (ctypes.c_void_p * k)(*[_p(t) for t in scales])
     ap = (ctypes.c_void_p * len(acc_ptrs))(*acc_ptrs)
     bp = (ctypes.c_int64 * len(bounds))(*bounds)
     _chk(_L().opk_clip_accumulate_group_push(gp, sp, k, ap, bp, len(acc_ptrs), rank, n, _s(gs[0])), "clip_accumulate_group_push")
@@ -408,8 +407,8 @@ def dp_step(*, grad_src: list[int], shard_begin: int, shard_len: int, inv_batch:
     if group:
         if len(group) != len(group_scales) or len(group) > 8 or any(g.numel() < group_len for g in group):
             raise ValueError("a group holds 1 to 8 gradient buffers of at least group_len elements with one scale each")
-        a.group_g = (ctypes.c_void_p * len(group))(*[g.data_ptr() for g in group])
-        a.group_scale = (ctypes.c_void_p * len(group))(*[t.data_ptr() for t in group_scales])
+        a.group_g = (ctypes.c_void_p * len(group))(*[_p(g) for g in group])
+        a.group_scale = (ctypes.c_void_p * len(group))(*[_p(t) for t in group_scales])
     a.n_group, a.group_len, a.skip_sum = len(group), group_len, int(skip_sum)
     dev = device if device is not None else (m.device if m is not None else torch.device("cuda"))
     _chk(_L().opk_dp_step(ctypes.byref(a), _lib.stream_ptr(dev)), "dp_step")

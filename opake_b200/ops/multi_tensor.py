@@ -56,7 +56,7 @@ def _pack(rows) -> bytes:
         ptrs, mask = [0] * 6, 0
         for i, t in enumerate(bufs):
             if t is not None:
-                ptrs[i] = t.data_ptr()
+                ptrs[i] = _lib.ptr(t)
                 if t.dtype is torch.bfloat16:
                     mask |= 1 << i
         # c_float rounds and overflows to infinity like a scalar next to an fp32 tensor; struct refuses what is out of range
@@ -90,10 +90,10 @@ def clip_and_sum(leaves, clip: float, guards, outs, *, prev=None, scale: float =
     norms = torch.empty(B, dtype=torch.float64, device=dev)
     clipped = torch.empty(B, dtype=torch.bool, device=dev)
     post = torch.empty(B, n_ap, dtype=torch.float64, device=dev) if with_postsq else None
-    _call("opk_mt_sumsq_partial", dev, blob, len(leaves), B, n_sq, partial.data_ptr())
+    _call("opk_mt_sumsq_partial", dev, blob, len(leaves), B, n_sq, _lib.ptr(partial))
     (kb, tb), (kf, tf) = guards
-    _call("opk_mt_clip_factors", dev, partial.data_ptr(), n_sq, B, clip, kb, tb, kf, tf, factors[0].data_ptr(), factors[1].data_ptr(),
-          norms.data_ptr(), clipped.data_ptr())
+    _call("opk_mt_clip_factors", dev, _lib.ptr(partial), n_sq, B, clip, kb, tb, kf, tf, factors[0].data_ptr(), factors[1].data_ptr(),
+          _lib.ptr(norms), _lib.ptr(clipped))
     _call("opk_mt_apply_sum", dev, blob, len(leaves), B, n_ap, factors[0].data_ptr(), factors[1].data_ptr(), scale, _lib.ptr(post))
     return norms, clipped, (None if post is None else post.sum(1))
 

@@ -115,3 +115,23 @@ def test_text_argument_and_saved_outputs():
         plain = lambda a, x: lin(fn(lin(x, p[0], a)) * lin(x, p[1], p[1][1]), p[2], p[2][1]).pow(2).sum()
         got, want = (vmap(grad(f, (0, 1)), (None, 0))(p[0][1], X) for f in (fused, plain))
         assert all((g - w).norm() <= 1e-5 * w.norm() for g, w in zip(got, want))        # the activation is formed in fp32
+
+
+@pytest.mark.parametrize("through_dispatcher", [False, True])
+def test_tensors_without_memory_are_refused(through_dispatcher):
+    """Under a tracer's FakeTensorMode no kernel may be launched: a fake tensor has the address zero."""
+    from torch._subclasses.fake_tensor import FakeTensorMode, UnsupportedOperatorException
+
+    from opake_b200.ops import flash, gemm, lce
+    from opake_b200.patches.kernels import functions as fns, lora
+
+    run = (lambda op, *a: op.call(*a)) if through_dispatcher else (lambda op, *a: op(*a))
+    with FakeTensorMode():
+        x = torch.empty(128, 64, device="cuda", dtype=torch.bfloat16)
+        label = torch.empty(128, device="cuda", dtype=torch.int64)
+        for f in (lambda: run(fns._Glu, x, x, 0), lambda: run(fns._RMSNorm, x, x[0], 1e-5, 0.0), lambda: run(fns._AddRMSNorm, x, x, x[0], 1e-5, 0.0),
+                  lambda: run(fns._CE, x, label, 1.0, 0.0), lambda: run(fns._RopeQK, x, x.float(), 1, 64),
+                  lambda: run(lce._LinearCE, x, x, label, 1.0, 0.0, True), lambda: lora._LoRA(x, x[:64], x[:8], x[:64, :8], 1.0),
+                  lambda: gemm.gemm(x, x), lambda: flash.flash_fwd(torch.empty(128, 192, device="cuda", dtype=torch.bfloat16), 1, 1, 64)):
+            with pytest.raises((NotImplementedError, UnsupportedOperatorException)):
+                f()
