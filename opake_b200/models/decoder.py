@@ -73,7 +73,7 @@ class DecoderRuntime:
         self.clip_count = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._ws: dict[tuple[int, int], dict] = {}
         self._parts: dict[tuple, dict] = {}
-        self._rope = None
+        self._rope = K.RopeTables(cfg.head_dim, cfg.rope_theta, cfg.rope_scaling, cfg.max_seq)
         # weights to pull from their owner during the NEXT forward pass (name -> the owner's copy, a peer-mapped
         # tensor): the consuming GEMM copies the matrix into this rank's replica band by band while it multiplies
         self._fetch: dict[str, torch.Tensor] | None = None
@@ -243,11 +243,7 @@ class DecoderRuntime:
         return ws["z"]
 
     def _rope_table(self, T: int):
-        cfg = self.cfg
-        if self._rope is None or self._rope.shape[0] < T:
-            self._rope = K.rope_table(max(T, cfg.max_seq), cfg.head_dim, cfg.rope_theta, device=self.device,
-                                      scaling=cfg.rope_scaling)
-        return self._rope
+        return self._rope.get(T, self.device)
 
     def _vec(self, ws, name: str) -> torch.Tensor:
         """Gradient of a vector parameter: ``[numel]``, or ``[n, numel]`` for ``n`` sequences."""

@@ -13,7 +13,7 @@ from typing import Any, Mapping
 import torch
 from torch import nn
 
-from ..ops.kernels import rope_table
+from ..ops.kernels import RopeTables
 from .config import DecoderConfig
 from .flat import build_layout
 from .reference_torch import decoder_hidden
@@ -27,7 +27,7 @@ class NativeCausalLM(nn.Module):
         self.cfg = cfg
         self.layout = build_layout(cfg)
         self.flat = nn.Parameter(torch.zeros(self.layout.total, dtype=dtype, device=device))
-        self._rope = None
+        self._rope = RopeTables(cfg.head_dim, cfg.rope_theta, cfg.rope_scaling, cfg.max_seq)
         if init_seed is not None:
             from .decoder import init_params_
             with torch.no_grad():
@@ -42,12 +42,7 @@ class NativeCausalLM(nn.Module):
         return self.layout.views(self.flat if flat is None else flat)
 
     def _rope_table(self, T: int, device) -> torch.Tensor | None:
-        if self.cfg.pos != "rope":
-            return None
-        if self._rope is None or self._rope.shape[0] < T or self._rope.device != device:
-            self._rope = rope_table(max(T, self.cfg.max_seq), self.cfg.head_dim, self.cfg.rope_theta, device=device,
-                                    scaling=self.cfg.rope_scaling)
-        return self._rope
+        return self._rope.get(T, device) if self.cfg.pos == "rope" else None
 
     def hidden_states(self, input_ids: torch.Tensor) -> torch.Tensor:
         """Final-norm hidden states ``[..., T, d]``."""

@@ -136,6 +136,24 @@ def rope_table(seq_len: int, head_dim: int, theta: float = 10000.0, device=None,
     return torch.stack([ang.cos(), ang.sin()], dim=-1).to(torch.float32).to(device).contiguous()
 
 
+class RopeTables:
+    """The rotary tables of one model, longer ones as longer sequences come. None is dropped: a CUDA graph that was captured for shorter
+    sequences reads the table of its time. Each is at least twice as long as the one before it, so all together are less than two of
+    the longest."""
+
+    def __init__(self, head_dim: int, theta: float, scaling: dict | None, rows: int):
+        self.args, self.rows = (head_dim, theta), rows
+        self.scaling = scaling
+        self.tables: dict[str, list[torch.Tensor]] = {}
+
+    def get(self, T: int, device) -> torch.Tensor:
+        kept = self.tables.setdefault(str(device), [])
+        if not kept or kept[-1].shape[0] < T:
+            rows = max(T, 2 * kept[-1].shape[0] if kept else self.rows)
+            kept.append(rope_table(rows, *self.args, device=device, scaling=self.scaling))
+        return kept[-1]
+
+
 def rope_(qk, table, n_heads: int, head_dim: int, pos=None, backward: bool = False, period: int = 0):
     """Rotate the first ``n_heads`` heads of every row of ``qk`` in place (rotate-half convention). Row ``t`` sits at
     position ``pos[t]``, else ``t % period`` (``period`` rows per sequence), else ``t``."""

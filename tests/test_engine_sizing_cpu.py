@@ -55,3 +55,24 @@ def test_consolidate_per_rank_shards_into_one_state():
     import pytest
     with pytest.raises(ValueError):
         ShardedDPEngine.consolidate(shards[:2])
+
+
+def test_rotary_tables_that_a_graph_may_read_are_kept():
+    """A longer sequence needs a longer table; a graph that was captured before still reads the address of the shorter one."""
+    import weakref
+
+    from opake_b200.models.config import tiny_llama
+    from opake_b200.models.decoder import DecoderRuntime
+    from opake_b200.models.flat import build_layout
+    from opake_b200.models.native import NativeCausalLM
+
+    cfg = tiny_llama()
+    layout = build_layout(cfg)
+    rt = DecoderRuntime(cfg, torch.zeros(layout.total, dtype=torch.bfloat16), layout=layout)
+    model = NativeCausalLM(cfg, init_seed=None)
+    for table in (rt._rope_table, lambda T: model._rope_table(T, torch.device("cpu"))):
+        short = weakref.ref(table(16))
+        long = table(cfg.max_seq + 1)
+        assert short() is not None and long.shape[0] > cfg.max_seq and torch.equal(long[: cfg.max_seq], short())
+        seen = {table(T).data_ptr() for T in range(cfg.max_seq + 1, 4 * cfg.max_seq)}
+        assert len(seen) <= 3                      # each at least twice as long as the one before
