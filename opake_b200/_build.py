@@ -119,7 +119,10 @@ def build_nodes(force: bool = False) -> Path:
         f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(NODES_LIB), *(f"-L{p}" for p in library_paths()),
         "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10",
     ]
-    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    try:
+        r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    except OSError as exc:
+        raise RuntimeError(f"build of the autograd nodes failed: no C++ compiler ({exc})") from exc
     if r.returncode != 0:
         raise RuntimeError(f"build of the autograd nodes failed:\n{r.stdout}")
     return NODES_LIB

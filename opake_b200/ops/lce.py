@@ -24,13 +24,14 @@ IGNORE_INDEX = -100
 # Logits of one loss that may wait for its backward pass. They are twice the bf16 gradient that the backward pass
 # writes anyway; beyond this size the second product is the smaller price.
 KEEP_BYTES = 1 << 30
+_TOP_HOOKS = getattr(torch._C._autograd, "_top_saved_tensors_default_hooks", None)       # without it nothing is kept
 
 
 def _keep_logits(hidden, weight) -> bool:
     """Whether the forward pass leaves its logits for a backward pass: one is coming, and nobody is moving or replacing what
     autograd saves (offloading hooks would carry the logits around)."""
     return (torch.is_grad_enabled() and (hidden.requires_grad or weight.requires_grad)
-            and torch._C._autograd._top_saved_tensors_default_hooks(True) is None)
+            and _TOP_HOOKS is not None and _TOP_HOOKS(True) is None)
 
 
 def native_available(hidden: torch.Tensor, weight: torch.Tensor) -> bool:
