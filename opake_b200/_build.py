@@ -19,8 +19,6 @@ OUT = Path(__file__).resolve().parent / "_C"
 KERNEL_LIB = OUT / "libopake_kernels.so"
 # same sources with -DOPK_DEBUG_BOUNDS: data-dependent indices are checked, a bad one is recorded and its access skipped
 KERNEL_LIB_DEBUG = OUT / "libopake_kernels_debug.so"
-# autograd nodes of the operators of ops/nodes.py: the one library here that is compiled against torch's headers
-NODES_LIB = OUT / ("_opake_nodes" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 ACCOUNTING_LIB = OUT / ("_opake_accounting" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC_FLAGS = [
@@ -104,28 +102,46 @@ def build_accounting(force: bool = False) -> Path:
     return ACCOUNTING_LIB
 
 
+def nodes_lib() -> Path:
+    """The autograd nodes of the operators of ops/nodes.py: the one library here that is compiled against torch's headers. Its name tells
+    the torch and the source that it was built from, so one of another torch or of an older source is never taken for it."""
+    import hashlib
+
+    import torch
+
+    source = hashlib.sha256((CSRC / "host" / "nodes.cpp").read_bytes()).hexdigest()[:12]
+    torch_version = "".join(c if c.isalnum() or c == "." else "_" for c in torch.__version__)
+    return OUT / f"_opake_nodes-torch{torch_version}-{source}{sysconfig.get_config_var('EXT_SUFFIX') or '.so'}"
+
+
 def build_nodes(force: bool = False) -> Path:
-    """Compile the autograd nodes of the dispatcher operators (host code on torch's C++ API)."""
-    src = CSRC / "host" / "nodes.cpp"
-    if not force and _newer(NODES_LIB, [src]):
-        return NODES_LIB
+    """Compile the autograd nodes of the dispatcher operators (host code on torch's C++ API). The library appears whole or not at all:
+    several ranks may look for it, and build it, at once."""
+    src, target = CSRC / "host" / "nodes.cpp", nodes_lib()
+    if not force and target.exists():
+        return target
     import torch
     from torch.utils.cpp_extension import include_paths, library_paths
+
+    part = target.with_name(f"{target.name}.{os.getpid()}.part")
 
     OUT.mkdir(parents=True, exist_ok=True)
     cmd = [
         os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=_opake_nodes",
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{p}" for p in include_paths()),
-        f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(NODES_LIB), *(f"-L{p}" for p in library_paths()),
+        f"-I{sysconfig.get_paths()['include']}", str(src), "-o", str(part), *(f"-L{p}" for p in library_paths()),
         "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10",
     ]
     try:
         r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"build of the autograd nodes failed:\n{r.stdout}")
+        os.replace(part, target)
     except OSError as exc:
         raise RuntimeError(f"build of the autograd nodes failed: no C++ compiler ({exc})") from exc
-    if r.returncode != 0:
-        raise RuntimeError(f"build of the autograd nodes failed:\n{r.stdout}")
-    return NODES_LIB
+    finally:
+        part.unlink(missing_ok=True)
+    return target
 
 
 def build_all(force: bool = False, verbose: bool = False) -> None:

@@ -14,7 +14,7 @@ import warnings
 
 import torch
 
-from .._build import NODES_LIB, build_nodes
+from .._build import build_nodes, nodes_lib
 
 _LIB = torch.library.Library("opake_b200", "DEF")
 
@@ -46,9 +46,10 @@ def _native():
 
     name = "opake_b200._C._opake_nodes"
     if name not in sys.modules:
-        if not NODES_LIB.exists():
+        path = nodes_lib()
+        if not path.exists():
             build_nodes()
-        spec = importlib.util.spec_from_file_location(name, NODES_LIB)
+        spec = importlib.util.spec_from_file_location(name, path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         sys.modules[name] = module

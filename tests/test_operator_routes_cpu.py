@@ -32,7 +32,7 @@ def test_without_library_and_compiler(tmp_path):
 import warnings
 from pathlib import Path
 from opake_b200 import _build
-_build.OUT = Path(%r); _build.NODES_LIB = _build.OUT / _build.NODES_LIB.name
+_build.OUT = Path(%r)
 warnings.simplefilter("error")
 import torch
 import opake_b200.patches, opake_b200.patches.kernels, opake_b200.ops.lce, opake_b200.alignment.logprob, opake_b200.alignment.sft.loss
@@ -52,3 +52,46 @@ print("fell back")
 """ % str(tmp_path)
     run = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env={**os.environ, "CXX": "/nonexistent/compiler"}, capture_output=True, text=True)
     assert run.returncode == 0 and "fell back" in run.stdout, run.stderr[-2000:]
+
+
+def test_library_of_another_torch_or_source_is_not_taken(tmp_path, monkeypatch):
+    import torch
+
+    from opake_b200 import _build
+
+    name = _build.nodes_lib().name
+    monkeypatch.setattr(torch, "__version__", "9.9.9+other")
+    other_torch = _build.nodes_lib().name
+    monkeypatch.undo()
+    (tmp_path / "host").mkdir()
+    (tmp_path / "host" / "nodes.cpp").write_bytes((_build.CSRC / "host" / "nodes.cpp").read_bytes() + b"\n")
+    monkeypatch.setattr(_build, "CSRC", tmp_path)
+    assert len({name, other_torch, _build.nodes_lib().name}) == 3
+
+
+@pytest.mark.parametrize("status", [0, 1])
+def test_library_appears_whole(tmp_path, monkeypatch, status):
+    """While the compiler writes, nothing stands where the library will be; a failed build leaves nothing behind."""
+    from opake_b200 import _build
+
+    monkeypatch.setattr(_build, "OUT", tmp_path / "out")
+    seen = tmp_path / "seen"
+    compiler = tmp_path / "cxx"
+    compiler.write_text(f'''#!{sys.executable}
+import os, sys
+out = sys.argv[sys.argv.index("-o") + 1]
+open(out, "w").write("half")
+open({str(seen)!r}, "w").write(str(os.path.exists({str(_build.nodes_lib())!r})))
+open(out, "a").write(" and half")
+sys.exit({status})
+''')
+    compiler.chmod(0o755)
+    monkeypatch.setenv("CXX", str(compiler))
+    if status:
+        with pytest.raises(RuntimeError, match="build of the autograd nodes failed"):
+            _build.build_nodes()
+        assert not list((tmp_path / "out").iterdir())
+    else:
+        path = _build.build_nodes()
+        assert path.read_text() == "half and half" and list((tmp_path / "out").iterdir()) == [path]
+    assert seen.read_text() == "False"
