@@ -5,8 +5,9 @@ linear_cross_entropy.py:1223-1276, kernels :101-247 and :292-528). The reference
 program and merges partial log-sum-exps under a spin lock; here the vocabulary GEMM runs on the tcgen05 kernel with
 two epilogues: the forward epilogue reduces every 256-column tile to (max, sum-exp, target logit) per row, a tiny
 finalize kernel merges the tiles, and the backward epilogue recomputes the logits tile and writes
-``coef * (softmax - onehot)`` in bf16, from which dH and dW are two more GEMMs. Up to ``KEEP_BYTES`` of logits are left
-behind by the forward epilogue for one backward pass instead (same bits, a pass over memory in place of the product).
+``coef * (softmax - onehot)`` in bf16, from which dH and dW are two more GEMMs. Up to ``KEEP_BYTES`` of logits, over all losses
+that wait for their backward pass, are left behind by the forward epilogue instead where memory is plenty (same bits, a pass
+over memory in place of the product).
 
 Both directions are dispatcher operators (``ops/nodes.py``) with ``vmap`` rules so that ``vmap(grad(loss))`` works: a
 batch of examples sharing one weight is flattened into rows for the forward and dH; the per-example weight gradient
@@ -15,15 +16,22 @@ the same ``(B, V, D)`` result).
 """
 from __future__ import annotations
 
+import threading
+
 import torch
+from torch.multiprocessing.reductions import StorageWeakRef
 
 from .nodes import Operator, front
 
 IGNORE_INDEX = -100
 
-# Logits of one loss that may wait for its backward pass. They are twice the bf16 gradient that the backward pass
-# writes anyway; beyond this size the second product is the smaller price.
+# Logits that may wait for their backward passes at a time, over all losses on a device. They are twice the bf16 gradient that a
+# backward pass writes anyway; beyond this size the second product is the smaller price.
 KEEP_BYTES = 1 << 30
+# Up to here nobody asks how much memory is left: the count takes 60 us on the host.
+_UNASKED_BYTES = 256 << 20
+_WAITING: list[tuple[torch.device, StorageWeakRef, int]] = []
+_WAITING_LOCK = threading.Lock()
 _TOP_HOOKS = getattr(torch._C._autograd, "_top_saved_tensors_default_hooks", None)       # without it nothing is kept
 
 
@@ -56,8 +64,29 @@ def _chunked_nll(hidden, weight, labels, logit_scale, softcap, chunk: int = 4096
 
 
 # ------------------------------------------------------------------------------------------- native forward
-def _native_fwd(hidden, weight, labels, logit_scale, softcap, keep):
-    """``(nll, lse, int32 labels, logits)``; the last one is empty unless ``keep`` and the size allows it."""
+def _logits_buffer(rows: int, vocab: int, dim: int, examples: int, device) -> torch.Tensor:
+    """fp32 buffer in which the logits wait for their backward pass; empty where the losses that are waiting already leave no room for
+    them, or the device would not have as much memory again as they and the backward pass take. (They stay through all of the backward
+    pass: it may be asked for a second time.)"""
+    from . import _lib, gemm as G
+    n = G.lce_logits_floats(rows, vocab)
+    # d logits, d hidden, d weight per example and its scaled copy
+    needed = 4 * n + 2 * (n + rows * dim + 2 * examples * vocab * dim)
+    with _WAITING_LOCK:
+        _WAITING[:] = [w for w in _WAITING if not w[1].expired()]
+        waiting = 4 * n + sum(size for dev, _, size in _WAITING if dev == device)
+        if waiting <= KEEP_BYTES and (waiting <= _UNASKED_BYTES or 2 * needed <= _lib.free_bytes(device, plenty=16 * needed)):
+            try:
+                z = torch.empty(n, dtype=torch.float32, device=device)
+                _WAITING.append((device, StorageWeakRef(z.untyped_storage()), 4 * n))
+                return z
+            except torch.cuda.OutOfMemoryError:
+                pass
+    return torch.empty(0, dtype=torch.float32, device=device)
+
+
+def _native_fwd(hidden, weight, labels, logit_scale, softcap, keep, examples=1):
+    """``(nll, lse, int32 labels, logits)``; the last one is empty unless ``keep`` and there is room for them."""
     from . import gemm as G, kernels as K
     T, V = hidden.shape[0], weight.shape[0]
     tiles = G.lce_tiles(V, parts=2 if softcap else 1)
@@ -65,11 +94,9 @@ def _native_fwd(hidden, weight, labels, logit_scale, softcap, keep):
     psum = torch.empty_like(pmax)
     tgt = torch.empty(T, dtype=torch.float32, device=hidden.device)
     lab = labels.to(torch.int32, copy=True).contiguous()      # kept for the backward pass: never the caller's buffer
-    n = G.lce_logits_floats(T, V)
-    try:
-        keep = keep and 4 * n <= KEEP_BYTES and G.lce_keeps_logits(T, V, hidden.shape[1], softcap)
-        z = torch.empty(n if keep else 0, dtype=torch.float32, device=hidden.device)
-    except torch.cuda.OutOfMemoryError:
+    if keep and G.lce_keeps_logits(T, V, hidden.shape[1], softcap):
+        z = _logits_buffer(T, V, hidden.shape[1], examples, hidden.device)
+    else:
         z = torch.empty(0, dtype=torch.float32, device=hidden.device)
     G.gemm(hidden, weight, epilogue=G.EPI_LCE_FWD, labels=lab, pmax=pmax, psum=psum, tgt=tgt, alpha=logit_scale,
            softcap=softcap, z=z if z.numel() else None)
@@ -132,7 +159,7 @@ def _linear_ce_vmap(B, in_dims, hidden, weight, labels, logit_scale, softcap, ke
         raise NotImplementedError("fused linear cross-entropy under vmap needs one shared weight")
     h, lb = front(hidden, in_dims[0], B), front(labels, in_dims[2], B)
     T, D = h.shape[1], h.shape[2]
-    nll, lse, lab, z = _native_fwd(h.reshape(B * T, D).contiguous(), weight, lb.reshape(B * T), logit_scale, softcap, keep)
+    nll, lse, lab, z = _native_fwd(h.reshape(B * T, D).contiguous(), weight, lb.reshape(B * T), logit_scale, softcap, keep, B)
     return (nll.view(B, T), lse.view(B, T), lab.view(B, T), z), (0, 0, 0, None)
 
 

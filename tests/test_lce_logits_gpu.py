@@ -70,3 +70,35 @@ def test_loss_gradients_do_not_depend_on_kept_logits(cuda, cap, monkeypatch):
     with torch.no_grad():
         lce.linear_cross_entropy(h[0], w, lab[0])
     assert kept[-1][3].numel() == 0
+
+
+def test_losses_that_wait_share_one_limit_and_give_way_to_scarce_memory(cuda, monkeypatch):
+    """Several losses before one backward pass (preference pairs, sums of losses) keep no more logits together than one may, none at all
+    where memory is short, and the same bits come out; the room is free again when their graphs are gone."""
+    from opake_b200.ops import _lib, gemm as G, lce
+
+    torch.manual_seed(1)
+    T, D, V = 40, 64, 700
+    one = 4 * G.lce_logits_floats(T, V)
+    hs, w = [_rand((T, D), cuda) for _ in range(4)], _rand((V, D), cuda, 0.2).requires_grad_()
+    lab = torch.randint(0, V, (T,), device=cuda)
+    sizes = []
+    inner = lce._native_fwd
+    monkeypatch.setattr(lce, "_native_fwd", lambda *a: (r := inner(*a), sizes.append(4 * r[3].numel()))[0])
+
+    def run():
+        sizes.clear()
+        grads = torch.autograd.grad(sum(lce.linear_cross_entropy(h, w, lab).sum() for h in hs), w)
+        return grads[0], list(sizes)
+
+    want, all_kept = run()
+    assert all_kept == [one] * 4
+    monkeypatch.setattr(lce, "KEEP_BYTES", 5 * one // 2)
+    for _ in range(2):                                   # the first pass's logits are gone when the second one begins
+        got, kept = run()
+        assert kept == [one, one, 0, 0] and torch.equal(got, want)
+    monkeypatch.setattr(lce, "_UNASKED_BYTES", 0)
+    assert run()[1] == [one, one, 0, 0]
+    monkeypatch.setattr(_lib, "free_bytes", lambda device, plenty=None: 2 * one)
+    got, kept = run()
+    assert kept == [0] * 4 and torch.equal(got, want)
