@@ -19,6 +19,7 @@ from dataclasses import dataclass
 
 import torch
 
+from ..ops import _lib
 from ..ops import attention as A
 from ..ops import gemm as G
 from ..ops import kernels as K
@@ -73,6 +74,8 @@ class DecoderRuntime:
         self.clip_count = torch.zeros(1, dtype=torch.int32, device=self.device)
         self._ws: dict[tuple[int, int], dict] = {}
         self._parts: dict[tuple, dict] = {}
+        self._logits: list[torch.Tensor] = []
+        self._logits_limit: int | None = None            # floats
         self._rope = K.RopeTables(cfg.head_dim, cfg.rope_theta, cfg.rope_scaling, cfg.max_seq)
         # weights to pull from their owner during the NEXT forward pass (name -> the owner's copy, a peer-mapped
         # tensor): the consuming GEMM copies the matrix into this rank's replica band by band while it multiplies
@@ -224,23 +227,38 @@ class DecoderRuntime:
 
     def _logits_buffer(self, ws: dict) -> torch.Tensor | None:
         """fp32 logits that the loss leaves for its backward pass, which then needs no second product with the head. ``None``,
-        for good, where the product is the cheaper one or they would take more than a quarter of the memory that is free."""
+        for good, where the product is the cheaper one or the memory for them is not there (see :meth:`_shared_logits`)."""
         ws = self._ws[ws["key"]]          # the whole set, T its rows
         T = ws["labels"].numel()
         if "z" in ws or self.device.type != "cuda":
             return ws.get("z")
         if torch.cuda.is_current_stream_capturing():
             return None
-        dev = self.device
-        free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-        n = G.lce_logits_floats(T, self.cfg.vocab_size)
-        ws["z"] = None
-        if 16 * n <= free and G.lce_keeps_logits(T, self.cfg.vocab_size, self.cfg.d_model):
-            try:
-                ws["z"] = self._alloc(n, dtype=torch.float32, name=f"logits[rows={T}]")
-            except torch.cuda.OutOfMemoryError:
-                pass
+        keep = G.lce_keeps_logits(T, self.cfg.vocab_size, self.cfg.d_model)
+        ws["z"] = self._shared_logits(G.lce_logits_floats(T, self.cfg.vocab_size)) if keep else None
         return ws["z"]
+
+    def _shared_logits(self, n: int) -> torch.Tensor | None:
+        """At least ``n`` floats, the same for all lengths: they are live between the loss of a pass and its gradient only. A buffer that has
+        become too short stays, because graphs may read it; the next one is twice as long where it may be. All of them together
+        take at most a quarter of the memory that was free when the first was asked for, and each a quarter of what is free."""
+        exact = self.canaries is not None                # guard bands have to begin behind the last logit
+        for z in self._logits:
+            if z.numel() == n if exact else z.numel() >= n:
+                return z
+        free = _lib.free_bytes(self.device) // 16
+        if self._logits_limit is None:
+            self._logits_limit = free
+        room = min(free, self._logits_limit - sum(z.numel() for z in self._logits))
+        longest = max((z.numel() for z in self._logits), default=0)
+        size = 2 * longest if n < 2 * longest <= room and not exact else n
+        if size > room:
+            return None
+        try:
+            self._logits.append(self._alloc(size, dtype=torch.float32, name=f"logits[{n}]"))
+        except torch.cuda.OutOfMemoryError:
+            return None
+        return self._logits[-1]
 
     def _rope_table(self, T: int):
         return self._rope.get(T, self.device)

@@ -39,3 +39,35 @@ def test_sequences_longer_than_the_rotary_table(cuda):
         junk = [torch.full((1 << k,), float("nan"), device=cuda) for k in range(8, 20)]         # what was given back is taken again
         del junk
     _same(a, b)
+
+
+def _kept_logits(eng):
+    """Bytes of the distinct buffers in which workspaces leave logits."""
+    zs = {ws["z"].untyped_storage().data_ptr(): ws["z"].untyped_storage().nbytes() for ws in eng.runtime._ws.values() if ws.get("z") is not None}
+    return sum(zs.values())
+
+
+@pytest.mark.parametrize("lengths", [(100, 90, 75, 61, 50, 41, 33), (33, 41, 50, 61, 75, 90, 100)])
+def test_stored_logits_of_all_lengths_share_their_memory(cuda, lengths, monkeypatch):
+    """Steps of many lengths, each twice (captured, replayed): at most four times what the longest needs, within the limit where memory is
+    short, and the bits of an engine without stored logits."""
+    from opake_b200.models.decoder import DecoderRuntime
+    from opake_b200.ops import _lib, gemm as G
+
+    a, b, c = _engine(cuda), _engine(cuda), _engine(cuda)
+    vocab = a.model_cfg.vocab_size
+    one = 4 * G.lce_logits_floats(3 * max(lengths), vocab)         # three examples go through the model together
+    steps = [_batch(a.model_cfg, 4, T, T + i) for i in range(2) for T in lengths]
+    for batch in steps:
+        a.step(*batch)
+    assert 0 < _kept_logits(a) <= 4 * one
+    with monkeypatch.context() as m:
+        m.setattr(_lib, "free_bytes", lambda device, plenty=None: 4 * one // 2)
+        for batch in steps:
+            b.step(*batch)
+    assert 0 < _kept_logits(b) <= one // 2
+    monkeypatch.setattr(DecoderRuntime, "_logits_buffer", lambda self, ws: None)
+    for batch in steps:
+        c.step(*batch)
+    _same(a, c)
+    _same(b, c)
