@@ -76,6 +76,8 @@ class DecoderRuntime:
         self._parts: dict[tuple, dict] = {}
         self._logits: list[torch.Tensor] = []
         self._logits_limit: int | None = None            # floats
+        self.lean = False                                # after release(): nothing that only makes passes faster
+        self.on_release = lambda: None                   # a weakref.WeakMethod of the owner's: no cycle, whose end would be a matter of chance
         self._rope = K.RopeTables(cfg.head_dim, cfg.rope_theta, cfg.rope_scaling, cfg.max_seq)
         # weights to pull from their owner during the NEXT forward pass (name -> the owner's copy, a peer-mapped
         # tensor): the consuming GEMM copies the matrix into this rank's replica band by band while it multiplies
@@ -110,7 +112,7 @@ class DecoderRuntime:
         """Whether several sequences can go through the model in one pass: experts of its own, native attention, slots in one
         buffer."""
         impl = A.resolve_impl(self.cfg.head_dim) if self.attn_impl == "auto" else self.attn_impl
-        return self.G_all is not None and self.ep is None and impl == "flash" and self.device.type == "cuda"
+        return not self.lean and self.G_all is not None and self.ep is None and impl == "flash" and self.device.type == "cuda"
 
     @property
     def sumsq(self):
@@ -132,13 +134,53 @@ class DecoderRuntime:
     # ------------------------------------------------------------------ workspaces
     def workspace(self, T: int, n: int = 1) -> dict:
         """Buffers for sequences of ``T`` tokens, ``n`` of them going through the model together: one set of ``n * T`` rows
-        per length. A smaller ``n`` gets views of a larger set."""
+        per length. A smaller ``n`` gets views of a larger set. Sets for several sequences raise ``OutOfMemoryError`` where they do not
+        leave as much memory as they take; one for a single sequence that finds no more than that makes the others give way."""
         ws = self._ws.get((T, n))
         if ws is not None:
             return ws
         wider = [m for t, m in self._ws if t == T and m > n]
         if wider:
             return self.part(self._ws[(T, max(wider))], n)
+        optional = n > 1 or self._has_optional()
+        watch = optional and self.device.type == "cuda" and not torch.cuda.is_current_stream_capturing()
+        before = _lib.free_bytes(self.device) if watch else 0
+        try:
+            ws = self._new_workspace(T, n)
+        except torch.cuda.OutOfMemoryError:
+            if n > 1 or not watch:
+                raise
+            ws = None
+        # a pass allocates as well (scratch of the attention kernels, graph pools): as much again has to be left
+        if watch and (ws is None or 2 * _lib.free_bytes(self.device) < before):
+            if n > 1:
+                raise torch.cuda.OutOfMemoryError(f"buffers for {n} sequences of {T} tokens leave too little memory for a pass")
+            self.release()
+            if ws is None:
+                ws = self._new_workspace(T, n)
+        self._ws[(T, n)] = ws
+        return ws
+
+    def _has_optional(self) -> bool:
+        return bool(self._logits) or any(n > 1 for _, n in self._ws)
+
+    def release(self) -> None:
+        """Gives back what only makes passes faster, for good: the sets for several sequences and the stored logits. ``on_release`` (the owner
+        of graphs that read them) is called first."""
+        torch.cuda.synchronize(self.device)
+        self.lean = True
+        drop = self.on_release()
+        if drop is not None:
+            drop()
+        self._ws = {key: ws for key, ws in self._ws.items() if key[1] == 1}
+        self._parts.clear()
+        self._logits.clear()
+        self._norm_scratch = {n: t for n, t in self._norm_scratch.items() if n == 1}
+        for ws in self._ws.values():
+            ws["z"] = None
+        torch.cuda.empty_cache()
+
+    def _new_workspace(self, T: int, n: int) -> dict:
         cfg, dev = self.cfg, self.device
         d, F, L = cfg.d_model, cfg.ffn, cfg.n_layers
         seq, T = T, n * T
@@ -197,7 +239,6 @@ class DecoderRuntime:
             R, I = layers[0]["plan"].R, cfg.expert_ffn
             ws.update(dye=e(R, d), dgu=e(R, 2 * I).zero_(), dxs=e(R, d).zero_(),
                       dwts=e(T, cfg.top_k, dtype=torch.float32), drl=e(T, cfg.n_experts))
-        self._ws[(seq, n)] = ws
         return ws
 
     def part(self, ws: dict, n: int) -> dict:
@@ -207,7 +248,7 @@ class DecoderRuntime:
         out = self._parts.get((ws["key"], n))
         if out is not None:
             return out
-        out = self._parts[(ws["key"], n)] = dict(ws, n=n)
+        out = self._parts[(ws["key"], n)] = dict(ws, n=n, whole=ws)
         rows = n * ws["key"][0]
         layers, plans = [], [a["plan"].part(n) for a in ws["layers"] if "plan" in a]
         for li, a in enumerate(ws["layers"]):
@@ -228,7 +269,7 @@ class DecoderRuntime:
     def _logits_buffer(self, ws: dict) -> torch.Tensor | None:
         """fp32 logits that the loss leaves for its backward pass, which then needs no second product with the head. ``None``,
         for good, where the product is the cheaper one or the memory for them is not there (see :meth:`_shared_logits`)."""
-        ws = self._ws[ws["key"]]          # the whole set, T its rows
+        ws = ws.get("whole", ws)          # T its rows
         T = ws["labels"].numel()
         if "z" in ws or self.device.type != "cuda":
             return ws.get("z")
@@ -242,6 +283,8 @@ class DecoderRuntime:
         """At least ``n`` floats, the same for all lengths: they are live between the loss of a pass and its gradient only. A buffer that has
         become too short stays, because graphs may read it; the next one is twice as long where it may be. All of them together
         take at most a quarter of the memory that was free when the first was asked for, and each a quarter of what is free."""
+        if self.lean:
+            return None
         exact = self.canaries is not None                # guard bands have to begin behind the last logit
         for z in self._logits:
             if z.numel() == n if exact else z.numel() >= n:

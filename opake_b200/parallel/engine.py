@@ -19,6 +19,7 @@ gradients.py:150-200) with CPU-generated noise (packages/opake-dpsgd/src/opake/a
 from __future__ import annotations
 
 import math
+import weakref
 from dataclasses import dataclass, field
 
 import torch
@@ -168,6 +169,7 @@ class ShardedDPEngine:
             self.canaries = CanaryPool(device)
         self.runtime = DecoderRuntime(model_cfg, self.params, layout=self.layout, attn_impl=cfg.attn_impl, n_slots=self.group,
                                       ep=self.ep, canaries=self.canaries)
+        self.runtime.on_release = weakref.WeakMethod(self._drop_graphs)
         self._side = torch.cuda.Stream(device=device)
         self._warm: dict[tuple, bool] = {}
         self._join_limit: dict[int, int] = {}
@@ -342,6 +344,10 @@ class ShardedDPEngine:
         torch.cuda.empty_cache()
         return 1, self.runtime.workspace(T)
 
+    def _drop_graphs(self) -> None:
+        self._graphs.clear()
+        self._warm.clear()
+
     def _joined_body(self, ws, n: int, slot: int, drain_prev: bool, first: bool) -> None:
         """``_example_body`` for the ``n`` examples in slots ``slot ..``: one pass through the model."""
         rt, cfg = self.runtime, self.cfg
@@ -384,7 +390,7 @@ class ShardedDPEngine:
 
             if warm_key is not None and not self._warm.get(warm_key):
                 # eager warm-up (lazy workspaces, library autotuning) on a side stream, state restored afterwards
-                saved = ws["loss_sum"].clone()
+                saved, clipped = ws["loss_sum"].clone(), self.runtime.clip_count.clone()
                 s = torch.cuda.Stream(device=self.device)
                 s.wait_stream(torch.cuda.current_stream(self.device))
                 with torch.cuda.stream(s):
@@ -392,7 +398,7 @@ class ShardedDPEngine:
                 torch.cuda.current_stream(self.device).wait_stream(s)
                 torch.cuda.synchronize(self.device)
                 ws["loss_sum"].copy_(saved)
-                self.runtime.clip_count.zero_()
+                self.runtime.clip_count.copy_(clipped)
                 if self.ep is not None:
                     # warm-ups only ever happen on the first example of a step, where the expert sums are still zero
                     self.ep.acc.zero_()

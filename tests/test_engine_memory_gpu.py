@@ -1,4 +1,6 @@
 """Buffers of the one-rank engine over steps of different lengths: what graphs read stays, what is optional gives way."""
+import gc
+
 import pytest
 import torch
 
@@ -71,3 +73,82 @@ def test_stored_logits_of_all_lengths_share_their_memory(cuda, lengths, monkeypa
         c.step(*batch)
     _same(a, c)
     _same(b, c)
+
+
+@pytest.fixture(autouse=True)
+def _no_garbage():
+    """A patched method makes a cycle of its engine, whose graphs must not go while another test captures."""
+    yield
+    gc.collect()
+
+
+def _scarce(monkeypatch, eng, room):
+    """``room`` bytes more for this engine's runtime than torch has handed out now: what the device says and what allocations do."""
+    from opake_b200.ops import _lib
+
+    cap, inner = torch.cuda.memory_allocated() + room, eng.runtime._alloc
+
+    def alloc(*shape, dtype, name):
+        t = inner(*shape, dtype=dtype, name=name)
+        if torch.cuda.memory_allocated() > cap:
+            raise torch.cuda.OutOfMemoryError("the test's limit")
+        return t
+
+    monkeypatch.setattr(eng.runtime, "_alloc", alloc)
+    monkeypatch.setattr(_lib, "free_bytes", lambda device, plenty=None: max(0, cap - torch.cuda.memory_allocated()))
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_examples_go_one_by_one_where_several_do_not_fit(cuda, graph, monkeypatch):
+    """Whole and partial groups, a step of one example first; the bits of an engine that never takes several."""
+    from opake_b200.parallel import engine as E
+
+    a, b = _engine(cuda, use_cuda_graph=graph), _engine(cuda, use_cuda_graph=graph)
+    inner = a.runtime._alloc
+
+    def alloc(*shape, dtype, name):
+        if name.startswith("workspace[T=144]"):          # three examples of 48 tokens
+            raise torch.cuda.OutOfMemoryError("the test's limit")
+        return inner(*shape, dtype=dtype, name=name)
+
+    monkeypatch.setattr(a.runtime, "_alloc", alloc)
+    steps = [_batch(a.model_cfg, B, 48, B) for B in (1, 7, 4, 2)]
+    for batch in steps:
+        a.step(*batch)
+    monkeypatch.setattr(E, "_JOIN_VALUES", 0)
+    for batch in steps:
+        b.step(*batch)
+    assert a._join_limit == {48: 1} and set(a.runtime._ws) == {(48, 1)}
+    _same(a, b)
+
+
+@pytest.mark.parametrize("experts", [False, True])
+def test_what_is_optional_gives_way_to_more_lengths(cuda, experts, monkeypatch):
+    """Every length fits one by one; with the sets and logits of the earlier ones it does not. Captured steps, a sequence that is only
+    evaluated among them, then the earlier lengths again."""
+    from opake_b200.models.config import tiny_llama
+
+    cfg = tiny_llama(n_experts=8, top_k=2, expert_ffn=64) if experts else tiny_llama()
+    lengths = (64, 60, 56, 52, 48, 44)
+    plain, empty = _engine(cuda, cfg), torch.cuda.memory_allocated()
+    probe = _engine(cuda, cfg)
+    before = torch.cuda.memory_allocated()
+    for T in (*lengths, 70):
+        probe.runtime.workspace(T)
+    room = torch.cuda.memory_allocated() - before + (1 << 20)         # the scratch of a pass is not in it
+    del probe
+    assert torch.cuda.memory_allocated() <= empty                     # nothing waits for a garbage collection
+    steps = [_batch(cfg, B, T, T + B) for B in (4, 7) for T in lengths]
+    tok = _batch(cfg, 1, 70, 0)[0][0].to(cuda)
+    for batch in steps:
+        plain.step(*batch)
+    want = plain.runtime.logits(tok)
+    eng = _engine(cuda, cfg)
+    with monkeypatch.context() as m:
+        _scarce(m, eng, room)
+        for batch in steps:
+            eng.step(*batch)
+        got = eng.runtime.logits(tok)
+    assert eng.runtime.lean and all(n == 1 for _, n in eng.runtime._ws) and not eng.runtime._logits
+    assert torch.equal(got, want)
+    _same(eng, plain)
