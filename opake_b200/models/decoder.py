@@ -57,13 +57,12 @@ class DecoderRuntime:
         # With two slots the clipped accumulation of example i can run on a side stream while example i+1 is
         # being computed into the other slot.
         self.n_slots = n_slots
-        # The slots are one buffer, so that one launch can write the gradients of several (guard bands need them apart).
+        # The slots are rows of one buffer, so that one launch can write the gradients of several.
         if canaries is None:
             self.G_all = torch.empty(n_slots, self.layout.dense_total, dtype=_bf16, device=self.device)
-            self.Gs = list(self.G_all.unbind(0))
         else:
-            self.G_all = None
-            self.Gs = [self._alloc(self.layout.dense_total, dtype=_bf16, name=f"grad_slot{i}") for i in range(n_slots)]
+            self.G_all = canaries.rows(n_slots, self.layout.dense_total, dtype=_bf16, name="grad_slot")
+        self.Gs = list(self.G_all.unbind(0))
         self.gs = [self.layout.views(G_, dense_only=True) for G_ in self.Gs]
         self._g_stacks: dict[tuple[int, int], dict] = {}
         self.attn_impl = attn_impl
@@ -109,10 +108,9 @@ class DecoderRuntime:
         return self.gs[0]
 
     def can_join(self) -> bool:
-        """Whether several sequences can go through the model in one pass: experts of its own, native attention, slots in one
-        buffer."""
+        """Whether several sequences can go through the model in one pass: experts of its own, native attention."""
         impl = A.resolve_impl(self.cfg.head_dim) if self.attn_impl == "auto" else self.attn_impl
-        return not self.lean and self.G_all is not None and self.ep is None and impl == "flash" and self.device.type == "cuda"
+        return not self.lean and self.ep is None and impl == "flash" and self.device.type == "cuda"
 
     @property
     def sumsq(self):

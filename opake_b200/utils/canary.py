@@ -56,6 +56,17 @@ class CanaryPool:
         self._meta.append((name or f"buffer{len(self._raw) - 1}", nbytes))
         return raw[GUARD_BYTES : GUARD_BYTES + nbytes].view(dtype).view(*shape)
 
+    def rows(self, n: int, width: int, *, dtype: torch.dtype = torch.bfloat16, name: str = "row") -> torch.Tensor:
+        """``[n, width]`` for kernels that write several rows in one launch: each row between bands of its own, buffer ``name + index``."""
+        itemsize = torch.empty((), dtype=dtype).element_size()
+        nbytes = width * itemsize
+        pitch = (nbytes + GUARD_BYTES - 1) // GUARD_BYTES * GUARD_BYTES + GUARD_BYTES
+        raw = torch.full((GUARD_BYTES + n * pitch,), PATTERN, dtype=torch.uint8, device=self.device)
+        for j in range(n):
+            self._raw.append(raw[j * pitch : (j + 1) * pitch + GUARD_BYTES])       # neighbours share the band between them
+            self._meta.append((f"{name}{j}", nbytes))
+        return raw[GUARD_BYTES:].view(dtype).view(n, pitch // itemsize)[:, :width]
+
     def zeros(self, *shape: int, dtype: torch.dtype = torch.bfloat16, name: str | None = None) -> torch.Tensor:
         return self.empty(*shape, dtype=dtype, name=name).zero_()
 

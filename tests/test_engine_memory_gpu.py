@@ -152,3 +152,26 @@ def test_what_is_optional_gives_way_to_more_lengths(cuda, experts, monkeypatch):
     assert eng.runtime.lean and all(n == 1 for _, n in eng.runtime._ws) and not eng.runtime._logits
     assert torch.equal(got, want)
     _same(eng, plain)
+
+
+@pytest.mark.parametrize("name", ["llama", "tied", "experts", "biases"])
+def test_guard_bands_watch_the_passes_that_steps_take(cuda, name):
+    """With guard bands, examples go through the model together as they do without: the same bits, every band intact, and a write behind
+    a gradient slot is reported."""
+    from opake_b200.models.config import tiny_llama
+    from opake_b200.utils import DeviceIntegrityError
+
+    cfg = {"llama": tiny_llama(), "tied": tiny_llama(tie_embeddings=True), "biases": tiny_llama(qkv_bias=True),
+           "experts": tiny_llama(n_experts=8, top_k=2, expert_ffn=64)}[name]
+    for graph in (False, True):
+        a, b = _engine(cuda, cfg, use_cuda_graph=graph, debug_canaries=True), _engine(cuda, cfg, use_cuda_graph=graph)
+        for B, T in ((7, 45), (4, 45), (1, 33)):
+            batch = _batch(cfg, B, T, B)
+            a.step(*batch), b.step(*batch)
+        assert a._joined(45) == b._joined(45) == 3 and (45, 3) in a.runtime._ws
+        if name != "biases":                                   # whose gradients are added by fp32 atomics
+            _same(a, b)
+        slot = a.runtime.Gs[1]
+        slot.as_strided((1,), (1,), slot.storage_offset() + slot.numel()).zero_()
+        with pytest.raises(DeviceIntegrityError, match="grad_slot1: after the buffer"):
+            a.step(*batch)

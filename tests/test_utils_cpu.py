@@ -28,3 +28,16 @@ def test_canary_pool_detects_writes_on_both_sides_and_repairs():
     pool.repair()
     assert pool.check() == []
     assert float(b.sum()) == 6.0 and float(c.sum()) == 12.0           # payloads untouched by the repair
+
+
+def test_rows_of_one_buffer_have_guard_bands_of_their_own():
+    pool = CanaryPool("cpu")
+    x = pool.rows(3, 130, dtype=torch.bfloat16, name="slot")
+    assert x.shape == (3, 130) and x.stride(1) == 1 and all(r.data_ptr() % 16 == 0 for r in x)
+    x.copy_(torch.arange(390).view(3, 130))
+    assert pool.check() == [] and float(x.float().sum()) == float(torch.arange(390).to(torch.bfloat16).float().sum())
+    x.as_strided((131,), (1,))[130] = 1.0                      # one element behind the first row: the band between the first two
+    assert {(v.name, v.side) for v in pool.check()} == {("slot0", "after")}
+    pool.repair()
+    x.as_strided((1,), (1,), x[2].storage_offset() - 1).fill_(1.0)
+    assert {(v.name, v.side) for v in pool.check()} == {("slot1", "after"), ("slot2", "before")}
