@@ -259,7 +259,7 @@ __device__ __forceinline__ void ld_stream(const __nv_bfloat16* p, uint32_t (&o)[
 __device__ __forceinline__ float2 unpack2(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
 
 // The rows of correlation state that a vector needs first are loaded with everything else (four rows: BLT with up to four buffers
-// needs no other access before its stores; two next to eight gradient buffers, which leave no registers for more).
+// needs no other access before its stores; two in vectors of eight next to eight gradient buffers, which leave no registers for more).
 template <int CORR, int VEC, int ROWS>
 struct CorrIn {
   float row[ROWS][VEC];
@@ -351,7 +351,7 @@ template <int NG, int CORR, int VEC>
 struct VecIn {
   float g[VEC], m[VEC], v[VEC], mw[VEC];
   uint32_t pw[VEC / 2], gr[NG > 0 ? NG : 1][VEC / 2];
-  CorrIn<CORR, VEC, (NG > 2 && CORR == CORR_BLT ? 2 : 4)> corr;
+  CorrIn<CORR, VEC, (NG > 2 && CORR == CORR_BLT && VEC == 8 ? 2 : 4)> corr;
 };
 // NG > 0 (the most buffers the variant takes: 2, or all 8): the last group of per-example gradients is clipped and added here
 // instead of in a pass of its own. A separate pass reads and writes the fp32 sums once more and the step reads them again: 12 bytes
@@ -477,15 +477,25 @@ __device__ __forceinline__ void finish_vec(const OpkDpStepArgs& a, const opk::Ph
   }
 }
 
-// CTAs per SM that the registers must allow: what the variant fits without spilling.
+// Whether a thread holds two vectors of four at a time. With a group to add and much state next to it there are no registers for two,
+// and four rows of BLT state take those of the second; the loads of more CTAs are in flight instead. (us at 2^26 elements off a 32-byte
+// boundary: quads of the kernel before -> two vectors -> one: SGD with five buffers 290 -> 320 -> 260; AdamW with master weights and two
+// 364 -> 382 -> 352; four BLT rows, AdamW with five 809 -> 979 -> 732, SGD with eight 713 -> 853 -> 628, AdamW alone 692 -> 668 -> 644.
+// Two is the better one for SGD alone, 146 -> 121 -> 130 to 194, and for AdamW with eight and Toeplitz rows, 891 -> 613 -> 624 to 673.)
+__host__ __device__ constexpr bool step_two(bool adam, bool master, int corr, int ng) {
+  return corr == CORR_TOEPLITZ || (corr == CORR_NONE && ng <= 2 && !(adam && master && ng > 0));
+}
+// CTAs per SM that the registers must allow: what the variant fits with a few bytes of spills at most.
 constexpr int step_min_ctas(bool adam, bool master, int corr, int ng, int vec) {
-  return vec == 8 || ng > 2 || corr != CORR_NONE || (adam && master && ng > 0) ? 2 : adam ? 3 : 4;
+  if (vec == 8 || corr == CORR_TOEPLITZ) return 2;
+  if (corr == CORR_BLT) return 3;
+  return adam && (step_two(adam, master, corr, ng) || (master && ng > 2)) ? 3 : 4;
 }
 template <bool ADAM, bool MASTER, int CORR, int NG, int VEC>
 __global__ void __launch_bounds__(256, step_min_ctas(ADAM, MASTER, CORR, NG, VEC))
 dp_step_kernel(const OpkDpStepArgs a, const opk::PhiloxKeys key, const PeerTable pt, const StepGroup grp) {
-  // Each thread owns aligned vectors of the shard: eight elements an iteration, or two times four; a ragged end takes the scalar
-  // path.
+  // Each thread owns aligned vectors of the shard: eight elements an iteration, or four, or two times four (step_two); a ragged end
+  // takes the scalar path.
   //
   // What bounds it: memory, 28 bytes per parameter with two gradient buffers, and next to it the issue slots: 118 instructions per
   // parameter kept 72 % of them busy at full clock, and a step under the power cap runs at two thirds of that. Eight elements per
@@ -501,7 +511,7 @@ dp_step_kernel(const OpkDpStepArgs a, const opk::PhiloxKeys key, const PeerTable
   for (int j = 0; j < NG; ++j) gs[j] = j < grp.n ? *grp.scale[j] : 0.f;
   const long long stride = (long long)gridDim.x * 256;
   long long q = blockIdx.x * 256ll + threadIdx.x;
-  if constexpr (VEC == 4) {
+  if constexpr (VEC == 4 && step_two(ADAM, MASTER, CORR, NG)) {
 #pragma unroll 1
     for (; q + stride < nfull; q += 2 * stride) {
       const long long q2 = q + stride;

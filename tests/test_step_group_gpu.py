@@ -194,3 +194,9 @@ def test_vectors_of_eight_and_of_four_give_the_same_bits(cuda, n_group, group_le
         out.append((p, *full.values()))
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n_group,group_len", [(0, 0), (2, 4096), (3, 7000)])
+@pytest.mark.parametrize("noise", ["independent", "blt 4", "toeplitz 3"])
+def test_vectors_of_eight_and_of_four_with_master_weights_under_sgd(cuda, n_group, group_len, noise):
+    test_vectors_of_eight_and_of_four_give_the_same_bits(cuda, n_group, group_len, noise, True, True)
