@@ -345,8 +345,8 @@ class ShardedDPEngine:
         return 1, self.runtime.workspace(T)
 
     def _drop_graphs(self) -> None:
+        # What has been warmed up stays so: with experts on several ranks a warm-up exchanges rows with the others, who may not make one.
         self._graphs.clear()
-        self._warm.clear()
 
     def _joined_body(self, ws, n: int, slot: int, drain_prev: bool, first: bool) -> None:
         """``_example_body`` for the ``n`` examples in slots ``slot ..``: one pass through the model."""

@@ -150,7 +150,7 @@ def test_what_is_optional_gives_way_to_more_lengths(cuda, experts, monkeypatch):
             eng.step(*batch)
         got = eng.runtime.logits(tok)
     assert eng.runtime.lean and all(n == 1 for _, n in eng.runtime._ws) and not eng.runtime._logits
-    assert torch.equal(got, want)
+    assert torch.equal(got, want) and ("joined", 64) in eng._warm          # a rank must not warm up again by itself
     _same(eng, plain)
 
 
