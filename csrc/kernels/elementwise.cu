@@ -59,7 +59,8 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
 constexpr int NT = 256;
 
 // ------------------------------------------------------------------------------------------- RMSNorm
-template <bool ADD>
+// COPY: sum_out receives x.
+template <bool ADD, bool COPY>
 __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
                                                          const __nv_bfloat16* __restrict__ r,
                                                          const __nv_bfloat16* __restrict__ w,
@@ -72,14 +73,14 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __
   const long long row = blockIdx.x;
   const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * ldx);
   const bf16x8* rr = ADD ? reinterpret_cast<const bf16x8*>(r + row * D) : nullptr;
-  bf16x8* sr = sum_out ? reinterpret_cast<bf16x8*>(sum_out + row * ld_sum) : nullptr;     // without ADD: a copy of x
+  bf16x8* sr = ADD || COPY ? reinterpret_cast<bf16x8*>(sum_out + row * (COPY ? ld_sum : D)) : nullptr;
   const int nv = D >> 3;
   float ss = 0.f;
   for (int i = threadIdx.x; i < nv; i += NT) {
     float f[8];
     const bf16x8 in = xr[i];
     unpack8(in, f);
-    if (!ADD && sr) sr[i] = in;
+    if (COPY) sr[i] = in;
     if (ADD) {
       float g[8];
       unpack8(rr[i], g);
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(NT) rmsnorm_fwd_kernel(const __nv_bfloat16* __
 //
 // `copy` (optional) receives the row as it was read, for a norm in place whose input the backward pass needs (query and key columns
 // of a fused projection: 4096 x 4096 values took 107 us in a strided copy of their own, 428 us of a 22.6 ms OLMoE step).
-template <int VPL>
+template <int VPL, bool COPY>
 __global__ void __launch_bounds__(256, VPL >= 16 ? 2 : 4) rmsnorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x,
                                                                const __nv_bfloat16* __restrict__ w,
                                                                __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int T,
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(256, VPL >= 16 ? 2 : 4) rmsnorm_fwd_warp_kerne
   bf16x8 v[VPL];
 #pragma unroll
   for (int i = 0; i < VPL; ++i) v[i] = xr[lane + 32 * i];
-  if (copy) {
+  if constexpr (COPY) {
     bf16x8* cr = reinterpret_cast<bf16x8*>(copy + row * ld_copy);
 #pragma unroll
     for (int i = 0; i < VPL; ++i) cr[lane + 32 * i] = v[i];
@@ -226,7 +227,8 @@ __global__ void __launch_bounds__(NT) add_rmsnorm_fwd_kernel(const __nv_bfloat16
 // an example's rows meet the same CTAs in the same order as in a launch of its own, so its weight gradient has the same bits.
 constexpr int MAX_COL_ITERS = 8;  // layernorm backward: D <= 8 * 2048
 constexpr int RMS_BWD_NT = 512;
-template <int ITERS>
+// (MANY: more than one; a single example keeps the shorter addresses.)
+template <int ITERS, bool MANY>
 __global__ void __launch_bounds__(RMS_BWD_NT) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                                  const __nv_bfloat16* __restrict__ x,
                                                                  const __nv_bfloat16* __restrict__ w,
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(RMS_BWD_NT) rmsnorm_bwd_kernel(const __nv_bflo
                                                                  long long ld_dx) {
   __shared__ float sh[32];
   const int nv = D >> 3;
-  const long long first = (long long)blockIdx.y * T;
+  const long long first = MANY ? (long long)blockIdx.y * T : 0;
   float wv[ITERS][8], acc[ITERS][8];
 #pragma unroll
   for (int it = 0; it < ITERS; ++it) {
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(RMS_BWD_NT) rmsnorm_bwd_kernel(const __nv_bflo
     for (int it = 0; it < ITERS; ++it) {
       const int v = threadIdx.x + it * RMS_BWD_NT;
       if (v < nv) {
-        float4* dst = reinterpret_cast<float4*>(partial + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * D + v * 8);
+        float4* dst = reinterpret_cast<float4*>(partial + ((MANY ? (long long)blockIdx.y * gridDim.x : 0ll) + blockIdx.x) * D + v * 8);
         dst[0] = make_float4(acc[it][0], acc[it][1], acc[it][2], acc[it][3]);
         dst[1] = make_float4(acc[it][4], acc[it][5], acc[it][6], acc[it][7]);
       }
@@ -313,23 +315,37 @@ __global__ void __launch_bounds__(RMS_BWD_NT) rmsnorm_bwd_kernel(const __nv_bflo
 }
 
 // dst[b][c] += sum_r partial[b][r][c] (b = blockIdx.y); CTA = 32 columns x 8 row groups.
+template <bool MANY>
 __global__ void __launch_bounds__(256) colsum_add_kernel(const float* __restrict__ partial, float* __restrict__ dst,
                                                          int rows, int D, long long dst_stride) {
   opk::pdl_trigger();
-  partial += (long long)blockIdx.y * rows * D;
-  dst += blockIdx.y * dst_stride;
   __shared__ float sh[8][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
   float s = 0.f;
-  if (c < D)
-    for (int r = ry; r < rows; r += 8) s += partial[(long long)r * D + c];
+  if (c < D) {
+    if constexpr (!MANY) {
+      for (int r = ry; r < rows; r += 8) s += partial[(long long)r * D + c];
+    } else {
+      // with one more term in the address the compiler has fewer loads in flight: eight are asked for ahead (1.0 us less for 296 rows)
+      const float* src = partial + ((long long)blockIdx.y * rows + ry) * D + c;
+      int r = ry;
+      for (; r + 56 < rows; r += 64, src += 64ll * D) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v[u]) : "l"(src + 8ll * u * D));
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += v[u];
+      }
+      for (; r < rows; r += 8, src += 8ll * D) s += *src;
+    }
+  }
   sh[ry][cx] = s;
   __syncthreads();
   if (ry == 0 && c < D) {
 #pragma unroll
     for (int k = 1; k < 8; ++k) s += sh[k][cx];
-    dst[c] += s;
+    dst[(MANY ? blockIdx.y * dst_stride : 0) + c] += s;
   }
 }
 
@@ -378,6 +394,7 @@ __global__ void __launch_bounds__(NT) layernorm_fwd_kernel(const __nv_bfloat16* 
   }
 }
 
+template <bool MANY>
 __global__ void __launch_bounds__(NT) layernorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
                                                            const __nv_bfloat16* __restrict__ x,
                                                            const __nv_bfloat16* __restrict__ w,
@@ -388,7 +405,7 @@ __global__ void __launch_bounds__(NT) layernorm_bwd_kernel(const __nv_bfloat16* 
                                                            float* __restrict__ db, int T, int D, long long stride) {
   __shared__ float sh[32];
   const int nv = D >> 3;
-  const long long first = (long long)blockIdx.y * T;       // gridDim.y examples of T rows, gradients `stride` floats apart
+  const long long first = MANY ? (long long)blockIdx.y * T : 0;       // gridDim.y examples of T rows, gradients `stride` floats apart
   float dwp[MAX_COL_ITERS][8], dbp[MAX_COL_ITERS][8];
 #pragma unroll
   for (int c = 0; c < MAX_COL_ITERS; ++c)
@@ -448,8 +465,8 @@ __global__ void __launch_bounds__(NT) layernorm_bwd_kernel(const __nv_bfloat16* 
     if (i < nv) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        if (dw) atomicAdd(&dw[blockIdx.y * stride + i * 8 + j], dwp[c][j]);
-        if (db) atomicAdd(&db[blockIdx.y * stride + i * 8 + j], dbp[c][j]);
+        if (dw) atomicAdd(&dw[(MANY ? blockIdx.y * stride : 0) + i * 8 + j], dwp[c][j]);
+        if (db) atomicAdd(&db[(MANY ? blockIdx.y * stride : 0) + i * 8 + j], dbp[c][j]);
       }
     }
   }
@@ -463,14 +480,14 @@ __global__ void __launch_bounds__(NT) layernorm_bwd_kernel(const __nv_bfloat16* 
 __device__ __forceinline__ void red_add_v4(float* dst, const float* v) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
 }
-template <int VPL>
+template <int VPL, bool MANY>
 __global__ void __launch_bounds__(256) layernorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                                  const __nv_bfloat16* __restrict__ w, const float* __restrict__ mean,
                                                                  const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dres,
                                                                  __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
                                                                  float* __restrict__ db, int T, int D, long long stride) {
   opk::pdl_trigger();
-  const long long first = (long long)blockIdx.y * T;       // gridDim.y examples of T rows, gradients `stride` floats apart
+  const long long first = MANY ? (long long)blockIdx.y * T : 0;       // gridDim.y examples of T rows, gradients `stride` floats apart
   constexpr int W = VPL * 256;
   __shared__ float sh[8 * W];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nv = D >> 3;
@@ -552,7 +569,7 @@ __global__ void __launch_bounds__(256) layernorm_bwd_warp_kernel(const __nv_bflo
       for (int k = 0; k < 8; ++k)
 #pragma unroll
         for (int j = 0; j < 4; ++j) a[j] += sh[k * W + c + j];
-      red_add_v4(out + blockIdx.y * stride + c, a);
+      red_add_v4(out + (MANY ? blockIdx.y * stride : 0) + c, a);
     }
   }
 }
@@ -780,6 +797,7 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const __nv_bfloat16* __re
 }
 
 // ------------------------------------------------------------------------------------------- embedding
+template <bool PERIODIC>
 __global__ void embedding_fwd_kernel(const int* __restrict__ tok, const __nv_bfloat16* __restrict__ table,
                                      const __nv_bfloat16* __restrict__ pos_table, __nv_bfloat16* __restrict__ out,
                                      int D, int vocab, int period) {
@@ -788,7 +806,7 @@ __global__ void embedding_fwd_kernel(const int* __restrict__ tok, const __nv_bfl
   const bool in_table = tok[t] >= 0 && tok[t] < vocab;
   (void)OPK_IDX_OK(tok[t], vocab);
   const bf16x8* src = reinterpret_cast<const bf16x8*>(table + (long long)(in_table ? tok[t] : 0) * D);
-  const bf16x8* ps = pos_table ? reinterpret_cast<const bf16x8*>(pos_table + (t % period) * D) : nullptr;
+  const bf16x8* ps = pos_table ? reinterpret_cast<const bf16x8*>(pos_table + (PERIODIC ? t % period : t) * D) : nullptr;
   bf16x8* dst = reinterpret_cast<bf16x8*>(out + t * D);
   for (int i = threadIdx.x; i < (D >> 3); i += blockDim.x) {
     if (ps || !in_table) {
@@ -873,11 +891,12 @@ __device__ __forceinline__ void load_vec16(const void* p, long long i, float (&f
     unpack8(*reinterpret_cast<const bf16x8*>(&raw), f);
   }
 }
-template <bool FP32, bool ROUND>
+// MANY: gridDim.y buffers with one sum each, on one 16-byte boundary. One buffer has no offset in its addresses: with it 8192 x 8192
+// values take 23 us instead of 21.
+template <bool FP32, bool ROUND, bool MANY>
 __global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, long long n, double* out, long long stride) {
   double acc = 0.0;
-  x = reinterpret_cast<const char*>(x) + blockIdx.y * stride * (FP32 ? 4 : 2);       // gridDim.y buffers, one sum each
-  out += blockIdx.y;
+  const long long first = MANY ? blockIdx.y * stride : 0;
   float part = 0.f;
   int cnt = 0;
   // 16-byte loads, four vectors in flight, when the base allows it; fp32 partials of at most 64 squares as below
@@ -886,7 +905,7 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, l
 #pragma unroll 4
   for (long long i = blockIdx.x * (long long)NT + threadIdx.x; i < nvec; i += (long long)gridDim.x * NT) {
     float f[8];
-    load_vec16<FP32>(x, i * VW, f);
+    load_vec16<FP32>(x, first + i * VW, f);
     float p8 = 0.f;
 #pragma unroll
     for (int j = 0; j < VW; ++j) {
@@ -896,7 +915,7 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, l
     acc += (double)p8;
   }
   for (long long i = nvec * VW + blockIdx.x * (long long)NT + threadIdx.x; i < n; i += (long long)gridDim.x * NT) {
-    float v = FP32 ? reinterpret_cast<const float*>(x)[i] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[i]);
+    float v = FP32 ? reinterpret_cast<const float*>(x)[first + i] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(x)[first + i]);
     if (ROUND) v = __bfloat162float(__float2bfloat16(v));
     part += v * v;
     if (++cnt == 64) { acc += (double)part; part = 0.f; cnt = 0; }
@@ -910,7 +929,7 @@ __global__ void __launch_bounds__(NT) sumsq_kernel(const void* __restrict__ x, l
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int w = 0; w < NT / 32; ++w) t += shd[w];
-    atomicAdd(out, t);
+    atomicAdd(MANY ? out + blockIdx.y : out, t);
   }
 }
 
@@ -1194,22 +1213,30 @@ __global__ void colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __res
                               long long out_stride) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= N) return;
-  dy += (long long)blockIdx.z * T * ld;        // gridDim.z examples of T rows
-  out += blockIdx.z * out_stride;
+  const long long first = (long long)blockIdx.z * T;        // gridDim.z examples of T rows
   float a = 0.f;
-  for (int t = blockIdx.y; t < T; t += gridDim.y) a += __bfloat162float(dy[(long long)t * ld + n]);
-  atomicAdd(&out[n], a);
+  for (int t = blockIdx.y; t < T; t += gridDim.y) a += __bfloat162float(dy[(first + t) * ld + n]);
+  atomicAdd(&out[blockIdx.z * out_stride + n], a);
 }
 
 // The same for a 16-byte aligned matrix whose width is a multiple of 8: a warp reads 256 columns of a row at a time, the
 // eight warps of a CTA take every eighth row of the CTA's row chunk and meet in shared memory, one vector reduction per
 // four columns and CTA. (2-byte loads and one atomic per column and row chunk measured 9.2 us on average over the
 // GPT-2-small bias gradients, 1024 x 768 .. 3072.)
-__global__ void __launch_bounds__(256) colsum_vec_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ out, int T, int N,
-                                                         long long ld, int rows_per_cta, long long out_stride) {
+//
+// What bounds it: the loads in flight of one CTA per SM. The compiler spread four unrolled loads over 32 registers, and fewer were in
+// flight as soon as the address had one more term; eight are asked for before the first is added (us, with one example: four unrolled
+// without that term -> with it -> eight ahead: 4007 x 6712 28.6 -> 37.3 -> 12.8, 2048 x 4096 9.7 -> 12.6 -> 5.8, 1024 x 3072 3.2 -> 3.5 -> 2.6,
+// 1024 x 768 2.2 each).
+__device__ __forceinline__ bf16x8 ld_vec(const bf16x8* p) {
+  uint4 q;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w) : "l"(p));
+  return *reinterpret_cast<const bf16x8*>(&q);
+}
+__global__ void __launch_bounds__(256, 4) colsum_vec_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ out, int T, int N,
+                                                            long long ld, int rows_per_cta, long long out_stride) {
   opk::pdl_trigger();
-  dy += (long long)blockIdx.z * T * ld;
-  out += blockIdx.z * out_stride;
+  const long long first = (long long)blockIdx.z * T;
   __shared__ float sh[8][256 + 4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = blockIdx.x * 256, c = c0 + lane * 8;
@@ -1218,10 +1245,23 @@ __global__ void __launch_bounds__(256) colsum_vec_kernel(const __nv_bfloat16* __
 #pragma unroll
   for (int j = 0; j < 8; ++j) a[j] = 0.f;
   if (c < N) {
-#pragma unroll 4
-    for (int t = t0 + warp; t < t1; t += 8) {
+    const bf16x8* src = reinterpret_cast<const bf16x8*>(dy + (first + t0 + warp) * ld + c);        // `ld` vectors are eight rows
+    int t = t0 + warp;
+    for (; t + 56 < t1; t += 64, src += 8 * ld) {
+      bf16x8 r[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) r[u] = ld_vec(src + u * ld);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        float f[8];
+        unpack8(r[u], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] += f[j];
+      }
+    }
+    for (; t < t1; t += 8, src += ld) {
       float f[8];
-      unpack8(*reinterpret_cast<const bf16x8*>(dy + (long long)t * ld + c), f);
+      unpack8(*src, f);
 #pragma unroll
       for (int j = 0; j < 8; ++j) a[j] += f[j];
     }
@@ -1235,7 +1275,7 @@ __global__ void __launch_bounds__(256) colsum_vec_kernel(const __nv_bfloat16* __
     for (int k = 0; k < 8; ++k)
 #pragma unroll
       for (int j = 0; j < 4; ++j) v[j] += sh[k][threadIdx.x * 4 + j];
-    red_add_v4(out + c0 + threadIdx.x * 4, v);
+    red_add_v4(out + blockIdx.z * out_stride + c0 + threadIdx.x * 4, v);
   }
 }
 
@@ -1263,20 +1303,28 @@ inline int grid_for(long long n, int block, int cap_blocks = 148 * 16) {
 #define BF(p) reinterpret_cast<const __nv_bfloat16*>(p)
 #define BFM(p) reinterpret_cast<__nv_bfloat16*>(p)
 
+template <bool FP32, bool ROUND>
+void launch_sumsq(int ctas, int batch, cudaStream_t st, const void* x, long long n, double* sums, long long stride) {
+  if (batch == 1) sumsq_kernel<FP32, ROUND, false><<<ctas, NT, 0, st>>>(x, n, sums, 0);
+  else sumsq_kernel<FP32, ROUND, true><<<dim3(ctas, batch), NT, 0, st>>>(x, n, sums, stride);
+}
+
+template <bool COPY>
+void launch_rmsnorm_fwd(cudaStream_t st, const __nv_bfloat16* x, const __nv_bfloat16* w, __nv_bfloat16* y, float* rstd, int T, int D, float eps,
+                        float w_offset, long long ldx, long long ldy, __nv_bfloat16* copy, long long ld_copy) {
+  const int warp_grid = (T + 7) / 8;
+  if (D == 4096) rmsnorm_fwd_warp_kernel<16, COPY><<<warp_grid, 256, 0, st>>>(x, w, y, rstd, T, eps, w_offset, ldx, ldy, copy, ld_copy);
+  else if (D == 2048) rmsnorm_fwd_warp_kernel<8, COPY><<<warp_grid, 256, 0, st>>>(x, w, y, rstd, T, eps, w_offset, ldx, ldy, copy, ld_copy);
+  else if (D == 1024) rmsnorm_fwd_warp_kernel<4, COPY><<<warp_grid, 256, 0, st>>>(x, w, y, rstd, T, eps, w_offset, ldx, ldy, copy, ld_copy);
+  else rmsnorm_fwd_kernel<false, COPY><<<T, NT, 0, st>>>(x, nullptr, w, copy, y, rstd, D, eps, w_offset, ldx, ldy, ld_copy);
+}
 extern "C" int opk_rmsnorm_fwd_ld(const void* x, int64_t ldx, const void* w, void* y, int64_t ldy, float* rstd, int T, int D,
                                   float eps, float w_offset, void* copy, int64_t ld_copy, void* stream) {
   if (T <= 0) return 0;
   if (D % 8 || ldx % 8 || ldy % 8 || ldx < D || ldy < D) return -1;
   if (copy && (ld_copy % 8 || ld_copy < D || (reinterpret_cast<uintptr_t>(copy) & 15))) return -1;
-  const int warp_grid = (T + 7) / 8;
-  if (D == 4096)
-    rmsnorm_fwd_warp_kernel<16><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy, BFM(copy), ld_copy);
-  else if (D == 2048)
-    rmsnorm_fwd_warp_kernel<8><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy, BFM(copy), ld_copy);
-  else if (D == 1024)
-    rmsnorm_fwd_warp_kernel<4><<<warp_grid, 256, 0, ST(stream)>>>(BF(x), BF(w), BFM(y), rstd, T, eps, w_offset, ldx, ldy, BFM(copy), ld_copy);
-  else
-    rmsnorm_fwd_kernel<false><<<T, NT, 0, ST(stream)>>>(BF(x), nullptr, BF(w), BFM(copy), BFM(y), rstd, D, eps, w_offset, ldx, ldy, ld_copy);
+  if (copy) launch_rmsnorm_fwd<true>(ST(stream), BF(x), BF(w), BFM(y), rstd, T, D, eps, w_offset, ldx, ldy, BFM(copy), ld_copy);
+  else launch_rmsnorm_fwd<false>(ST(stream), BF(x), BF(w), BFM(y), rstd, T, D, eps, w_offset, ldx, ldy, nullptr, 0);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1295,7 +1343,7 @@ extern "C" int opk_add_rmsnorm_fwd(const void* x, const void* r, const void* w, 
   else if (D <= 8192)
     add_rmsnorm_fwd_kernel<4><<<T, NT, 0, ST(stream)>>>(BF(x), BF(r), BF(w), BFM(sum_out), BFM(y), rstd, D, eps, w_offset);
   else
-    rmsnorm_fwd_kernel<true><<<T, NT, 0, ST(stream)>>>(BF(x), BF(r), BF(w), BFM(sum_out), BFM(y), rstd, D, eps, w_offset, D, D, D);
+    rmsnorm_fwd_kernel<true, false><<<T, NT, 0, ST(stream)>>>(BF(x), BF(r), BF(w), BFM(sum_out), BFM(y), rstd, D, eps, w_offset, D, D, D);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1312,15 +1360,26 @@ extern "C" int opk_rmsnorm_bwd_ld(const void* dy, int64_t ld_dy, const void* x, 
   const dim3 grid((unsigned)ctas, (unsigned)batch);
   float* part = dw ? workspace : nullptr;
   const int iters = (D / 8 + RMS_BWD_NT - 1) / RMS_BWD_NT;
+#define OPK_RMS_BWD(I)                                                                                                                 \
+  do {                                                                                                                                 \
+    if (batch == 1)                                                                                                                    \
+      rmsnorm_bwd_kernel<I, false><<<grid, RMS_BWD_NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), rstd, BF(dres), BFM(dx_out), part, T, D, \
+                                                                        w_offset, ld_dy, ldx, ld_dx);                                  \
+    else                                                                                                                               \
+      rmsnorm_bwd_kernel<I, true><<<grid, RMS_BWD_NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), rstd, BF(dres), BFM(dx_out), part, T, D,  \
+                                                                       w_offset, ld_dy, ldx, ld_dx);                                   \
+  } while (0)
   if (iters == 1)
-    rmsnorm_bwd_kernel<1><<<grid, RMS_BWD_NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), rstd, BF(dres), BFM(dx_out), part, T, D, w_offset, ld_dy, ldx, ld_dx);
+    OPK_RMS_BWD(1);
   else if (iters == 2)
-    rmsnorm_bwd_kernel<2><<<grid, RMS_BWD_NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), rstd, BF(dres), BFM(dx_out), part, T, D, w_offset, ld_dy, ldx, ld_dx);
+    OPK_RMS_BWD(2);
   else
-    rmsnorm_bwd_kernel<3><<<grid, RMS_BWD_NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), rstd, BF(dres), BFM(dx_out), part, T, D, w_offset, ld_dy, ldx, ld_dx);
+    OPK_RMS_BWD(3);
+#undef OPK_RMS_BWD
   OPK_LAUNCH_CHECK();
   if (dw) {
-    colsum_add_kernel<<<dim3((D + 31) / 32, batch), 256, 0, ST(stream)>>>(part, dw, ctas, D, dw_stride);
+    if (batch == 1) colsum_add_kernel<false><<<(D + 31) / 32, 256, 0, ST(stream)>>>(part, dw, ctas, D, 0);
+    else colsum_add_kernel<true><<<dim3((D + 31) / 32, batch), 256, 0, ST(stream)>>>(part, dw, ctas, D, dw_stride);
     OPK_LAUNCH_CHECK();
   }
   return 0;
@@ -1345,8 +1404,15 @@ extern "C" int opk_layernorm_bwd(const void* dy, const void* x, const void* w, c
   if (D % 8 || D > MAX_COL_ITERS * NT * 8 || batch > 65535) return -1;
   if (D <= 1024 && (batch == 1 || stride % 4 == 0) && (reinterpret_cast<uintptr_t>(dw) & 15) == 0 && (reinterpret_cast<uintptr_t>(db) & 15) == 0) {
     const int g = (T + 7) / 8 < 148 ? (T + 7) / 8 : 148;
-#define OPK_LN_BWD(V) \
-  layernorm_bwd_warp_kernel<V><<<dim3(g, batch), 256, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db, T, D, stride)
+#define OPK_LN_BWD(V)                                                                                                                  \
+  do {                                                                                                                                 \
+    if (batch == 1)                                                                                                                    \
+      layernorm_bwd_warp_kernel<V, false><<<g, 256, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db,  \
+                                                                     T, D, 0);                                                         \
+    else                                                                                                                               \
+      layernorm_bwd_warp_kernel<V, true><<<dim3(g, batch), 256, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres),           \
+                                                                                 BFM(dx_out), dw, db, T, D, stride);                   \
+  } while (0)
     if (D <= 256) OPK_LN_BWD(1);
     else if (D <= 512) OPK_LN_BWD(2);
     else if (D <= 768) OPK_LN_BWD(3);
@@ -1356,7 +1422,8 @@ extern "C" int opk_layernorm_bwd(const void* dy, const void* x, const void* w, c
     return 0;
   }
   const dim3 grid(T < 148 * 2 ? T : 148 * 2, batch);
-  layernorm_bwd_kernel<<<grid, NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db, T, D, stride);
+  if (batch == 1) layernorm_bwd_kernel<false><<<grid, NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db, T, D, 0);
+  else layernorm_bwd_kernel<true><<<grid, NT, 0, ST(stream)>>>(BF(dy), BF(x), BF(w), mean, rstd, BF(dres), BFM(dx_out), dw, db, T, D, stride);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1469,7 +1536,8 @@ extern "C" int opk_embedding_fwd(const int32_t* tok, const void* table, const vo
                                  int vocab, int period, void* stream) {
   if (T <= 0) return 0;
   if (D % 8 || vocab <= 0) return -1;
-  embedding_fwd_kernel<<<T, 128, 0, ST(stream)>>>(tok, BF(table), BF(pos_table), BFM(out), D, vocab, period > 0 ? period : T);
+  if (period > 0 && pos_table) embedding_fwd_kernel<true><<<T, 128, 0, ST(stream)>>>(tok, BF(table), BF(pos_table), BFM(out), D, vocab, period);
+  else embedding_fwd_kernel<false><<<T, 128, 0, ST(stream)>>>(tok, BF(table), BF(pos_table), BFM(out), D, vocab, 0);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1485,7 +1553,7 @@ extern "C" int opk_embedding_bwd_compact(const int32_t* tok, const void* dx, int
   emb_scatter_kernel<<<dim3(T, batch), 256, 0, st>>>(tok, BF(dx), first_pos, rep, gc, T, D, vocab);
   emb_reset_kernel<<<by_token, 256, 0, st>>>(tok, first_pos, T, vocab);
   const long long n = (long long)T * D;
-  if (sumsq) sumsq_kernel<true, true><<<dim3(grid_for(n, NT, 148 * 4), batch), NT, 0, st>>>(gc, n, sumsq, n);
+  if (sumsq) launch_sumsq<true, true>(grid_for(n, NT, 148 * 4), batch, st, gc, n, sumsq, n);
   OPK_LAUNCH_CHECK();
   return 0;
 }
@@ -1553,12 +1621,12 @@ extern "C" int opk_sumsq(const void* x, int is_fp32, int round_bf16, int64_t n, 
   if (n <= 0 || batch <= 0) return 0;
   // the 16-byte form is chosen by the base, so every buffer of a batch has to lie on the same boundary
   if (batch > 65535 || (batch > 1 && stride % 8)) return -1;
-  const dim3 g(grid_for(n, NT, 148 * 8), batch);
+  const int g = grid_for(n, NT, 148 * 8);
   if (is_fp32) {
-    if (round_bf16) sumsq_kernel<true, true><<<g, NT, 0, ST(stream)>>>(x, n, sumsq, stride);
-    else sumsq_kernel<true, false><<<g, NT, 0, ST(stream)>>>(x, n, sumsq, stride);
+    if (round_bf16) launch_sumsq<true, true>(g, batch, ST(stream), x, n, sumsq, stride);
+    else launch_sumsq<true, false>(g, batch, ST(stream), x, n, sumsq, stride);
   } else {
-    sumsq_kernel<false, false><<<g, NT, 0, ST(stream)>>>(x, n, sumsq, stride);
+    launch_sumsq<false, false>(g, batch, ST(stream), x, n, sumsq, stride);
   }
   OPK_LAUNCH_CHECK();
   return 0;
@@ -1643,7 +1711,7 @@ extern "C" int opk_embedding_bwd_compact_noalloc(const int32_t* tok, const void*
   emb_first_pos_kernel<<<(T + 255) / 256, 256, 0, st>>>(tok, first_pos, T, vocab);
   emb_scatter_kernel<<<T, 256, 0, st>>>(tok, BF(dx), first_pos, rep, gc, T, D, vocab);
   emb_reset_kernel<<<(T + 255) / 256, 256, 0, st>>>(tok, first_pos, T, vocab);
-  if (sumsq) sumsq_kernel<true, true><<<grid_for((long long)T * D, NT, 148 * 4), NT, 0, st>>>(gc, (long long)T * D, sumsq, 0);
+  if (sumsq) launch_sumsq<true, true>(grid_for((long long)T * D, NT, 148 * 4), 1, st, gc, (long long)T * D, sumsq, 0);
   OPK_LAUNCH_CHECK();
   return 0;
 }
