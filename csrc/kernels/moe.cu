@@ -142,10 +142,11 @@ __global__ void __launch_bounds__(256) moe_route_bwd_kernel(const float* __restr
 //
 // What bounds it: latency, it stands alone in the chain between router and products. Expert ids are loaded eight at a time (a load per
 // step of 32 entries waited for memory each time), segments are placed by a scan over the experts instead of one thread, and the
-// matching of equal experts, the longest part on one SM, is spread over eight: 64 experts, 32768 entries 60 -> 13 us, 16384 38 -> 10,
-// 1024 21 -> 7.
-template <bool CLUSTER>
-__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, int n_entries, int E, int examples, int r_cap,
+// matching of equal experts, the longest part on one SM, is spread over eight: 64 experts, 32768 entries 38 -> 9.3 us, 16384 22 -> 7.3,
+// 1024 7.3 -> 5.2. Without MANY there is one example and no division per entry, which had made few experts slower than one thread's
+// placement (8 experts, 512 entries 3.5 -> 4.4 -> 3.5 us, 2048 4.1 -> 5.4 -> 4.2).
+template <bool CLUSTER, bool MANY>
+__global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ idx, int n_entries, int E, int n_examples, int r_cap,
                                                         int* __restrict__ dest, int* __restrict__ src_entry,
                                                         int* __restrict__ tile_group, int* __restrict__ group_k,
                                                         int* __restrict__ counts_out) {
@@ -156,7 +157,8 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
   __shared__ int prior[MAX_E];        // entries per key in the CTAs before this one
   const int ctas = CLUSTER ? (int)gridDim.x : 1, rank = CLUSTER ? (int)blockIdx.x : 0;               // the grid is one cluster
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gwarp = rank * 32 + warp, warps = ctas * 32;
-  const int keys = E * examples, per_example = n_entries / examples;
+  const int examples = MANY ? n_examples : 1, keys = E * examples, per_example = MANY ? n_entries / examples : 1;
+  auto key_of = [&](int id, int n) { return MANY ? id * examples + n / per_example : id; };
   for (int i = threadIdx.x; i < 32 * MAX_E; i += blockDim.x) (&hist[0][0])[i] = 0;
   __syncthreads();
   const int chunk = ((n_entries + warps - 1) / warps + 31) / 32 * 32;      // entries per warp, a multiple of 32
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
     for (int u = 0; u < U; ++u) {
       const int n = base + 32 * u + lane;
       if (base + 32 * u >= c1) break;
-      if (n < c1 && OPK_IDX_OK(id[u], E) && (unsigned)id[u] < (unsigned)E) atomicAdd(&hist[warp][id[u] * examples + n / per_example], 1);
+      if (n < c1 && OPK_IDX_OK(id[u], E) && (unsigned)id[u] < (unsigned)E) atomicAdd(&hist[warp][key_of(id[u], n)], 1);
     }
   }
   __syncthreads();
@@ -260,7 +262,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
       if (base + 32 * u >= c1) break;
       const bool valid = (unsigned)id[u] < (unsigned)E;
       if (n < c1 && !valid) dest[n] = -1;
-      const int e = valid ? id[u] * examples + n / per_example : -1 - lane;     // invalid lanes match nobody
+      const int e = valid ? key_of(id[u], n) : -1 - lane;     // invalid lanes match nobody
       const unsigned m = __match_any_sync(0xffffffffu, e);
       if (valid) {
         const int row = offs[e] + (CLUSTER ? prior[e] : 0) + hist[warp][e] + __popc(m & ((1u << lane) - 1u));
@@ -401,10 +403,11 @@ extern "C" int opk_moe_plan(const int32_t* idx, int n_entries, int E, int exampl
       r_cap < opk_moe_rows_capacity(n_entries, E, examples))
     return -1;
   if (n_entries == 0 && examples > 1) return -1;
-  // From 4096 entries on a cluster (64 experts, us, one CTA -> cluster): 4096 11.1 -> 8.9, 8192 16.6 -> 8.9, 16384 25 -> 10, 32768
-  // 45 -> 13; 2048 takes 8.8 on one CTA.
+  // From 4096 entries on a cluster (us, one CTA -> cluster: 64 experts 2048 6.3 -> 6.1, 4096 8.6 -> 6.4, 8192 12.8 -> 6.4, 32768 37 -> 9.3;
+  // 8 experts 2048 4.2 -> 5.1, 4096 5.0 -> 5.2, 8192 6.8 -> 5.2).
   if (n_entries < 4096) {
-    moe_plan_kernel<false><<<1, 1024, 0, ST(stream)>>>(idx, n_entries, E, examples, r_cap, dest, src_entry, tile_group, group_k, counts);
+    if (examples == 1) moe_plan_kernel<false, false><<<1, 1024, 0, ST(stream)>>>(idx, n_entries, E, 1, r_cap, dest, src_entry, tile_group, group_k, counts);
+    else moe_plan_kernel<false, true><<<1, 1024, 0, ST(stream)>>>(idx, n_entries, E, examples, r_cap, dest, src_entry, tile_group, group_k, counts);
     return (int)cudaGetLastError();
   }
   const int ctas = 8;
@@ -418,7 +421,7 @@ extern "C" int opk_moe_plan(const int32_t* idx, int n_entries, int E, int exampl
   cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
   cfg.attrs = &cluster;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, moe_plan_kernel<true>, idx, n_entries, E, examples, r_cap, dest, src_entry, tile_group, group_k, counts);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, examples == 1 ? moe_plan_kernel<true, false> : moe_plan_kernel<true, true>, idx, n_entries, E, examples, r_cap, dest, src_entry, tile_group, group_k, counts);
   if (e != cudaSuccess) return (int)e;
   return (int)cudaGetLastError();
 }
