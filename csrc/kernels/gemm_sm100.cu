@@ -367,8 +367,10 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
       case opk::EPI_LCE_FWD:
         if (!a->labels || !a->pmax || !a->psum || !a->tgt) { set_err("opk_gemm: lce fwd buffers required"); return -1; }
         if (key == 0)
-          return a->lce_parts == 2 ? launch2<false, false, opk::EPI_LCE_FWD2>(ta, tb, p, mc, st)
-                                   : launch2<false, false, opk::EPI_LCE_FWD>(ta, tb, p, mc, st);
+          return a->z ? a->lce_parts == 2 ? launch2<false, false, opk::EPI_LCE_KEEP2>(ta, tb, p, mc, st)
+                                          : launch2<false, false, opk::EPI_LCE_KEEP>(ta, tb, p, mc, st)
+                 : a->lce_parts == 2 ? launch2<false, false, opk::EPI_LCE_FWD2>(ta, tb, p, mc, st)
+                                     : launch2<false, false, opk::EPI_LCE_FWD>(ta, tb, p, mc, st);
         break;
       case opk::EPI_LCE_BWD:
         if (!a->labels || !a->lse || !a->coef) { set_err("opk_gemm: lce bwd buffers required"); return -1; }
@@ -404,8 +406,10 @@ extern "C" int opk_gemm(const OpkGemmArgs* a, void* stream) {
     case opk::EPI_LCE_FWD:
       if (!a->labels || !a->pmax || !a->psum || !a->tgt) { set_err("opk_gemm: lce fwd buffers required"); return -1; }
       if (key == 0)
-        return a->lce_parts == 2 ? launch<false, false, 256, opk::EPI_LCE_FWD2>(ta, tb, p, mc, st)
-                                 : launch<false, false, 256, opk::EPI_LCE_FWD>(ta, tb, p, mc, st);
+        return a->z ? a->lce_parts == 2 ? launch<false, false, 256, opk::EPI_LCE_KEEP2>(ta, tb, p, mc, st)
+                                        : launch<false, false, 256, opk::EPI_LCE_KEEP>(ta, tb, p, mc, st)
+               : a->lce_parts == 2 ? launch<false, false, 256, opk::EPI_LCE_FWD2>(ta, tb, p, mc, st)
+                                   : launch<false, false, 256, opk::EPI_LCE_FWD>(ta, tb, p, mc, st);
       break;
     case opk::EPI_LCE_BWD:
       if (!a->labels || !a->lse || !a->coef) { set_err("opk_gemm: lce bwd buffers required"); return -1; }

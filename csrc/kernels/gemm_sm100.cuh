@@ -28,6 +28,10 @@ enum GemmEpilogue : int {
   EPI_SWIGLU_BWD = 5,  // acc = d(act); act = saved (gate, up) pairs [M][2N]; C[m][2n], C[m][2n+1] = d(gate), d(up)
   EPI_LCE_FWD2 = 6,    // EPI_LCE_FWD with two column parts per tile (twice the epilogue warps), chosen by lce_parts == 2
   EPI_LCE_GRAD = 7,    // EPI_LCE_BWD on logits that the forward pass stored (lce_grad_kernel): no product
+  // Forms of their own: asking in every chunk whether to store cost the products that store nothing 2 to 3 % (us, before there was
+  // anything to store -> asked -> now: 2048 x 50257 x 768 139.5 -> 142.0 -> 139.5, 1520 x 11421 x 128 25.2 -> 26.0 -> 25.2).
+  EPI_LCE_KEEP = 8,    // EPI_LCE_FWD that also stores the logits (`z`)
+  EPI_LCE_KEEP2 = 9,   // EPI_LCE_FWD2 that does
 };
 
 struct GemmParams {
@@ -47,7 +51,7 @@ struct GemmParams {
   float* pmax;           // EPI_LCE_FWD: [M][parts * tiles_n], parts = 1 (EPI_LCE_FWD) or 2 (EPI_LCE_FWD2)
   float* psum;           // EPI_LCE_FWD: [M][parts * tiles_n], parts = 1 (EPI_LCE_FWD) or 2 (EPI_LCE_FWD2)
   float* tgt;            // EPI_LCE_FWD: [M] target logit (written by the tile that owns the label)
-  float* z;              // EPI_LCE_FWD, optional: fp32 logits for the backward pass in blocks of 32 x 32 (see z_block)
+  float* z;              // EPI_LCE_KEEP: fp32 logits for the backward pass in blocks of 32 x 32 (see z_block)
   const float* lse;      // EPI_LCE_BWD: [M]
   const float* coef;     // EPI_LCE_BWD: [M] per-row scale (mask / divisor * upstream grad)
   float softcap;         // EPI_LCE_*: 0 = off, else z = cap * tanh(z / cap)
@@ -79,12 +83,14 @@ struct GemmParams {
 // takes eight too: with four it set the pace up to K = 4096 (2048 x 16384 x 2048 116 us, 97 with eight; 2048 x 28672 x 4096
 // 324 and 319). (With eight warps the store-only kernels measured 3-5 % slower; the
 // plain forward cross-entropy hides under its main loop with four.)
+__host__ __device__ constexpr bool lce_keeps(int epi) { return epi == EPI_LCE_KEEP || epi == EPI_LCE_KEEP2; }
+__host__ __device__ constexpr bool lce_forward(int epi) { return epi == EPI_LCE_FWD || epi == EPI_LCE_FWD2 || lce_keeps(epi); }
 __host__ __device__ constexpr int gemm_epi_warps(int epi) {
-  return epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD || epi == EPI_LCE_FWD2 || epi == EPI_LCE_BWD ? 8 : 4;
+  return epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD || epi == EPI_LCE_FWD2 || epi == EPI_LCE_KEEP2 || epi == EPI_LCE_BWD ? 8 : 4;
 }
 // The single-CTA kernel serves the grouped (mixture-of-experts) modes, whose per-expert reductions are only a few
 // k-blocks long while every tile is still written in full: there the epilogue, not the main loop, sets the pace.
-__host__ __device__ constexpr int gemm1_epi_warps(int epi) { return epi == EPI_LCE_FWD ? 4 : 8; }
+__host__ __device__ constexpr int gemm1_epi_warps(int epi) { return epi == EPI_LCE_FWD || epi == EPI_LCE_KEEP ? 4 : 8; }
 
 constexpr int kEpiScratch = 2048;      // bytes of shared memory per epilogue warp (see store_pieces)
 
@@ -212,7 +218,7 @@ __device__ __forceinline__ EpiState epi_begin(const GemmParams& p, uint8_t* scr,
   e.run_sum = 0.f;
   e.label = -1;
   e.lse = e.coef = 0.f;
-  if (EPI == EPI_LCE_FWD || EPI == EPI_LCE_FWD2 || EPI == EPI_LCE_BWD || EPI == EPI_LCE_GRAD) {
+  if (lce_forward(EPI) || EPI == EPI_LCE_BWD || EPI == EPI_LCE_GRAD) {
     if (e.row_ok) e.label = p.labels[e.row];
     if ((EPI == EPI_LCE_BWD || EPI == EPI_LCE_GRAD) && e.row_ok) { e.lse = p.lse[e.row]; e.coef = p.coef[e.row]; }
   }
@@ -367,19 +373,22 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, EpiState& e, floa
           drow[2 * j + 1] = __float2bfloat16(d * (g * sg));
         }
     }
-  } else if (EPI == EPI_LCE_FWD || EPI == EPI_LCE_FWD2) {
+  } else if (lce_forward(EPI)) {
     if (p.softcap > 0.f) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = tanhf(cap_quotient(p, v[j]));
+      for (int j = 0; j < 32; ++j) {
+        v[j] = tanhf(cap_quotient(p, v[j]));
+        if (!lce_keeps(EPI)) v[j] *= p.softcap;
+      }
     }
-    if (p.z) {      // the scaled logit, or the hyperbolic tangent of the soft cap: what EPI_LCE_GRAD starts from
+    if constexpr (lce_keeps(EPI)) {      // the scaled logit, or the hyperbolic tangent of the soft cap: what EPI_LCE_GRAD starts from
       float4* z = z_block(p.z, p.N, e.row - (int)(threadIdx.x & 31), col0);
 #pragma unroll
       for (int q = 0; q < 8; ++q) __stcs(z + 32 * q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
-    }
-    if (p.softcap > 0.f) {
+      if (p.softcap > 0.f) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] *= p.softcap;
+        for (int j = 0; j < 32; ++j) v[j] *= p.softcap;
+      }
     }
     float cmax = -INFINITY;
 #pragma unroll
@@ -423,7 +432,7 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& p, EpiState& e, floa
 // part: index of this (column tile, column part of the tile); parts: their number per row.
 template <int EPI>
 __device__ __forceinline__ void epi_end(const GemmParams& p, const EpiState& e, int part, int parts) {
-  if ((EPI == EPI_LCE_FWD || EPI == EPI_LCE_FWD2) && e.row_ok) {
+  if (lce_forward(EPI) && e.row_ok) {
     p.pmax[(long long)e.row * parts + part] = e.run_max;
     p.psum[(long long)e.row * parts + part] = e.run_sum;
   }
