@@ -51,8 +51,14 @@ __global__ void philox_normal_kernel(float* __restrict__ out, long long n, uint6
 // accumulation, of the fp32 multiply and of the bf16 store, so that the norm of the *stored* clipped gradient
 // is <= clip. AUTO-S (mode_auto): R / (norm + gamma) with the same guard and no clamp to one.
 __global__ void clip_scale_kernel(double* sumsq, float clip, int mode_auto, float gamma, int n_leaves,
-                                  long long widest_leaf, float* scale_out, float* norm_out, int* counters, int reset) {
+                                  long long widest_leaf, float* scale_out, float* norm_out, int* counters, int reset,
+                                  const float* loss, float* loss_sum) {
   const int j = threadIdx.x;             // one example per thread
+  if (loss_sum && j == 0) {              // in the order of the examples, as one by one
+    float sum = *loss_sum;
+    for (int k = 0; k < (int)blockDim.x; ++k) sum += loss[k];
+    *loss_sum = sum;
+  }
   const double sq = sumsq[j];
   if (reset) sumsq[j] = 0.0;
   const double norm = sqrt(sq > 0.0 ? sq : 0.0);
@@ -668,10 +674,11 @@ extern "C" int opk_philox_normal(float* out, int64_t n, uint64_t seed, uint32_t 
 }
 
 extern "C" int opk_clip_scale(double* sumsq, float clip, int mode_auto, float gamma, int n_leaves, int64_t widest_leaf,
-                              float* scale_out, float* norm_out, int32_t* counters, int reset, int batch, void* stream) {
-  if (batch < 1 || batch > 32) return -1;
+                              float* scale_out, float* norm_out, int32_t* counters, int reset, int batch, const float* loss,
+                              float* loss_sum, void* stream) {
+  if (batch < 1 || batch > 32 || (loss_sum && !loss)) return -1;
   clip_scale_kernel<<<1, batch, 0, ST(stream)>>>(sumsq, clip, mode_auto, gamma, n_leaves, widest_leaf, scale_out, norm_out,
-                                            counters, reset);
+                                            counters, reset, loss, loss_sum);
   OPK_LAUNCH_CHECK();
   return 0;
 }

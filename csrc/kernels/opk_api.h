@@ -270,9 +270,10 @@ int opk_moe_combine_bwd(const void* dy, const void* y, const int32_t* dest, int 
 // ---- DP clipping / noise / optimizer (csrc/kernels/dp_step.cu) ---------------------------------------------
 // scale = guarded min(1, C / sqrt(sumsq)) (fixed) or R / (sqrt(sumsq) + gamma) (auto); see dp_step.cu.
 // Also: norm_out[0] = sqrt(sumsq), counters[0] += (norm > C), and *sumsq is reset to 0 when reset != 0. `batch` (1 .. 32)
-// consecutive sums, factors and norms.
+// consecutive sums, factors and norms. loss_sum (may be NULL): the `batch` losses are added to it, in order.
 int opk_clip_scale(double* sumsq, float clip, int mode_auto, float gamma, int n_leaves, int64_t widest_leaf,
-                   float* scale_out, float* norm_out, int32_t* counters, int reset, int batch, void* stream);
+                   float* scale_out, float* norm_out, int32_t* counters, int reset, int batch, const float* loss, float* loss_sum,
+                   void* stream);
 // acc[i] += float(bf16(float(g[i]) * scale)) with bf16 subnormals that rounded up flushed to zero.
 int opk_clip_accumulate(const void* g, const float* scale, float* acc, int64_t n, void* stream);
 // Same with overwrite != 0 meaning acc = bf16(g * scale) (first example of a step: no separate zeroing pass).

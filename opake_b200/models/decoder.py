@@ -639,11 +639,12 @@ class DecoderRuntime:
         return ExampleStats(loss=loss, n_tokens=ntok)
 
     # ------------------------------------------------------------------ clip + accumulate
-    def clip_factor(self, clip: float, *, auto: bool = False, gamma: float = 0.01, slot: int = 0, n: int = 1) -> None:
-        """Turns the squared norms of ``n`` slots into the guarded clip factors (device scalars) and resets the accumulators."""
+    def clip_factor(self, clip: float, *, auto: bool = False, gamma: float = 0.01, slot: int = 0, n: int = 1, loss=None, loss_sum=None) -> None:
+        """Turns the squared norms of ``n`` slots into the guarded clip factors (device scalars) and resets the accumulators. ``loss_sum``:
+        the ``n`` losses are added to it, one after the other."""
         K.clip_scale(self.sumsq_all[slot : slot + n], clip, scale_out=self.scales[slot], norm_out=self.norms[slot],
                      counters=self.clip_count, auto=auto, gamma=gamma, n_leaves=self._n_leaves,
-                     widest_leaf=self._widest, reset=True)
+                     widest_leaf=self._widest, reset=True, loss=loss, loss_sum=loss_sum)
 
     def accumulate(self, acc: torch.Tensor, ws: dict, tok: torch.Tensor, *, slot: int = 0, overwrite: bool = False) -> None:
         """``acc`` (fp32, full flat layout) ``+= clip_factor * G[slot]`` with the conservative storage rounding."""

@@ -98,7 +98,7 @@ PROTOTYPES: dict = {
     "opk_scatter_rows_cast_sumsq": (I, [P, P, P, P, I, I, P, I, L, P]),
     "opk_colsum": (I, [P, P, I, I, L, I, L, P]),
     "opk_embedding_add_rows": (I, [P, P, P, P, I, I, I, L, P]),
-    "opk_clip_scale": (I, [P, F, I, F, I, L, P, P, P, I, I, P]),
+    "opk_clip_scale": (I, [P, F, I, F, I, L, P, P, P, I, I, P, P, P]),
     "opk_clip_accumulate": (I, [P, P, P, L, P]),
     "opk_clip_accumulate2": (I, [P, P, P, L, I, P]),
     "opk_clip_accumulate_group": (I, [POINTER(c_void_p), POINTER(c_void_p), I, P, L, I, P]),

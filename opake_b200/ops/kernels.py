@@ -340,10 +340,13 @@ def embedding_add_rows(tok, ws, dense, T: int):
 
 
 def clip_scale(sumsq, clip: float, *, scale_out, norm_out=None, counters=None, auto: bool = False, gamma: float = 0.01,
-               n_leaves: int = 1, widest_leaf: int = 1, reset: bool = True):
-    """``sumsq`` of several elements: one factor (and norm) for each."""
+               n_leaves: int = 1, widest_leaf: int = 1, reset: bool = True, loss=None, loss_sum=None):
+    """``sumsq`` of several elements: one factor (and norm) for each. ``loss_sum`` (fp32 scalar): ``loss``, one per sum, is added to it
+    in order."""
+    if loss_sum is not None and (loss is None or loss.numel() != sumsq.numel()):
+        raise ValueError("one loss for each squared norm")
     _chk(_L().opk_clip_scale(_p(sumsq), clip, int(auto), gamma, n_leaves, widest_leaf, _p(scale_out), _p(norm_out),
-                             _p(counters), int(reset), sumsq.numel(), _s(sumsq)), "clip_scale")
+                             _p(counters), int(reset), sumsq.numel(), _p(loss), _p(loss_sum), _s(sumsq)), "clip_scale")
 
 
 def clip_accumulate(g, scale, acc, overwrite: bool = False):

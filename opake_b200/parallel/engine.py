@@ -360,8 +360,7 @@ class ShardedDPEngine:
             hook = lambda: main.wait_stream(self._side)
         toks = ws["tok_all"][slot : slot + n]
         st = rt.example_grad(toks.view(-1), part["labels"], ws=part, slot=slot, before_wgrad=hook)
-        rt.clip_factor(cfg.clip_norm, auto=cfg.auto_clip, gamma=cfg.auto_gamma, slot=slot, n=n)
-        ws["loss_sum"].add_(st.loss.sum())
+        rt.clip_factor(cfg.clip_norm, auto=cfg.auto_clip, gamma=cfg.auto_gamma, slot=slot, n=n, loss=st.loss, loss_sum=ws["loss_sum"])
         ws["tok_keep"][slot : slot + n].copy_(toks)      # the slots' tokens are replaced before their deferred pass runs
 
     def _run_joined(self, ws, tok_host: torch.Tensor, labels_host: torch.Tensor, index: int) -> None:

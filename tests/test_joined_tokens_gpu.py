@@ -85,3 +85,20 @@ def test_one_example_before_several(cuda, name, monkeypatch):
     for x, y in ((a.params, b.params), (a.m, b.m), (a.v, b.v)):
         for p, q in zip(a.layout.views(x).values(), b.layout.views(y).values()):
             assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_losses_are_added_in_the_order_of_the_examples(cuda, graph, monkeypatch):
+    """The loss of a step has the bits that the examples one by one give."""
+    from opake_b200.parallel import engine as E
+
+    cfg, losses = _model("llama"), []
+    for values in (1 << 23, 0):
+        monkeypatch.setattr(E, "_JOIN_VALUES", values)
+        eng = E.ShardedDPEngine(cfg, E.EngineConfig(logical_batch=4, noise_multiplier=0.1, accumulate_group=5, lr=1e-3, use_cuda_graph=graph), cuda)
+        gen = torch.Generator().manual_seed(1)
+        for B in (1, 5, 9, 13, 13, 13, 2):
+            tok = torch.rand(B, cfg.vocab_size, generator=gen).argsort(1)[:, :77].to(torch.int32).contiguous().pin_memory()
+            losses.append(eng.step(tok, torch.roll(tok, -1, 1).clone()).clone())
+    half = len(losses) // 2
+    assert all(torch.equal(a, b) for a, b in zip(losses[:half], losses[half:]))
